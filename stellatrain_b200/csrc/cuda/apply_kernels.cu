@@ -6,7 +6,8 @@
 //                                   backend/src/engine/modules/cpu_optimize.cpp:40-72
 //   sparse SGD / sparse Adam        backend/src/optim/sgd.cpp:221-262, backend/src/optim/adam.cpp:19-87
 //   H2D copy of updated parameters  backend/src/engine/modules/h2d_copy.cpp:31-56  (no longer needed)
-// by two kernels per bucket (three when the optimiser state is partitioned over the ranks):
+// by two kernels per bucket (one when there is a single source, three when the optimiser state is partitioned over the
+// ranks):
 //   wait     one warp waits (bounded) for the arrival flags of all sources (only when flags are in use)
 //   scatter  adds every source's weighted values into a dense accumulator with red.global.add.f32
 //   apply    walks the same streams again; the first thread to stamp an index with the current epoch
@@ -96,6 +97,56 @@ __device__ __forceinline__ void finish_apply(const ApplyArgs& A, uint32_t epoch,
   }
 }
 
+// What one update needs besides its entry: the bias corrections of this step (Adam) and the host's options.
+struct StepConsts {
+  float bc1, bc2, lr;
+  uint32_t m_iter;
+};
+
+// 1 - beta^tick in double, as the reference computes it (adam.cpp:41-42).  Two double-precision powers take about
+// 1.5 us: every kernel below sends its own loads off first and computes them while those travel.
+__device__ __forceinline__ void bias_corrections(const OptState& o, float* bc) {
+  bc[0] = (float)(1.0 - pow((double)o.beta1, (double)o.tick));
+  bc[1] = (float)(1.0 - pow((double)o.beta2, (double)o.tick));
+}
+
+// The optimiser rule for element `s` of the state range (`rc`: its record with the merged gradient in x, `x`: its
+// parameter).  Writes the record back with the accumulator cleared and the stamp of this epoch; returns the new value.
+__device__ __forceinline__ float update_element(const ApplyArgs& A, const OptState& o, const StepConsts& c, uint32_t s,
+                                                uint32_t epoch, const float4& rc, float x) {
+  float g = rc.x, m_new = rc.z, v_new = rc.w, xn;
+  if (o.kind == 0) {
+    float mu = o.momentum;
+    if (o.smart_momentum && A.last != nullptr && c.m_iter != 0u)
+      mu = powf(o.momentum, (float)(c.m_iter - A.last[s]));
+    if (o.weight_decay != 0.f) g += o.weight_decay * x;
+    if (o.momentum != 0.f) {
+      const float b = o.first ? g : rc.z * mu + (1.f - o.dampening) * g;
+      g = o.nesterov ? g + mu * b : b;
+      m_new = b;
+    }
+    xn = x - c.lr * g;
+    if (o.smart_momentum && A.last != nullptr) A.last[s] = c.m_iter;
+  } else {
+    if (o.maximize) g = -g;
+    if (o.weight_decay != 0.f) g += o.weight_decay * x;
+    const float mt = o.beta1 * rc.z + (1.f - o.beta1) * g;
+    const float vt = o.beta2 * rc.w + (1.f - o.beta2) * g * g;
+    const float mh = mt / c.bc1;
+    float vh = vt / c.bc2;
+    if (o.amsgrad && A.vmax != nullptr) {
+      vh = fmaxf(A.vmax[s], vh);
+      A.vmax[s] = vh;
+    }
+    xn = x - o.lr * mh / (sqrtf(vh) + o.eps);
+    m_new = mt;
+    v_new = vt;
+  }
+  // accumulator cleared, stamp kept (a late loser's exchange writes the same epoch again)
+  A.rec[s] = make_float4(0.f, __uint_as_float(epoch), m_new, v_new);
+  return xn;
+}
+
 __global__ void __launch_bounds__(kThreads) k_apply(ApplyArgs A) {
   __shared__ float s_bc[2];
   const int src = blockIdx.y;
@@ -106,70 +157,50 @@ __global__ void __launch_bounds__(kThreads) k_apply(ApplyArgs A) {
   const OptState o = *A.opt;
 
   if (ok) {
-    if (threadIdx.x == 0) {
-      // bias corrections in double, as the reference computes them (adam.cpp:41-42)
-      s_bc[0] = (float)(1.0 - pow((double)o.beta1, (double)o.tick));
-      s_bc[1] = (float)(1.0 - pow((double)o.beta2, (double)o.tick));
-    }
-    __syncthreads();
-    const float bc1 = s_bc[0], bc2 = s_bc[1];
-    const uint32_t m_iter = o.tick - 1u;
-    const float lr = (o.kind == 0 && o.maximize) ? -o.lr : o.lr;
     const uint64_t src_off = (size_t)slot * A.slot_stride + (size_t)src * A.cap;
     uint2* in = A.recv + src_off;
+    const uint32_t step = gridDim.x * kThreads;
+    uint32_t i = A.ent_lo + blockIdx.x * kThreads + threadIdx.x;
+    // Everything an entry needs leaves in one go: the exchange that decides whether this thread owns the element, its
+    // record and its parameter.  A thread that wins may use what it read before: the record's accumulator was complete
+    // when this kernel began, and only the winner writes record and parameter.
+    uint32_t idx = kSentinelIdx, s = 0u, old = 0u;
+    float4 rc = make_float4(0.f, 0.f, 0.f, 0.f);
+    float x = 0.f;
+    bool in_range = false;
+    auto fetch = [&]() {
+      idx = load_entry(A, in, i).x;
+      s = idx - A.state_base;        // sentinel or invalid indices (already reported) fall outside
+      in_range = s < A.state_len;
+      if (in_range) {
+        rc = __ldcg(A.rec + s);      // accumulator, stamp, m, v in one 16-byte load
+        x = __ldcg(A.param + idx);
+        // the first thread to stamp an index with this epoch owns it
+        old = atomicExch(reinterpret_cast<uint32_t*>(&A.rec[s].y), epoch);
+      }
+    };
+    if (i < A.ent_hi) fetch();
+    if (threadIdx.x == 0 && o.kind != 0) bias_corrections(o, s_bc);
     if (A.cksum_local != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
       // the scatter kernel has read the whole stream of this source: does it add up to what was sent?
       const uint32_t got = atomicExch(A.rsum + src, 0u);
       const uint32_t want = __ldcg(A.cksum_local + (size_t)slot * A.world + src);
       if (got != want) set_status(A.status, kBadChecksum);
     }
-    for (uint32_t i = A.ent_lo + blockIdx.x * kThreads + threadIdx.x; i < A.ent_hi; i += gridDim.x * kThreads) {
-      const uint2 e = load_entry(A, in, i);
-      const uint32_t idx = e.x;
-      const uint32_t s = idx - A.state_base;        // sentinel or invalid indices (already reported) fall outside
-      // the first thread to stamp an index with this epoch owns it
-      const bool won = s < A.state_len &&
-                       atomicExch(reinterpret_cast<uint32_t*>(&A.rec[s].y), epoch) != epoch;
+    __syncthreads();
+    const StepConsts c = {s_bc[0], s_bc[1], o.maximize ? -o.lr : o.lr, o.tick - 1u};
+    while (i < A.ent_hi) {
+      const bool won = in_range && old != epoch;
       float xn = 0.f;
       if (won) {
-        const float4 rc = __ldcg(A.rec + s);     // accumulator, stamp, m, v in one 16-byte load
-        float g = rc.x;
-        float m_new = rc.z, v_new = rc.w;
-        const float x = A.param[idx];
-        if (o.kind == 0) {
-          float mu = o.momentum;
-          if (o.smart_momentum && A.last != nullptr && m_iter != 0u)
-            mu = powf(o.momentum, (float)(m_iter - A.last[s]));
-          if (o.weight_decay != 0.f) g += o.weight_decay * x;
-          if (o.momentum != 0.f) {
-            const float b = o.first ? g : rc.z * mu + (1.f - o.dampening) * g;
-            g = o.nesterov ? g + mu * b : b;
-            m_new = b;
-          }
-          xn = x - lr * g;
-          if (o.smart_momentum && A.last != nullptr) A.last[s] = m_iter;
-        } else {
-          if (o.maximize) g = -g;
-          if (o.weight_decay != 0.f) g += o.weight_decay * x;
-          const float mt = o.beta1 * rc.z + (1.f - o.beta1) * g;
-          const float vt = o.beta2 * rc.w + (1.f - o.beta2) * g * g;
-          const float mh = mt / bc1;
-          float vh = vt / bc2;
-          if (o.amsgrad && A.vmax != nullptr) {
-            vh = fmaxf(A.vmax[s], vh);
-            A.vmax[s] = vh;
-          }
-          xn = x - o.lr * mh / (sqrtf(vh) + o.eps);
-          m_new = mt;
-          v_new = vt;
-        }
-        // accumulator cleared, stamp kept (a late loser's exchange writes the same epoch again)
-        A.rec[s] = make_float4(0.f, __uint_as_float(epoch), m_new, v_new);
+        xn = update_element(A, o, c, s, epoch, rc, x);
         A.param[idx] = xn;
       }
       // every consumed position is rewritten each epoch, so a stale value can never be read back
       if (A.owner_mode) emit_writeback(A, src_off + i, won ? idx : kSentinelIdx, xn);
       if (A.poison && !A.narrow) in[i] = make_uint2(kSentinelIdx, 0u);
+      i += step;
+      if (i < A.ent_hi) fetch();
     }
   }
 
@@ -188,6 +219,60 @@ __global__ void __launch_bounds__(kThreads) k_apply(ApplyArgs A) {
         for (int p = 0; p < A.world; ++p)
           st_release_sys_u64(A.pflag[p] + (size_t)slot * A.pflag_slot_stride, (uint64_t)epoch);
       }
+    }
+  }
+}
+
+// One source: its stream names every element at most once (each select emits an element once, random-k strides
+// through the tensor with a step coprime to its size), so there is nothing to merge: no accumulator, no stamp to
+// compete for, one kernel instead of two.
+__global__ void __launch_bounds__(kThreads) k_apply_single(ApplyArgs A) {
+  __shared__ float s_bc[2];
+  const uint32_t epoch = *A.epoch;
+  const uint32_t slot = epoch & 1u;
+  if (epoch >= ld_volatile_u32(A.sel_epoch)) return;
+  const bool ok = ld_volatile_u32(A.status) == kOk;
+  const OptState o = *A.opt;
+  if (A.stamps != nullptr && !A.use_flags && blockIdx.x == 0 && threadIdx.x == 0) A.stamps[2] = global_timer_ns();
+  if (ok) {
+    const uint2* in = A.recv + (size_t)slot * A.slot_stride;
+    const float w = A.weight[slot];
+    const uint32_t step = gridDim.x * kThreads;
+    uint32_t i = blockIdx.x * kThreads + threadIdx.x;
+    uint2 e = make_uint2(kSentinelIdx, 0u);
+    float4 rc = make_float4(0.f, 0.f, 0.f, 0.f);
+    float x = 0.f;
+    bool in_range = false;
+    auto fetch = [&]() {
+      e = load_entry(A, in, i);
+      in_range = e.x < A.n_total;
+      if (in_range) {
+        rc = __ldcg(A.rec + e.x);
+        x = __ldcg(A.param + e.x);
+      } else if (e.x != kSentinelIdx) {
+        set_status(A.status, kBadIndex);
+      }
+    };
+    if (i < A.ent_hi) fetch();
+    if (threadIdx.x == 0 && o.kind != 0) bias_corrections(o, s_bc);
+    __syncthreads();
+    const StepConsts c = {s_bc[0], s_bc[1], o.maximize ? -o.lr : o.lr, o.tick - 1u};
+    while (i < A.ent_hi) {
+      if (in_range) {
+        rc.x += __uint_as_float(e.y) * w;      // what the merge would have left in the accumulator
+        A.param[e.x] = update_element(A, o, c, e.x, epoch, rc, x);
+      }
+      i += step;
+      if (i < A.ent_hi) fetch();
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    const uint32_t prev = atomicAdd(A.done_ctr, 1u);
+    if (prev == gridDim.x - 1) {
+      *A.done_ctr = 0;
+      finish_apply(A, epoch, o.tick);
     }
   }
 }
@@ -230,6 +315,10 @@ __global__ void __launch_bounds__(kThreads) k_param_scatter(ApplyArgs A) {
   }
 }
 
+// One source has nothing to merge.  The debug checks keep the two kernels: the stream's checksum has to be known
+// before its first entry is applied.
+bool apply_merges_nothing(const ApplyArgs& A) { return A.world == 1 && !A.owner_mode && A.cksum_local == nullptr && !A.poison; }
+
 // phase 0: the whole chain; 1: scatter + apply only; 2: the parameter copy of partitioned state only
 // (split launches let a test run several emulated ranks on one GPU without a kernel waiting for a later one).
 cudaError_t launch_apply(const ApplyArgs& A, int max_ctas_per_source, int phase, cudaStream_t stream) {
@@ -244,6 +333,10 @@ cudaError_t launch_apply(const ApplyArgs& A, int max_ctas_per_source, int phase,
     if (parts > max_ctas_per_source) parts = max_ctas_per_source;
     dim3 grid(parts, A.world);
     if (A.use_flags) k_wait_streams<<<1, 32, 0, stream>>>(A);
+    if (apply_merges_nothing(A)) {
+      k_apply_single<<<parts, kThreads, 0, stream>>>(A);
+      return cudaGetLastError();
+    }
     if (A.deterministic) {
       ApplyArgs one = A;
       for (int src = 0; src < A.world; ++src) {   // one launch per source: a fixed order of additions

@@ -39,6 +39,7 @@ struct BucketHandle {
   cudaError_t apply(cudaStream_t stream, int phase) { return launch_apply(app, max_ctas_per_source, phase, stream); }
 
   int apply_kernels() const {
+    if (apply_merges_nothing(app)) return 1 + (app.use_flags ? 1 : 0);
     return (app.owner_mode ? 3 : 2) + (app.deterministic ? app.world - 1 : 0) + (app.use_flags ? 1 : 0);
   }
 

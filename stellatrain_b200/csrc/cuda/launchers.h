@@ -18,6 +18,9 @@ cudaError_t launch_select_fused(const SelectArgs& args, cudaStream_t stream);
 // apply only, 2 = parameter copy only.
 cudaError_t launch_apply(const ApplyArgs& args, int max_ctas_per_source, int phase, cudaStream_t stream);
 
+// True when launch_apply runs its single kernel for one source (no merge).
+bool apply_merges_nothing(const ApplyArgs& args);
+
 // max |a - b| as float bits, atomically folded into *out_bits (caller zeroes it).
 cudaError_t launch_max_abs_diff(const float* a, const float* b, uint64_t n, uint32_t* out_bits,
                                 cudaStream_t stream);

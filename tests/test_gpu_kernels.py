@@ -184,6 +184,45 @@ def test_apply_options_nesterov_smart_amsgrad():
         torch.testing.assert_close(b.param, p_ref, rtol=1e-4, atol=1e-6)
 
 
+@pytest.mark.parametrize("optimizer,options,extra", [
+    ("sgd", dict(lr=0.1, momentum=0.9, weight_decay=1e-4), {}),
+    ("sgd", dict(lr=0.05, momentum=0.8, nesterov=1, dampening=0.1), dict(smart_momentum=True)),
+    ("adam", dict(lr=1e-3, weight_decay=1e-2), {}),
+    ("adam", dict(lr=1e-2, maximize=1), dict(amsgrad=True)),
+])
+@pytest.mark.parametrize("compressor,narrow", [("topk", False), ("thresholdv", True), ("randomk", False)])
+@pytest.mark.parametrize("ctas", [1, 148 * 16])
+def test_single_source_apply_equals_the_merging_one(optimizer, options, extra, compressor, narrow, ctas):
+    """The one-kernel apply of a single source against scatter + apply (which debug checks keep): the same bits, with one
+    entry per thread and with a grid that walks the stream.  Both do the same operations in the same order."""
+    from stellatrain_b200.parallel.gpu_bucket import GpuBucket
+
+    pair = []
+    for debug in (False, True):
+        gen = torch.Generator(device="cuda").manual_seed(21)
+        layout = B.BucketLayout([f"t{i}" for i in range(4)], [1, 300, 5000, 70001], chunk_elems=4096, narrow_wire=narrow)
+        b = GpuBucket(0, layout, torch.device("cuda:0"), compressor=compressor, ratio=0.9, optimizer=optimizer, **extra)
+        b.wire_local(debug_checks=debug)
+        assert b.apply_kernels == (2 if debug else 1)
+        b.handle.max_ctas_per_source = ctas
+        b.set_optimizer_options(**options)
+        b.param.copy_(torch.randn(layout.n_total, generator=gen, device="cuda"))
+        for _ in range(5):
+            fill_grads(b, gen)
+            b.select()
+            b.apply()
+        b.apply()                      # nothing selected: leaves everything alone
+        torch.cuda.synchronize()
+        b.check_status()
+        pair.append(b)
+    one, two = pair
+    assert torch.equal(one.param, two.param) and torch.equal(one.rec, two.rec)
+    assert torch.equal(one.opt, two.opt) and torch.equal(one.counters[:4], two.counters[:4])
+    for name in ("vmax", "last"):
+        if getattr(one, name) is not None:
+            assert torch.equal(getattr(one, name), getattr(two, name))
+
+
 def test_randomk_stream_is_valid():
     b = make_bucket("randomk", 0.9, sizes=[1000, 4096, 17])
     gen = torch.Generator(device="cuda").manual_seed(3)
