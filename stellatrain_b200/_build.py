@@ -50,7 +50,7 @@ def _pybind_includes() -> list[str]:
 
 EXTENSIONS = {
     "_C": {
-        "cu": ["cuda/select_kernels.cu", "cuda/apply_kernels.cu", "cuda/aux_kernels.cu", "cuda/noalloc_entry.cu"],
+        "cu": ["cuda/select_kernels.cu", "cuda/one_pass_select.cu", "cuda/apply_kernels.cu", "cuda/aux_kernels.cu", "cuda/noalloc_entry.cu"],
         "cpp": ["cuda/bindings.cpp"],
         # compiled against the torch headers and linked with the torch libraries: the native step engine registers
         # C++ hooks on autograd's accumulation nodes (the reference links its engine against torch the same way,

@@ -51,9 +51,15 @@ struct BucketHandle : public st::BucketHandle {
 
   void set_tables(uint64_t segs, uint64_t state, uint64_t work, uint64_t chunks, uint64_t chunk_cnt,
                   uint64_t chunk_pos, uint64_t hist, uint32_t n_segs, uint32_t n_chunks, uint32_t cap,
-                  uint64_t chunk_state, uint32_t max_chunk) {
-    sel.chunk_state = as_ptr<uint64_t>(chunk_state);
-    max_chunk_len = max_chunk;
+                  uint64_t pieces, uint64_t run_cnt, uint64_t piece_cnt, uint64_t hist_top, uint64_t hist_rest, uint64_t refills,
+                  uint32_t n_pieces) {
+    sel.pieces = as_ptr<const st::Piece>(pieces);
+    sel.run_cnt = as_ptr<uint32_t>(run_cnt);
+    sel.piece_cnt = as_ptr<uint64_t>(piece_cnt);
+    sel.hist_top = as_ptr<uint32_t>(hist_top);
+    sel.hist_rest = as_ptr<uint32_t>(hist_rest);
+    sel.refills = as_ptr<uint32_t>(refills);
+    sel.n_pieces = n_pieces;
     sel.segs = as_ptr<const st::SegDesc>(segs);
     sel.state = as_ptr<st::SegState>(state);
     sel.work = as_ptr<st::SegWork>(work);
@@ -247,6 +253,9 @@ PYBIND11_MODULE(_C, m) {
   m.attr("SIZEOF_SEG_STATE") = sizeof(st::SegState);
   m.attr("SIZEOF_SEG_WORK") = sizeof(st::SegWork);
   m.attr("SIZEOF_CHUNK") = sizeof(st::Chunk);
+  m.attr("SIZEOF_PIECE") = sizeof(st::Piece);
+  m.attr("PIECE_RUNS") = st::kPieceRuns;
+  m.attr("RUN_ELEMS") = st::kRunElems;
   m.attr("SIZEOF_OPT_STATE") = sizeof(st::OptState);
 
   py::class_<BucketHandle>(m, "BucketHandle")
@@ -255,7 +264,8 @@ PYBIND11_MODULE(_C, m) {
            py::arg("param"), py::arg("rec"), py::arg("vmax"), py::arg("last"), py::arg("n_total"))
       .def("set_tables", &BucketHandle::set_tables, py::arg("segs"), py::arg("state"), py::arg("work"),
            py::arg("chunks"), py::arg("chunk_cnt"), py::arg("chunk_pos"), py::arg("hist"), py::arg("n_segs"),
-           py::arg("n_chunks"), py::arg("cap"), py::arg("chunk_state") = 0, py::arg("max_chunk") = 0)
+           py::arg("n_chunks"), py::arg("cap"), py::arg("pieces") = 0, py::arg("run_cnt") = 0,
+           py::arg("piece_cnt") = 0, py::arg("hist_top") = 0, py::arg("hist_rest") = 0, py::arg("refills") = 0, py::arg("n_pieces") = 0)
       .def("set_scratch", &BucketHandle::set_scratch, py::arg("cand"), py::arg("cand_cursor"), py::arg("cand_cap"))
       .def("set_control", &BucketHandle::set_control, py::arg("counters"), py::arg("status"), py::arg("opt"),
            py::arg("weight"), py::arg("timeout_ns"), py::arg("stamps") = 0)

@@ -16,25 +16,28 @@ struct BucketHandle {
   bool has_group = false;
   uint32_t randomk_seed = 0x5DEECE66u;
   int max_ctas_per_source = 148 * 16;
-  uint32_t max_chunk_len = 0;      // longest chunk of the chunk table (decides whether the one-pass select may run)
-  // One-pass select of the threshold compressors: allowed by configuration, and possible once every tensor of
-  // the bucket has its threshold (one select through the four-kernel chain, or a restored checkpoint).
+  // One-pass select: allowed by configuration, and possible once every tensor of the bucket has its threshold
+  // (one select through the four-kernel chain, or a restored checkpoint).
   bool fused_enabled = true;
   bool thresholds_ready = false;
   bool last_select_fused = false;
 
-  bool can_fuse() const { return fused_select_possible(sel, max_chunk_len); }
+  bool can_fuse() const { return one_pass_possible(sel); }
 
   cudaError_t select(cudaStream_t stream) {
     const bool fused = fused_enabled && thresholds_ready && can_fuse();
-    const cudaError_t e = fused ? launch_select_fused(sel, stream) : launch_select(sel, randomk_seed, stream);
+    const cudaError_t e = fused ? launch_select_one_pass(sel, stream) : launch_select(sel, randomk_seed, stream);
     thresholds_ready = true;       // the four-kernel chain leaves every tensor with a threshold
     last_select_fused = fused;
     return e;
   }
 
   // kernels of the last select (telemetry's launch count)
-  int select_kernels() const { return (sel.compressor == kRandomk || last_select_fused) ? 2 : 4; }
+  int select_kernels() const {
+    if (sel.compressor == kRandomk) return 2;
+    if (!last_select_fused) return 4;
+    return sel.compressor == kTopk ? 3 : 2;
+  }
 
   cudaError_t apply(cudaStream_t stream, int phase) { return launch_apply(app, max_ctas_per_source, phase, stream); }
 

@@ -46,6 +46,14 @@ __device__ __forceinline__ uint32_t ld_volatile_u32(const uint32_t* p) {
   return *reinterpret_cast<const volatile uint32_t*>(p);
 }
 
+// Counter by which CTAs of one grid hand their results over: releases this thread's (and, behind a CTA barrier, its CTA's)
+// stores to whoever adds later, and acquires those of whoever added earlier.
+__device__ __forceinline__ uint32_t atom_add_acq_rel_gpu(uint32_t* p, uint32_t v) {
+  uint32_t old;
+  asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+  return old;
+}
+
 // One 8-byte store that NVSwitch replicates into every GPU bound to the multicast object.
 __device__ __forceinline__ void multimem_st_pair(uint2* mc_addr, uint2 v) {
   asm volatile("multimem.st.relaxed.sys.global.v2.f32 [%0], {%1, %2};" ::"l"(mc_addr),
@@ -98,10 +106,8 @@ __device__ __forceinline__ void emit_entry(const SelectArgs& A, int dest, uint32
     } else if (A.out_mc != nullptr) {
       multimem_st_u32(reinterpret_cast<uint32_t*>(A.out_mc + slot_off) + pos, w);
     } else {
-#pragma unroll
-      for (int p = 0; p < kMaxWorld; ++p) {
-        if (p < A.world) reinterpret_cast<uint32_t*>(A.out[p] + slot_off)[pos] = w;
-      }
+#pragma unroll 1
+      for (int p = 0; p < A.world; ++p) reinterpret_cast<uint32_t*>(A.out[p] + slot_off)[pos] = w;
     }
     return;
   }
@@ -111,10 +117,8 @@ __device__ __forceinline__ void emit_entry(const SelectArgs& A, int dest, uint32
   } else if (A.out_mc != nullptr) {
     multimem_st_pair(A.out_mc + slot_off + pos, e);
   } else {
-#pragma unroll
-    for (int p = 0; p < kMaxWorld; ++p) {
-      if (p < A.world) A.out[p][slot_off + pos] = e;
-    }
+#pragma unroll 1
+    for (int p = 0; p < A.world; ++p) A.out[p][slot_off + pos] = e;
   }
 }
 

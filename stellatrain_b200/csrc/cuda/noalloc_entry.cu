@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(256) k_noalloc_setup(const float* values, uint
   for (uint32_t c = tid; c < n_chunks; c += stride) {
     const uint32_t start = c * kChunkElems;
     st::Chunk ch;
-    ch.seg = 0; ch.start = start; ch.len = min(kChunkElems, n_pad - start); ch.reserved = 0;
+    ch.seg = 0; ch.start = start; ch.len = min(kChunkElems, n_pad - start); ch.run0 = 0;
     chunks[c] = ch;
     chunk_cnt[c] = 0;
     chunk_pos[c] = 0;

@@ -1,0 +1,1058 @@
+// One-pass select: the steady state of top-k, threshold-v and threshold-v16.
+//
+// Every tensor remembers the threshold of its previous select, so one pass over gradient and residual can already tell
+// the few items that matter from the rest:
+//   scan    a = g + r, r <- a; every warp walks one run of 1024 consecutive elements and lists the run's items at or over
+//           a cut, without a word to any other warp.  The cut is the persistent threshold (threshold-v and threshold-v16,
+//           backend/src/compress/thresholdv.cpp:44-52, backend/src/compress/thresholdv16.cpp:81-97; the latter also lists
+//           near-miss blocks just under it) or a little less than the previous k-th largest value (top-k, which also
+//           counts its candidates in a histogram around that value).
+//   emit    one CTA per piece (up to 128 runs) of a tensor turns the lists into stream entries, stores them into the
+//           destinations' receive areas and clears them in r.  The CTA that finishes a tensor last settles what is left:
+//           the exact cut inside the threshold's bin (top-k), the best of the near misses when the blocks over the
+//           threshold fall short of the budget (the reference's heap, backend/src/compress/thresholdv16.cpp:261-293),
+//           the step of the threshold (AIMD).  Threshold-v pads a short stream instead
+//           (backend/src/compress/thresholdv.cpp:82).
+//   refill  top-k only: tensors whose candidates fell short of k (the distribution dropped below the cut) are selected
+//           from r itself.  Their histogram was taken by `emit`; with no such tensor this kernel returns at once.
+// 12 bytes per element cross HBM (read g, read r, write r) against 16 to 20 of the four-kernel chain, which remains for a
+// tensor's first select.  The results are those of the four-kernel chain; only the order of a top-k stream differs.
+#include "select_common.cuh"
+
+namespace st {
+
+namespace {
+
+enum ScanMode : int { kScanTop = 0, kScanElem = 1, kScanBlock = 2 };
+
+constexpr int kScanThreads = 256;
+constexpr int kScanWarps = kScanThreads / 32;
+constexpr uint32_t kHalf = kRunElems / 2;      // a run is read in two halves: four float4 of r and of g per lane in flight
+constexpr uint32_t kRunBlocks = kRunElems / 16;
+constexpr uint32_t kPieceElems = kPieceRuns * kRunElems;
+
+constexpr int kEmitThreads = 256;
+constexpr uint32_t kStageItems = 2048;         // entries staged at a time
+constexpr uint32_t kPickMax = 2048;            // candidates that a CTA holds in registers to pick the best from
+
+// Top-k of a tensor this small is picked from registers by its one CTA of `emit`: its k-th largest value moves too much from
+// step to step to be worth predicting, and no list, histogram or cut is needed.
+constexpr uint32_t kTopDirect = 4096;
+constexpr float kTopWindowDefault = 0.1f;
+constexpr float kTopWindowMin = 1e-3f;
+constexpr float kTopWindowMax = 0.45f;         // the histogram reaches down to half the previous threshold
+
+__device__ __forceinline__ float window_or(uint32_t bits, float fallback) {
+  const float w = __uint_as_float(bits);
+  return (w > 0.f && w <= 1.f) ? w : fallback;
+}
+
+// Lowest key top-k lists: a little under the previous k-th largest value, and never zero.
+__device__ __forceinline__ uint32_t top_cut(const SegState& ss, uint32_t n_pad) {
+  if (n_pad <= kTopDirect) return 0xFFFFFFFFu;     // lists nothing
+  const float t = __uint_as_float(ss.reserved[1]);
+  const float w = fminf(window_or(ss.reserved[0], kTopWindowDefault), kTopWindowMax);
+  const uint32_t cut = t < __uint_as_float(0x7f800000u) ? __float_as_uint(t * (1.f - w)) : ss.reserved[1];
+  return cut ? cut : 1u;
+}
+
+// Histogram of top-k's candidates around the previous threshold c (float bits), three widths of bins: 1024 of 2^-17
+// (relative) within 0.4 % of it, 256 of 2^-13 on either side as far as 3 %, 256 of 2^-8 on either side as far as an octave,
+// everything beyond in the end bins.  Error feedback piles items up at the threshold: with bins of 2^-10 throughout a few of
+// them took most of the counts (L2 adds to one address one after the other: 239 us for a scan of 38.6 M elements, of
+// which the traffic needs 75) and the threshold's bin held thousands of undecided items.
+// c = 0 stands for "no usable threshold": 2048 even bins over all keys.
+// A tensor of several pieces spreads its counts over up to eight such histograms (one per piece modulo eight): 500,000
+// adds into the 64 cache lines of a single one still took 60 us longer than the traffic.
+constexpr int kNearShift = 6, kMidShift = 10, kFarShift = 15;
+constexpr uint32_t kNear = 512u << kNearShift, kMid = kNear + (256u << kMidShift);     // distances where the widths change
+
+__device__ __forceinline__ uint32_t top_centre(const SegState& ss) {
+  return ss.reserved[1] >= (1u << 24) ? ss.reserved[1] : 0u;      // all bins under it fit
+}
+
+// Histogram of what lies under the cut, for a tensor whose candidates fell short: bins of 2^15 key units for the four octaves
+// under the cut (2^-8 relative; coarser ones would put most elements on a few shared-memory addresses), four bins per octave
+// below, bin 0 for zeros alone.  Monotone in key; key < cut.
+__device__ __forceinline__ uint32_t rest_bin(uint32_t key, uint32_t cut) {
+  const uint32_t d = cut - 1u - key;
+  if (d < 1u << 25) return key ? 2047u - (d >> 15) : 0u;
+  return key ? max(1u, min(1023u, key >> 21)) : 0u;
+}
+
+__device__ __forceinline__ void rest_bin_range(uint32_t bin, uint32_t cut, uint32_t& lo, uint32_t& hi) {
+  if (bin == 0u) { lo = 0u; hi = 1u; return; }
+  if (bin >= 1024u) {
+    const uint32_t from = (2047u - bin) << 15;         // distances [from, from + 2^15)
+    hi = cut - from;
+    lo = hi > 1u << 15 ? hi - (1u << 15) : 1u;
+  } else {
+    lo = bin == 1u ? 1u : bin << 21;
+    hi = (bin + 1u) << 21;
+  }
+  if (cut > 1u << 25) {                                // the four octaves end where the coarse bins begin
+    const uint32_t edge = cut - (1u << 25);
+    if (bin >= 1024u) lo = max(lo, edge); else hi = min(hi, edge);
+  }
+}
+
+__device__ __forceinline__ uint32_t hist_copies(uint32_t pieces) {
+  return pieces >= 8u ? 8u : pieces >= 4u ? 4u : pieces >= 2u ? 2u : 1u;
+}
+
+// Monotone in key.
+__device__ __forceinline__ uint32_t top_bin(uint32_t key, uint32_t c) {
+  if (c == 0u) return key >> kHistShift;
+  const bool above = key >= c;
+  const uint32_t d = above ? key - c : c - key - 1u;
+  const uint32_t b = d < kNear ? d >> kNearShift : d < kMid ? 512u + ((d - kNear) >> kMidShift) : min(1023u, 768u + ((d - kMid) >> kFarShift));
+  return above ? 1024u + b : 1023u - b;
+}
+
+// Key range [lo, hi) of a bin; keys are below 2^31, so 2^31 stands for "none above".
+__device__ __forceinline__ void top_bin_range(uint32_t bin, uint32_t c, uint32_t& lo, uint32_t& hi) {
+  if (c == 0u) {
+    lo = bin << kHistShift;
+    hi = (bin + 1u) << kHistShift;
+    return;
+  }
+  const bool above = bin >= 1024u;
+  const uint32_t b = above ? bin - 1024u : 1023u - bin;
+  const int shift = b < 512u ? kNearShift : b < 768u ? kMidShift : kFarShift;
+  const uint32_t from = b < 512u ? b << kNearShift : b < 768u ? kNear + ((b - 512u) << kMidShift) : kMid + ((b - 768u) << kFarShift);
+  const uint32_t to = from + (1u << shift);          // distances [from, to)
+  lo = above ? c + from : b == 1023u ? 0u : c - to;
+  hi = above ? (b == 1023u ? 0x80000000u : c + to) : c - from;
+}
+static_assert(kHistBins == 2048 && kHistShift == 20 && kMid + (256u << kFarShift) < 1u << 24, "bins of top_bin");
+
+}  // namespace
+
+// ------------------------------------------------------------------------------------------------
+// scan
+// ------------------------------------------------------------------------------------------------
+template <int MODE>
+__global__ void __launch_bounds__(kScanThreads, 4) k_scan(SelectArgs A) {
+  // The run's place is all the first loads of r need: they are on their way while the tensor's descriptor, threshold and
+  // gradient pointer (a second level of dependent loads) are fetched.
+  const Chunk ch = A.chunks[blockIdx.x];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  // Listed elements of half a run meet here, so that all lanes take part in storing (and, top-k, counting) them.  A fuller
+  // half goes straight to the list.
+  constexpr uint32_t kStage = MODE == kScanBlock ? 1u : 96u;
+  __shared__ uint2 s_stage[kScanWarps][kStage];
+  uint2* const stage = s_stage[warp];
+  if (blockIdx.x == 0 && threadIdx.x == 0 && A.stamps != nullptr) A.stamps[0] = global_timer_ns();
+
+  for (uint32_t rel = warp * kRunElems; rel < ch.len; rel += kScanWarps * kRunElems) {
+    const uint32_t start = ch.start + rel;
+    const uint32_t len = min(kRunElems, ch.len - rel);     // multiple of 16
+    float* r = A.resid + start;
+    float4 rv[4], gv[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t i = j * 128u + lane * 4u;
+      rv[j] = i < len ? *reinterpret_cast<const float4*>(r + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const SegDesc sd = A.segs[ch.seg];
+    const bool tab = A.grad_tab != nullptr;
+    const uint32_t seg_rel = start - sd.off, piece_of_seg = seg_rel / kPieceElems;
+    float* g = tab ? A.grad_tab[ch.seg] + seg_rel : A.grad + start;
+    const SegState ss = A.state[ch.seg];
+    if (sd.reserved & kSegSkip) {
+      // a tensor another rank of the group is responsible for: only clear the consumed gradient
+      if (A.zero_grad && !tab)
+        for (uint32_t i = lane * 4u; i < len; i += 128u) *reinterpret_cast<float4*>(g + i) = make_float4(0.f, 0.f, 0.f, 0.f);
+      continue;
+    }
+    const uint32_t n_valid = sd.n > seg_rel ? min(len, sd.n - seg_rel) : 0u;
+    const uint32_t g_valid = tab ? n_valid : len;          // gradients handed over per tensor are not padded
+    const bool add = !A.skip_ef;
+    // a tensor without a threshold yet lists nothing: `emit` then takes the exact top items from the residual
+    const uint32_t tau_bits = ss.inited ? __float_as_uint(ss.tau) : 0xFFFFFFFFu;
+    uint32_t cut = tau_bits, near_lo = 0xFFFFFFFFu;
+    if (MODE == kScanTop) cut = top_cut(ss, sd.n_pad);
+    if (MODE == kScanBlock && ss.inited)
+      near_lo = __float_as_uint(fmaxf(ss.tau * (1.f - window_or(ss.reserved[0], kWindowDefault)), 0.f));
+
+    uint32_t n_list = 0, mx = 0;        // entries listed so far; largest key of this lane
+    uint32_t own[2] = {0u, 0u};         // block mode: keys of two of the run's blocks, numbers h * 32 + (lane & 3) * 8 + lane / 4
+    uint2* list = A.cand + (MODE == kScanBlock ? start >> 4 : start);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t h0 = h * kHalf + lane * 4u;
+      if (h == 1) {
+        if (len <= kHalf) break;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t i = h0 + j * 128u;
+          rv[j] = i < len ? *reinterpret_cast<const float4*>(r + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+      }
+      if (add) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t i = h0 + j * 128u;
+          gv[j] = i < len ? load4_guarded(g, i, g_valid) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+      }
+      uint32_t mask = 0;                // bit 4 j + e: element e of float4 j is listed
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t i = h0 + j * 128u;
+        float4 a = rv[j];
+        if (add) {
+          a.x += gv[j].x; a.y += gv[j].y; a.z += gv[j].z; a.w += gv[j].w;
+          // NaN policy: a NaN is dropped (neither sent nor kept), so it cannot poison the residual.  The sum of the
+          // magnitudes is NaN exactly when one of them is.
+          const float s = (fabsf(a.x) + fabsf(a.y)) + (fabsf(a.z) + fabsf(a.w));
+          if (!(s == s)) {
+            if (!(a.x == a.x)) a.x = 0.f;
+            if (!(a.y == a.y)) a.y = 0.f;
+            if (!(a.z == a.z)) a.z = 0.f;
+            if (!(a.w == a.w)) a.w = 0.f;
+          }
+          if (i < len) {
+            *reinterpret_cast<float4*>(r + i) = a;
+            if (A.zero_grad) store4_guarded(g, i, g_valid, make_float4(0.f, 0.f, 0.f, 0.f));
+          }
+          rv[j] = a;
+        }
+        if (MODE == kScanBlock) {
+          const uint32_t key = __float_as_uint(quad_l1(a));   // the same value in the four lanes of a block
+          if ((lane & 3u) == (uint32_t)j) own[h] = key;
+        } else {
+          const uint32_t k0 = key_bits(a.x), k1 = key_bits(a.y), k2 = key_bits(a.z), k3 = key_bits(a.w);
+          mask |= (k0 >= cut ? 1u << (4 * j) : 0u) | (k1 >= cut ? 2u << (4 * j) : 0u) |
+                  (k2 >= cut ? 4u << (4 * j) : 0u) | (k3 >= cut ? 8u << (4 * j) : 0u);
+          if (MODE == kScanElem) mx = max(mx, max(max(k0, k1), max(k2, k3)));
+        }
+      }
+      if (MODE == kScanElem && n_valid < (h + 1) * kHalf) {
+        // the padding behind the tensor never counts, whatever the threshold
+#pragma unroll
+        for (int b = 0; b < 16; ++b)
+          if (h0 + (b >> 2) * 128u + (b & 3) >= n_valid) mask &= ~(1u << b);
+      }
+      if (MODE != kScanBlock && __any_sync(0xffffffffu, mask != 0u)) {
+        // places in index order: one scan carries the counts of the four float4 in its four bytes (at most 128 each)
+        uint32_t n4 = mask - ((mask >> 1) & 0x5555u);
+        n4 = (n4 & 0x3333u) + ((n4 >> 2) & 0x3333u);
+        n4 = (n4 & 0xFu) | (n4 & 0xF0u) << 4 | (n4 & 0xF00u) << 8 | (n4 & 0xF000u) << 12;
+        const uint32_t incl = warp_incl_scan(n4), ex = incl - n4;
+        const uint32_t all = __shfl_sync(0xffffffffu, incl, 31);
+        const uint32_t n_half = (all & 0xFFu) + ((all >> 8) & 0xFFu) + ((all >> 16) & 0xFFu) + (all >> 24);
+        uint2* const dst = list + n_list;
+        uint2* const first = n_half <= kStage ? stage : dst;
+        uint32_t before = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (mask & (15u << (4 * j))) {
+            const uint32_t at = start + h0 + j * 128u;
+            uint2* to = first + before + ((ex >> (8 * j)) & 0xFFu);
+            if (mask & (1u << (4 * j))) *to++ = make_uint2(at, __float_as_uint(rv[j].x));
+            if (mask & (2u << (4 * j))) *to++ = make_uint2(at + 1u, __float_as_uint(rv[j].y));
+            if (mask & (4u << (4 * j))) *to++ = make_uint2(at + 2u, __float_as_uint(rv[j].z));
+            if (mask & (8u << (4 * j))) *to++ = make_uint2(at + 3u, __float_as_uint(rv[j].w));
+          }
+          before += (all >> (8 * j)) & 0xFFu;
+        }
+        __syncwarp();
+        // Histogram of the candidates.  The top bin, which holds many of them, is not counted: `emit` knows their number.
+        const uint32_t centre = top_centre(ss);
+        const uint32_t copy = piece_of_seg & (hist_copies((sd.n_pad + kPieceElems - 1u) / kPieceElems) - 1u);
+        uint32_t* const gh = A.hist_top + (size_t)((ch.run0 + rel / kRunElems) / kPieceRuns - piece_of_seg + copy) * kHistBins;
+        for (uint32_t q0 = 0; q0 < n_half; q0 += 32u) {
+          const uint32_t q = q0 + lane;
+          uint32_t b = kHistBins - 1;
+          if (q < n_half) {
+            const uint2 e = first[q];
+            if (n_half <= kStage) dst[q] = e;
+            b = top_bin(e.y & 0x7fffffffu, centre);
+          }
+          if (MODE == kScanTop) {
+            if (b != (uint32_t)(kHistBins - 1)) atomicAdd(gh + b, 1u);
+          } else if (n_half > kStage) {
+            break;
+          }
+        }
+        __syncwarp();
+        n_list += n_half;
+      }
+    }
+    uint32_t n_near = 0;
+    if (MODE == kScanBlock) {
+      // selected blocks fill the run's area from the front, near misses from the back: together they are at most all
+      const uint32_t n_blk = len >> 4;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint32_t b = h * 32u + lane;    // block of the run this lane answers for now: lanes in index order
+        const uint32_t key = __shfl_sync(0xffffffffu, own[h], (lane & 7u) * 4u + (lane >> 3));
+        const bool sel = b < n_blk && key >= tau_bits;
+        const bool near = b < n_blk && !sel && key >= near_lo && key != 0u;
+        const uint32_t bs = __ballot_sync(0xffffffffu, sel), bn = __ballot_sync(0xffffffffu, near);
+        const uint32_t below = (1u << lane) - 1u;
+        const uint2 e = make_uint2((start >> 4) + b, key);
+        if (sel) list[n_list + __popc(bs & below)] = e;
+        if (near) list[n_blk - 1u - n_near - __popc(bn & below)] = e;
+        n_list += __popc(bs);
+        n_near += __popc(bn);
+      }
+    }
+    if (MODE == kScanElem) {
+      mx = __reduce_max_sync(0xffffffffu, mx);
+      // runs that do not raise the maximum leave its one address alone
+      if (lane == 0 && mx > ld_volatile_u32(&A.work[ch.seg].max_bits)) atomicMax(&A.work[ch.seg].max_bits, mx);
+    }
+    if (lane == 0) {
+      const uint32_t run = ch.run0 + rel / kRunElems;
+      A.run_cnt[run] = n_list | n_near << 16;
+      // tensors of several pieces: every piece's total, so that each CTA of `emit` can place itself
+      if (sd.n_pad > kPieceElems && (n_list | n_near))
+        atomicAdd(reinterpret_cast<unsigned long long*>(A.piece_cnt + run / kPieceRuns),
+                  (unsigned long long)n_near << 32 | n_list);
+    }
+  }
+}
+
+// ------------------------------------------------------------------------------------------------
+// emit
+// ------------------------------------------------------------------------------------------------
+namespace {
+
+struct EmitShared {
+  uint2 stage[kStageItems];
+  uint32_t hist[2048];
+  uint32_t pre[kPieceRuns + 1];     // listed items in front of each run of the piece
+  uint32_t near[kPieceRuns + 1];    // near misses in front of each run of the piece
+  uint32_t tmp[kEmitThreads / 32 + 1];
+  uint32_t res[4];
+  uint32_t cnt[64];                 // counts of the bitwise searches
+  uint32_t word[4];                 // [0] may emit, [1] last CTA of the tensor, [2], [3] bases of a batch
+  unsigned long long sum[2];        // [0] totals of the tensor
+  uint32_t at[2];                   // piece of the tensor that holds a position, positions in front of it
+};
+
+// Run (of the piece) that holds item j: the last one that starts at or in front of it and is not empty.
+__device__ __forceinline__ uint32_t run_of(const uint32_t* pre, uint32_t j) {
+  uint32_t lo = 0, hi = kPieceRuns;
+#pragma unroll
+  for (int s = 0; s < 7; ++s) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (pre[mid] <= j) lo = mid; else hi = mid;
+  }
+  return lo;
+}
+static_assert(kPieceRuns == 128, "run_of halves 128 runs seven times");
+
+// What a CTA of `emit` / `refill` works on.
+struct Job {
+  Piece pc;
+  SegDesc sd;
+  SegWork* wp;
+  uint32_t epoch, kk;
+  uint64_t slot_off;
+  int dest;
+  uint32_t nb;
+};
+
+__device__ __forceinline__ Job job_of(const SelectArgs& A, bool block) {
+  Job J;
+  J.pc = A.pieces[blockIdx.x];
+  J.sd = A.segs[J.pc.seg];
+  J.wp = &A.work[J.pc.seg];
+  J.epoch = *A.epoch;
+  J.kk = block ? (J.sd.k + 15u) / 16u : J.sd.k;
+  J.slot_off = (uint64_t)(J.epoch & 1u) * A.slot_stride + J.sd.out_off;
+  J.dest = dest_of(A, J.sd);
+  J.nb = narrow_base_of(J.sd);
+  return J;
+}
+
+__device__ __forceinline__ void emit_and_keep(const SelectArgs& A, const Job& J, uint32_t pos, uint32_t gi, float a) {
+  const float sv = wire_value(J.nb, a);
+  emit_entry(A, J.dest, J.nb, J.slot_off, pos, gi, sv);
+  A.resid[gi] = a - sv;     // exactly zero unless the wire format rounds
+}
+
+// True in every thread of the CTA that finishes its tensor last; orders the other CTAs' stores in front of what follows.
+// The CTA barrier orders a CTA's stores before its thread 0, whose release and acquire on the counter order the CTAs.
+__device__ __forceinline__ bool last_of_tensor(const Job& J, EmitShared& S) {
+  __syncthreads();
+  if (J.pc.count == 1u) return true;
+  if (threadIdx.x == 0) {
+    const bool last = atom_add_acq_rel_gpu(&J.wp->pieces_done, 1u) == J.pc.count - 1u;
+    if (last) J.wp->pieces_done = 0u;
+    S.word[1] = last ? 1u : 0u;
+  }
+  __syncthreads();
+  return S.word[1] != 0u;
+}
+
+// Picks the bin of `gh` that holds the kk-th largest of n_items keys: S.res = {bin, items still to be taken from it, items
+// in it}.  One end bin is not counted and holds what the others do not: the top one or, for the histogram of the rest, bin 0.
+__device__ __forceinline__ void plan_top(const uint32_t* gh, uint32_t copies, uint32_t n_items, uint32_t kk, bool rest_hist,
+                                         EmitShared& S) {
+  constexpr int kPer = kHistBins / kEmitThreads;
+  const uint32_t tid = threadIdx.x;
+  static_assert(kPer == 8, "two 16-byte loads per thread");
+  // thread t owns the bins 2047 - 8 t ... 2040 - 8 t, highest first
+  uint32_t h[kPer] = {};
+#pragma unroll
+  for (uint32_t r = 0; r < 8u; ++r) {
+    if (r < copies) {
+      const uint4* row = reinterpret_cast<const uint4*>(gh + (size_t)r * kHistBins + kHistBins - kPer * (tid + 1));
+      const uint4 lo = __ldcg(row), hi = __ldcg(row + 1);
+      h[0] += hi.w; h[1] += hi.z; h[2] += hi.y; h[3] += hi.x;
+      h[4] += lo.w; h[5] += lo.z; h[6] += lo.y; h[7] += lo.x;
+    }
+  }
+  if (tid == 0 && !rest_hist) h[0] = 0u;
+  if (tid == kEmitThreads - 1 && rest_hist) h[kPer - 1] = 0u;
+  uint32_t local = 0;
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) local += h[j];
+  uint32_t total;
+  uint32_t running = block_excl_scan(local, S.tmp, total);
+  const uint32_t rest = n_items > total ? n_items - total : 0u;
+  if (rest_hist) {
+    if (tid == kEmitThreads - 1) h[kPer - 1] = rest;
+  } else {
+    if (tid == 0) h[0] = rest;
+    else running += rest;
+  }
+  if (tid == 0) { S.res[0] = 0u; S.res[1] = 0u; S.res[2] = 0u; }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    if (running < kk && running + h[j] >= kk) {
+      S.res[0] = kHistBins - 1 - (tid * kPer + j);
+      S.res[1] = kk - running;
+      S.res[2] = h[j];
+    }
+    running += h[j];
+  }
+  __syncthreads();
+}
+
+// Sends the `n` marked items of a CTA's batch at positions base, base + 1, ...: bit u of `sel` marks the thread's item u, `ex`
+// is the number of marked items in front of the thread's first.  They go through shared memory, so that the stores into the
+// destinations are consecutive and stand in the code once (unrolled per item they took 10 us in instruction fetches alone).
+template <int N>
+__device__ __forceinline__ void send_marked(const SelectArgs& A, const Job& J, EmitShared& S, const uint32_t (&idx)[N],
+                                            const uint32_t (&bits)[N], uint32_t sel, uint32_t ex, uint32_t n, uint32_t base) {
+  uint2* const stage = S.stage;
+  for (uint32_t w = 0; w < n; w += kStageItems) {
+    uint32_t p = ex - w;
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+      if (sel >> u & 1u) {
+        if (p < kStageItems) stage[p] = make_uint2(idx[u], bits[u]);
+        ++p;
+      }
+    }
+    __syncthreads();
+    const uint32_t m = min(kStageItems, n - w);
+#pragma unroll 1
+    for (uint32_t q = threadIdx.x; q < m; q += kEmitThreads)
+      emit_and_keep(A, J, base + w + q, stage[q].x, __uint_as_float(stage[q].y));
+    __syncthreads();
+  }
+}
+
+// Sends the items over the threshold's bin and notes those inside it.  `emitted` / `noted`: counts so far when one CTA
+// has the whole tensor; several CTAs draw theirs from the tensor's counters, once per batch.
+template <int N>
+__device__ __forceinline__ void emit_top_batch(const SelectArgs& A, const Job& J, EmitShared& S, uint2* undecided,
+                                               const uint32_t (&idx)[N], const uint32_t (&bits)[N], uint32_t key_lo,
+                                               uint32_t key_hi, uint32_t& emitted, uint32_t& noted) {
+  uint32_t sel = 0, und = 0;
+#pragma unroll
+  for (int u = 0; u < N; ++u) {
+    const uint32_t key = bits[u] & 0x7fffffffu;
+    const bool there = idx[u] != kSentinelIdx;
+    sel |= (uint32_t)(there && key >= key_hi) << u;
+    und |= (uint32_t)(there && key >= key_lo && key < key_hi) << u;
+  }
+  uint32_t total;
+  const uint32_t ex = block_excl_scan(__popc(sel) | __popc(und) << 16, S.tmp, total);
+  const uint32_t t_sel = total & 0xffffu, t_und = total >> 16;
+  uint32_t b_sel = emitted, b_und = noted;
+  if (J.pc.count > 1u) {
+    if (threadIdx.x == 0) {
+      S.word[2] = t_sel ? atomicAdd(&J.wp->out_cursor, t_sel) : 0u;
+      S.word[3] = t_und ? atomicAdd(&J.wp->cand_cnt, t_und) : 0u;
+    }
+    __syncthreads();
+    b_sel = S.word[2];
+    b_und = S.word[3];
+  }
+  emitted += t_sel;
+  noted += t_und;
+  uint32_t q = b_und + (ex >> 16);
+#pragma unroll
+  for (int u = 0; u < N; ++u)
+    if (und >> u & 1u) undecided[q++] = make_uint2(idx[u], bits[u] & 0x7fffffffu);
+  send_marked<N>(A, J, S, idx, bits, sel, ex & 0xffffu, t_sel, b_sel);
+}
+
+// Where the best `take` of the CTA's (key, id) pairs end (larger key first, equal keys by lower id): the lowest-ranked one
+// taken.  `there`: bit u says whether pair u counts; 1 <= take <= number of pairs.  The CTA holds the pairs in registers and
+// finds the key bit by bit, as many bits as [key_lo, key_hi), which holds all keys, leaves open; a step is a count over the
+// CTA with one barrier, about 0.1 us whatever the data (ranking 400 pairs against one another took 25 us).  The caller has
+// cleared S.cnt behind a barrier.
+template <int N>
+__device__ __forceinline__ uint2 cut_of_best(const uint32_t (&key)[N], const uint32_t (&id)[N], uint32_t there, uint32_t take,
+                                             uint32_t key_lo, uint32_t key_hi, EmitShared& S) {
+  auto count = [&](int slot, auto pred) {
+    uint32_t n = 0;
+#pragma unroll
+    for (int u = 0; u < N; ++u) n += (there >> u & 1u) && pred(key[u], id[u]) ? 1u : 0u;
+    n = __reduce_add_sync(0xffffffffu, n);
+    if ((threadIdx.x & 31u) == 0u && n) atomicAdd(&S.cnt[slot], n);
+    __syncthreads();
+    return S.cnt[slot];
+  };
+  uint32_t t = key_lo, n_ge = 0xFFFFFFFFu;      // a key that at least `take` pairs reach
+  for (int bit = 31 - __clz((key_hi - key_lo) | 1u); bit >= 0 && n_ge != take; --bit) {
+    const uint32_t trial = t + (1u << bit);
+    const uint32_t n = count(bit, [&](uint32_t k, uint32_t) { return k >= trial; });
+    if (n >= take) { t = trial; n_ge = n; }
+  }
+  uint32_t last;
+  if (n_ge == take) {
+    // exactly the pairs from t upwards: the smallest key among them, and the highest id that has it
+    uint32_t mn = 0xFFFFFFFFu, mx = 0;
+#pragma unroll
+    for (int u = 0; u < N; ++u)
+      if ((there >> u & 1u) && key[u] >= t) mn = min(mn, key[u]);
+    t = ~block_max_u32(~mn, S.tmp);
+#pragma unroll
+    for (int u = 0; u < N; ++u)
+      if ((there >> u & 1u) && key[u] == t) mx = max(mx, id[u]);
+    last = block_max_u32(mx, S.tmp);
+  } else {
+    // t is the take-th largest key itself and more pairs share it than are wanted
+    const uint32_t need = take - count(31, [&](uint32_t k, uint32_t) { return k > t; });
+    last = 0;                      // the need-th smallest id among equal keys: the largest that fewer ids lie under
+    for (int bit = 31; bit >= 0; --bit) {
+      const uint32_t trial = last | 1u << bit;
+      if (count(32 + bit, [&](uint32_t k, uint32_t i) { return k == t && i < trial; }) < need) last = trial;
+    }
+  }
+  return make_uint2(t, last);
+}
+
+// The best `take` of c candidates: their ids go to S.hist, the lowest-ranked one last.  Returns its key.
+// 1 <= take <= c <= N * kEmitThreads.
+template <int N>
+__device__ __forceinline__ uint32_t pick_best(const uint2* cand, uint32_t c, uint32_t take, uint32_t key_lo, uint32_t key_hi,
+                                              EmitShared& S) {
+  static_assert(N * kEmitThreads <= (int)kPickMax && kPickMax <= 2048, "the ids fit EmitShared::hist");
+  const uint32_t tid = threadIdx.x;
+  uint32_t key[N], id[N], there = 0;
+#pragma unroll
+  for (int u = 0; u < N; ++u) {
+    const uint32_t i = u * kEmitThreads + tid;
+    const uint2 e = i < c ? __ldcg(cand + i) : make_uint2(0u, 0u);
+    there |= (uint32_t)(i < c) << u;
+    id[u] = e.x;
+    key[u] = e.y;
+  }
+  if (tid < 64u) S.cnt[tid] = 0u;
+  if (tid == 64u) S.word[2] = 0u;
+  __syncthreads();
+  const uint2 cut = cut_of_best<N>(key, id, there, take, key_lo, key_hi, S);
+#pragma unroll
+  for (int u = 0; u < N; ++u) {
+    if ((there >> u & 1u) && (key[u] > cut.x || (key[u] == cut.x && id[u] <= cut.y))) {
+      const bool is_last = key[u] == cut.x && id[u] == cut.y;
+      S.hist[is_last ? take - 1u : atomicAdd(&S.word[2], 1u)] = id[u];
+    }
+  }
+  __syncthreads();
+  return cut.x;
+}
+
+__device__ __forceinline__ uint32_t pick_few(const uint2* cand, uint32_t c, uint32_t take, uint32_t key_lo, uint32_t key_hi,
+                                             EmitShared& S) {
+  return c <= (uint32_t)kEmitThreads ? pick_best<1>(cand, c, take, key_lo, key_hi, S)
+                                     : pick_best<kPickMax / kEmitThreads>(cand, c, take, key_lo, key_hi, S);
+}
+
+// Top-k of a small tensor, from registers: every thread holds N of its elements.  Returns the k-th largest key.
+template <int N>
+__device__ __forceinline__ uint32_t top_direct(const SelectArgs& A, const Job& J, EmitShared& S) {
+  const uint32_t tid = threadIdx.x;
+  uint32_t key[N], id[N], bits[N], there = 0;
+#pragma unroll
+  for (int u = 0; u < N / 4; ++u) {
+    const uint32_t i = (u * kEmitThreads + tid) * 4u;
+    const bool act = i < J.sd.n_pad;
+    const float4 a = act ? *reinterpret_cast<const float4*>(A.resid + J.sd.off + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    there |= (act ? 15u : 0u) << (4 * u);
+    const float v[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      id[4 * u + e] = J.sd.off + i + e;
+      bits[4 * u + e] = __float_as_uint(v[e]);
+      key[4 * u + e] = key_bits(v[e]);
+    }
+  }
+  if (tid < 64u) S.cnt[tid] = 0u;
+  __syncthreads();
+  const uint2 cut = cut_of_best<N>(key, id, there, J.kk, 0u, 0x7fffffffu, S);
+  uint32_t take = 0;
+#pragma unroll
+  for (int u = 0; u < N; ++u)
+    take |= (uint32_t)((there >> u & 1u) && (key[u] > cut.x || (key[u] == cut.x && id[u] <= cut.y))) << u;
+  uint32_t total;
+  const uint32_t ex = block_excl_scan(__popc(take), S.tmp, total);
+  send_marked<N>(A, J, S, id, bits, take, ex, total, 0u);
+  return cut.x;
+}
+
+// Top-k, last CTA of a tensor: the best `rem` of the `c` undecided items complete the stream.  Returns the k-th largest key.
+__device__ __forceinline__ uint32_t settle_top(const SelectArgs& A, const Job& J, EmitShared& S, const uint2* undecided,
+                                               uint32_t c, uint32_t rem, uint32_t key_lo, uint32_t key_hi) {
+  const uint32_t done = J.kk - rem;
+  if (c <= kPickMax) {
+    const uint32_t t_key = pick_few(undecided, c, rem, key_lo, key_hi, S);
+#pragma unroll 1
+    for (uint32_t q = threadIdx.x; q < rem; q += kEmitThreads) {
+      const uint32_t gi = S.hist[q];
+      emit_and_keep(A, J, done + q, gi, __ldcg(A.resid + gi));
+    }
+    return t_key;
+  }
+  if (threadIdx.x == 0) J.wp->out_cursor = done;
+  __syncthreads();
+  return take_top<kEmitThreads>(A, J.sd, J.wp, undecided, c, rem, false, J.kk, J.kk - 1u, J.slot_off, J.dest, J.nb, S.hist,
+                                S.tmp, S.res);
+}
+
+// Sends the items [j0, j1) of one piece at positions base + j; items and positions are in index order.  The dependent loads
+// (list, residual) of four entries per thread travel together; the entries then pass through shared memory as above.
+template <bool kBlock>
+__device__ __forceinline__ void send_range(const SelectArgs& A, const Job& J, EmitShared& S, const uint2* lists,
+                                           uint32_t base, uint32_t j0, uint32_t j1) {
+  constexpr uint32_t kPerItem = kBlock ? 16u : 1u, kArea = kBlock ? kRunBlocks : kRunElems;
+  constexpr uint32_t kIlp = kStageItems / kEmitThreads;
+  uint2* const stage = S.stage;
+  const uint32_t end = j1 * kPerItem;
+  for (uint32_t t0 = j0 * kPerItem; t0 < end; t0 += kStageItems) {
+    uint2 e[kIlp];
+#pragma unroll
+    for (int u = 0; u < (int)kIlp; ++u) {
+      const uint32_t t = t0 + u * kEmitThreads + threadIdx.x;
+      e[u] = make_uint2(0u, 0u);
+      if (t < end) {
+        const uint32_t j = t / kPerItem, run = run_of(S.pre, j);
+        e[u] = lists[run * kArea + (j - S.pre[run])];
+        if (kBlock) e[u].x = e[u].x * 16u + (t & 15u);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < (int)kIlp; ++u) {
+      if (kBlock && t0 + u * kEmitThreads + threadIdx.x < end) e[u].y = __float_as_uint(__ldcg(A.resid + e[u].x));
+      stage[u * kEmitThreads + threadIdx.x] = e[u];
+    }
+    __syncthreads();
+    // a truncated last block leaves the residual exact: only emitted elements are cleared
+    const uint32_t p0 = base * kPerItem + t0, m = min(min(kStageItems, end - t0), J.sd.k > p0 ? J.sd.k - p0 : 0u);
+#pragma unroll 1
+    for (uint32_t q = threadIdx.x; q < m; q += kEmitThreads)
+      emit_and_keep(A, J, p0 + q, stage[q].x, __uint_as_float(stage[q].y));
+    __syncthreads();
+  }
+}
+
+// Thread 0 of the last CTA of a top-k tensor: what the next select starts from.  Every candidate costs a list entry and a
+// histogram count, candidates that fall short cost two more passes over the tensor (twice the time).  How many more
+// candidates there were than entries says how near the cut came to falling short.  The threshold of one batch differs from
+// that of the next, so the window grows at once when few were spare and shrinks by a few per cent a step when many were.
+__device__ __forceinline__ void step_top(const SelectArgs& A, const Job& J, SegState ss, uint32_t t_key, uint32_t listed) {
+  float w = fminf(window_or(ss.reserved[0], kTopWindowDefault), kTopWindowMax);
+  const float k = (float)J.kk, spare = (float)listed - k, noise = 4.f * sqrtf(k);
+  if (spare < 0.f) w *= 2.f;
+  else if (spare < noise + 0.15f * k) w *= 1.3f;
+  else if (spare > 2.f * noise + 0.3f * k) w *= 0.97f;
+  if (J.sd.n_pad > kTopDirect) ss.reserved[0] = __float_as_uint(fminf(fmaxf(w, kTopWindowMin), kTopWindowMax));
+  ss.reserved[1] = t_key;
+  if (t_key < (uint32_t)(kHistBins / 2) << (kFineShift + 1)) { ss.hist_shift = 0; ss.hist_base = 0; }
+  else centre_window(ss, t_key);
+  A.state[J.pc.seg] = ss;
+}
+
+}  // namespace
+
+template <int MODE>
+__global__ void __launch_bounds__(kEmitThreads, 4) k_emit(SelectArgs A) {
+  __shared__ EmitShared S;
+  constexpr bool kBlock = MODE == kScanBlock;
+  const uint32_t tid = threadIdx.x;
+  const Job J = job_of(A, kBlock);
+  const uint32_t cnt = tid < J.pc.n_runs ? A.run_cnt[blockIdx.x * kPieceRuns + tid] : 0u;
+  const bool ok = ld_volatile_u32(A.status) == kOk;
+
+  if (!(J.sd.reserved & kSegSkip)) {
+    const SegState ss = A.state[J.pc.seg];
+    // listed items and near misses of this piece and of the tensor
+    unsigned long long all = 0ull;
+    if (J.pc.count > 1u)
+      for (uint32_t t = tid; t < J.pc.count; t += kEmitThreads) all += A.piece_cnt[J.pc.first + t];
+    if (tid < 2) S.sum[tid] = 0ull;
+    uint32_t total, near_total = 0;
+    uint32_t ex = block_excl_scan(cnt & 0xffffu, S.tmp, total);
+    if (tid <= kPieceRuns) S.pre[tid] = ex;
+    if (kBlock) {
+      const uint32_t nex = block_excl_scan(cnt >> 16, S.tmp, near_total);
+      if (tid <= kPieceRuns) S.near[tid] = nex;
+    }
+    uint32_t found = total, c_near = near_total;
+    if (J.pc.count > 1u) {
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) all += __shfl_xor_sync(0xffffffffu, all, d);
+      if ((tid & 31u) == 0u && all) atomicAdd(&S.sum[0], all);
+      __syncthreads();
+      found = (uint32_t)S.sum[0];
+      c_near = (uint32_t)(S.sum[0] >> 32);
+    }
+    const bool short_of = found < J.kk;
+    // will this CTA store into the destinations?  Then they must have consumed the slot.
+    if (tid == 0) S.word[0] = ok && acks_arrived(A, J.epoch) ? 1u : 0u;
+    __syncthreads();
+    const bool may = S.word[0] != 0u;
+    uint2* const area = A.cand + (kBlock ? J.pc.start >> 4 : J.pc.start);
+    constexpr uint32_t kArea = kBlock ? kRunBlocks : kRunElems;      // list slots per run
+
+    if (MODE == kScanTop) {
+      uint2* const undecided = A.cand + A.n_total + J.sd.off;
+      uint32_t emitted = 0, noted = 0, key_lo = 0, key_hi = 0;
+      const bool direct = J.sd.n_pad <= kTopDirect;
+      if (direct) {
+        if (may) {
+          const uint32_t t_key = J.sd.n_pad <= 4u * kEmitThreads ? top_direct<4>(A, J, S) : top_direct<16>(A, J, S);
+          if (tid == 0) step_top(A, J, ss, t_key, 0u);
+        }
+      } else if (short_of && ok) {
+        // the candidates do not reach down to the k-th largest value: a histogram of the rest, for `refill`
+        const uint32_t cut = top_cut(ss, J.sd.n_pad);
+        for (uint32_t b = tid; b < (uint32_t)kHistBins; b += kEmitThreads) S.hist[b] = 0u;
+        __syncthreads();
+        const uint32_t len = min(kPieceElems, J.sd.off + J.sd.n_pad - J.pc.start);
+        uint32_t zeros = 0;
+#pragma unroll 4
+        for (uint32_t i = tid * 4u; i < len; i += kEmitThreads * 4u) {
+          const float4 a = *reinterpret_cast<const float4*>(A.resid + J.pc.start + i);
+          const uint32_t key[4] = {key_bits(a.x), key_bits(a.y), key_bits(a.z), key_bits(a.w)};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            if (key[e] == 0u) ++zeros;
+            else if (key[e] < cut) atomicAdd(&S.hist[rest_bin(key[e], cut)], 1u);
+          }
+        }
+        block_excl_scan(zeros, S.tmp, zeros);
+        uint32_t* gh = A.hist_rest + (size_t)J.pc.seg * kHistBins;
+        for (uint32_t b = tid; b < (uint32_t)kHistBins; b += kEmitThreads)
+          if (S.hist[b]) atomicAdd(gh + b, S.hist[b]);
+        if (tid == 0) A.run_cnt[blockIdx.x * kPieceRuns] = zeros;     // this CTA has read its own counts
+      } else if (!short_of) {
+        plan_top(A.hist_top + (size_t)J.pc.first * kHistBins, hist_copies(J.pc.count), found, J.kk, false, S);
+        top_bin_range(S.res[0], top_centre(ss), key_lo, key_hi);
+        if (may) {
+          constexpr int kItems = 8;
+          for (uint32_t j0 = 0; j0 < total; j0 += kEmitThreads * kItems) {
+            uint32_t idx[kItems], bits[kItems];
+#pragma unroll
+            for (int u = 0; u < kItems; ++u) {
+              const uint32_t j = j0 + tid * kItems + u;     // the stream keeps the lists' order: the update reads it faster
+              idx[u] = kSentinelIdx;
+              bits[u] = 0u;
+              if (j < total) {
+                const uint32_t run = run_of(S.pre, j);
+                const uint2 e = area[run * kArea + (j - S.pre[run])];
+                idx[u] = e.x;
+                bits[u] = e.y;
+              }
+            }
+            emit_top_batch<kItems>(A, J, S, undecided, idx, bits, key_lo, key_hi, emitted, noted);
+          }
+        }
+      }
+      const uint32_t rem = S.res[1];     // read before the helpers below reuse the words
+      if (!direct && last_of_tensor(J, S)) {
+        if (!short_of) {
+          const uint32_t c = J.pc.count == 1u ? noted : __ldcg(&J.wp->cand_cnt);
+          if (may && rem != 0u && rem <= c) {
+            const uint32_t t_key = settle_top(A, J, S, undecided, c, rem, key_lo, key_hi);
+            if (tid == 0) step_top(A, J, ss, t_key, found);
+          } else if (may && tid == 0) {
+            set_status(A.status, kBadCandidate);   // cannot happen: the histogram counted these very items
+          }
+        } else if (tid == 0 && ok) {
+          J.wp->refill = 1u;                       // `refill` selects this tensor
+          J.wp->found = found;
+          atomicAdd(A.refills, 1u);
+        }
+        __syncthreads();
+        if (tid == 0) { J.wp->out_cursor = 0u; J.wp->cand_cnt = 0u; }
+        for (uint32_t t = tid; t < J.pc.count; t += kEmitThreads) A.piece_cnt[J.pc.first + t] = 0ull;
+        uint4* gh = reinterpret_cast<uint4*>(A.hist_top + (size_t)J.pc.first * kHistBins);
+        for (uint32_t b = tid; b < hist_copies(J.pc.count) * (kHistBins / 4); b += kEmitThreads) gh[b] = make_uint4(0u, 0u, 0u, 0u);
+      }
+    } else {
+      uint2* const nears = A.cand + (A.n_total >> 4) + (J.sd.off >> 4);     // block mode: one slot per block of the tensor
+      if (kBlock && short_of && near_total) {
+        // the fill needs the tensor's near misses in one place
+        if (tid == 0) S.word[2] = J.pc.count == 1u ? 0u : atomicAdd(&J.wp->cand_cnt, near_total);
+        __syncthreads();
+        const uint32_t nb0 = S.word[2];
+        for (uint32_t j = tid; j < near_total; j += kEmitThreads) {
+          const uint32_t run = run_of(S.near, j);
+          const uint32_t in_seg = J.pc.start - J.sd.off + run * kRunElems;
+          const uint32_t n_blk = min(kRunElems, J.sd.n_pad - in_seg) >> 4;
+          nears[nb0 + j] = area[run * kArea + n_blk - 1u - (j - S.near[run])];
+        }
+      }
+      // The first kk items in index order are sent.  A threshold that lags behind lets nearly everything pass, and the budget
+      // then ends within the tensor's first piece: the positions, not the pieces, are shared out among its CTAs.
+      const uint32_t n_send = min(found, J.kk);
+      const uint32_t lo = (uint32_t)((uint64_t)n_send * J.pc.index / J.pc.count);
+      const uint32_t hi = (uint32_t)((uint64_t)n_send * (J.pc.index + 1u) / J.pc.count);
+      if (may && lo < hi) {
+        uint32_t piece = 0, base = 0;
+        if (J.pc.count > 1u) {
+          uint32_t carry = 0;
+          for (uint32_t t0 = 0; t0 < J.pc.count && carry <= lo; t0 += kEmitThreads) {
+            const uint32_t t = t0 + tid;
+            const uint32_t v = t < J.pc.count ? (uint32_t)A.piece_cnt[J.pc.first + t] : 0u;
+            uint32_t sum;
+            const uint32_t at = carry + block_excl_scan(v, S.tmp, sum);
+            if (at <= lo && lo < at + v) { S.at[0] = t; S.at[1] = at; }
+            carry += sum;
+          }
+          __syncthreads();
+          piece = S.at[0];
+          base = S.at[1];
+        }
+        for (;;) {
+          if (J.pc.count > 1u) {
+            const uint32_t v = tid < kPieceRuns ? A.run_cnt[(J.pc.first + piece) * kPieceRuns + tid] & 0xffffu : 0u;
+            const uint32_t n_runs = (min(kPieceElems, J.sd.n_pad - piece * kPieceElems) + kRunElems - 1u) / kRunElems;
+            ex = block_excl_scan(tid < n_runs ? v : 0u, S.tmp, total);
+            if (tid <= kPieceRuns) S.pre[tid] = ex;
+            __syncthreads();
+          }
+          const uint2* const lists = A.cand + (kBlock ? J.sd.off >> 4 : J.sd.off) + (size_t)piece * (kPieceRuns * kArea);
+          send_range<kBlock>(A, J, S, lists, base, lo > base ? lo - base : 0u, min(hi - base, total));
+          base += total;
+          ++piece;
+          if (base >= hi || piece >= J.pc.count) break;
+          __syncthreads();     // S.pre is rewritten
+        }
+      }
+      if (!kBlock && short_of && may) {
+        // pad the fixed-size stream, every CTA its share
+#pragma unroll 1
+        for (uint32_t p = found + J.pc.index * kEmitThreads + tid; p < J.sd.k; p += J.pc.count * kEmitThreads)
+          emit_entry(A, J.dest, J.nb, J.slot_off, p, kSentinelIdx, 0.f);
+      }
+      if (last_of_tensor(J, S)) {
+        uint32_t t_key = 0;
+        bool scanned = false;
+        if (kBlock && short_of && may) {
+          const uint32_t need = J.kk - found, n_blocks = J.sd.n_pad / 16u;
+          uint32_t c = c_near;
+          if (!ss.inited || c < need) {
+            // every block that still holds something is a candidate: the blocks over the threshold were all
+            // emitted (the stream is short of them) and are zero in the residual by now
+            scanned = true;
+            if (tid == 0) S.word[3] = 0u;
+            __syncthreads();
+            constexpr uint32_t kRound = kEmitThreads / 4;   // blocks per round, four lanes each
+            const float* src = A.resid + J.sd.off + (tid & 3u) * 4u;
+            for (uint32_t b0 = 0; b0 < n_blocks; b0 += 8u * kRound) {
+              float4 a[8];
+#pragma unroll
+              for (int u = 0; u < 8; ++u) {   // independent loads in flight
+                const uint32_t b = b0 + u * kRound + (tid >> 2);
+                a[u] = b < n_blocks ? __ldcg(reinterpret_cast<const float4*>(src + (size_t)b * 16u)) : make_float4(0.f, 0.f, 0.f, 0.f);
+              }
+#pragma unroll
+              for (int u = 0; u < 8; ++u) {
+                const uint32_t b = b0 + u * kRound + (tid >> 2);
+                const uint32_t key = __float_as_uint(quad_l1(a[u]));
+                if (b < n_blocks && (tid & 3u) == 0u && key != 0u)
+                  nears[atomicAdd(&S.word[3], 1u)] = make_uint2((J.sd.off >> 4) + b, key);
+              }
+            }
+            __syncthreads();
+            c = S.word[3];
+          }
+          const uint32_t take = min(need, c);
+          if (take && c <= kPickMax) {
+            t_key = pick_few(nears, c, take, 0u, 0x7fffffffu, S);
+#pragma unroll 1
+            for (uint32_t e = tid; e < take * 16u; e += kEmitThreads) {
+              const uint32_t q = e >> 4, p = (found + q) * 16u + (e & 15u);
+              if (p < J.sd.k) {   // only the lowest-ranked block can be cut off
+                const uint32_t gi = S.hist[q] * 16u + (e & 15u);
+                emit_and_keep(A, J, p, gi, __ldcg(A.resid + gi));
+              }
+            }
+          } else if (take) {
+            if (tid == 0) J.wp->out_cursor = found;
+            __syncthreads();
+            t_key = take_top<kEmitThreads>(A, J.sd, J.wp, nears, c, take, true, J.kk, found + take - 1u, J.slot_off, J.dest,
+                                           J.nb, S.hist, S.tmp, S.res);
+          }
+          // fewer blocks with anything in them than the budget: the rest of the stream says "no entry"
+#pragma unroll 1
+          for (uint32_t p = (found + take) * 16u + tid; p < J.sd.k; p += kEmitThreads)
+            emit_entry(A, J.dest, J.nb, J.slot_off, p, kSentinelIdx, 0.f);
+        }
+        __syncthreads();
+        if (tid == 0 && ok) {
+          SegState st = ss;
+          if (!kBlock) {
+            const float max_abs = __uint_as_float(__ldcg(&J.wp->max_bits));
+            if (st.inited) {   // AIMD of thresholdv.cpp:70-76
+              if (J.sd.k > found) st.tau *= 0.99f;
+              else if (J.sd.k < found) st.tau = st.tau + 0.01f * ((float)found / (float)J.sd.k) * max_abs;
+            }
+          } else if (!st.inited) {
+            if (short_of && may) {   // first threshold: the smallest selected key plus the first additive step
+              const float t0 = __uint_as_float(t_key);
+              st.tau_inc = 0.01f * t0;
+              st.tau = t0 + st.tau_inc;
+              st.inited = 1;
+            }
+          } else {
+            if (short_of) st.tau *= 0.99f;      // "must drop less" (thresholdv16.cpp:245-248)
+            else st.tau += st.tau_inc;          // thresholdv16.cpp:249-252
+            // Keep a sixteenth to a quarter of the budget in near-miss blocks, and at least twice what this fill took:
+            // the additive and multiplicative steps of the threshold move the count of blocks over it by a few per
+            // cent, which is all a fill ever needs, and ranking the candidates costs time in proportion to their number.
+            float w = window_or(st.reserved[0], kWindowDefault);
+            const uint32_t needed = short_of ? J.kk - found : 0u;
+            if (scanned) w *= 2.f;
+            else if (c_near < J.kk / 16u + 8u || c_near < 2u * needed) w *= 1.5f;
+            else if (c_near > J.kk / 4u + 32u) w *= 0.75f;
+            st.reserved[0] = __float_as_uint(fminf(fmaxf(w, 1e-3f), 1.f));
+          }
+          A.state[J.pc.seg] = st;
+        }
+        if (tid == 0) { J.wp->cand_cnt = 0u; J.wp->out_cursor = 0u; J.wp->max_bits = 0u; }
+        for (uint32_t t = tid; t < J.pc.count; t += kEmitThreads) A.piece_cnt[J.pc.first + t] = 0ull;
+      }
+    }
+  }
+
+  __syncthreads();
+  if (tid == 0) finish_select(A, J.epoch, MODE == kScanTop ? A.refills : nullptr);
+}
+
+// Top-k tensors whose candidates fell short: the exact selection from the residual, with the histogram that `emit` took.
+__global__ void __launch_bounds__(kEmitThreads, 2) k_refill(SelectArgs A) {
+  __shared__ EmitShared S;
+  if (ld_volatile_u32(A.refills) == 0u) return;     // the same for every CTA: it is cleared behind the last one
+  const uint32_t tid = threadIdx.x;
+  const Job J = job_of(A, false);
+  const bool ok = ld_volatile_u32(A.status) == kOk;
+  if (!(J.sd.reserved & kSegSkip) && J.wp->refill != 0u) {
+    if (tid == 0) S.word[0] = ok && acks_arrived(A, J.epoch) ? 1u : 0u;
+    const SegState ss = A.state[J.pc.seg];
+    const uint32_t cut = top_cut(ss, J.sd.n_pad), found = J.wp->found;      // found < kk items reach the cut
+    uint32_t* gh = A.hist_rest + (size_t)J.pc.seg * kHistBins;
+    plan_top(gh, 1u, J.sd.n_pad - found, J.kk - found, true, S);
+    const bool may = S.word[0] != 0u, zero_fill = S.res[0] == 0u;
+    uint32_t key_lo, key_hi, emitted = 0, noted = 0;
+    rest_bin_range(S.res[0], cut, key_lo, key_hi);
+    const uint32_t rem = S.res[1];
+    uint2* const undecided = A.cand + A.n_total + J.sd.off;
+    const uint32_t len = min(kPieceElems, J.sd.off + J.sd.n_pad - J.pc.start);
+    if (may && zero_fill) {
+      // fewer non-zero elements than the budget: zeros complete it, lowest index first; `emit` left their number per piece.
+      // This comes first, because what is sent below becomes zero in the residual.
+      uint32_t before = 0, base;
+      for (uint32_t t = tid; t < J.pc.index; t += kEmitThreads) before += A.run_cnt[(J.pc.first + t) * kPieceRuns];
+      block_excl_scan(before, S.tmp, base);
+      for (uint32_t i0 = 0; i0 < len && base < rem; i0 += kEmitThreads * 4u) {
+        const uint32_t i = i0 + tid * 4u;
+        const bool act = i < len;
+        const float4 a = act ? *reinterpret_cast<const float4*>(A.resid + J.pc.start + i) : make_float4(1.f, 1.f, 1.f, 1.f);
+        const uint32_t at = J.pc.start + i, idx[4] = {at, at + 1u, at + 2u, at + 3u};
+        const uint32_t bits[4] = {__float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(a.z), __float_as_uint(a.w)};
+        uint32_t zero = 0, total;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) zero |= (uint32_t)((bits[e] & 0x7fffffffu) == 0u) << e;
+        const uint32_t ex = block_excl_scan(__popc(zero), S.tmp, total);
+        while (zero && base + ex + __popc(zero) > rem) zero &= ~(0x80000000u >> __clz(zero));      // the budget ends here
+        send_marked<4>(A, J, S, idx, bits, zero, ex, min(total, rem - base), J.kk - rem + base);
+        base += total;
+      }
+    }
+    if (may) {
+      constexpr int kItems = 16;
+      for (uint32_t i0 = 0; i0 < len; i0 += kEmitThreads * kItems) {
+        uint32_t idx[kItems], bits[kItems];
+#pragma unroll
+        for (int u = 0; u < kItems / 4; ++u) {
+          const uint32_t i = i0 + (u * kEmitThreads + tid) * 4u;
+          const bool act = i < len;
+          const float4 a = act ? *reinterpret_cast<const float4*>(A.resid + J.pc.start + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+          const float v[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            bits[4 * u + e] = __float_as_uint(v[e]);
+            idx[4 * u + e] = act && (bits[4 * u + e] & 0x7fffffffu) ? J.pc.start + i + e : kSentinelIdx;
+          }
+        }
+        emit_top_batch<kItems>(A, J, S, undecided, idx, bits, key_lo, key_hi, emitted, noted);
+      }
+    }
+    if (last_of_tensor(J, S)) {
+      const uint32_t c = J.pc.count == 1u ? noted : __ldcg(&J.wp->cand_cnt);
+      if (may && rem != 0u && (zero_fill || rem <= c)) {
+        const uint32_t t_key = zero_fill ? 0u : settle_top(A, J, S, undecided, c, rem, key_lo, key_hi);
+        if (tid == 0) step_top(A, J, ss, t_key, 0u);
+      } else if (may && tid == 0) {
+        set_status(A.status, kBadCandidate);
+      }
+      __syncthreads();
+      if (tid == 0) { J.wp->out_cursor = 0u; J.wp->cand_cnt = 0u; J.wp->refill = 0u; J.wp->found = 0u; }
+      for (uint32_t b = tid; b < (uint32_t)kHistBins; b += kEmitThreads) gh[b] = 0u;
+    }
+  }
+  __syncthreads();
+  if (tid == 0) finish_select(A, J.epoch, A.refills, true);
+}
+
+// ------------------------------------------------------------------------------------------------
+// host launchers
+// ------------------------------------------------------------------------------------------------
+bool one_pass_possible(const SelectArgs& A) {
+  // list positions and counts are 32-bit, top-k keeps its undecided items behind the lists (2 n slots)
+  return A.compressor != kRandomk && A.pieces != nullptr && A.n_total < (1u << 30) &&
+         (A.compressor != kTopk || (uint64_t)A.cand_cap >= 2ull * A.n_total);
+}
+
+cudaError_t launch_select_one_pass(const SelectArgs& A, cudaStream_t stream) {
+  if (A.n_chunks == 0 || A.n_segs == 0) return cudaSuccess;
+  if (A.world > kMaxWorld || !one_pass_possible(A)) return cudaErrorInvalidValue;
+  if (A.compressor == kThresholdv16) {
+    k_scan<kScanBlock><<<A.n_chunks, kScanThreads, 0, stream>>>(A);
+    k_emit<kScanBlock><<<A.n_pieces, kEmitThreads, 0, stream>>>(A);
+  } else if (A.compressor == kThresholdv) {
+    k_scan<kScanElem><<<A.n_chunks, kScanThreads, 0, stream>>>(A);
+    k_emit<kScanElem><<<A.n_pieces, kEmitThreads, 0, stream>>>(A);
+  } else {
+    k_scan<kScanTop><<<A.n_chunks, kScanThreads, 0, stream>>>(A);
+    k_emit<kScanTop><<<A.n_pieces, kEmitThreads, 0, stream>>>(A);
+    k_refill<<<A.n_pieces, kEmitThreads, 0, stream>>>(A);
+  }
+  return cudaGetLastError();
+}
+
+}  // namespace st

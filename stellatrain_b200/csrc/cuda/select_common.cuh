@@ -1,0 +1,250 @@
+// What the select chains share: guarded float4 accesses, block keys, the histogram window, the exact selection among a
+// list of candidates, and the completion of a stream.
+#pragma once
+#include "device_utils.cuh"
+
+namespace st {
+
+constexpr float kWindowDefault = 0.05f;        // threshold-v16's near misses: keys in [tau * (1 - window), tau)
+
+__device__ __forceinline__ uint32_t key_bits(float a) { return __float_as_uint(a) & 0x7fffffffu; }
+
+// Gradients are read once: streaming loads and stores (evict-first) keep them from pushing the
+// residual, which pass 2 reads again, out of L2.
+__device__ __forceinline__ float4 load4_guarded(const float* p, uint32_t i, uint32_t valid) {
+  if (i + 4 <= valid) return __ldcs(reinterpret_cast<const float4*>(p + i));
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (i + 0 < valid) v.x = p[i + 0];
+  if (i + 1 < valid) v.y = p[i + 1];
+  if (i + 2 < valid) v.z = p[i + 2];
+  return v;
+}
+
+__device__ __forceinline__ void store4_guarded(float* p, uint32_t i, uint32_t valid, float4 v) {
+  if (i + 4 <= valid) {
+    __stcs(reinterpret_cast<float4*>(p + i), v);
+    return;
+  }
+  if (i + 0 < valid) p[i + 0] = v.x;
+  if (i + 1 < valid) p[i + 1] = v.y;
+  if (i + 2 < valid) p[i + 2] = v.z;
+}
+
+// L1 norm of the 16-element block held by four consecutive lanes (one float4 each).  The
+// reduction tree is fixed, so the value is identical in all four lanes and reproducible.
+__device__ __forceinline__ float quad_l1(const float4& a) {
+  float s = (fabsf(a.x) + fabsf(a.y)) + (fabsf(a.z) + fabsf(a.w));
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  return s;
+}
+
+// ------------------------------------------------------------------------------------------------
+// histogram window
+// ------------------------------------------------------------------------------------------------
+struct HistWindow {
+  uint32_t base, shift;
+};
+
+__device__ __forceinline__ HistWindow window_of(const SegState& ss) {
+  HistWindow w;
+  w.base = ss.hist_shift ? ss.hist_base : 0u;
+  w.shift = ss.hist_shift ? ss.hist_shift : (uint32_t)kHistShift;
+  return w;
+}
+
+// Monotone in key, so "bin > b" implies "key above every key of bin b".
+__device__ __forceinline__ uint32_t bin_of(uint32_t key, const HistWindow& w) {
+  if (key < w.base) return 0u;
+  const uint32_t b = (key - w.base) >> w.shift;
+  return b < (uint32_t)(kHistBins - 1) ? b : (uint32_t)(kHistBins - 1);
+}
+
+// Window for the next select: 2048 bins of 2^13 key units (2^-10 relative) centred on `key`,
+// i.e. one octave to either side; keys outside fall into the two end bins.
+__device__ __forceinline__ void centre_window(SegState& ss, uint32_t key) {
+  const uint32_t half = (uint32_t)(kHistBins / 2) << kFineShift;
+  ss.hist_shift = kFineShift;
+  ss.hist_base = key > half ? key - half : 0u;
+}
+
+// Debug checks: hand every destination the sum over the entries this select stored into it, and clear
+// the accumulators for the next select.  Called by the one thread that publishes the arrival flags, before
+// them (their release orders these stores too).
+__device__ __forceinline__ void publish_checksums(const SelectArgs& A, uint32_t epoch) {
+  if (A.stamps != nullptr) {
+    A.stamps[1] = global_timer_ns();
+    A.stamps[4] = epoch;
+  }
+  if (A.cksum_acc == nullptr) return;
+  for (int p = 0; p < A.world; ++p) {
+    const uint32_t sum = atomicAdd(A.cksum_acc + (A.owner_mode ? p : 0), 0u);
+    if (A.cksum[p] != nullptr) A.cksum[p][(size_t)(epoch & 1u) * A.cksum_slot_stride] = sum;
+  }
+  for (int p = 0; p < kMaxWorld; ++p) A.cksum_acc[p] = 0u;
+  __threadfence_system();
+}
+
+// The receive slot about to be overwritten was last used two epochs ago; every destination must have consumed
+// it.  One thread calls this right before its CTA stores into the destinations.
+__device__ __forceinline__ bool acks_arrived(const SelectArgs& A, uint32_t epoch) {
+  if (!A.use_acks || epoch <= 2u) return true;
+  const uint64_t want = (uint64_t)epoch - 2u;
+  for (int p = 0; p < A.world; ++p) {
+    if (!wait_ge_bounded(A.ack_local + (size_t)(epoch & 1u) * A.world + p, want, A.timeout_ns)) {
+      set_status(A.status, kTimeoutAck);
+      return false;
+    }
+  }
+  return true;
+}
+
+// Called by a whole CTA of T threads.  Among cand[0..c) takes the `rem` largest keys (equal keys: lowest
+// item id first; 1 <= rem <= c) and emits them: stream positions come from wp->out_cursor, except that the
+// lowest-ranked taken block of threshold-v16 goes to `last_pos`, where it may be cut off at sd.k.  Returns the key
+// of the lowest-ranked taken item.  s_hist: 2048 words, s_tmp: T / 32 + 1 words, s_res: 4 words.
+template <int T>
+__device__ __forceinline__ uint32_t take_top(const SelectArgs& A, const SegDesc& sd, SegWork* wp, const uint2* cand,
+                                             uint32_t c, uint32_t rem, bool b16, uint32_t kk, uint32_t last_pos,
+                                             uint64_t slot_off, int dest, uint32_t nb, uint32_t* s_hist,
+                                             uint32_t* s_tmp, uint32_t* s_res) {
+  constexpr int kIlp = 4;              // independent loads in flight per thread
+  constexpr int kPer = 2048 / T;       // bins per thread, descending from the highest
+  const uint32_t tid = threadIdx.x;
+  uint32_t ties = 0;
+  uint32_t prefix = 0, mask = 0;
+  // radix select over the full 31-bit key, largest first: digits of 11, 11 and 9 bits
+  const int shifts[3] = {20, 9, 0};
+  const uint32_t widths[3] = {2048u, 2048u, 512u};
+  for (int pass = 0; pass < 3; ++pass) {
+    const int shift = shifts[pass];
+    const uint32_t nbins = widths[pass];
+    for (uint32_t b = tid; b < nbins; b += T) s_hist[b] = 0;
+    __syncthreads();
+    for (uint32_t i0 = tid; i0 < c; i0 += T * kIlp) {
+      uint32_t key[kIlp];
+#pragma unroll
+      for (int u = 0; u < kIlp; ++u) {
+        const uint32_t i = i0 + u * T;
+        key[u] = i < c ? __ldcg(&cand[i].y) : 0xFFFFFFFFu;
+      }
+#pragma unroll
+      for (int u = 0; u < kIlp; ++u)
+        if (key[u] != 0xFFFFFFFFu && (key[u] & mask) == prefix) atomicAdd(&s_hist[(key[u] >> shift) & (nbins - 1)], 1u);
+    }
+    __syncthreads();
+    uint32_t h[kPer], local = 0;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const uint32_t d = kPer * tid + j;
+      h[j] = d < nbins ? s_hist[nbins - 1 - d] : 0u;
+      local += h[j];
+    }
+    uint32_t total;
+    uint32_t ex = block_excl_scan(local, s_tmp, total);
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      if (ex < rem && ex + h[j] >= rem) {
+        s_res[0] = nbins - 1 - (kPer * tid + j); s_res[1] = rem - ex; s_res[2] = h[j];
+      }
+      ex += h[j];
+    }
+    __syncthreads();
+    prefix |= s_res[0] << shift;
+    mask |= (nbins - 1) << shift;
+    rem = s_res[1];
+    ties = s_res[2];
+    __syncthreads();
+  }
+  const uint32_t t_key = prefix;
+  // among equal keys take the lowest item ids: radix select on the id, smallest first
+  uint32_t id_thr = 0xFFFFFFFFu;
+  if (rem < ties) {
+    uint32_t ipre = 0, imask = 0, irem = rem;
+    for (int pass = 0; pass < 4; ++pass) {
+      const int shift = 24 - 8 * pass;
+      for (uint32_t b = tid; b < 256; b += T) s_hist[b] = 0;
+      __syncthreads();
+      for (uint32_t i = tid; i < c; i += T) {
+        const uint2 e = __ldcg(cand + i);
+        if (e.y == t_key && (e.x & imask) == ipre) atomicAdd(&s_hist[(e.x >> shift) & 255u], 1u);
+      }
+      __syncthreads();
+      const uint32_t h = tid < 256 ? s_hist[tid] : 0u;
+      uint32_t total;
+      const uint32_t ex = block_excl_scan(h, s_tmp, total);
+      if (tid < 256 && ex < irem && ex + h >= irem) { s_res[0] = tid; s_res[1] = irem - ex; }
+      __syncthreads();
+      ipre |= s_res[0] << shift;
+      imask |= 255u << shift;
+      irem = s_res[1];
+      __syncthreads();
+    }
+    id_thr = ipre;
+  }
+  // threshold-v16: the lowest-ranked taken block goes last and may be truncated
+  uint32_t last_id = id_thr;
+  if (b16 && rem >= ties) {
+    uint32_t mxid = 0;
+    for (uint32_t i = tid; i < c; i += T) {
+      const uint2 e = __ldcg(cand + i);
+      if (e.y == t_key) mxid = max(mxid, e.x);
+    }
+    last_id = block_max_u32(mxid, s_tmp);
+  }
+#pragma unroll 1
+  for (uint32_t i = tid; i < c; i += T) {
+    const uint2 e = __ldcg(cand + i);
+    const bool take = e.y > t_key || (e.y == t_key && e.x <= id_thr);
+    if (!take) continue;
+    if (!b16) {
+      const uint32_t pos = atomicAdd(&wp->out_cursor, 1u);
+      if (pos < kk) {
+        const float a = __ldcg(A.resid + e.x), sv = wire_value(nb, a);
+        emit_entry(A, dest, nb, slot_off, pos, e.x, sv);
+        A.resid[e.x] = a - sv;
+      }
+    } else {
+      const bool is_last = (e.y == t_key && e.x == last_id);
+      const uint32_t pos = is_last ? last_pos : atomicAdd(&wp->out_cursor, 1u);
+      if (pos < kk) {
+        const uint32_t base = e.x * 16u;
+#pragma unroll 1
+        for (uint32_t j = 0; j < 16u; ++j) {
+          if (pos * 16u + j < sd.k) {
+            const float a = __ldcg(A.resid + base + j), sv = wire_value(nb, a);
+            emit_entry(A, dest, nb, slot_off, pos * 16u + j, base + j, sv);
+            A.resid[base + j] = a - sv;
+          }
+        }
+      }
+    }
+  }
+  return t_key;
+}
+
+// Completion of a select chain, called by thread 0 of every CTA of its last kernel after a CTA barrier: the last
+// CTA publishes the arrival flags and advances the epoch.  The CTA barrier orders the CTA's stores before this
+// thread's system-scope fence, the counter orders the CTAs.  `refills`: when the word is not zero the stream is not
+// complete yet and the chain's next kernel finishes it, unless `is_refill` says that this is that kernel.
+__device__ __forceinline__ void finish_select(const SelectArgs& A, uint32_t epoch, uint32_t* refills = nullptr,
+                                              bool is_refill = false) {
+  if (A.publish) __threadfence_system();   // stores into peers' memory; without peers the counter's own order is enough
+  const uint32_t prev = atom_add_acq_rel_gpu(A.done_ctr, 1u);
+  if (prev == gridDim.x - 1) {
+    *A.done_ctr = 0;
+    __threadfence_system();
+    if (refills != nullptr) {
+      if (is_refill) *refills = 0;
+      else if (ld_volatile_u32(refills) != 0u) return;
+    }
+    publish_checksums(A, epoch);
+    if (A.publish && ld_volatile_u32(A.status) == kOk) {
+      for (int p = 0; p < A.world; ++p)
+        st_release_sys_u64(A.flag[p] + (size_t)(epoch & 1u) * A.flag_slot_stride, (uint64_t)epoch);
+    }
+    *A.epoch = epoch + 1;
+  }
+}
+
+}  // namespace st

@@ -28,7 +28,6 @@ enum Status : uint32_t {
   kBadCandidate = 4,  // candidate scratch exhausted (cannot happen with a correctly sized scratch)
   kBadSize = 5,       // request exceeds a compiled-in limit
   kBadChecksum = 6,   // debug checks: a received stream does not add up to what its source sent
-  kTimeoutScan = 7,   // one-pass select: a chunk never saw the item count of the chunk in front of it
 };
 
 struct SegDesc {          // static per segment (re-uploaded when the compression ratio changes)
@@ -65,8 +64,9 @@ struct SegState {         // persistent per segment, saved in checkpoints
   // holds the next threshold is 2^-10 wide (relative) and the candidate set is tiny.
   uint32_t hist_base;
   uint32_t hist_shift;
-  // reserved[0]: float bits of the one-pass select's candidate window (blocks with a key in
-  // [tau * (1 - window), tau) are noted for the fill); 0 = not set yet.
+  // reserved[0]: float bits of the one-pass select's candidate window (threshold-v16: blocks with a key in
+  // [tau * (1 - window), tau) are noted for the fill; top-k: items down to (1 - window) times the k-th largest
+  // key of the previous select are listed); 0 = not set yet.  reserved[1]: that key (top-k).
   uint32_t reserved[3];
 };
 
@@ -81,14 +81,31 @@ struct SegWork {          // scratch per segment, valid within one select
   uint32_t max_bits;      // running max |x| of the segment as float bits (reset by plan)
   uint32_t max_saved;     // max |x| of the current select
   uint32_t tau_bits;      // threshold the current select was counted with
-  uint32_t reserved[2];
+  uint32_t pieces_done;   // one-pass chain: pieces of the tensor that are through
+  uint32_t refill;        // one-pass top-k: the candidates fell short, the refill kernel selects this tensor
 };
 
 struct Chunk {            // unit of work of the streaming passes; never spans two segments
   uint32_t seg;
   uint32_t start;         // bucket offset, multiple of 16
   uint32_t len;           // elements, multiple of 16
-  uint32_t reserved;
+  uint32_t run0;          // one-pass chain: number of the chunk's first run
+};
+
+// One-pass chain.  A run is 1024 consecutive elements of a tensor (fewer at its end), the work of one warp; chunk lengths
+// are multiples of it.  A piece is up to 128 runs of one tensor, the work of one CTA of the emitting kernels.  Run r of
+// piece p has the number 128 p + r.
+constexpr uint32_t kRunElems = 1024u;
+constexpr uint32_t kPieceRuns = 128u;
+
+struct Piece {
+  uint32_t seg;
+  uint32_t start;         // bucket offset of its first element
+  uint32_t n_runs;
+  uint32_t index;         // place among the tensor's pieces
+  uint32_t count;         // pieces of the tensor
+  uint32_t first;         // number of the tensor's first piece
+  uint32_t reserved[2];
 };
 
 // Hyper-parameters and counters of the sparse optimisers, resident on the device so that a step
@@ -113,7 +130,13 @@ struct SelectArgs {
   const Chunk* chunks;
   uint32_t* chunk_cnt;         // items over the threshold per chunk
   uint32_t* chunk_pos;         // exclusive prefix of chunk_cnt inside the segment
-  uint64_t* chunk_state;       // one-pass select: per chunk (epoch | kind | items), see chunk_word(); or null
+  const Piece* pieces;         // one-pass chain, or null: pieces of all tensors
+  uint32_t* run_cnt;           // [n_pieces][kPieceRuns] listed items | near misses << 16
+  uint64_t* piece_cnt;         // [n_pieces] the same summed, low and high word (tensors of several pieces only)
+  uint32_t* hist_top;          // [n_pieces][kHistBins] top-k: histograms of the candidates, see top_bin()
+  uint32_t* hist_rest;          // [n_segs][kHistBins] top-k whose candidates fell short: histogram of the rest, see rest_bin()
+  uint32_t* refills;           // number of tensors left to the refill kernel
+  uint32_t n_pieces;
   uint32_t* hist;              // [n_segs][kHistBins]
   uint2* cand;                 // candidate scratch: (item id, key)
   uint32_t* cand_cursor;       // bump pointer into cand

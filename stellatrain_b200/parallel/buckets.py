@@ -21,7 +21,13 @@ SEG_DESC_DTYPE = np.dtype(
 SEG_STATE_DTYPE = np.dtype([("tau", "<f4"), ("tau_inc", "<f4"), ("inited", "<u4"), ("hist_base", "<u4"),
                             ("hist_shift", "<u4"), ("r0", "<u4"), ("r1", "<u4"), ("r2", "<u4")])
 SEG_WORK_WORDS = 12
-CHUNK_DTYPE = np.dtype([("seg", "<u4"), ("start", "<u4"), ("len", "<u4"), ("reserved", "<u4")])
+CHUNK_DTYPE = np.dtype([("seg", "<u4"), ("start", "<u4"), ("len", "<u4"), ("run0", "<u4")])
+# One-pass select: a run is the work of one warp of the streaming kernel, a piece the work of one CTA of the emitting one;
+# run r of piece p has the number PIECE_RUNS * p + r (csrc/cuda/sparse_types.h)
+RUN_ELEMS = 1024
+PIECE_RUNS = 128
+PIECE_DTYPE = np.dtype([("seg", "<u4"), ("start", "<u4"), ("n_runs", "<u4"), ("index", "<u4"), ("count", "<u4"),
+                        ("first", "<u4"), ("r0", "<u4"), ("r1", "<u4")])
 OPT_STATE_DTYPE = np.dtype(
     [("lr", "<f4"), ("momentum", "<f4"), ("dampening", "<f4"), ("weight_decay", "<f4"),
      ("beta1", "<f4"), ("beta2", "<f4"), ("eps", "<f4"), ("reserved0", "<f4"),
@@ -159,15 +165,31 @@ class BucketLayout:
     def chunk_table(self) -> np.ndarray:
         t = np.zeros(self.n_chunks, dtype=CHUNK_DTYPE)
         c = 0
+        piece = 0
         for i, s in enumerate(self.segments):
             done = 0
             while done < s.n_pad:
                 ln = min(self.chunk_elems, s.n_pad - done)
-                t[c] = (i, s.off + done, ln, 0)
+                t[c] = (i, s.off + done, ln, piece * PIECE_RUNS + done // RUN_ELEMS)
                 done += ln
                 c += 1
+            piece += self._pieces_of(s)
         assert c == self.n_chunks
         return t
+
+    @staticmethod
+    def _pieces_of(s: Segment) -> int:
+        return -(-s.n_pad // (PIECE_RUNS * RUN_ELEMS))
+
+    def piece_table(self) -> np.ndarray:
+        rows = []
+        for i, s in enumerate(self.segments):
+            count, first = self._pieces_of(s), len(rows)
+            for q in range(count):
+                rel = q * PIECE_RUNS * RUN_ELEMS
+                n_runs = min(PIECE_RUNS, -(-(s.n_pad - rel) // RUN_ELEMS))
+                rows.append((i, s.off + rel, n_runs, q, count, first, 0, 0))
+        return np.array(rows, dtype=PIECE_DTYPE)
 
 
 def plan_buckets(numels: Sequence[int], bucket_elems: int) -> list[list[int]]:

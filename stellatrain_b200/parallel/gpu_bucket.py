@@ -23,7 +23,6 @@ STATUS_NAMES = {
     4: "candidate scratch exhausted",
     5: "size beyond a compiled-in limit",
     6: "a received stream does not match its source's checksum",
-    7: "one-pass select: a chunk never saw the count of the chunk before it",
 }
 
 
@@ -142,12 +141,19 @@ class GpuBucket:
         self.chunks = _dev_bytes(layout.chunk_table(), device)
         self.chunk_cnt = torch.zeros(layout.n_chunks, dtype=torch.int32, device=device)
         self.chunk_pos = torch.zeros(layout.n_chunks, dtype=torch.int32, device=device)
-        # One-pass select of the threshold compressors: one state word per chunk (epoch | kind | count).  It takes
-        # over once every tensor has a threshold: after the first select, or after a checkpoint that carries them.
-        self.chunk_state = torch.zeros(layout.n_chunks, dtype=torch.int64, device=device)
+        # One-pass select: it takes over once every tensor has a threshold, after the first select or (threshold
+        # compressors) after a checkpoint that carries them.
         self.fused_select = bool(fused_select)
+        pieces = layout.piece_table()
+        self.n_pieces = len(pieces)
+        self.pieces = _dev_bytes(pieces, device)
+        self.run_cnt = torch.zeros(self.n_pieces * B.PIECE_RUNS, dtype=torch.int32, device=device)
+        self.piece_cnt = torch.zeros(self.n_pieces, dtype=torch.int64, device=device)
+        one_pass_topk = compressor == "topk" and self.fused_select
+        self.hist_top = torch.zeros(self.n_pieces * 2048 if one_pass_topk else 1, dtype=torch.int32, device=device)
+        self.hist_rest = torch.zeros(n_segs * 2048 if one_pass_topk else 1, dtype=torch.int32, device=device)
         self.hist = torch.zeros(n_segs * 2048, dtype=torch.int32, device=device)
-        # [select epoch, apply epoch, select CTAs done, apply CTAs done, 4 spare]
+        # [select epoch, apply epoch, select CTAs done, apply CTAs done, tensors to refill (one-pass top-k), 3 spare]
         self.counters = torch.tensor([1, 1, 0, 0, 0, 0, 0, 0], dtype=torch.int32, device=device)
         self.status = torch.zeros(1, dtype=torch.int32, device=device)
         self.stamps = torch.zeros(8, dtype=torch.int64, device=device)    # device clock of the latest chain, see device_times()
@@ -163,7 +169,8 @@ class GpuBucket:
         self._opt_host = opt
         self.opt = _dev_bytes(opt, device)
         self.scratch = scratch if scratch is not None else CandidateScratch(device)
-        self.scratch.reserve(n)
+        # lists of the one-pass chain: a slot per element; top-k keeps its undecided items behind them
+        self.scratch.reserve(2 * n if one_pass_topk and n < 1 << 30 else n)
         self.handle = _ext().BucketHandle()
         self.wiring: Optional[Wiring] = None
         # library-collective baseline: a second handle whose only destination is a local send buffer
@@ -196,7 +203,8 @@ class GpuBucket:
             segs=self.segs.data_ptr(), state=self.state.data_ptr(), work=self.work.data_ptr(),
             chunks=self.chunks.data_ptr(), chunk_cnt=self.chunk_cnt.data_ptr(), chunk_pos=self.chunk_pos.data_ptr(),
             hist=self.hist.data_ptr(), n_segs=len(L.segments), n_chunks=L.n_chunks, cap=L.cap,
-            chunk_state=self.chunk_state.data_ptr(), max_chunk=min(L.chunk_elems, max(s.n_pad for s in L.segments)),
+            pieces=self.pieces.data_ptr(), run_cnt=self.run_cnt.data_ptr(), piece_cnt=self.piece_cnt.data_ptr(),
+            hist_top=self.hist_top.data_ptr(), hist_rest=self.hist_rest.data_ptr(), refills=self.counters.data_ptr() + 16, n_pieces=self.n_pieces,
         )
         self.scratch.bind(h)
         h.set_control(

@@ -198,3 +198,25 @@ def test_bundles_train_bit_for_bit_like_one_task_per_tensor(sizes, bundle_elems,
     assert n_plain == len(sizes) and n_units <= n_plain
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("chunk", [1024, 8192, 1 << 18])
+def test_runs_and_pieces_of_the_one_pass_select_tile_every_tensor(chunk):
+    """Every element belongs to exactly one run, and a run found through its chunk has the place its piece gives it."""
+    from stellatrain_b200.parallel import buckets as B
+
+    numels = [1, 16, 17, 1023, 1025, 131071, 131072, 131073, 500001]
+    L = B.BucketLayout([str(i) for i in range(len(numels))], numels, chunk_elems=chunk)
+    by_chunk, by_piece = {}, {}
+    for c in L.chunk_table():
+        for rel in range(0, int(c["len"]), B.RUN_ELEMS):
+            run = int(c["run0"]) + rel // B.RUN_ELEMS
+            assert run not in by_chunk
+            by_chunk[run] = (int(c["seg"]), int(c["start"]) + rel)
+    table = L.piece_table()
+    for p, row in enumerate(table):
+        assert table[int(row["first"])]["index"] == 0 and p == int(row["first"]) + int(row["index"]) < int(row["first"]) + int(row["count"])
+        for r in range(int(row["n_runs"])):
+            by_piece[p * B.PIECE_RUNS + r] = (int(row["seg"]), int(row["start"]) + r * B.RUN_ELEMS)
+    assert by_chunk == by_piece
+    assert sum(min(B.RUN_ELEMS, L.segments[s].off + L.segments[s].n_pad - at) for s, at in by_piece.values()) == L.n_total

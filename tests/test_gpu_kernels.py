@@ -103,6 +103,52 @@ def test_select_matches_oracle(compressor, mode, fused):
         assert torch.equal(b.resid, resid_ref), (compressor, mode, step)
 
 
+@pytest.mark.parametrize("compressor", ["topk", "thresholdv", "thresholdv16"])
+@pytest.mark.parametrize("mode", ["steady", "jumps", "ties", "mostly_zero", "huge"])
+@pytest.mark.parametrize("ratio,chunk", [(0.99, 8192), (0.5, 1024), (0.999, 1 << 18)])
+def test_one_pass_select_at_its_edges(compressor, mode, ratio, chunk):
+    """The one-pass chain against the plain rule at the edges of its runs (1024 elements), pieces (131072) and chunks:
+    the same entries bit for bit.  "jumps" moves the gradient scale up and down by large factors, so that top-k's
+    candidates fall short and the refill kernel selects; "mostly_zero" leaves fewer entries than the budget; "huge"
+    holds values far outside the histogram window."""
+    sizes = [1, 16, 1023, 1024, 1025, 8192, 9001, 131071, 131072, 131073, 400001]
+    gen = torch.Generator(device="cuda").manual_seed(99)
+    b = make_bucket(compressor, ratio, sizes=sizes, chunk=chunk)
+    resid_ref = torch.zeros_like(b.resid)
+    for step in range(7):
+        scale = [1.0, 1.0, 0.02, 0.02, 50.0, 0.5, 0.4][step] if mode == "jumps" else 1.0
+        fill_grads(b, gen, scale=1e-2 * scale, mode="ties" if mode == "ties" else "normal")
+        for s, sl, _ in seg_slices(b):
+            if mode == "mostly_zero":
+                b.grad[sl] *= (torch.rand(s.numel, generator=gen, device="cuda") < 0.2 * (1 - ratio)).float()
+            if mode == "huge" and step in (1, 4):
+                b.grad[s.off + s.numel // 2] = 1e30
+        grad, states = b.grad.clone(), oracle_states(b)
+        b.select()
+        torch.cuda.synchronize()
+        b.check_status()
+        assert b.last_select_fused == (step > 0)
+        idx_all, val_all = read_stream(b, step + 1)
+        for si, (s, sl, slp) in enumerate(seg_slices(b)):
+            own = slp if compressor == "thresholdv16" else sl
+            # top-k of a tensor with fewer entries than the budget sends zeros, lowest index first
+            want_idx, want_val, new_r = O.compress_step(compressor, grad[own], resid_ref[own], s.k, states[si], one_pass=step > 0)
+            got = torch.from_numpy(idx_all[s.out_off : s.out_off + s.k])
+            valid = got != O.SENTINEL
+            got, order = got[valid].sort()
+            want, worder = (want_idx.cpu() + s.off).sort()
+            assert torch.equal(got, want), (s.numel, step)
+            assert torch.equal(val_all[s.out_off : s.out_off + s.k][valid][order], want_val.cpu()[worder]), (s.numel, step)
+            resid_ref[own] = new_r
+            if compressor != "topk":
+                assert b.seg_state()[si]["tau"] == pytest.approx(states[si].tau, rel=1e-5, abs=1e-30)
+        assert torch.equal(b.resid, resid_ref), step
+    # the chain leaves its counters as it found them
+    assert int(b.hist.abs().max()) == 0 and int(b.hist_top.abs().max()) == 0 and int(b.hist_rest.abs().max()) == 0 and int(b.piece_cnt.abs().max()) == 0
+    work = b.work.view(len(sizes), B.SEG_WORK_WORDS)
+    assert int(work[:, 4:6].abs().max()) == 0 and int(work[:, 10:].abs().max()) == 0 and int(b.counters[4]) == 0
+
+
 def test_select_drops_nan():
     b = make_bucket("topk", 0.9, sizes=[1000, 5000])
     g = torch.randn(b.layout.n_total, device="cuda")
