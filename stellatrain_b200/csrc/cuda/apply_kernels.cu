@@ -364,6 +364,34 @@ cudaError_t launch_apply(const ApplyArgs& A, int max_ctas_per_source, int phase,
 }
 
 // ------------------------------------------------------------------------------------------------
+// Single-tensor compression: the pairs of a wide stream as two arrays, in stream order.  Entries without an element ("no
+// entry" of a short stream, zero padding behind the tensor) are counted; the caller drops them when there are any.
+// ------------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(kThreads) k_unpack(UnpackArgs A) {
+  const uint32_t epoch = A.epoch[0];      // the select has advanced it
+  const uint2* in = A.recv + (size_t)((epoch - 1u) & 1u) * A.slot_stride;
+  uint32_t none = 0;
+  for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < A.k; i += gridDim.x * kThreads) {
+    const uint2 e = __ldcg(in + i);
+    const bool there = e.x < A.n;
+    A.idx[i] = there ? (int32_t)e.x : -1;
+    A.val[i] = __uint_as_float(e.y);
+    none += there ? 0u : 1u;
+  }
+  none = __reduce_add_sync(0xffffffffu, none);
+  if ((threadIdx.x & 31) == 0 && none) atomicAdd(A.left_out, none);
+  if (blockIdx.x == 0 && threadIdx.x == 0) A.epoch[1] = epoch;      // both advance together, as in the engine
+}
+
+cudaError_t launch_unpack(const UnpackArgs& A, cudaStream_t stream) {
+  if (A.k == 0) return cudaSuccess;
+  int grid = (int)((A.k + kThreads * 2 - 1) / (kThreads * 2));
+  if (grid > 148 * 8) grid = 148 * 8;
+  k_unpack<<<grid, kThreads, 0, stream>>>(A);
+  return cudaGetLastError();
+}
+
+// ------------------------------------------------------------------------------------------------
 // Replica parity: max |mine - peer| over a flat range, read through a peer pointer.  The
 // reference checks cross-node divergence by shipping whole tensors to the broker
 // (backend/src/engine/core.cpp:843-847, 874-878); here one kernel reads the peer over NVLink.

@@ -207,6 +207,33 @@ struct BucketHandle : public st::BucketHandle {
   void py_select(uint64_t stream) {
     check(st::BucketHandle::select(as_ptr<CUstream_st>(stream)), "launch_select");
   }
+  // Compression of one tensor by itself: select from `input` (n elements, 16-byte aligned) without a residual, unpack the k
+  // pairs into idx / val.  The bucket's status word has the left-out counter right behind it.  Returns (status, entries
+  // without an element) once the stream is done.
+  py::tuple compress(uint64_t input, uint32_t n, uint64_t idx, uint64_t val, uint64_t stream) {
+    cudaStream_t s = as_ptr<CUstream_st>(stream);
+    const uint32_t zero_grad = sel.zero_grad;
+    float* const grad = sel.grad;
+    sel.grad = as_ptr<float>(input);
+    sel.fresh = 1u;
+    sel.zero_grad = 0u;
+    uint32_t words[2] = {0u, 0u};
+    cudaError_t e = cudaMemsetAsync(sel.status + 1, 0, sizeof(uint32_t), s);
+    if (e == cudaSuccess) e = st::BucketHandle::select(s);
+    sel.grad = grad;
+    sel.fresh = 0u;
+    sel.zero_grad = zero_grad;
+    st::UnpackArgs U = {app.recv, app.slot_stride, app.cap, n, sel.epoch, as_ptr<int32_t>(idx), as_ptr<float>(val), sel.status + 1};
+    if (e == cudaSuccess) e = st::launch_unpack(U, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(words, sel.status, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) {
+      py::gil_scoped_release nogil;
+      e = cudaStreamSynchronize(s);
+    }
+    check(e, "compress");
+    return py::make_tuple(words[0], words[1]);
+  }
+
   // Debug checks.  cksum areas are [2][world] u32 indexed [slot][source]; cksum_acc has MAX_WORLD words, rsum `world`.
   void set_debug(uint64_t cksum_acc, uint64_t rsum, uint64_t cksum_local, const std::vector<uint64_t>& peer_cksum, bool poison) {
     const int world = app.world;
@@ -281,6 +308,7 @@ PYBIND11_MODULE(_C, m) {
            py::arg("group_done_ctr"))
       .def("group_reduce", &BucketHandle::py_group_reduce, py::arg("stream"))
       .def("select", &BucketHandle::py_select, py::arg("stream"))
+      .def("compress", &BucketHandle::compress, py::arg("input"), py::arg("n"), py::arg("idx"), py::arg("val"), py::arg("stream"))
       .def("can_fuse", [](const BucketHandle& h) { return h.can_fuse(); })
       .def_readwrite("fused_enabled", &BucketHandle::fused_enabled)
       .def_readwrite("thresholds_ready", &BucketHandle::thresholds_ready)

@@ -21,6 +21,9 @@ cudaError_t launch_apply(const ApplyArgs& args, int max_ctas_per_source, int pha
 // True when launch_apply runs its single kernel for one source (no merge).
 bool apply_merges_nothing(const ApplyArgs& args);
 
+// Index and value arrays of a one-tensor stream; *left_out counts entries without an element.
+cudaError_t launch_unpack(const UnpackArgs& args, cudaStream_t stream);
+
 // max |a - b| as float bits, atomically folded into *out_bits (caller zeroes it).
 cudaError_t launch_max_abs_diff(const float* a, const float* b, uint64_t n, uint32_t* out_bits,
                                 cudaStream_t stream);

@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(kScanThreads, 4) k_scan(SelectArgs A) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const uint32_t i = j * 128u + lane * 4u;
-      rv[j] = i < len ? *reinterpret_cast<const float4*>(r + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      rv[j] = i < len && !A.fresh ? *reinterpret_cast<const float4*>(r + i) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     const SegDesc sd = A.segs[ch.seg];
     const bool tab = A.grad_tab != nullptr;
@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(kScanThreads, 4) k_scan(SelectArgs A) {
       continue;
     }
     const uint32_t n_valid = sd.n > seg_rel ? min(len, sd.n - seg_rel) : 0u;
-    const uint32_t g_valid = tab ? n_valid : len;          // gradients handed over per tensor are not padded
+    const uint32_t g_valid = tab || A.fresh ? n_valid : len;   // gradients handed over per tensor are not padded
     const bool add = !A.skip_ef;
     // a tensor without a threshold yet lists nothing: `emit` then takes the exact top items from the residual
     const uint32_t tau_bits = ss.inited ? __float_as_uint(ss.tau) : 0xFFFFFFFFu;
@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(kScanThreads, 4) k_scan(SelectArgs A) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const uint32_t i = h0 + j * 128u;
-          rv[j] = i < len ? *reinterpret_cast<const float4*>(r + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+          rv[j] = i < len && !A.fresh ? *reinterpret_cast<const float4*>(r + i) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
       }
       if (add) {

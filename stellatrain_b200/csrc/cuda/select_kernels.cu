@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(kThreads) k_pass1(SelectArgs A) {
   // Gradients handed over per tensor are not padded: guard the tail.  Flat buckets are.
   const bool tab = A.grad_tab != nullptr;
   float* g = tab ? A.grad_tab[ch.seg] + seg_rel : A.grad + ch.start;
-  const uint32_t g_valid = tab ? (sd.n > seg_rel ? min(ch.len, sd.n - seg_rel) : 0u) : ch.len;
+  const uint32_t g_valid = tab || A.fresh ? (sd.n > seg_rel ? min(ch.len, sd.n - seg_rel) : 0u) : ch.len;
   float* r = A.resid + ch.start;
 
   // Bin 0 is never counted (plan derives it from the item count) and the top bin is counted in a
@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(kThreads) k_pass1(SelectArgs A) {
     const bool act = i < ch.len;
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
     if (act) {
-      a = *reinterpret_cast<const float4*>(r + i);
+      if (!A.fresh) a = *reinterpret_cast<const float4*>(r + i);
       if (!A.skip_ef) {
         const float4 gv = load4_guarded(g, i, g_valid);
         a.x += gv.x; a.y += gv.y; a.z += gv.z; a.w += gv.w;
@@ -683,7 +683,7 @@ __global__ void __launch_bounds__(kThreads) k_ef_only(SelectArgs A) {
   const uint32_t seg_rel = ch.start - sd.off;
   const bool tab = A.grad_tab != nullptr;
   float* g = tab ? A.grad_tab[ch.seg] + seg_rel : A.grad + ch.start;
-  const uint32_t g_valid = tab ? (sd.n > seg_rel ? min(ch.len, sd.n - seg_rel) : 0u) : ch.len;
+  const uint32_t g_valid = tab || A.fresh ? (sd.n > seg_rel ? min(ch.len, sd.n - seg_rel) : 0u) : ch.len;
   float* r = A.resid + ch.start;
   if (blockIdx.x == 0 && threadIdx.x == 0 && A.stamps != nullptr) A.stamps[0] = global_timer_ns();
   if (blockIdx.x == 0 && threadIdx.x == 0 && A.use_acks) {
@@ -697,7 +697,8 @@ __global__ void __launch_bounds__(kThreads) k_ef_only(SelectArgs A) {
     }
   }
   for (uint32_t i = threadIdx.x * 4; i < ch.len; i += kPerIter) {
-    float4 a = *reinterpret_cast<const float4*>(r + i);
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (!A.fresh) a = *reinterpret_cast<const float4*>(r + i);
     const float4 gv = load4_guarded(g, i, g_valid);
     a.x += gv.x; a.y += gv.y; a.z += gv.z; a.w += gv.w;
     if (!(a.x == a.x)) a.x = 0.f;

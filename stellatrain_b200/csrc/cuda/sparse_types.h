@@ -145,6 +145,7 @@ struct SelectArgs {
   uint32_t compressor;         // Compressor
   uint32_t zero_grad;          // write zeros over consumed gradients
   uint32_t skip_ef;            // 1: the residual already holds g + r (re-selection), skip the add
+  uint32_t fresh;              // 1: there is no residual yet (r is written, not read); `grad` holds exactly one tensor
   // exchange
   int32_t world, rank;
   uint2* out[kMaxWorld];       // per destination: its receive area for source `rank`, slot 0
@@ -170,6 +171,17 @@ struct SelectArgs {
   // complete, flags published), [2] apply start (first stream seen), [3] apply end, [4] epoch of the
   // select, [5] epoch of the apply.  Feeds the telemetry (push duration, exposed wait).
   uint64_t* stamps;
+};
+
+// Unpacking of the stream of a bucket of one tensor into separate index and value arrays (single-tensor compression).
+struct UnpackArgs {
+  const uint2* recv;           // slot 0
+  uint64_t slot_stride;
+  uint32_t k, n;               // entries of the stream, elements of the tensor
+  uint32_t* epoch;             // [0] select epoch, one past the stream's; [1] apply epoch, set to the same
+  int32_t* idx;
+  float* val;
+  uint32_t* left_out;          // number of entries without an element (counted up from zero by the caller)
 };
 
 struct ApplyArgs {

@@ -40,7 +40,7 @@ def _compress_cuda(name: str, flat: torch.Tensor, k: int, method: str):
     b = _gpu_cache.get(key)
     if b is None:
         layout = B.BucketLayout([name], [n])
-        b = GpuBucket(0, layout, flat.device, compressor=method, ratio=0.0, world=1, rank=0)
+        b = GpuBucket(0, layout, flat.device, compressor=method, ratio=1.0, world=1, rank=0, select_only=True)
         b.wire_local()
         _gpu_cache[key] = b
     # one tensor, explicit k: patch the segment table
@@ -50,18 +50,10 @@ def _compress_cuda(name: str, flat: torch.Tensor, k: int, method: str):
         from ..parallel.gpu_bucket import _dev_bytes
         b.segs.copy_(_dev_bytes(b.layout.seg_table(), flat.device))
         b._bind()
-    b.resid.zero_()
-    b.grad[:n].copy_(flat)
-    epoch = int(b.counters[0].item())
-    b.select()
-    torch.cuda.current_stream(flat.device).synchronize()
-    b.check_status()
-    idx, val = b.stream_of(epoch & 1, 0)
-    # the epochs of select and apply advance together in the engine; keep them aligned here too
-    b.counters[1] = b.counters[0]
-    keep = idx != -1
-    keep &= idx < n   # threshold-v16 may name zero padding behind the tensor
-    return idx[keep].to(torch.int32), val[keep]
+        if k > b.cap_max:           # room for the pairs of this call (every call has waited for its stream)
+            b.cap_max = k
+            b.wire_local()
+    return b.compress(flat)
 
 
 def _compress_cpu(name: str, flat: torch.Tensor, k: int, method: str):

@@ -96,7 +96,9 @@ class GpuBucket:
         partition_state: bool = False,
         deterministic_merge: bool = False,
         fused_select: bool = True,
+        select_only: bool = False,
     ) -> None:
+        """``select_only``: for `compress`, which has no use for gradients, parameters and optimiser state of its own."""
         self.index = index
         self.layout = layout
         self.device = device
@@ -110,9 +112,10 @@ class GpuBucket:
         self.deterministic_merge = bool(deterministic_merge)   # scatter one source after the other: bit-equal replicas
         n = layout.n_total
         f32 = dict(dtype=torch.float32, device=device)
-        self.grad = torch.zeros(n, **f32)
+        n_state = B.ALIGN if select_only else n
+        self.grad = torch.zeros(n_state, **f32)
         self.resid = torch.zeros(n, **f32)
-        self.param = torch.zeros(n, **f32)
+        self.param = torch.zeros(n_state, **f32)
         # Accumulator, stamps and optimiser state cover the whole bucket, or with partitioned state only the
         # contiguous element range of the tensors this rank owns (1/world of the memory).
         self.partition_state = bool(partition_state) and world > 1
@@ -120,7 +123,7 @@ class GpuBucket:
             layout.assign_state_owners(world)
             self.state_lo, self.state_hi = layout.state_range(rank)
         else:
-            self.state_lo, self.state_hi = 0, n
+            self.state_lo, self.state_hi = 0, n_state
         ns = max(self.state_hi - self.state_lo, B.ALIGN)
         # One 16-byte record per element, {accumulator, stamp, m, v}: an update touches one sector of state.
         # acc / stamp / m / v are strided views of it (v stays unused by SGD).
@@ -155,7 +158,8 @@ class GpuBucket:
         self.hist = torch.zeros(n_segs * 2048, dtype=torch.int32, device=device)
         # [select epoch, apply epoch, select CTAs done, apply CTAs done, tensors to refill (one-pass top-k), 3 spare]
         self.counters = torch.tensor([1, 1, 0, 0, 0, 0, 0, 0], dtype=torch.int32, device=device)
-        self.status = torch.zeros(1, dtype=torch.int32, device=device)
+        self._status_words = torch.zeros(2, dtype=torch.int32, device=device)    # status, counter of `compress`
+        self.status = self._status_words[:1]
         self.stamps = torch.zeros(8, dtype=torch.int64, device=device)    # device clock of the latest chain, see device_times()
         # merge weight of every source, one row per epoch parity (the scatter of epoch e reads row e & 1)
         self.weight = torch.full((2, world), 1.0 / world, **f32)
@@ -341,6 +345,22 @@ class GpuBucket:
         """phase 0: the whole chain; 1: scatter + optimiser only; 2: copy of the owners' values only."""
         s = stream if stream is not None else torch.cuda.current_stream(self.device)
         self.handle.apply(s.cuda_stream, phase)
+
+    def compress(self, flat: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
+        """(idx:int32, val) of a one-tensor bucket for a flat tensor, without a residual; waits for the stream."""
+        if not flat.is_contiguous() or flat.data_ptr() & 15:        # the kernels use 16-byte loads
+            flat = flat.clone(memory_format=torch.contiguous_format)
+        n, k = self.layout.segments[0].numel, self.layout.cap
+        idx = torch.empty(k, dtype=torch.int32, device=self.device)
+        val = torch.empty(k, dtype=torch.float32, device=self.device)
+        s = torch.cuda.current_stream(self.device)
+        code, left_out = self.handle.compress(flat.data_ptr(), n, idx.data_ptr(), val.data_ptr(), s.cuda_stream)
+        if code != 0:
+            raise SparseStepError(self.index, code)
+        if left_out:
+            keep = torch.nonzero(idx != -1).flatten()
+            idx, val = idx[keep], val[keep]
+        return idx, val
 
     @property
     def apply_kernels(self) -> int:

@@ -149,6 +149,39 @@ def test_one_pass_select_at_its_edges(compressor, mode, ratio, chunk):
     assert int(work[:, 4:6].abs().max()) == 0 and int(work[:, 10:].abs().max()) == 0 and int(b.counters[4]) == 0
 
 
+@pytest.mark.parametrize("compressor", ["topk", "thresholdv", "thresholdv16", "randomk"])
+@pytest.mark.parametrize("n", [17, 1000, 4097, 131089])
+@pytest.mark.parametrize("form", ["plain", "unaligned", "strided"])
+def test_compress_reads_the_tensor_in_place(compressor, n, form):
+    """Single-tensor compression takes the caller's tensor as the gradient of a bucket without a residual: the pairs of the
+    plain rule, for aligned, unaligned and strided tensors, a ratio that changes from call to call, and NaNs dropped."""
+    import stellatrain_b200 as st
+
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    name, state = f"{compressor} {n} {form}", O.ThresholdState()
+    st.configure_compression(compressor)
+    try:
+        for call in range(5):
+            store = torch.randn(2 * n + 1, generator=gen, device="cuda") * 1e-2
+            store[5] = float("nan")
+            x = {"plain": store[:n], "unaligned": store[1 : n + 1], "strided": store[: 2 * n : 2]}[form]
+            before = store.clone()
+            ratio = 0.9 if call < 3 else 0.75
+            k = int((1.0 - ratio) * n)
+            idx, val = st.compress(name, x, ratio)
+            assert torch.equal(store.nan_to_num(7.0), before.nan_to_num(7.0)) and idx.dtype == torch.int32
+            x = x.nan_to_num(0.0)
+            assert torch.equal(val, x[idx.long()]) and len(torch.unique(idx)) == len(idx)
+            if compressor == "randomk":
+                assert len(idx) == k
+                continue
+            want, _, _ = O.compress_step(compressor, x, torch.zeros_like(x), k, state, one_pass=call > 0)
+            want = want[want < n].sort().values
+            assert torch.equal(idx.long().sort().values, want), call
+    finally:
+        st.configure_compression("thresholdv16")
+
+
 def test_select_drops_nan():
     b = make_bucket("topk", 0.9, sizes=[1000, 5000])
     g = torch.randn(b.layout.n_total, device="cuda")
