@@ -44,6 +44,7 @@ struct BucketRec {
   bool select_done_set = false;
   bool has_pending_apply = false;
   int64_t select_count = 0, apply_count = 0;
+  cudaStream_t lane = nullptr;             // stream of the bucket's chains
 };
 
 // Shared between the engine and its hooks: a hook that outlives the engine (a parameter that is still referenced
@@ -57,7 +58,11 @@ struct Shared {
 
 struct NativeEngine::Impl {
   int device = 0;
-  cudaStream_t sparse = nullptr;
+  // Streams of the bucket chains.  With one rank consecutive buckets take turns on two of them: the short kernels of one
+  // bucket's chain (update, emission) are bound by latency and leave the memory to the streaming kernel of the next one.
+  // `second` is null when there is one stream: buckets of several ranks stay in one order for all of them, and an emulated
+  // slow link has one token bucket.
+  cudaStream_t sparse = nullptr, second = nullptr;
   int staleness = 1, ga = 1;
   std::vector<BucketRec> buckets;
   std::vector<ParamRec> params;
@@ -93,8 +98,8 @@ struct NativeEngine::Impl {
   }
 
   void apply(BucketRec& b) {
-    check(b.spec.handle->apply(sparse, 0));
-    check(cudaEventRecord(b.apply_done, sparse));
+    check(b.spec.handle->apply(b.lane, 0));
+    check(cudaEventRecord(b.apply_done, b.lane));
     b.apply_done_set = true;
     b.has_pending_apply = false;
     b.apply_count += 1;
@@ -104,17 +109,17 @@ struct NativeEngine::Impl {
   void select(BucketRec& b) {
     BucketHandle* h = b.spec.select_handle ? b.spec.select_handle : b.spec.handle;
     if (b.spec.handle->has_group) {
-      check(b.spec.handle->group_reduce(sparse));
+      check(b.spec.handle->group_reduce(b.lane));
       kernels += 3;
     }
     if (shaper != nullptr && b.spec.shaped_bytes) {
-      check(launch_shape(static_cast<ShaperState*>(shaper), b.spec.shaped_bytes, shaper_cap_ns, sparse));
+      check(launch_shape(static_cast<ShaperState*>(shaper), b.spec.shaped_bytes, shaper_cap_ns, b.lane));
       shaped += b.spec.shaped_bytes;
       kernels += 1;
     }
-    check(h->select(sparse));
+    check(h->select(b.lane));
     if (!capturing) {
-      check(cudaEventRecord(b.select_done, sparse));
+      check(cudaEventRecord(b.select_done, b.lane));
       b.select_done_set = true;
     }
     b.select_count += 1;
@@ -174,7 +179,7 @@ struct NativeEngine::Impl {
         b.tab_slot = (b.tab_slot + 1) % b.spec.table_ring;
         // the copy that last used the next row must be done before the hooks rewrite it
         if (b.tab_event_set[b.tab_slot]) check(cudaEventSynchronize(b.tab_events[b.tab_slot]));
-        const c10::cuda::CUDAStream sparse_s = c10::cuda::getStreamFromExternal(sparse, (c10::DeviceIndex)device);
+        const c10::cuda::CUDAStream sparse_s = c10::cuda::getStreamFromExternal(b.lane, (c10::DeviceIndex)device);
         for (auto& g : b.held)   // the allocator must not reuse them before the select has read them
           c10::cuda::CUDACachingAllocator::recordStream(g.storage().data_ptr(), sparse_s);
         release.swap(b.held);
@@ -185,7 +190,7 @@ struct NativeEngine::Impl {
       for (int pi : b.params) params[pi].tensor.mutable_grad().reset();
     }
     check(cudaEventRecord(b.grad_ready, cur));
-    check(cudaStreamWaitEvent(sparse, b.grad_ready, 0));
+    check(cudaStreamWaitEvent(b.lane, b.grad_ready, 0));
     if (staleness == 1 && b.has_pending_apply) apply(b);
     select(b);
     if (staleness == 0) apply(b);
@@ -214,9 +219,11 @@ at::Tensor tensor_of(PyObject* obj, const char* what) {
 
 }  // namespace
 
-NativeEngine::NativeEngine(int device, uint64_t sparse_stream, int staleness, int grad_accumulation) : impl_(new Impl) {
+NativeEngine::NativeEngine(int device, uint64_t sparse_stream, uint64_t second_stream, int staleness, int grad_accumulation)
+    : impl_(new Impl) {
   impl_->device = device;
   impl_->sparse = reinterpret_cast<cudaStream_t>(static_cast<uintptr_t>(sparse_stream));
+  impl_->second = reinterpret_cast<cudaStream_t>(static_cast<uintptr_t>(second_stream));
   impl_->staleness = staleness;
   impl_->ga = grad_accumulation < 1 ? 1 : grad_accumulation;
   impl_->shared = std::make_shared<Shared>();
@@ -254,6 +261,7 @@ int NativeEngine::add_bucket(const NativeBucketSpec& spec) {
       cudaEventCreateWithFlags(&b.apply_done, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&b.select_done, cudaEventDisableTiming) != cudaSuccess)
     throw std::runtime_error("cudaEventCreate failed");
+  b.lane = impl_->second != nullptr && (impl_->buckets.size() & 1u) ? impl_->second : impl_->sparse;
   impl_->buckets.push_back(std::move(b));
   return (int)impl_->buckets.size() - 1;
 }
@@ -295,6 +303,19 @@ void NativeEngine::remove_hooks() {
 
 void NativeEngine::set_shaper(void* shaper_state, uint64_t cap_ns) {
   std::lock_guard<std::mutex> lock(impl_->mu);
+  if (shaper_state != nullptr && impl_->second != nullptr) {
+    // one token bucket, one stream: what the second stream still holds goes first
+    c10::cuda::CUDAGuard guard((c10::DeviceIndex)impl_->device);
+    cudaEvent_t ev = nullptr;
+    impl_->check(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    if (ev != nullptr) {
+      impl_->check(cudaEventRecord(ev, impl_->second));
+      impl_->check(cudaStreamWaitEvent(impl_->sparse, ev, 0));
+      cudaEventDestroy(ev);
+    }
+    impl_->second = nullptr;
+    for (auto& b : impl_->buckets) b.lane = impl_->sparse;
+  }
   impl_->shaper = shaper_state;
   impl_->shaper_cap_ns = cap_ns;
 }
@@ -326,10 +347,14 @@ void NativeEngine::flush(uint64_t stream) {
   if (ev == nullptr) return;
   impl_->check(cudaEventRecord(ev, s));
   impl_->check(cudaStreamWaitEvent(impl_->sparse, ev, 0));
+  if (impl_->second) impl_->check(cudaStreamWaitEvent(impl_->second, ev, 0));
   for (auto& b : impl_->buckets)
     if (b.has_pending_apply) impl_->apply(b);
-  impl_->check(cudaEventRecord(ev, impl_->sparse));
-  impl_->check(cudaStreamWaitEvent(s, ev, 0));
+  for (cudaStream_t lane : {impl_->sparse, impl_->second}) {
+    if (lane == nullptr) continue;
+    impl_->check(cudaEventRecord(ev, lane));
+    impl_->check(cudaStreamWaitEvent(s, ev, 0));
+  }
   cudaEventDestroy(ev);     // released once the waits that refer to it have been enqueued
 }
 

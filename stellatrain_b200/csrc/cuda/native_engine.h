@@ -38,7 +38,7 @@ struct NativeBucketSpec {
 
 class NativeEngine {
  public:
-  NativeEngine(int device, uint64_t sparse_stream, int staleness, int grad_accumulation);
+  NativeEngine(int device, uint64_t sparse_stream, uint64_t second_stream, int staleness, int grad_accumulation);
   ~NativeEngine();
   NativeEngine(const NativeEngine&) = delete;
   NativeEngine& operator=(const NativeEngine&) = delete;

@@ -195,6 +195,11 @@ class SparseDPEngine:
         self._shaped_bytes = 0
         low, high = torch.cuda.Stream.priority_range()
         self.sparse_stream = torch.cuda.Stream(device=self.device, priority=high)
+        # With one rank the native engine lets consecutive buckets take turns on two streams, each with a candidate scratch
+        # of its own: the latency-bound kernels of one bucket's chain run under the streaming kernel of the next.  Several
+        # ranks, Python hooks and a shaped link keep one stream.
+        self._second_stream: Optional[torch.cuda.Stream] = None
+        self._second_high = high
         self.iteration = 0            # completed optimiser iterations (selects issued per bucket)
         self.micro_step = 0
         self._failed: Optional[SparseStepError] = None
@@ -225,6 +230,9 @@ class SparseDPEngine:
         numels = [params[i][1].numel() for i in order]
         groups = B.plan_buckets(numels, int(cfg.bucket_mb * (1 << 20) / 4))
         self.scratch = CandidateScratch(self.device)
+        if self.transport == "local" and self._use_native() and len(groups) > 1:
+            self._second_stream = torch.cuda.Stream(device=self.device, priority=self._second_high)
+        scratches = [self.scratch, CandidateScratch(self.device) if self._second_stream is not None else self.scratch]
         self.buckets: list[_BucketRuntime] = []
         self.param_names: list[list[str]] = []
         self._param_to_bucket: dict[int, int] = {}
@@ -237,7 +245,7 @@ class SparseDPEngine:
             bucket = GpuBucket(
                 bi, layout, self.device, compressor=cfg.compressor, ratio=cfg.ratio, world=self.world,
                 rank=self.rank, optimizer=cfg.optimizer, amsgrad=cfg.amsgrad,
-                smart_momentum=cfg.smart_momentum, min_ratio=cfg.min_ratio, scratch=self.scratch,
+                smart_momentum=cfg.smart_momentum, min_ratio=cfg.min_ratio, scratch=scratches[bi & 1],
                 timeout_s=cfg.timeout_s, divide_k_by_world=cfg.divide_k_by_world,
                 k_world=(self.groups if (self.group_size > 1 and cfg.divide_k_by_world) else None),
                 partition_state=self.partitioned, deterministic_merge=cfg.deterministic_merge,
@@ -375,6 +383,8 @@ class SparseDPEngine:
         if self.native is None or self.shaper is None:
             return
         self.native.set_shaper(self.shaper.state.data_ptr(), self.shaper.MAX_HOLD_NS)
+        if self._second_stream is not None:
+            self._second_stream = None          # the native engine has moved every bucket to the first stream
         for bi, rt in enumerate(self.buckets):
             self.native.set_shaped_bytes(bi, rt.bucket.layout.wire_bytes(owned_only=True) * self._remote_ranks())
 
@@ -440,7 +450,9 @@ class SparseDPEngine:
         C = _build.load_extension("_C")
         steal = self.cfg.grad_mode != "flat"
         self.native = C.NativeEngine(self.device.index if self.device.index is not None else torch.cuda.current_device(),
-                                     self.sparse_stream.cuda_stream, self.cfg.staleness, self.cfg.grad_accumulation)
+                                     self.sparse_stream.cuda_stream,
+                                     self._second_stream.cuda_stream if self._second_stream is not None else 0,
+                                     self.cfg.staleness, self.cfg.grad_accumulation)
         for bi, rt in enumerate(self.buckets):
             b = rt.bucket
             segs = b.layout.segments
@@ -688,6 +700,14 @@ class SparseDPEngine:
         self.stats["kernels"] += rt.bucket.apply_kernels
 
     # ------------------------------------------------------------------ public control
+    @property
+    def sparse_streams(self) -> list:
+        """The streams that carry bucket chains."""
+        return [self.sparse_stream] if self._second_stream is None else [self.sparse_stream, self._second_stream]
+
+    def stream_of_bucket(self, bi: int) -> torch.cuda.Stream:
+        return self.sparse_streams[bi % len(self.sparse_streams)]
+
     def synchronize(self) -> None:
         """Flush every pending update and wait for the sparse stream
         (role of backend/src/engine/core.cpp:1097-1140)."""
@@ -703,12 +723,14 @@ class SparseDPEngine:
                 if rt.has_pending_apply:
                     self._apply(rt)
             cur.wait_stream(self.sparse_stream)
-        self.sparse_stream.synchronize()
+        for s in self.sparse_streams:
+            s.synchronize()
         self.check_status()
 
     def device_timeline(self) -> list:
         """Per bucket: device-clock durations of the latest select + push and apply (``GpuBucket.device_times``)."""
-        self.sparse_stream.synchronize()
+        for s in self.sparse_streams:
+            s.synchronize()
         return [rt.bucket.device_times() for rt in self.buckets]
 
     def export_stats(self, path: Optional[str] = None) -> str:
@@ -732,7 +754,7 @@ class SparseDPEngine:
                 raise self._failed
             self._status_event = None
         if self._status_event is None:
-            s = self.sparse_stream
+            s = self.sparse_stream          # words of buckets on the other stream are looked at as they stand
             with torch.cuda.stream(s):
                 torch.stack([rt.bucket.status[0] for rt in self.buckets], out=self._status_dev)
                 self._status_host.copy_(self._status_dev, non_blocking=True)
@@ -808,15 +830,14 @@ class SparseDPEngine:
         if not self._pending_weights:
             return
         it = self.iterations_started()
-        # eager: the sparse stream carries the applies; a replayed graph carries them on the stream it is launched on
-        stream = stream if stream is not None else self.sparse_stream
+        # eager: the bucket's own stream carries the applies; a replayed graph carries them on the stream it is launched on
         keep = []
         for entry in self._pending_weights:
             since, w, done = entry
             for step in (0, 1):
                 if it == since + step and done == step:
-                    with torch.cuda.stream(stream):
-                        for rt in self.buckets:
+                    for bi, rt in enumerate(self.buckets):
+                        with torch.cuda.stream(stream if stream is not None else self.stream_of_bucket(bi)):
                             rt.bucket.set_weight_row((since + step + 1) & 1, w)
                     entry[2] = done = step + 1
             if done < 2:

@@ -50,7 +50,12 @@ class GraphedStep:
         try:
             with torch.cuda.graph(self.graph, stream=side):
                 self.loss = step_fn(*self.static_inputs)
-                torch.cuda.current_stream(dev).wait_stream(engine.sparse_stream)
+                cur = torch.cuda.current_stream(dev)
+                for s in engine.sparse_streams:
+                    with torch.cuda.stream(s):      # the second one takes part only when a bucket on it was ready
+                        joins = s is engine.sparse_stream or torch.cuda.is_current_stream_capturing()
+                    if joins:
+                        cur.wait_stream(s)
                 if engine.cfg.step_clock:
                     engine.stamp(4)      # behind the join: (4) - (2) is the time the iteration waited for its bucket chains
         finally:
