@@ -13,7 +13,7 @@ cudaError_t launch_select(const SelectArgs& args, uint32_t randomk_seed, cudaStr
 bool one_pass_possible(const SelectArgs& args);
 cudaError_t launch_select_one_pass(const SelectArgs& args, cudaStream_t stream);
 
-// Bounded wait + scatter-add + sparse optimiser of one bucket: two kernels on `stream`, plus the copy of
+// Bounded wait + scatter-add + sparse optimiser of one bucket: two kernels on `stream` (one for a single source), plus the copy of
 // the owners' new parameter values when the optimiser state is partitioned.  phase 0 = all, 1 = scatter and
 // apply only, 2 = parameter copy only.
 cudaError_t launch_apply(const ApplyArgs& args, int max_ctas_per_source, int phase, cudaStream_t stream);

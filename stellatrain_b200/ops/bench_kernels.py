@@ -7,7 +7,7 @@ Times, with CUDA events after warm-up, the select chain and the apply chain (sca
 of a parameter-size list, and reports achieved HBM bandwidth against the measured copy bandwidth of the
 machine (``MEASURED_PEAKS.json`` next to the repository root when present).  Algorithmic traffic of one select,
 per element: the two-pass chain (pass1, plan, pass2, cand) reads g and r and writes r in pass 1 and reads r
-again in pass 2 = 16 bytes; the one-pass chain of the threshold compressors (fused, finish) reads g and r and
+again in pass 2 = 16 bytes; the one-pass chain (scan, emit and, top-k, refill) reads g and r and
 writes r = 12 bytes; both write 4 more when the consumed gradient is zeroed (``--zero-grad 1``, the engine's
 "flat" gradient mode; its default mode hands the kernels autograd's own tensors and zeroes nothing).  The sparse
 outputs are below 1 % of that.  Between iterations the gradient buffers are refilled, which also evicts the
@@ -54,7 +54,7 @@ def main() -> None:
     ap.add_argument("--bucket-mb", type=float, default=64.0)
     ap.add_argument("--chunk-elems", type=int, default=8192)
     ap.add_argument("--zero-grad", type=int, default=0, help="1: the select also writes zeros over the gradients it consumed")
-    ap.add_argument("--fused", type=int, default=1, help="0: keep the threshold compressors on the two-pass chain")
+    ap.add_argument("--fused", type=int, default=1, help="0: stay on the four-kernel chain")
     ap.add_argument("--iters", type=int, default=10)
     ap.add_argument("--warmup", type=int, default=3)
     args = ap.parse_args()
@@ -108,13 +108,13 @@ def main() -> None:
     out = {
         "compressor": args.compressor, "optimizer": args.optimizer, "elements": n_total, "buckets": len(buckets),
         "segments": len(numels), "entries_per_step": entries,
-        "select_chain": "one-pass (fused, finish)" if one_pass else "two-pass (pass1, plan, pass2, cand)",
+        "select_chain": "one-pass (scan, emit)" if one_pass else "two-pass (pass1, plan, pass2, cand)",
         "select_bytes_per_element": sel_bytes / n_total,
         "select_ms": sel, "select_GBps": sel_bytes / sel / 1e6,
         "select_frac_of_measured_copy": sel_bytes / sel / 1e6 / peaks["hbm_gbs"],
         "apply_ms": app, "apply_sector_GBps": app_bytes / app / 1e6,
         "hbm_gbs_measured": peaks["hbm_gbs"], "peaks_are_fallback": bool(peaks.get("fallback", False)),
-        "kernel_launches_per_step": len(buckets) * (4 if one_pass else 6),
+        "kernel_launches_per_step": sum(b.handle.select_kernels + b.apply_kernels for b in buckets),
     }
     print(json.dumps(out))
 

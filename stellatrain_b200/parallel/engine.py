@@ -56,8 +56,8 @@ class EngineConfig:
     status_poll_interval: int = 16        # forwards between non-blocking looks at the status words
     deterministic_merge: bool = False     # add the sources' contributions in rank order (one scatter launch per source):
                                           # replicas with replicated state stay bit-equal; world - 1 more launches per bucket
-    fused_select: bool = True             # threshold compressors: one pass over gradient and residual once every tensor
-                                          # has its threshold (12 bytes per element instead of 16 to 20)
+    fused_select: bool = True             # one pass over gradient and residual once every tensor has its threshold
+                                          # (12 bytes per element instead of 16 to 20)
     debug_checks: bool = False            # every stream carries a checksum that the receiver verifies (status 6), consumed
                                           # entries are overwritten with the "no entry" marker; slower, for debugging
     native_hooks: bool = True             # C++ hooks on the parameters and C++ bucket scheduling (csrc/cuda/native_engine.cpp);

@@ -208,7 +208,8 @@ class GpuBucket:
             chunks=self.chunks.data_ptr(), chunk_cnt=self.chunk_cnt.data_ptr(), chunk_pos=self.chunk_pos.data_ptr(),
             hist=self.hist.data_ptr(), n_segs=len(L.segments), n_chunks=L.n_chunks, cap=L.cap,
             pieces=self.pieces.data_ptr(), run_cnt=self.run_cnt.data_ptr(), piece_cnt=self.piece_cnt.data_ptr(),
-            hist_top=self.hist_top.data_ptr(), hist_rest=self.hist_rest.data_ptr(), refills=self.counters.data_ptr() + 16, n_pieces=self.n_pieces,
+            hist_top=self.hist_top.data_ptr(), hist_rest=self.hist_rest.data_ptr(), refills=self.counters.data_ptr() + 16,
+            n_pieces=self.n_pieces,
         )
         self.scratch.bind(h)
         h.set_control(
@@ -326,7 +327,7 @@ class GpuBucket:
 
     @property
     def thresholds_ready(self) -> bool:
-        """Every tensor has its threshold: the one-pass chain of the threshold compressors may take over."""
+        """Every tensor has its threshold: the one-pass chain may take over."""
         return bool(self._select_h.thresholds_ready)
 
     @thresholds_ready.setter
@@ -450,8 +451,8 @@ class GpuBucket:
 
 
 class CandidateScratch:
-    """Scratch for the undecided items of the threshold bin, shared by all buckets that run their
-    selects on one stream (worst case: every item of the largest bucket)."""
+    """Scratch for the lists and undecided items of a select, shared by all buckets that run their selects on one
+    stream (worst case: every item of the largest bucket)."""
 
     def __init__(self, device: torch.device) -> None:
         self.device = device

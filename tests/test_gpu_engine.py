@@ -632,3 +632,39 @@ def test_rank_weights_switch_at_a_named_iteration_without_draining(staleness):
         eng = make_engine(model, compressor="topk", ratio=0.9, optimizer="sgd")
         model([torch.randn(p.numel(), device="cuda") for p in model.ps]).backward()
         eng.set_rank_weights([1.0], from_iteration=0)
+
+
+@pytest.mark.parametrize("staleness", [0, 1])
+@pytest.mark.parametrize("grad_mode", ["steal", "flat"])
+def test_bucket_chains_on_two_streams_equal_one_stream(staleness, grad_mode):
+    """One rank, several buckets: the native engine lets them take turns on two streams, Python hooks use one.  Same bits,
+    also after a link shaper has moved every bucket to one stream and after new merge weights for a named iteration."""
+    import torch.nn as nn
+    import torch.nn.functional as F
+
+    from stellatrain_b200.control.shaper import BandwidthSchedule, DeviceTokenBucket
+    from stellatrain_b200.parallel.engine import EngineConfig, SparseDPEngine
+
+    def run(native):
+        torch.manual_seed(11)
+        m = nn.Sequential(nn.Linear(64, 200), nn.ReLU(), nn.Linear(200, 150), nn.ReLU(), nn.Linear(150, 10)).cuda()
+        e = SparseDPEngine(m, EngineConfig(compressor="topk", ratio=0.9, optimizer="adam", staleness=staleness, bucket_mb=0.02,
+                                           chunk_elems=1024, optimizer_options={"lr": 1e-2}, native_hooks=native,
+                                           grad_mode=grad_mode))
+        assert len(e.buckets) > 2 and len(e.sparse_streams) == (2 if native else 1)
+        g = torch.Generator(device="cuda").manual_seed(5)
+        for it in range(14):
+            x, y = torch.randn(32, 64, device="cuda", generator=g), torch.randint(0, 10, (32,), device="cuda", generator=g)
+            if it == 5:
+                e.set_rank_weights([0.5], from_iteration=7)
+            if it == 9:
+                e.set_link_shaper(DeviceTokenBucket(BandwidthSchedule(seed=1, lo_gbps=5.0, hi_gbps=9.0), e.device), destinations=1)
+                assert len(e.sparse_streams) == 1
+            F.cross_entropy(m(x), y).backward()
+        e.synchronize()
+        out = [p.detach().clone() for p in m.parameters()] + [rt.bucket.resid.clone() for rt in e.buckets]
+        e.close()
+        return out
+
+    for a, b in zip(run(True), run(False)):
+        assert torch.equal(a, b)
