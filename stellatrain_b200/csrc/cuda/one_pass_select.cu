@@ -64,15 +64,16 @@ __device__ __forceinline__ uint32_t top_cut(const SegState& ss, uint32_t n_pad) 
 }
 
 // Histogram of top-k's candidates around the previous threshold c (float bits), three widths of bins: 1024 of 2^-17
-// (relative) within 0.4 % of it, 256 of 2^-13 on either side as far as 3 %, 256 of 2^-8 on either side as far as an octave,
-// everything beyond in the end bins.  Error feedback piles items up at the threshold: with bins of 2^-10 throughout a few of
+// (relative) within 0.4 % of it, 256 of 2^-13 on either side as far as 3 %, 128 of 2^-7 on either side as far as an octave,
+// 128 of an eighth of an octave each beyond (gradients that jump up), the rest in the end bins.  Error feedback piles items up at the threshold: with bins of 2^-10 throughout a few of
 // them took most of the counts (L2 adds to one address one after the other: 239 us for a scan of 38.6 M elements, of
 // which the traffic needs 75) and the threshold's bin held thousands of undecided items.
 // c = 0 stands for "no usable threshold": 2048 even bins over all keys.
 // A tensor of several pieces spreads its counts over up to eight such histograms (one per piece modulo eight): 500,000
 // adds into the 64 cache lines of a single one still took 60 us longer than the traffic.
-constexpr int kNearShift = 6, kMidShift = 10, kFarShift = 15;
+constexpr int kNearShift = 6, kMidShift = 10, kFarShift = 16, kBeyondShift = 20;
 constexpr uint32_t kNear = 512u << kNearShift, kMid = kNear + (256u << kMidShift);     // distances where the widths change
+constexpr uint32_t kFar = kMid + (128u << kFarShift);
 
 __device__ __forceinline__ uint32_t top_centre(const SegState& ss) {
   return ss.reserved[1] >= (1u << 24) ? ss.reserved[1] : 0u;      // all bins under it fit
@@ -112,7 +113,10 @@ __device__ __forceinline__ uint32_t top_bin(uint32_t key, uint32_t c) {
   if (c == 0u) return key >> kHistShift;
   const bool above = key >= c;
   const uint32_t d = above ? key - c : c - key - 1u;
-  const uint32_t b = d < kNear ? d >> kNearShift : d < kMid ? 512u + ((d - kNear) >> kMidShift) : min(1023u, 768u + ((d - kMid) >> kFarShift));
+  const uint32_t b = d < kNear  ? d >> kNearShift
+                     : d < kMid ? 512u + ((d - kNear) >> kMidShift)
+                     : d < kFar ? 768u + ((d - kMid) >> kFarShift)
+                                : min(1023u, 896u + ((d - kFar) >> kBeyondShift));
   return above ? 1024u + b : 1023u - b;
 }
 
@@ -125,13 +129,21 @@ __device__ __forceinline__ void top_bin_range(uint32_t bin, uint32_t c, uint32_t
   }
   const bool above = bin >= 1024u;
   const uint32_t b = above ? bin - 1024u : 1023u - bin;
-  const int shift = b < 512u ? kNearShift : b < 768u ? kMidShift : kFarShift;
-  const uint32_t from = b < 512u ? b << kNearShift : b < 768u ? kNear + ((b - 512u) << kMidShift) : kMid + ((b - 768u) << kFarShift);
+  const int shift = b < 512u ? kNearShift : b < 768u ? kMidShift : b < 896u ? kFarShift : kBeyondShift;
+  const uint32_t from = b < 512u   ? b << kNearShift
+                        : b < 768u ? kNear + ((b - 512u) << kMidShift)
+                        : b < 896u ? kMid + ((b - 768u) << kFarShift)
+                                   : kFar + ((b - 896u) << kBeyondShift);
   const uint32_t to = from + (1u << shift);          // distances [from, to)
-  lo = above ? c + from : b == 1023u ? 0u : c - to;
-  hi = above ? (b == 1023u ? 0x80000000u : c + to) : c - from;
+  if (above) {
+    lo = min(c + from, 0x80000000u);
+    hi = b == 1023u ? 0x80000000u : min(c + to, 0x80000000u);
+  } else {
+    lo = b == 1023u || to >= c ? 0u : c - to;
+    hi = from >= c ? 0u : c - from;
+  }
 }
-static_assert(kHistBins == 2048 && kHistShift == 20 && kMid + (256u << kFarShift) < 1u << 24, "bins of top_bin");
+static_assert(kHistBins == 2048 && kHistShift == 20 && kFar < 1u << 24, "bins of top_bin");
 
 }  // namespace
 
