@@ -223,8 +223,9 @@ __global__ void __launch_bounds__(kThreads) k_apply(ApplyArgs A) {
   }
 }
 
-// One source: its stream names every element at most once (each select emits an element once, random-k strides
-// through the tensor with a step coprime to its size), so there is nothing to merge: no accumulator, no stamp to
+// One source: its stream names every element at most once (each select emits an element once, also where the narrow wire
+// format's rounding leaves something of it in the residual; random-k strides through the tensor with a step coprime to its
+// size), so there is nothing to merge: no accumulator, no stamp to
 // compete for, one kernel instead of two.  Bound by DRAM accesses to single records: 168,000 entries of a 64 MB bucket take
 // 10.8 us as blocks of 16 neighbours (threshold-v16; 13 us with scatter and apply) and 16.5 us one by one (top-k; 19 us).
 __global__ void __launch_bounds__(kThreads) k_apply_single(ApplyArgs A) {

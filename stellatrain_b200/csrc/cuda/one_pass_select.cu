@@ -686,6 +686,60 @@ __device__ __forceinline__ void send_range(const SelectArgs& A, const Job& J, Em
   }
 }
 
+// Threshold-v16: the blocks of a piece that hold something and are not on its lists (`total` listed blocks), as candidates of
+// the fill.  A listed block is sent whenever the stream is short; what the narrow wire format's rounding leaves of it in the
+// residual waits for the next select, so that a stream names an element once.  The lists, and not the residual, say which
+// blocks these are: other CTAs of the tensor may be sending them now.  Returns the number collected by this CTA.
+__device__ __forceinline__ uint32_t collect_unlisted(const SelectArgs& A, const Job& J, EmitShared& S, const uint2* area,
+                                                     uint32_t total, uint2* cand) {
+  constexpr uint32_t kQuads = kEmitThreads / 4, kKeys = 8;      // blocks side by side; keys a lane keeps per round
+  static_assert(kPieceElems / 16u / 32u <= 2048u, "a bit per block of a piece fits EmitShared::hist");
+  const uint32_t tid = threadIdx.x, first = J.pc.start >> 4;
+  const uint32_t n_blk = min(kPieceElems, J.sd.off + J.sd.n_pad - J.pc.start) >> 4;
+  for (uint32_t w = tid; w < kPieceElems / 16u / 32u; w += kEmitThreads) S.hist[w] = 0u;
+  __syncthreads();
+  for (uint32_t j = tid; j < total; j += kEmitThreads) {
+    const uint32_t run = run_of(S.pre, j), b = area[run * kRunBlocks + (j - S.pre[run])].x - first;
+    atomicOr(&S.hist[b >> 5], 1u << (b & 31u));
+  }
+  __syncthreads();
+  const float* src = A.resid + J.pc.start + (tid & 3u) * 4u;
+  uint32_t done = 0;
+  for (uint32_t b0 = 0; b0 < n_blk; b0 += kQuads * kKeys * 4u) {
+    uint32_t key[kKeys], there = 0;
+#pragma unroll
+    for (uint32_t s = 0; s < kKeys; ++s) {
+      float4 a[4];
+#pragma unroll
+      for (uint32_t q = 0; q < 4u; ++q) {   // independent loads in flight
+        const uint32_t b = b0 + (s * 4u + q) * kQuads + (tid >> 2);
+        const bool take = b < n_blk && !(S.hist[b >> 5] >> (b & 31u) & 1u);
+        a[q] = take ? __ldcg(reinterpret_cast<const float4*>(src + b * 16u)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (uint32_t q = 0; q < 4u; ++q) {
+        const uint32_t k = __float_as_uint(quad_l1(a[q]));
+        if ((tid & 3u) == q) key[s] = k;
+      }
+      there |= (key[s] != 0u ? 1u : 0u) << s;
+    }
+    uint32_t n;
+    const uint32_t ex = block_excl_scan(__popc(there), S.tmp, n);
+    uint32_t base = done;
+    if (J.pc.count > 1u) {
+      if (tid == 0) S.word[2] = n ? atomicAdd(&J.wp->cand_cnt, n) : 0u;
+      __syncthreads();
+      base = S.word[2];
+    }
+    uint32_t at = base + ex;
+#pragma unroll
+    for (uint32_t s = 0; s < kKeys; ++s)
+      if (there >> s & 1u) cand[at++] = make_uint2(first + b0 + (s * 4u + (tid & 3u)) * kQuads + (tid >> 2), key[s]);
+    done += n;
+  }
+  return done;
+}
+
 // Thread 0 of the last CTA of a top-k tensor: what the next select starts from.  Every candidate costs a list entry and a
 // histogram count, candidates that fall short cost two more passes over the tensor (twice the time).  How many more
 // candidates there were than entries says how near the cut came to falling short.  The threshold of one batch differs from
@@ -822,7 +876,13 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(SelectArgs A) {
       }
     } else {
       uint2* const nears = A.cand + (A.n_total >> 4) + (J.sd.off >> 4);     // block mode: one slot per block of the tensor
-      if (kBlock && short_of && near_total) {
+      // Do the near misses not suffice (or is there no threshold yet), then every block that holds something and is not over
+      // the threshold is a candidate.  Each CTA collects those of its own piece.
+      const bool rescan = kBlock && short_of && (!ss.inited || c_near < J.kk - found);
+      uint32_t collected = 0;
+      if (rescan) {
+        collected = collect_unlisted(A, J, S, area, total, nears);
+      } else if (kBlock && short_of && near_total) {
         // the fill needs the tensor's near misses in one place
         if (tid == 0) S.word[2] = J.pc.count == 1u ? 0u : atomicAdd(&J.wp->cand_cnt, near_total);
         __syncthreads();
@@ -879,36 +939,9 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(SelectArgs A) {
       }
       if (last_of_tensor(J, S)) {
         uint32_t t_key = 0;
-        bool scanned = false;
         if (kBlock && short_of && may) {
-          const uint32_t need = J.kk - found, n_blocks = J.sd.n_pad / 16u;
-          uint32_t c = c_near;
-          if (!ss.inited || c < need) {
-            // every block that still holds something is a candidate: the blocks over the threshold were all
-            // emitted (the stream is short of them) and are zero in the residual by now
-            scanned = true;
-            if (tid == 0) S.word[3] = 0u;
-            __syncthreads();
-            constexpr uint32_t kRound = kEmitThreads / 4;   // blocks per round, four lanes each
-            const float* src = A.resid + J.sd.off + (tid & 3u) * 4u;
-            for (uint32_t b0 = 0; b0 < n_blocks; b0 += 8u * kRound) {
-              float4 a[8];
-#pragma unroll
-              for (int u = 0; u < 8; ++u) {   // independent loads in flight
-                const uint32_t b = b0 + u * kRound + (tid >> 2);
-                a[u] = b < n_blocks ? __ldcg(reinterpret_cast<const float4*>(src + (size_t)b * 16u)) : make_float4(0.f, 0.f, 0.f, 0.f);
-              }
-#pragma unroll
-              for (int u = 0; u < 8; ++u) {
-                const uint32_t b = b0 + u * kRound + (tid >> 2);
-                const uint32_t key = __float_as_uint(quad_l1(a[u]));
-                if (b < n_blocks && (tid & 3u) == 0u && key != 0u)
-                  nears[atomicAdd(&S.word[3], 1u)] = make_uint2((J.sd.off >> 4) + b, key);
-              }
-            }
-            __syncthreads();
-            c = S.word[3];
-          }
+          const uint32_t need = J.kk - found;
+          const uint32_t c = !rescan ? c_near : J.pc.count == 1u ? collected : __ldcg(&J.wp->cand_cnt);
           const uint32_t take = min(need, c);
           if (take && c <= kPickMax) {
             t_key = pick_few(nears, c, take, 0u, 0x7fffffffu, S);
@@ -955,7 +988,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(SelectArgs A) {
             // cent, which is all a fill ever needs, and ranking the candidates costs time in proportion to their number.
             float w = window_or(st.reserved[0], kWindowDefault);
             const uint32_t needed = short_of ? J.kk - found : 0u;
-            if (scanned) w *= 2.f;
+            if (rescan) w *= 2.f;
             else if (c_near < J.kk / 16u + 8u || c_near < 2u * needed) w *= 1.5f;
             else if (c_near > J.kk / 4u + 32u) w *= 0.75f;
             st.reserved[0] = __float_as_uint(fminf(fmaxf(w, 1e-3f), 1.f));

@@ -11,13 +11,13 @@ pytestmark = pytest.mark.gpu
 SIZES = [1, 15, 16, 17, 1000, 4096, 65535, 65536, 70001, 300000]
 
 
-def make_bucket(compressor, ratio, optimizer="sgd", sizes=SIZES, chunk=4096, **kw):
+def make_bucket(compressor, ratio, optimizer="sgd", sizes=SIZES, chunk=4096, narrow=False, debug=False, **kw):
     from stellatrain_b200.parallel.gpu_bucket import GpuBucket
 
     dev = torch.device("cuda:0")
-    layout = B.BucketLayout([f"t{i}" for i in range(len(sizes))], sizes, chunk_elems=chunk)
+    layout = B.BucketLayout([f"t{i}" for i in range(len(sizes))], sizes, chunk_elems=chunk, narrow_wire=narrow)
     b = GpuBucket(0, layout, dev, compressor=compressor, ratio=ratio, optimizer=optimizer, **kw)
-    b.wire_local()
+    b.wire_local(debug_checks=debug)
     return b
 
 
@@ -105,15 +105,17 @@ def test_select_matches_oracle(compressor, mode, fused):
 
 @pytest.mark.parametrize("compressor", ["topk", "thresholdv", "thresholdv16"])
 @pytest.mark.parametrize("mode", ["steady", "jumps", "ties", "mostly_zero", "huge"])
-@pytest.mark.parametrize("ratio,chunk", [(0.99, 8192), (0.5, 1024), (0.999, 1 << 18)])
-def test_one_pass_select_at_its_edges(compressor, mode, ratio, chunk):
+@pytest.mark.parametrize("ratio,chunk,narrow", [(0.99, 8192, False), (0.5, 1024, False), (0.999, 1 << 18, False),
+                                                (0.99, 8192, True), (0.5, 1024, True)])
+def test_one_pass_select_at_its_edges(compressor, mode, ratio, chunk, narrow):
     """The one-pass chain against the plain rule at the edges of its runs (1024 elements), pieces (131072) and chunks:
     the same entries bit for bit.  "jumps" moves the gradient scale up and down by large factors, so that top-k's
     candidates fall short and the refill kernel selects; "mostly_zero" leaves fewer entries than the budget; "huge"
-    holds values far outside the histogram window."""
-    sizes = [1, 16, 1023, 1024, 1025, 8192, 9001, 131071, 131072, 131073, 400001]
+    holds values far outside the histogram window.  ``narrow``: tensors of fewer than 65536 elements send bf16 values and keep
+    the rounding error."""
+    sizes = [1, 16, 1023, 1024, 1025, 8192, 9001, 65519, 131071, 131072, 131073, 400001]
     gen = torch.Generator(device="cuda").manual_seed(99)
-    b = make_bucket(compressor, ratio, sizes=sizes, chunk=chunk)
+    b = make_bucket(compressor, ratio, sizes=sizes, chunk=chunk, narrow=narrow)
     resid_ref = torch.zeros_like(b.resid)
     for step in range(7):
         scale = [1.0, 1.0, 0.02, 0.02, 50.0, 0.5, 0.4][step] if mode == "jumps" else 1.0
@@ -133,6 +135,10 @@ def test_one_pass_select_at_its_edges(compressor, mode, ratio, chunk):
             own = slp if compressor == "thresholdv16" else sl
             # top-k of a tensor with fewer entries than the budget sends zeros, lowest index first
             want_idx, want_val, new_r = O.compress_step(compressor, grad[own], resid_ref[own], s.k, states[si], one_pass=step > 0)
+            if b.layout.is_narrow(s):
+                sent = want_val.bfloat16().float()
+                new_r[want_idx] = want_val - sent
+                want_val = sent
             got = torch.from_numpy(idx_all[s.out_off : s.out_off + s.k])
             valid = got != O.SENTINEL
             got, order = got[valid].sort()
@@ -261,6 +267,49 @@ def test_apply_options_nesterov_smart_amsgrad():
         g, touched = O.merge_streams(b.layout.n_total, [(torch.from_numpy(idx).cuda(), val.cuda())], [1.0])
         O.sparse_adam(p_ref, g, touched, cfg, st)
         torch.testing.assert_close(b.param, p_ref, rtol=1e-4, atol=1e-6)
+
+
+@pytest.mark.parametrize("compressor", ["topk", "thresholdv", "thresholdv16"])
+@pytest.mark.parametrize("optimizer", ["sgd", "adam"])
+@pytest.mark.parametrize("narrow,infinite", [(True, False), (False, False), (False, True)])
+def test_a_stream_names_an_element_once(compressor, optimizer, narrow, infinite):
+    """What the single-source apply rests on.  Gradients that are dense at first and then live in a few blocks only (an
+    embedding, a mostly frozen tensor) leave the near misses short of the budget, so that threshold-v16 fills its stream from
+    all blocks; neither the remainders of the narrow format's rounding nor inf - inf in the residual may be sent again in the
+    same stream.  Against the merging apply, which would add such entries up."""
+    sizes = [5, 3000, 40000, 65000, 200000, 300001]
+    pair = [make_bucket(compressor, 0.9, optimizer, sizes=sizes, chunk=8192, narrow=narrow, debug=d) for d in (False, True)]
+    assert [b.apply_kernels for b in pair] == [1, 2]
+    gen = torch.Generator(device="cuda").manual_seed(17)
+    start = torch.randn(pair[0].layout.n_total, generator=gen, device="cuda")
+    live = (torch.rand(pair[0].layout.n_total // 16, generator=gen, device="cuda") < 0.01).repeat_interleave(16)
+    for b in pair:
+        b.set_optimizer_options(lr=1e-2, momentum=0.9)
+        b.param.copy_(start)
+    for step in range(50):
+        fill_grads(pair[0], gen)
+        if step >= 5:
+            pair[0].grad *= live
+        if infinite and step in (10, 30):
+            for s, _, _ in seg_slices(pair[0]):
+                pair[0].grad[s.off + s.numel // 2] = float("inf")
+        pair[1].grad.copy_(pair[0].grad)
+        for b in pair:
+            a = b.grad + b.resid
+            b.select()
+            idx, val = b.stream_of((step + 1) & 1, 0)
+            there = idx != -1
+            idx, val = idx[there].long(), val[there]
+            assert len(torch.unique(idx)) == len(idx), step
+            if not infinite:
+                # the wire format's rounding error is a float32 value, so nothing gets lost
+                assert torch.equal(b.resid.index_add(0, idx, val), a), step
+            b.apply()
+    for b in pair:
+        torch.cuda.synchronize()
+        b.check_status()
+    for name in ("param", "rec", "resid"):
+        torch.testing.assert_close(getattr(pair[0], name), getattr(pair[1], name), rtol=0, atol=0, equal_nan=True)
 
 
 @pytest.mark.parametrize("optimizer,options,extra", [
