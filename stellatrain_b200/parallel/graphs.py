@@ -51,11 +51,14 @@ class GraphedStep:
             with torch.cuda.graph(self.graph, stream=side):
                 self.loss = step_fn(*self.static_inputs)
                 cur = torch.cuda.current_stream(dev)
+                # a stream takes part only when a bucket on it was ready
+                taking_part = []
                 for s in engine.sparse_streams:
-                    with torch.cuda.stream(s):      # the second one takes part only when a bucket on it was ready
-                        joins = s is engine.sparse_stream or torch.cuda.is_current_stream_capturing()
-                    if joins:
-                        cur.wait_stream(s)
+                    with torch.cuda.stream(s):
+                        if torch.cuda.is_current_stream_capturing():
+                            taking_part.append(s)
+                for s in taking_part or [engine.sparse_stream]:      # no bucket at all: refused by the wait
+                    cur.wait_stream(s)
                 if engine.cfg.step_clock:
                     engine.stamp(4)      # behind the join: (4) - (2) is the time the iteration waited for its bucket chains
         finally:

@@ -668,3 +668,48 @@ def test_bucket_chains_on_two_streams_equal_one_stream(staleness, grad_mode):
 
     for a, b in zip(run(True), run(False)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("used", ["all", "bucket on the second stream only"])
+def test_captured_iteration_joins_the_streams_that_took_part(used):
+    """The native engine's two streams under capture against the one stream of the Python hooks: the same bits.  Also when
+    only a bucket on the second stream has its gradients, so that the first one is not part of the capture."""
+    import torch.nn as nn
+
+    from stellatrain_b200.parallel.engine import EngineConfig, SparseDPEngine
+    from stellatrain_b200.parallel.graphs import GraphedStep
+
+    class Net(nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.a, self.b = nn.Linear(64, 80, bias=False), nn.Linear(80, 65, bias=False)
+
+        def forward(self, x):
+            h = self.a(x)
+            return self.b(torch.relu(h)) if used == "all" else h
+
+    def run(native):
+        torch.manual_seed(3)
+        m = Net().cuda()
+        e = SparseDPEngine(m, EngineConfig(compressor="thresholdv", ratio=0.9, optimizer="adam", staleness=0, bucket_mb=0.02,
+                                           chunk_elems=1024, optimizer_options={"lr": 1e-2}, native_hooks=native))
+        assert len(e.buckets) == 2 and len(e.sparse_streams) == (2 if native else 1)      # b comes first
+
+        def step(x):
+            loss = m(x).square().mean()
+            loss.backward()
+            return loss
+
+        gen = torch.Generator(device="cuda").manual_seed(8)
+        xs = [torch.randn(32, 64, device="cuda", generator=gen) for _ in range(6)]
+        graphed = GraphedStep(e, step, [xs[0]], warmup=3)
+        for x in xs:
+            graphed.copy_inputs(x)
+            graphed.replay()
+        e.synchronize()
+        out = [p.detach().clone() for p in m.parameters()] + [rt.bucket.resid.clone() for rt in e.buckets]
+        e.close()
+        return out
+
+    for a, b in zip(run(True), run(False)):
+        assert torch.equal(a, b)
