@@ -35,6 +35,9 @@ def compress_tensor(name: str, tensor: torch.Tensor, ratio: float, method: str =
 def _compress_cuda(name: str, flat: torch.Tensor, k: int, method: str):
     from ..parallel.gpu_bucket import GpuBucket
 
+    if torch.cuda.is_current_stream_capturing():
+        # the caller gets as many pairs as the stream turns out to hold, which takes a wait; refused before any state moves on
+        raise RuntimeError("compress waits for its result: it cannot be captured in a CUDA graph")
     n = flat.numel()
     key = (name, n, method, flat.device.index)
     b = _gpu_cache.get(key)

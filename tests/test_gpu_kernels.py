@@ -188,6 +188,28 @@ def test_compress_reads_the_tensor_in_place(compressor, n, form):
         st.configure_compression("thresholdv16")
 
 
+@pytest.mark.parametrize("compressor", ["topk", "thresholdv", "thresholdv16"])
+def test_compress_under_capture_is_refused_and_leaves_no_trace(compressor):
+    """The refused call must not count as the tensor's first select, which is the one that measures the threshold."""
+    import stellatrain_b200 as st
+
+    n, name = 5000, f"captured {compressor}"
+    gen, state = torch.Generator(device="cuda").manual_seed(2), O.ThresholdState()
+    st.configure_compression(compressor)
+    try:
+        for call in range(4):
+            x = torch.randn(n, generator=gen, device="cuda")
+            if call in (0, 2):
+                with pytest.raises(RuntimeError, match="captured"), torch.cuda.graph(torch.cuda.CUDAGraph()):
+                    st.compress(name, x, 0.9)
+            idx, val = st.compress(name, x, 0.9)
+            want, _, _ = O.compress_step(compressor, x, torch.zeros_like(x), int((1 - 0.9) * n), state, one_pass=call > 0)
+            assert torch.equal(idx.long().sort().values, want[want < n].sort().values), call
+            assert torch.equal(val, x[idx.long()])
+    finally:
+        st.configure_compression("thresholdv16")
+
+
 def test_select_drops_nan():
     b = make_bucket("topk", 0.9, sizes=[1000, 5000])
     g = torch.randn(b.layout.n_total, device="cuda")
