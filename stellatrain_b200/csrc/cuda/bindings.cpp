@@ -52,7 +52,11 @@ struct BucketHandle : public st::BucketHandle {
   void set_tables(uint64_t segs, uint64_t state, uint64_t work, uint64_t chunks, uint64_t chunk_cnt,
                   uint64_t chunk_pos, uint64_t hist, uint32_t n_segs, uint32_t n_chunks, uint32_t cap,
                   uint64_t pieces, uint64_t run_cnt, uint64_t piece_cnt, uint64_t hist_top, uint64_t hist_rest, uint64_t refills,
-                  uint32_t n_pieces) {
+                  uint32_t n_pieces, uint32_t piece_runs) {
+    if (piece_runs == 0 || piece_runs > st::kMaxPieceRuns || (piece_runs & (piece_runs - 1u)) != 0u)
+      throw std::invalid_argument("a piece is a power of two of runs, at most 128");
+    sel.piece_shift = 0;
+    while (1u << sel.piece_shift < piece_runs) ++sel.piece_shift;
     sel.pieces = as_ptr<const st::Piece>(pieces);
     sel.run_cnt = as_ptr<uint32_t>(run_cnt);
     sel.piece_cnt = as_ptr<uint64_t>(piece_cnt);
@@ -281,7 +285,7 @@ PYBIND11_MODULE(_C, m) {
   m.attr("SIZEOF_SEG_WORK") = sizeof(st::SegWork);
   m.attr("SIZEOF_CHUNK") = sizeof(st::Chunk);
   m.attr("SIZEOF_PIECE") = sizeof(st::Piece);
-  m.attr("PIECE_RUNS") = st::kPieceRuns;
+  m.attr("MAX_PIECE_RUNS") = st::kMaxPieceRuns;
   m.attr("RUN_ELEMS") = st::kRunElems;
   m.attr("SIZEOF_OPT_STATE") = sizeof(st::OptState);
 
@@ -292,7 +296,8 @@ PYBIND11_MODULE(_C, m) {
       .def("set_tables", &BucketHandle::set_tables, py::arg("segs"), py::arg("state"), py::arg("work"),
            py::arg("chunks"), py::arg("chunk_cnt"), py::arg("chunk_pos"), py::arg("hist"), py::arg("n_segs"),
            py::arg("n_chunks"), py::arg("cap"), py::arg("pieces") = 0, py::arg("run_cnt") = 0,
-           py::arg("piece_cnt") = 0, py::arg("hist_top") = 0, py::arg("hist_rest") = 0, py::arg("refills") = 0, py::arg("n_pieces") = 0)
+           py::arg("piece_cnt") = 0, py::arg("hist_top") = 0, py::arg("hist_rest") = 0, py::arg("refills") = 0, py::arg("n_pieces") = 0,
+           py::arg("piece_runs") = st::kMaxPieceRuns)
       .def("set_scratch", &BucketHandle::set_scratch, py::arg("cand"), py::arg("cand_cursor"), py::arg("cand_cap"))
       .def("set_control", &BucketHandle::set_control, py::arg("counters"), py::arg("status"), py::arg("opt"),
            py::arg("weight"), py::arg("timeout_ns"), py::arg("stamps") = 0)

@@ -7,7 +7,7 @@
 //           backend/src/compress/thresholdv.cpp:44-52, backend/src/compress/thresholdv16.cpp:81-97; the latter also lists
 //           near-miss blocks just under it) or a little less than the previous k-th largest value (top-k, which also
 //           counts its candidates in a histogram around that value).
-//   emit    one CTA per piece (up to 128 runs) of a tensor turns the lists into stream entries, stores them into the
+//   emit    one CTA per piece (8 to 128 runs) of a tensor turns the lists into stream entries, stores them into the
 //           destinations' receive areas and clears them in r.  The CTA that finishes a tensor last settles what is left:
 //           the exact cut inside the threshold's bin (top-k), the best of the near misses when the blocks over the
 //           threshold fall short of the budget (the reference's heap, backend/src/compress/thresholdv16.cpp:261-293),
@@ -36,7 +36,7 @@ constexpr int kScanThreads = 256;
 constexpr int kScanWarps = kScanThreads / 32;
 constexpr uint32_t kHalf = kRunElems / 2;      // a run is read in two halves: four float4 of r and of g per lane in flight
 constexpr uint32_t kRunBlocks = kRunElems / 16;
-constexpr uint32_t kPieceElems = kPieceRuns * kRunElems;
+constexpr uint32_t kMaxPieceElems = kMaxPieceRuns * kRunElems;
 
 constexpr int kEmitThreads = 256;
 constexpr uint32_t kStageItems = 2048;         // entries staged at a time
@@ -69,7 +69,7 @@ __device__ __forceinline__ uint32_t top_cut(const SegState& ss, uint32_t n_pad) 
 // them took most of the counts (L2 adds to one address one after the other: 239 us for a scan of 38.6 M elements, of
 // which the traffic needs 75) and the threshold's bin held thousands of undecided items.
 // c = 0 stands for "no usable threshold": 2048 even bins over all keys.
-// A tensor of several pieces spreads its counts over up to eight such histograms (one per piece modulo eight): 500,000
+// A tensor of several pieces spreads its counts over up to eight such histograms (one per piece modulo their number): 500,000
 // adds into the 64 cache lines of a single one still took 60 us longer than the traffic.
 constexpr int kNearShift = 6, kMidShift = 10, kFarShift = 16, kBeyondShift = 20;
 constexpr uint32_t kNear = 512u << kNearShift, kMid = kNear + (256u << kMidShift);     // distances where the widths change
@@ -104,8 +104,10 @@ __device__ __forceinline__ void rest_bin_range(uint32_t bin, uint32_t cut, uint3
   }
 }
 
-__device__ __forceinline__ uint32_t hist_copies(uint32_t pieces) {
-  return pieces >= 8u ? 8u : pieces >= 4u ? 4u : pieces >= 2u ? 2u : 1u;
+// By the tensor's size and not its number of pieces, which is never smaller: every CTA of `emit` reads them all.
+__device__ __forceinline__ uint32_t hist_copies(uint32_t n_pad) {
+  const uint32_t full = (n_pad + kMaxPieceElems - 1u) / kMaxPieceElems;
+  return full >= 8u ? 8u : full >= 4u ? 4u : full >= 2u ? 2u : 1u;
 }
 
 // Monotone in key.
@@ -163,6 +165,7 @@ __global__ void __launch_bounds__(kScanThreads, 4) k_scan(SelectArgs A) {
   uint2* const stage = s_stage[warp];
   if (blockIdx.x == 0 && threadIdx.x == 0 && A.stamps != nullptr) A.stamps[0] = global_timer_ns();
 
+  const uint32_t piece_shift = A.piece_shift + kRunShift;      // of elements
   for (uint32_t rel = warp * kRunElems; rel < ch.len; rel += kScanWarps * kRunElems) {
     const uint32_t start = ch.start + rel;
     const uint32_t len = min(kRunElems, ch.len - rel);     // multiple of 16
@@ -175,7 +178,7 @@ __global__ void __launch_bounds__(kScanThreads, 4) k_scan(SelectArgs A) {
     }
     const SegDesc sd = A.segs[ch.seg];
     const bool tab = A.grad_tab != nullptr;
-    const uint32_t seg_rel = start - sd.off, piece_of_seg = seg_rel / kPieceElems;
+    const uint32_t seg_rel = start - sd.off;
     float* g = tab ? A.grad_tab[ch.seg] + seg_rel : A.grad + start;
     const SegState ss = A.state[ch.seg];
     if (sd.reserved & kSegSkip) {
@@ -279,8 +282,9 @@ __global__ void __launch_bounds__(kScanThreads, 4) k_scan(SelectArgs A) {
         __syncwarp();
         // Histogram of the candidates.  The top bin, which holds many of them, is not counted: `emit` knows their number.
         const uint32_t centre = top_centre(ss);
-        const uint32_t copy = piece_of_seg & (hist_copies((sd.n_pad + kPieceElems - 1u) / kPieceElems) - 1u);
-        uint32_t* const gh = A.hist_top + (size_t)((ch.run0 + rel / kRunElems) / kPieceRuns - piece_of_seg + copy) * kHistBins;
+        const uint32_t piece = seg_rel >> piece_shift;      // of the tensor
+        const uint32_t first_piece = ((ch.run0 + rel / kRunElems) >> A.piece_shift) - piece;
+        uint32_t* const gh = A.hist_top + (size_t)(first_piece + (piece & (hist_copies(sd.n_pad) - 1u))) * kHistBins;
         for (uint32_t q0 = 0; q0 < n_half; q0 += 32u) {
           const uint32_t q = q0 + lane;
           uint32_t b = kHistBins - 1;
@@ -327,8 +331,8 @@ __global__ void __launch_bounds__(kScanThreads, 4) k_scan(SelectArgs A) {
       const uint32_t run = ch.run0 + rel / kRunElems;
       A.run_cnt[run] = n_list | n_near << 16;
       // tensors of several pieces: every piece's total, so that each CTA of `emit` can place itself
-      if (sd.n_pad > kPieceElems && (n_list | n_near))
-        atomicAdd(reinterpret_cast<unsigned long long*>(A.piece_cnt + run / kPieceRuns),
+      if (sd.n_pad > 1u << piece_shift && (n_list | n_near))
+        atomicAdd(reinterpret_cast<unsigned long long*>(A.piece_cnt + (run >> A.piece_shift)),
                   (unsigned long long)n_near << 32 | n_list);
     }
   }
@@ -342,8 +346,8 @@ namespace {
 struct EmitShared {
   uint2 stage[kStageItems];
   uint32_t hist[2048];
-  uint32_t pre[kPieceRuns + 1];     // listed items in front of each run of the piece
-  uint32_t near[kPieceRuns + 1];    // near misses in front of each run of the piece
+  uint32_t pre[kMaxPieceRuns + 1];     // listed items in front of each run of the piece
+  uint32_t near[kMaxPieceRuns + 1];    // near misses in front of each run of the piece
   uint32_t tmp[kEmitThreads / 32 + 1];
   uint32_t res[4];
   uint32_t cnt[64];                 // counts of the bitwise searches
@@ -354,7 +358,7 @@ struct EmitShared {
 
 // Run (of the piece) that holds item j: the last one that starts at or in front of it and is not empty.
 __device__ __forceinline__ uint32_t run_of(const uint32_t* pre, uint32_t j) {
-  uint32_t lo = 0, hi = kPieceRuns;
+  uint32_t lo = 0, hi = kMaxPieceRuns;
 #pragma unroll
   for (int s = 0; s < 7; ++s) {
     const uint32_t mid = (lo + hi) >> 1;
@@ -362,7 +366,7 @@ __device__ __forceinline__ uint32_t run_of(const uint32_t* pre, uint32_t j) {
   }
   return lo;
 }
-static_assert(kPieceRuns == 128, "run_of halves 128 runs seven times");
+static_assert(kMaxPieceRuns == 128, "run_of halves 128 runs seven times");
 
 // What a CTA of `emit` / `refill` works on.
 struct Job {
@@ -373,6 +377,8 @@ struct Job {
   uint64_t slot_off;
   int dest;
   uint32_t nb;
+  uint32_t piece_elems;       // of a full piece
+  uint32_t len;               // elements of this one
 };
 
 __device__ __forceinline__ Job job_of(const SelectArgs& A, bool block) {
@@ -385,6 +391,8 @@ __device__ __forceinline__ Job job_of(const SelectArgs& A, bool block) {
   J.slot_off = (uint64_t)(J.epoch & 1u) * A.slot_stride + J.sd.out_off;
   J.dest = dest_of(A, J.sd);
   J.nb = narrow_base_of(J.sd);
+  J.piece_elems = kRunElems << A.piece_shift;
+  J.len = min(J.piece_elems, J.sd.off + J.sd.n_pad - J.pc.start);
   return J;
 }
 
@@ -693,10 +701,10 @@ __device__ __forceinline__ void send_range(const SelectArgs& A, const Job& J, Em
 __device__ __forceinline__ uint32_t collect_unlisted(const SelectArgs& A, const Job& J, EmitShared& S, const uint2* area,
                                                      uint32_t total, uint2* cand) {
   constexpr uint32_t kQuads = kEmitThreads / 4, kKeys = 8;      // blocks side by side; keys a lane keeps per round
-  static_assert(kPieceElems / 16u / 32u <= 2048u, "a bit per block of a piece fits EmitShared::hist");
+  static_assert(kMaxPieceElems / 16u / 32u <= 2048u, "a bit per block of a piece fits EmitShared::hist");
   const uint32_t tid = threadIdx.x, first = J.pc.start >> 4;
-  const uint32_t n_blk = min(kPieceElems, J.sd.off + J.sd.n_pad - J.pc.start) >> 4;
-  for (uint32_t w = tid; w < kPieceElems / 16u / 32u; w += kEmitThreads) S.hist[w] = 0u;
+  const uint32_t n_blk = J.len >> 4;
+  for (uint32_t w = tid; w < kMaxPieceElems / 16u / 32u; w += kEmitThreads) S.hist[w] = 0u;
   __syncthreads();
   for (uint32_t j = tid; j < total; j += kEmitThreads) {
     const uint32_t run = run_of(S.pre, j), b = area[run * kRunBlocks + (j - S.pre[run])].x - first;
@@ -765,7 +773,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(SelectArgs A) {
   constexpr bool kBlock = MODE == kScanBlock;
   const uint32_t tid = threadIdx.x;
   const Job J = job_of(A, kBlock);
-  const uint32_t cnt = tid < J.pc.n_runs ? A.run_cnt[blockIdx.x * kPieceRuns + tid] : 0u;
+  const uint32_t cnt = tid < J.pc.n_runs ? A.run_cnt[(blockIdx.x << A.piece_shift) + tid] : 0u;
   const bool ok = ld_volatile_u32(A.status) == kOk;
 
   if (!(J.sd.reserved & kSegSkip)) {
@@ -777,10 +785,10 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(SelectArgs A) {
     if (tid < 2) S.sum[tid] = 0ull;
     uint32_t total, near_total = 0;
     uint32_t ex = block_excl_scan(cnt & 0xffffu, S.tmp, total);
-    if (tid <= kPieceRuns) S.pre[tid] = ex;
+    if (tid <= kMaxPieceRuns) S.pre[tid] = ex;
     if (kBlock) {
       const uint32_t nex = block_excl_scan(cnt >> 16, S.tmp, near_total);
-      if (tid <= kPieceRuns) S.near[tid] = nex;
+      if (tid <= kMaxPieceRuns) S.near[tid] = nex;
     }
     uint32_t found = total, c_near = near_total;
     if (J.pc.count > 1u) {
@@ -813,10 +821,9 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(SelectArgs A) {
         const uint32_t cut = top_cut(ss, J.sd.n_pad);
         for (uint32_t b = tid; b < (uint32_t)kHistBins; b += kEmitThreads) S.hist[b] = 0u;
         __syncthreads();
-        const uint32_t len = min(kPieceElems, J.sd.off + J.sd.n_pad - J.pc.start);
         uint32_t zeros = 0;
 #pragma unroll 4
-        for (uint32_t i = tid * 4u; i < len; i += kEmitThreads * 4u) {
+        for (uint32_t i = tid * 4u; i < J.len; i += kEmitThreads * 4u) {
           const float4 a = *reinterpret_cast<const float4*>(A.resid + J.pc.start + i);
           const uint32_t key[4] = {key_bits(a.x), key_bits(a.y), key_bits(a.z), key_bits(a.w)};
 #pragma unroll
@@ -829,9 +836,9 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(SelectArgs A) {
         uint32_t* gh = A.hist_rest + (size_t)J.pc.seg * kHistBins;
         for (uint32_t b = tid; b < (uint32_t)kHistBins; b += kEmitThreads)
           if (S.hist[b]) atomicAdd(gh + b, S.hist[b]);
-        if (tid == 0) A.run_cnt[blockIdx.x * kPieceRuns] = zeros;     // this CTA has read its own counts
+        if (tid == 0) A.run_cnt[blockIdx.x << A.piece_shift] = zeros;     // this CTA has read its own counts
       } else if (!short_of) {
-        plan_top(A.hist_top + (size_t)J.pc.first * kHistBins, hist_copies(J.pc.count), found, J.kk, false, S);
+        plan_top(A.hist_top + (size_t)J.pc.first * kHistBins, hist_copies(J.sd.n_pad), found, J.kk, false, S);
         top_bin_range(S.res[0], top_centre(ss), key_lo, key_hi);
         if (may) {
           constexpr int kItems = 8;
@@ -872,7 +879,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(SelectArgs A) {
         if (tid == 0) { J.wp->out_cursor = 0u; J.wp->cand_cnt = 0u; }
         for (uint32_t t = tid; t < J.pc.count; t += kEmitThreads) A.piece_cnt[J.pc.first + t] = 0ull;
         uint4* gh = reinterpret_cast<uint4*>(A.hist_top + (size_t)J.pc.first * kHistBins);
-        for (uint32_t b = tid; b < hist_copies(J.pc.count) * (kHistBins / 4); b += kEmitThreads) gh[b] = make_uint4(0u, 0u, 0u, 0u);
+        for (uint32_t b = tid; b < hist_copies(J.sd.n_pad) * (kHistBins / 4); b += kEmitThreads) gh[b] = make_uint4(0u, 0u, 0u, 0u);
       }
     } else {
       uint2* const nears = A.cand + (A.n_total >> 4) + (J.sd.off >> 4);     // block mode: one slot per block of the tensor
@@ -917,13 +924,13 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(SelectArgs A) {
         }
         for (;;) {
           if (J.pc.count > 1u) {
-            const uint32_t v = tid < kPieceRuns ? A.run_cnt[(J.pc.first + piece) * kPieceRuns + tid] & 0xffffu : 0u;
-            const uint32_t n_runs = (min(kPieceElems, J.sd.n_pad - piece * kPieceElems) + kRunElems - 1u) / kRunElems;
-            ex = block_excl_scan(tid < n_runs ? v : 0u, S.tmp, total);
-            if (tid <= kPieceRuns) S.pre[tid] = ex;
+            const uint32_t n_runs = (min(J.piece_elems, J.sd.n_pad - piece * J.piece_elems) + kRunElems - 1u) / kRunElems;
+            const uint32_t v = tid < n_runs ? A.run_cnt[((J.pc.first + piece) << A.piece_shift) + tid] & 0xffffu : 0u;
+            ex = block_excl_scan(v, S.tmp, total);
+            if (tid <= kMaxPieceRuns) S.pre[tid] = ex;
             __syncthreads();
           }
-          const uint2* const lists = A.cand + (kBlock ? J.sd.off >> 4 : J.sd.off) + (size_t)piece * (kPieceRuns * kArea);
+          const uint2* const lists = A.cand + (kBlock ? J.sd.off >> 4 : J.sd.off) + (size_t)piece * (kArea << A.piece_shift);
           send_range<kBlock>(A, J, S, lists, base, lo > base ? lo - base : 0u, min(hi - base, total));
           base += total;
           ++piece;
@@ -1023,12 +1030,12 @@ __global__ void __launch_bounds__(kEmitThreads, 2) k_refill(SelectArgs A) {
     rest_bin_range(S.res[0], cut, key_lo, key_hi);
     const uint32_t rem = S.res[1];
     uint2* const undecided = A.cand + A.n_total + J.sd.off;
-    const uint32_t len = min(kPieceElems, J.sd.off + J.sd.n_pad - J.pc.start);
+    const uint32_t len = J.len;
     if (may && zero_fill) {
       // fewer non-zero elements than the budget: zeros complete it, lowest index first; `emit` left their number per piece.
       // This comes first, because what is sent below becomes zero in the residual.
       uint32_t before = 0, base;
-      for (uint32_t t = tid; t < J.pc.index; t += kEmitThreads) before += A.run_cnt[(J.pc.first + t) * kPieceRuns];
+      for (uint32_t t = tid; t < J.pc.index; t += kEmitThreads) before += A.run_cnt[(J.pc.first + t) << A.piece_shift];
       block_excl_scan(before, S.tmp, base);
       for (uint32_t i0 = 0; i0 < len && base < rem; i0 += kEmitThreads * 4u) {
         const uint32_t i = i0 + tid * 4u;
@@ -1092,7 +1099,7 @@ bool one_pass_possible(const SelectArgs& A) {
 
 cudaError_t launch_select_one_pass(const SelectArgs& A, cudaStream_t stream) {
   if (A.n_chunks == 0 || A.n_segs == 0) return cudaSuccess;
-  if (A.world > kMaxWorld || !one_pass_possible(A)) return cudaErrorInvalidValue;
+  if (A.world > kMaxWorld || !one_pass_possible(A) || (1u << A.piece_shift) > kMaxPieceRuns) return cudaErrorInvalidValue;
   if (A.compressor == kThresholdv16) {
     k_scan<kScanBlock><<<A.n_chunks, kScanThreads, 0, stream>>>(A);
     k_emit<kScanBlock><<<A.n_pieces, kEmitThreads, 0, stream>>>(A);

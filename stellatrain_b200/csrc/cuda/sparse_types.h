@@ -93,10 +93,11 @@ struct Chunk {            // unit of work of the streaming passes; never spans t
 };
 
 // One-pass chain.  A run is 1024 consecutive elements of a tensor (fewer at its end), the work of one warp; chunk lengths
-// are multiples of it.  A piece is up to 128 runs of one tensor, the work of one CTA of the emitting kernels.  Run r of
-// piece p has the number 128 p + r.
-constexpr uint32_t kRunElems = 1024u;
-constexpr uint32_t kPieceRuns = 128u;
+// are multiples of it.  A piece is up to 2^shift runs of one tensor, the work of one CTA of the emitting kernels; the shift is
+// one for the whole bucket (BucketLayout.piece_runs says how it is chosen).  Run r of piece p has the number (p << shift) + r.
+constexpr uint32_t kRunShift = 10u;
+constexpr uint32_t kRunElems = 1u << kRunShift;
+constexpr uint32_t kMaxPieceRuns = 128u;
 
 struct Piece {
   uint32_t seg;
@@ -131,7 +132,8 @@ struct SelectArgs {
   uint32_t* chunk_cnt;         // items over the threshold per chunk
   uint32_t* chunk_pos;         // exclusive prefix of chunk_cnt inside the segment
   const Piece* pieces;         // one-pass chain, or null: pieces of all tensors
-  uint32_t* run_cnt;           // [n_pieces][kPieceRuns] listed items | near misses << 16
+  uint32_t piece_shift;        // a piece is 1 << piece_shift runs (at most kMaxPieceRuns)
+  uint32_t* run_cnt;           // [n_pieces][1 << piece_shift] listed items | near misses << 16
   uint64_t* piece_cnt;         // [n_pieces] the same summed, low and high word (tensors of several pieces only)
   uint32_t* hist_top;          // [n_pieces][kHistBins] top-k: histograms of the candidates, see top_bin()
   uint32_t* hist_rest;          // [n_segs][kHistBins] top-k whose candidates fell short: histogram of the rest, see rest_bin()

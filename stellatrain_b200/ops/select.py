@@ -46,16 +46,7 @@ def _compress_cuda(name: str, flat: torch.Tensor, k: int, method: str):
         b = GpuBucket(0, layout, flat.device, compressor=method, ratio=1.0, world=1, rank=0, select_only=True)
         b.wire_local()
         _gpu_cache[key] = b
-    # one tensor, explicit k: patch the segment table
-    seg = b.layout.segments[0]
-    if seg.k != k:
-        seg.k, seg.out_off, b.layout.cap = k, 0, k
-        from ..parallel.gpu_bucket import _dev_bytes
-        b.segs.copy_(_dev_bytes(b.layout.seg_table(), flat.device))
-        b._bind()
-        if k > b.cap_max:           # room for the pairs of this call (every call has waited for its stream)
-            b.cap_max = k
-            b.wire_local()
+    b.set_entries(k)        # every call has waited for its stream
     return b.compress(flat)
 
 

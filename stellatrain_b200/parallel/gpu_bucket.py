@@ -141,19 +141,13 @@ class GpuBucket:
         self.segs = _dev_bytes(layout.seg_table(), device)
         self.state = torch.zeros(n_segs * B.SEG_STATE_DTYPE.itemsize, dtype=torch.uint8, device=device)
         self.work = torch.zeros(n_segs * B.SEG_WORK_WORDS, dtype=torch.int32, device=device)
-        self.chunks = _dev_bytes(layout.chunk_table(), device)
         self.chunk_cnt = torch.zeros(layout.n_chunks, dtype=torch.int32, device=device)
         self.chunk_pos = torch.zeros(layout.n_chunks, dtype=torch.int32, device=device)
         # One-pass select: it takes over once every tensor has a threshold, after the first select or (threshold
         # compressors) after a checkpoint that carries them.
         self.fused_select = bool(fused_select)
-        pieces = layout.piece_table()
-        self.n_pieces = len(pieces)
-        self.pieces = _dev_bytes(pieces, device)
-        self.run_cnt = torch.zeros(self.n_pieces * B.PIECE_RUNS, dtype=torch.int32, device=device)
-        self.piece_cnt = torch.zeros(self.n_pieces, dtype=torch.int64, device=device)
         one_pass_topk = compressor == "topk" and self.fused_select
-        self.hist_top = torch.zeros(self.n_pieces * 2048 if one_pass_topk else 1, dtype=torch.int32, device=device)
+        self._make_pieces()
         self.hist_rest = torch.zeros(n_segs * 2048 if one_pass_topk else 1, dtype=torch.int32, device=device)
         self.hist = torch.zeros(n_segs * 2048, dtype=torch.int32, device=device)
         # [select epoch, apply epoch, select CTAs done, apply CTAs done, tensors to refill (one-pass top-k), 3 spare]
@@ -187,6 +181,18 @@ class GpuBucket:
         self.grad_tab_dev: Optional[torch.Tensor] = None
         self._bind()
 
+    def _make_pieces(self) -> None:
+        """Tables of the streaming and emitting kernels' work, and the counters of the latter."""
+        L, i32 = self.layout, dict(dtype=torch.int32, device=self.device)
+        self._piece_runs = L.piece_runs
+        pieces = L.piece_table()
+        self.n_pieces = len(pieces)
+        self.chunks = _dev_bytes(L.chunk_table(), self.device)
+        self.pieces = _dev_bytes(pieces, self.device)
+        self.run_cnt = torch.zeros(self.n_pieces * self._piece_runs, **i32)
+        self.piece_cnt = torch.zeros(self.n_pieces, dtype=torch.int64, device=self.device)
+        self.hist_top = torch.zeros(self.n_pieces * 2048 if self.compressor == "topk" and self.fused_select else 1, **i32)
+
     # ------------------------------------------------------------------ wiring
     def _ptr(self, t: Optional[torch.Tensor]) -> int:
         return 0 if t is None else t.data_ptr()
@@ -209,7 +215,7 @@ class GpuBucket:
             hist=self.hist.data_ptr(), n_segs=len(L.segments), n_chunks=L.n_chunks, cap=L.cap,
             pieces=self.pieces.data_ptr(), run_cnt=self.run_cnt.data_ptr(), piece_cnt=self.piece_cnt.data_ptr(),
             hist_top=self.hist_top.data_ptr(), hist_rest=self.hist_rest.data_ptr(), refills=self.counters.data_ptr() + 16,
-            n_pieces=self.n_pieces,
+            n_pieces=self.n_pieces, piece_runs=self._piece_runs,
         )
         self.scratch.bind(h)
         h.set_control(
@@ -300,7 +306,23 @@ class GpuBucket:
             raise ValueError(f"ratio {ratio} is below the provisioned minimum {self.min_ratio}")
         self.ratio = ratio
         self.layout.set_ratio(ratio, self.k_world)
+        self._rebind_entries()
+
+    def set_entries(self, k: int) -> None:
+        """Entries of a bucket of one tensor; as `set_ratio`, and the receive area grows with them."""
+        seg = self.layout.segments[0]
+        if seg.k == k:
+            return
+        seg.k, seg.out_off, self.layout.cap = k, 0, k
+        self._rebind_entries()
+        if k > self.cap_max:
+            self.cap_max = k
+            self.wire_local()
+
+    def _rebind_entries(self) -> None:
         self.segs.copy_(_dev_bytes(self.layout.seg_table(), self.device))
+        if self.layout.piece_runs != self._piece_runs:
+            self._make_pieces()
         self._bind()
 
     def set_optimizer_options(self, **kw) -> None:

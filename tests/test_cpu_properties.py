@@ -200,13 +200,17 @@ def test_bundles_train_bit_for_bit_like_one_task_per_tensor(sizes, bundle_elems,
         assert torch.equal(a, b)
 
 
-@pytest.mark.parametrize("chunk", [1024, 8192, 1 << 18])
-def test_runs_and_pieces_of_the_one_pass_select_tile_every_tensor(chunk):
+@pytest.mark.parametrize("chunk,largest,ratio,piece_runs", [
+    (1024, 500_001, 0.99, 8), (8192, 500_001, 0.5, 8), (1 << 18, 500_001, 0.99, 8), (8192, 3_000_003, 0.99, 16),
+    (8192, 18_000_001, 0.99, 128), (1 << 18, 18_000_001, 0.97, 64), (1024, 18_000_001, 0.9, 32), (8192, 40_000_000, 0.5, 128)])
+def test_runs_and_pieces_of_the_one_pass_select_tile_every_tensor(chunk, largest, ratio, piece_runs):
     """Every element belongs to exactly one run, and a run found through its chunk has the place its piece gives it."""
     from stellatrain_b200.parallel import buckets as B
 
-    numels = [1, 16, 17, 1023, 1025, 131071, 131072, 131073, 500001]
+    numels = [1, 16, 17, 1023, 1025, 131071, 131072, 131073, largest]
     L = B.BucketLayout([str(i) for i in range(len(numels))], numels, chunk_elems=chunk)
+    L.set_ratio(ratio, 1)
+    assert L.piece_runs == piece_runs
     by_chunk, by_piece = {}, {}
     for c in L.chunk_table():
         for rel in range(0, int(c["len"]), B.RUN_ELEMS):
@@ -217,6 +221,6 @@ def test_runs_and_pieces_of_the_one_pass_select_tile_every_tensor(chunk):
     for p, row in enumerate(table):
         assert table[int(row["first"])]["index"] == 0 and p == int(row["first"]) + int(row["index"]) < int(row["first"]) + int(row["count"])
         for r in range(int(row["n_runs"])):
-            by_piece[p * B.PIECE_RUNS + r] = (int(row["seg"]), int(row["start"]) + r * B.RUN_ELEMS)
+            by_piece[p * L.piece_runs + r] = (int(row["seg"]), int(row["start"]) + r * B.RUN_ELEMS)
     assert by_chunk == by_piece
     assert sum(min(B.RUN_ELEMS, L.segments[s].off + L.segments[s].n_pad - at) for s, at in by_piece.values()) == L.n_total

@@ -105,15 +105,17 @@ def test_select_matches_oracle(compressor, mode, fused):
 
 @pytest.mark.parametrize("compressor", ["topk", "thresholdv", "thresholdv16"])
 @pytest.mark.parametrize("mode", ["steady", "jumps", "ties", "mostly_zero", "huge"])
-@pytest.mark.parametrize("ratio,chunk,narrow", [(0.99, 8192, False), (0.5, 1024, False), (0.999, 1 << 18, False),
-                                                (0.99, 8192, True), (0.5, 1024, True)])
-def test_one_pass_select_at_its_edges(compressor, mode, ratio, chunk, narrow):
-    """The one-pass chain against the plain rule at the edges of its runs (1024 elements), pieces (131072) and chunks:
+@pytest.mark.parametrize("ratio,chunk,narrow,piece_runs", [(0.99, 8192, False, 8), (0.5, 1024, False, 32), (0.999, 1 << 18, False, 128),
+                                                           (0.5, 8192, False, 128), (0.99, 8192, True, 128), (0.5, 1024, True, 8)])
+def test_one_pass_select_at_its_edges(compressor, mode, ratio, chunk, narrow, piece_runs, monkeypatch):
+    """The one-pass chain against the plain rule at the edges of its runs (1024 elements), pieces (of the named number of runs) and chunks:
     the same entries bit for bit.  "jumps" moves the gradient scale up and down by large factors, so that top-k's
     candidates fall short and the refill kernel selects; "mostly_zero" leaves fewer entries than the budget; "huge"
     holds values far outside the histogram window.  ``narrow``: tensors of fewer than 65536 elements send bf16 values and keep
     the rounding error."""
-    sizes = [1, 16, 1023, 1024, 1025, 8192, 9001, 65519, 131071, 131072, 131073, 400001]
+    sizes = [1, 16, 1023, 1024, 1025, 8192, 9001, 32769, 65519, 131071, 131072, 131073, 400001]
+    monkeypatch.setattr(B, "MIN_PIECE_RUNS", piece_runs)
+    monkeypatch.setattr(B, "MAX_PIECE_RUNS", piece_runs)
     gen = torch.Generator(device="cuda").manual_seed(99)
     b = make_bucket(compressor, ratio, sizes=sizes, chunk=chunk, narrow=narrow)
     resid_ref = torch.zeros_like(b.resid)
@@ -153,6 +155,32 @@ def test_one_pass_select_at_its_edges(compressor, mode, ratio, chunk, narrow):
     assert int(b.hist.abs().max()) == 0 and int(b.hist_top.abs().max()) == 0 and int(b.hist_rest.abs().max()) == 0 and int(b.piece_cnt.abs().max()) == 0
     work = b.work.view(len(sizes), B.SEG_WORK_WORDS)
     assert int(work[:, 4:6].abs().max()) == 0 and int(work[:, 10:].abs().max()) == 0 and int(b.counters[4]) == 0
+
+
+@pytest.mark.parametrize("compressor", ["topk", "thresholdv", "thresholdv16"])
+def test_a_ratio_change_cuts_the_bucket_anew(compressor):
+    """More entries want smaller pieces; thresholds and residuals stay."""
+    b = make_bucket(compressor, 0.995, sizes=[70001, 17_000_003], chunk=8192, min_ratio=0.9)
+    gen, resid_ref = torch.Generator(device="cuda").manual_seed(6), torch.zeros_like(b.resid)
+    cuts = []
+    for step, ratio in enumerate([0.995, 0.995, 0.9, 0.9, 0.97]):
+        if ratio != b.ratio:
+            b.set_ratio(ratio)
+        cuts.append(b.n_pieces)
+        fill_grads(b, gen)
+        grad, states = b.grad.clone(), oracle_states(b)
+        b.select()
+        torch.cuda.synchronize()
+        b.check_status()
+        idx_all, _ = b.stream_of((step + 1) & 1, 0)
+        for si, (s, sl, slp) in enumerate(seg_slices(b)):
+            own = slp if compressor == "thresholdv16" else sl
+            want, _, new_r = O.compress_step(compressor, grad[own], resid_ref[own], s.k, states[si], one_pass=step > 0)
+            got = idx_all[s.out_off : s.out_off + s.k]
+            assert torch.equal(got[got != -1].long().sort().values, want.sort().values + s.off), (step, s.name)
+            resid_ref[own] = new_r
+        assert torch.equal(b.resid, resid_ref), step
+    assert cuts[0] == cuts[1] < cuts[4] < cuts[2] == cuts[3]
 
 
 @pytest.mark.parametrize("compressor", ["topk", "thresholdv", "thresholdv16", "randomk"])
