@@ -352,7 +352,7 @@ struct EmitShared {
   uint32_t res[4];
   uint32_t cnt[64];                 // counts of the bitwise searches
   uint32_t word[4];                 // [0] may emit, [1] last CTA of the tensor, [2], [3] bases of a batch
-  unsigned long long sum[2];        // [0] totals of the tensor
+  unsigned long long sum;           // listed items | near misses << 32 of the tensor
   uint32_t at[2];                   // piece of the tensor that holds a position, positions in front of it
 };
 
@@ -639,6 +639,144 @@ __device__ __forceinline__ uint32_t top_direct(const SelectArgs& A, const Job& J
   return cut.x;
 }
 
+// The same for more pairs than registers hold: a radix search over the bits that the keys of `cand` leave open, 11 at a time.
+// Fixed digits of the whole key put nearly all pairs, which lie close together, on one counter: 25,000 adds to one address of
+// shared memory took longer than all passes over the pairs.  Ids lie in [id_lo, id_lo + n_ids).
+__device__ __forceinline__ uint2 cut_of_many(const uint2* cand, uint32_t c, uint32_t take, uint32_t id_lo, uint32_t n_ids,
+                                             EmitShared& S) {
+  constexpr int kIlp = 8;              // independent loads in flight per thread
+  constexpr uint32_t kDigit = 11u;
+  const uint32_t tid = threadIdx.x;
+  auto each = [&](auto f) {
+    for (uint32_t i0 = tid; i0 < c; i0 += kEmitThreads * kIlp) {
+      uint2 e[kIlp];
+#pragma unroll
+      for (int u = 0; u < kIlp; ++u) e[u] = i0 + u * kEmitThreads < c ? __ldcg(cand + i0 + u * kEmitThreads) : make_uint2(0u, 0u);
+#pragma unroll
+      for (int u = 0; u < kIlp; ++u)
+        if (i0 + u * kEmitThreads < c) f(e[u]);
+    }
+  };
+  // The digit of the rem-th value, counted from the largest (`down`) or the smallest one: S.res = {digit, values still to be
+  // taken among those that have it, their number}.
+  auto pick_digit = [&](uint32_t n_bins, uint32_t rem, bool down) {
+    constexpr int kPer = (1 << kDigit) / kEmitThreads;
+    uint32_t h[kPer], local = 0;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const uint32_t d = kPer * tid + j;
+      h[j] = d < n_bins ? S.hist[down ? n_bins - 1u - d : d] : 0u;
+      local += h[j];
+    }
+    uint32_t total;
+    uint32_t ex = block_excl_scan(local, S.tmp, total);
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const uint32_t d = kPer * tid + j;
+      if (ex < rem && ex + h[j] >= rem) { S.res[0] = down ? n_bins - 1u - d : d; S.res[1] = rem - ex; S.res[2] = h[j]; }
+      ex += h[j];
+    }
+    __syncthreads();
+  };
+  uint32_t mn = 0xFFFFFFFFu, mx = 0;
+  each([&](const uint2& e) { mn = min(mn, e.y); mx = max(mx, e.y); });
+  mn = ~block_max_u32(~mn, S.tmp);
+  mx = block_max_u32(mx, S.tmp);
+  uint32_t t = 0, rem = take, ties = c;
+  for (uint32_t open = 32u - __clz(mx - mn); open != 0u;) {
+    const uint32_t w = min(open, kDigit), shift = open - w, n_bins = 1u << w;
+    for (uint32_t b = tid; b < n_bins; b += kEmitThreads) S.hist[b] = 0u;
+    __syncthreads();
+    each([&](const uint2& e) {
+      const uint32_t v = e.y - mn;
+      if (v >> open == t) atomicAdd(&S.hist[v >> shift & (n_bins - 1u)], 1u);
+    });
+    __syncthreads();
+    pick_digit(n_bins, rem, true);
+    t = t << w | S.res[0];
+    rem = S.res[1];
+    ties = S.res[2];
+    open = shift;
+    __syncthreads();
+  }
+  const uint32_t key = mn + t;
+  if (rem == ties) {      // all pairs of this key: the highest id among them
+    uint32_t last = 0;
+    each([&](const uint2& e) { if (e.y == key) last = max(last, e.x); });
+    return make_uint2(key, block_max_u32(last, S.tmp));
+  }
+  uint32_t id = 0;        // the rem-th smallest id
+  for (uint32_t open = 32u - __clz(n_ids); open != 0u;) {
+    const uint32_t w = min(open, kDigit), shift = open - w, n_bins = 1u << w;
+    for (uint32_t b = tid; b < n_bins; b += kEmitThreads) S.hist[b] = 0u;
+    __syncthreads();
+    each([&](const uint2& e) {
+      const uint32_t v = e.x - id_lo;
+      if (e.y == key && v >> open == id) atomicAdd(&S.hist[v >> shift & (n_bins - 1u)], 1u);
+    });
+    __syncthreads();
+    pick_digit(n_bins, rem, false);
+    id = id << w | S.res[0];
+    rem = S.res[1];
+    open = shift;
+    __syncthreads();
+  }
+  return make_uint2(key, id_lo + id);
+}
+
+// Last CTA of a tensor, c > kPickMax candidates: sends the best `take` of them behind the `done` items that are in the stream,
+// the lowest-ranked one last.  Returns its key.  `list` is the area of the tensor's lists, which nobody reads any more.  Ranked
+// by one CTA of 1024 threads, which drew a stream position per item from one address and copied a block with one thread,
+// this took up to 0.1 ms for the 25,000 undecided items of a 64 MB bucket whose gradients had changed in scale.
+template <bool kBlock>
+__device__ __forceinline__ uint32_t send_best(const SelectArgs& A, const Job& J, EmitShared& S, const uint2* cand, uint32_t c,
+                                              uint32_t take, uint32_t done, uint2* list) {
+  constexpr uint32_t kPerItem = kBlock ? 16u : 1u;
+  constexpr int kIlp = kStageItems / kEmitThreads;
+  const uint32_t tid = threadIdx.x;
+  const uint2 cut = cut_of_many(cand, c, take, kBlock ? J.sd.off >> 4 : J.sd.off, kBlock ? J.sd.n_pad >> 4 : J.sd.n_pad, S);
+  uint32_t base = 0;
+  for (uint32_t i0 = 0; i0 < c; i0 += kStageItems) {
+    uint32_t id[kIlp], taken = 0;
+#pragma unroll
+    for (int u = 0; u < kIlp; ++u) {
+      const uint32_t i = i0 + u * kEmitThreads + tid;
+      const uint2 e = i < c ? __ldcg(cand + i) : make_uint2(0xFFFFFFFFu, 0u);
+      id[u] = e.x;
+      const bool is_last = e.y == cut.x && e.x == cut.y;
+      if (is_last) list[take - 1u].x = e.x;
+      taken |= (uint32_t)(i < c && !is_last && (e.y > cut.x || (e.y == cut.x && e.x < cut.y))) << u;
+    }
+    uint32_t n;
+    uint32_t at = base + block_excl_scan(__popc(taken), S.tmp, n);
+#pragma unroll
+    for (int u = 0; u < kIlp; ++u)
+      if (taken >> u & 1u) list[at++].x = id[u];
+    base += n;
+  }
+  __syncthreads();
+  uint2* const stage = S.stage;
+  for (uint32_t t0 = 0; t0 < take * kPerItem; t0 += kStageItems) {
+#pragma unroll
+    for (int u = 0; u < kIlp; ++u) {
+      const uint32_t t = t0 + u * kEmitThreads + tid;
+      uint2 e = make_uint2(0u, 0u);
+      if (t < take * kPerItem) {
+        e.x = __ldcg(&list[t / kPerItem].x) * kPerItem + t % kPerItem;
+        e.y = __float_as_uint(__ldcg(A.resid + e.x));
+      }
+      stage[u * kEmitThreads + tid] = e;
+    }
+    __syncthreads();
+    const uint32_t p0 = done * kPerItem + t0;      // the last block may be cut off at k
+    const uint32_t m = min(min(kStageItems, take * kPerItem - t0), J.sd.k > p0 ? J.sd.k - p0 : 0u);
+#pragma unroll 1
+    for (uint32_t q = tid; q < m; q += kEmitThreads) emit_and_keep(A, J, p0 + q, stage[q].x, __uint_as_float(stage[q].y));
+    __syncthreads();
+  }
+  return cut.x;
+}
+
 // Top-k, last CTA of a tensor: the best `rem` of the `c` undecided items complete the stream.  Returns the k-th largest key.
 __device__ __forceinline__ uint32_t settle_top(const SelectArgs& A, const Job& J, EmitShared& S, const uint2* undecided,
                                                uint32_t c, uint32_t rem, uint32_t key_lo, uint32_t key_hi) {
@@ -652,10 +790,7 @@ __device__ __forceinline__ uint32_t settle_top(const SelectArgs& A, const Job& J
     }
     return t_key;
   }
-  if (threadIdx.x == 0) J.wp->out_cursor = done;
-  __syncthreads();
-  return take_top<kEmitThreads>(A, J.sd, J.wp, undecided, c, rem, false, J.kk, J.kk - 1u, J.slot_off, J.dest, J.nb, S.hist,
-                                S.tmp, S.res);
+  return send_best<false>(A, J, S, undecided, c, rem, done, A.cand + J.sd.off);
 }
 
 // Sends the items [j0, j1) of one piece at positions base + j; items and positions are in index order.  The dependent loads
@@ -782,7 +917,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(SelectArgs A) {
     unsigned long long all = 0ull;
     if (J.pc.count > 1u)
       for (uint32_t t = tid; t < J.pc.count; t += kEmitThreads) all += A.piece_cnt[J.pc.first + t];
-    if (tid < 2) S.sum[tid] = 0ull;
+    if (tid == 0) S.sum = 0ull;
     uint32_t total, near_total = 0;
     uint32_t ex = block_excl_scan(cnt & 0xffffu, S.tmp, total);
     if (tid <= kMaxPieceRuns) S.pre[tid] = ex;
@@ -794,10 +929,10 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(SelectArgs A) {
     if (J.pc.count > 1u) {
 #pragma unroll
       for (int d = 16; d > 0; d >>= 1) all += __shfl_xor_sync(0xffffffffu, all, d);
-      if ((tid & 31u) == 0u && all) atomicAdd(&S.sum[0], all);
+      if ((tid & 31u) == 0u && all) atomicAdd(&S.sum, all);
       __syncthreads();
-      found = (uint32_t)S.sum[0];
-      c_near = (uint32_t)(S.sum[0] >> 32);
+      found = (uint32_t)S.sum;
+      c_near = (uint32_t)(S.sum >> 32);
     }
     const bool short_of = found < J.kk;
     // will this CTA store into the destinations?  Then they must have consumed the slot.
@@ -961,10 +1096,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(SelectArgs A) {
               }
             }
           } else if (take) {
-            if (tid == 0) J.wp->out_cursor = found;
-            __syncthreads();
-            t_key = take_top<kEmitThreads>(A, J.sd, J.wp, nears, c, take, true, J.kk, found + take - 1u, J.slot_off, J.dest,
-                                           J.nb, S.hist, S.tmp, S.res);
+            t_key = send_best<true>(A, J, S, nears, c, take, found, A.cand + (J.sd.off >> 4));
           }
           // fewer blocks with anything in them than the budget: the rest of the stream says "no entry"
 #pragma unroll 1

@@ -561,6 +561,130 @@ __global__ void __launch_bounds__(kThreads, 4) k_pass2(SelectArgs A) {
 // ------------------------------------------------------------------------------------------------
 constexpr int kCandThreads = 1024;
 
+// Called by a whole CTA.  Among cand[0..c) takes the `rem` largest keys (equal keys: lowest
+// item id first; 1 <= rem <= c) and emits them: stream positions come from wp->out_cursor, except that the
+// lowest-ranked taken block of threshold-v16 goes to `last_pos`, where it may be cut off at sd.k.  Returns the key
+// of the lowest-ranked taken item.  s_hist: 2048 words, s_tmp: kCandThreads / 32 + 1 words, s_res: 4 words.
+__device__ __forceinline__ uint32_t take_top(const SelectArgs& A, const SegDesc& sd, SegWork* wp, const uint2* cand,
+                                             uint32_t c, uint32_t rem, bool b16, uint32_t kk, uint32_t last_pos,
+                                             uint64_t slot_off, int dest, uint32_t nb, uint32_t* s_hist,
+                                             uint32_t* s_tmp, uint32_t* s_res) {
+  constexpr int kIlp = 4;              // independent loads in flight per thread
+  constexpr int T = kCandThreads;
+  constexpr int kPer = 2048 / T;       // bins per thread, descending from the highest
+  const uint32_t tid = threadIdx.x;
+  uint32_t ties = 0;
+  uint32_t prefix = 0, mask = 0;
+  // radix select over the full 31-bit key, largest first: digits of 11, 11 and 9 bits
+  const int shifts[3] = {20, 9, 0};
+  const uint32_t widths[3] = {2048u, 2048u, 512u};
+  for (int pass = 0; pass < 3; ++pass) {
+    const int shift = shifts[pass];
+    const uint32_t nbins = widths[pass];
+    for (uint32_t b = tid; b < nbins; b += T) s_hist[b] = 0;
+    __syncthreads();
+    for (uint32_t i0 = tid; i0 < c; i0 += T * kIlp) {
+      uint32_t key[kIlp];
+#pragma unroll
+      for (int u = 0; u < kIlp; ++u) {
+        const uint32_t i = i0 + u * T;
+        key[u] = i < c ? __ldcg(&cand[i].y) : 0xFFFFFFFFu;
+      }
+#pragma unroll
+      for (int u = 0; u < kIlp; ++u)
+        if (key[u] != 0xFFFFFFFFu && (key[u] & mask) == prefix) atomicAdd(&s_hist[(key[u] >> shift) & (nbins - 1)], 1u);
+    }
+    __syncthreads();
+    uint32_t h[kPer], local = 0;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const uint32_t d = kPer * tid + j;
+      h[j] = d < nbins ? s_hist[nbins - 1 - d] : 0u;
+      local += h[j];
+    }
+    uint32_t total;
+    uint32_t ex = block_excl_scan(local, s_tmp, total);
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      if (ex < rem && ex + h[j] >= rem) {
+        s_res[0] = nbins - 1 - (kPer * tid + j); s_res[1] = rem - ex; s_res[2] = h[j];
+      }
+      ex += h[j];
+    }
+    __syncthreads();
+    prefix |= s_res[0] << shift;
+    mask |= (nbins - 1) << shift;
+    rem = s_res[1];
+    ties = s_res[2];
+    __syncthreads();
+  }
+  const uint32_t t_key = prefix;
+  // among equal keys take the lowest item ids: radix select on the id, smallest first
+  uint32_t id_thr = 0xFFFFFFFFu;
+  if (rem < ties) {
+    uint32_t ipre = 0, imask = 0, irem = rem;
+    for (int pass = 0; pass < 4; ++pass) {
+      const int shift = 24 - 8 * pass;
+      for (uint32_t b = tid; b < 256; b += T) s_hist[b] = 0;
+      __syncthreads();
+      for (uint32_t i = tid; i < c; i += T) {
+        const uint2 e = __ldcg(cand + i);
+        if (e.y == t_key && (e.x & imask) == ipre) atomicAdd(&s_hist[(e.x >> shift) & 255u], 1u);
+      }
+      __syncthreads();
+      const uint32_t h = tid < 256 ? s_hist[tid] : 0u;
+      uint32_t total;
+      const uint32_t ex = block_excl_scan(h, s_tmp, total);
+      if (tid < 256 && ex < irem && ex + h >= irem) { s_res[0] = tid; s_res[1] = irem - ex; }
+      __syncthreads();
+      ipre |= s_res[0] << shift;
+      imask |= 255u << shift;
+      irem = s_res[1];
+      __syncthreads();
+    }
+    id_thr = ipre;
+  }
+  // threshold-v16: the lowest-ranked taken block goes last and may be truncated
+  uint32_t last_id = id_thr;
+  if (b16 && rem >= ties) {
+    uint32_t mxid = 0;
+    for (uint32_t i = tid; i < c; i += T) {
+      const uint2 e = __ldcg(cand + i);
+      if (e.y == t_key) mxid = max(mxid, e.x);
+    }
+    last_id = block_max_u32(mxid, s_tmp);
+  }
+#pragma unroll 1
+  for (uint32_t i = tid; i < c; i += T) {
+    const uint2 e = __ldcg(cand + i);
+    const bool take = e.y > t_key || (e.y == t_key && e.x <= id_thr);
+    if (!take) continue;
+    if (!b16) {
+      const uint32_t pos = atomicAdd(&wp->out_cursor, 1u);
+      if (pos < kk) {
+        const float a = __ldcg(A.resid + e.x), sv = wire_value(nb, a);
+        emit_entry(A, dest, nb, slot_off, pos, e.x, sv);
+        A.resid[e.x] = a - sv;
+      }
+    } else {
+      const bool is_last = (e.y == t_key && e.x == last_id);
+      const uint32_t pos = is_last ? last_pos : atomicAdd(&wp->out_cursor, 1u);
+      if (pos < kk) {
+        const uint32_t base = e.x * 16u;
+#pragma unroll 1
+        for (uint32_t j = 0; j < 16u; ++j) {
+          if (pos * 16u + j < sd.k) {
+            const float a = __ldcg(A.resid + base + j), sv = wire_value(nb, a);
+            emit_entry(A, dest, nb, slot_off, pos * 16u + j, base + j, sv);
+            A.resid[base + j] = a - sv;
+          }
+        }
+      }
+    }
+  }
+  return t_key;
+}
+
 __global__ void __launch_bounds__(kCandThreads) k_cand(SelectArgs A) {
   __shared__ uint32_t s_hist[2048];
   __shared__ uint32_t s_tmp[kCandThreads / 32 + 1];
@@ -580,7 +704,7 @@ __global__ void __launch_bounds__(kCandThreads) k_cand(SelectArgs A) {
   const uint32_t mode = wp->mode;
 
   if (ok && mode == kModeTop) {
-    const uint32_t t_key = take_top<kCandThreads>(A, sd, wp, A.cand + wp->cand_off, wp->cand_cnt, wp->k_rem, b16, kk, kk - 1u, slot_off,
+    const uint32_t t_key = take_top(A, sd, wp, A.cand + wp->cand_off, wp->cand_cnt, wp->k_rem, b16, kk, kk - 1u, slot_off,
                                     dest, nb, s_hist, s_tmp, s_res);
     if (tid == 0) {
       SegState ss = A.state[seg];
