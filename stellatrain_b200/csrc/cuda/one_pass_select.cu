@@ -63,17 +63,21 @@ __device__ __forceinline__ uint32_t top_cut(const SegState& ss, uint32_t n_pad) 
   return cut ? cut : 1u;
 }
 
-// Histogram of top-k's candidates around the previous threshold c (float bits), three widths of bins: 1024 of 2^-17
-// (relative) within 0.4 % of it, 256 of 2^-13 on either side as far as 3 %, 128 of 2^-7 on either side as far as an octave,
-// 128 of an eighth of an octave each beyond (gradients that jump up), the rest in the end bins.  Error feedback piles items up at the threshold: with bins of 2^-10 throughout a few of
-// them took most of the counts (L2 adds to one address one after the other: 239 us for a scan of 38.6 M elements, of
-// which the traffic needs 75) and the threshold's bin held thousands of undecided items.
+// Histogram of top-k's candidates around the previous threshold c (float bits), widths of bins that grow with the distance, on
+// either side 256 of 2^-16 (relative) as far as 0.4 %, 128 of 2^-12 as far as 3 %, 512 of 2^-9 as far as an octave, 128 of an
+// eighth of an octave each beyond (gradients that jump up), the rest in the end bins.  Error feedback piles items up at the
+// threshold: with bins of 2^-10 throughout a few of them took most of the counts (L2 adds to one address one after the other:
+// 239 us for a scan of 38.6 M elements, of which the traffic needs 75) and the threshold's bin held thousands of undecided
+// items.  A batch whose norm differs puts the threshold far from c: with bins of 2^-7 there, 25,000 of a 64 MB bucket's items
+// were undecided at 10 % kept.
 // c = 0 stands for "no usable threshold": 2048 even bins over all keys.
 // A tensor of several pieces spreads its counts over up to eight such histograms (one per piece modulo their number): 500,000
 // adds into the 64 cache lines of a single one still took 60 us longer than the traffic.
-constexpr int kNearShift = 6, kMidShift = 10, kFarShift = 16, kBeyondShift = 20;
-constexpr uint32_t kNear = 512u << kNearShift, kMid = kNear + (256u << kMidShift);     // distances where the widths change
-constexpr uint32_t kFar = kMid + (128u << kFarShift);
+constexpr int kNearShift = 7, kMidShift = 11, kFarShift = 14, kBeyondShift = 20;
+constexpr uint32_t kNearBins = 256u, kMidBins = 128u, kFarBins = 512u;
+constexpr uint32_t kMidFrom = kNearBins, kFarFrom = kMidFrom + kMidBins, kBeyondFrom = kFarFrom + kFarBins;      // of 1024 bins a side
+constexpr uint32_t kNear = kNearBins << kNearShift, kMid = kNear + (kMidBins << kMidShift);     // distances where the widths change
+constexpr uint32_t kFar = kMid + (kFarBins << kFarShift);
 
 __device__ __forceinline__ uint32_t top_centre(const SegState& ss) {
   return ss.reserved[1] >= (1u << 24) ? ss.reserved[1] : 0u;      // all bins under it fit
@@ -116,9 +120,9 @@ __device__ __forceinline__ uint32_t top_bin(uint32_t key, uint32_t c) {
   const bool above = key >= c;
   const uint32_t d = above ? key - c : c - key - 1u;
   const uint32_t b = d < kNear  ? d >> kNearShift
-                     : d < kMid ? 512u + ((d - kNear) >> kMidShift)
-                     : d < kFar ? 768u + ((d - kMid) >> kFarShift)
-                                : min(1023u, 896u + ((d - kFar) >> kBeyondShift));
+                     : d < kMid ? kMidFrom + ((d - kNear) >> kMidShift)
+                     : d < kFar ? kFarFrom + ((d - kMid) >> kFarShift)
+                                : min(1023u, kBeyondFrom + ((d - kFar) >> kBeyondShift));
   return above ? 1024u + b : 1023u - b;
 }
 
@@ -131,11 +135,11 @@ __device__ __forceinline__ void top_bin_range(uint32_t bin, uint32_t c, uint32_t
   }
   const bool above = bin >= 1024u;
   const uint32_t b = above ? bin - 1024u : 1023u - bin;
-  const int shift = b < 512u ? kNearShift : b < 768u ? kMidShift : b < 896u ? kFarShift : kBeyondShift;
-  const uint32_t from = b < 512u   ? b << kNearShift
-                        : b < 768u ? kNear + ((b - 512u) << kMidShift)
-                        : b < 896u ? kMid + ((b - 768u) << kFarShift)
-                                   : kFar + ((b - 896u) << kBeyondShift);
+  const int shift = b < kMidFrom ? kNearShift : b < kFarFrom ? kMidShift : b < kBeyondFrom ? kFarShift : kBeyondShift;
+  const uint32_t from = b < kMidFrom      ? b << kNearShift
+                        : b < kFarFrom    ? kNear + ((b - kMidFrom) << kMidShift)
+                        : b < kBeyondFrom ? kMid + ((b - kFarFrom) << kFarShift)
+                                          : kFar + ((b - kBeyondFrom) << kBeyondShift);
   const uint32_t to = from + (1u << shift);          // distances [from, to)
   if (above) {
     lo = min(c + from, 0x80000000u);
