@@ -708,14 +708,19 @@ def main() -> None:
     # The sparse path inside the step, from the device-clock stamps that the kernels of the last step wrote themselves:
     # select + push and scatter + apply of every bucket, and the select chain against the memory roofline at the measured
     # copy bandwidth.  Bytes per element: the one-pass chain reads gradient and residual and writes the residual (12), the
-    # two-pass chain reads the residual once more (16); 4 more where the consumed gradients are zeroed ("flat" gradient
-    # mode).  In the step these kernels share the GPU with the backward pass, so the fraction is a lower bound of what the
-    # kernels reach alone (profiles/ has those numbers).  Never allowed to break the result line.
+    # four-kernel chain reads the residual once more (16); 4 more where the consumed gradients are zeroed ("flat" gradient
+    # mode).  With one rank the chains of consecutive buckets overlap on two streams, so times are those during which some
+    # bucket was in the stage and not sums over buckets.  In the step these kernels share the GPU with the backward pass and
+    # with one another's updates, so the fraction is a lower bound of what the kernels reach alone (profiles/ has those
+    # numbers).  Never allowed to break the result line.
     sparse_path = None
     if engine is not None:
         try:
+            from stellatrain_b200.utils.stats import covered_ms
+
             rows = engine.device_timeline()
-            sel, app = sum(r["select_ms"] for r in rows), sum(r["apply_ms"] for r in rows)
+            sel_spans, app_spans = [r["select_span_ns"] for r in rows], [r["apply_span_ns"] for r in rows]
+            sel, app, both = covered_ms(sel_spans), covered_ms(app_spans), covered_ms(sel_spans + app_spans)
             hbm_gbs, peaks_src = 6650.0, "fallback"
             peaks_file = os.path.join(os.path.dirname(os.path.abspath(__file__)), "MEASURED_PEAKS.json")
             if os.path.exists(peaks_file):
@@ -724,8 +729,8 @@ def main() -> None:
             one_pass = all(getattr(rt.bucket, "last_select_fused", False) for rt in engine.buckets)
             per_elem = (12 if one_pass else 16) + (4 if engine.cfg.grad_mode == "flat" else 0)
             sparse_path = {"buckets": len(rows), "select_push_ms": sel, "scatter_apply_ms": app,
-                           "share_of_step": (sel + app) / per_step if per_step > 0 else None,
-                           "select_chain": "one-pass" if one_pass else "two-pass", "select_bytes_per_element": per_elem,
+                           "share_of_step": both / per_step if per_step > 0 else None,
+                           "select_chain": "one-pass" if one_pass else "four-kernel", "select_bytes_per_element": per_elem,
                            "select_bytes": per_elem * n_params,
                            "select_fraction_of_copy_bandwidth": (per_elem * n_params / (sel * 1e-3) / (hbm_gbs * 1e9)) if sel > 0 else None,
                            "copy_bandwidth_gbs": hbm_gbs, "of": peaks_src,

@@ -391,10 +391,11 @@ class GpuBucket:
 
     def device_times(self) -> dict:
         """Device-clock view of the latest select and apply of this bucket, in milliseconds (blocking read):
-        how long select + push took, how long the apply ran, and for which epochs the numbers stand."""
+        how long select + push took, how long the apply ran, and for which epochs the numbers stand; the spans are on the
+        clock that all buckets share (chains of consecutive buckets may overlap)."""
         t = self.stamps.cpu().tolist()
         return {"select_ms": max(0, t[1] - t[0]) / 1e6, "apply_ms": max(0, t[3] - t[2]) / 1e6,
-                "select_epoch": t[4], "apply_epoch": t[5],
+                "select_span_ns": (t[0], t[1]), "apply_span_ns": (t[2], t[3]), "select_epoch": t[4], "apply_epoch": t[5],
                 "select_end_to_apply_start_ms": (t[2] - t[1]) / 1e6 if t[4] == t[5] else None}
 
     def check_status(self) -> None:

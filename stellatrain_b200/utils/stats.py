@@ -15,9 +15,21 @@ import json
 import os
 import time
 from collections import OrderedDict, deque
-from typing import Deque, Dict, Optional, Tuple
+from typing import Deque, Dict, Iterable, Optional, Tuple
 
 import torch
+
+
+def covered_ms(spans_ns: Iterable[Tuple[int, int]]) -> float:
+    """Milliseconds that lie in at least one of the (begin, end) spans; a span that ends before it begins counts as empty."""
+    total, reached = 0, None
+    for begin, end in sorted(spans_ns):
+        if reached is not None:
+            begin = max(begin, reached)
+        if end > begin:
+            total += end - begin
+            reached = end
+    return total / 1e6
 
 
 @contextlib.contextmanager

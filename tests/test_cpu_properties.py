@@ -224,3 +224,12 @@ def test_runs_and_pieces_of_the_one_pass_select_tile_every_tensor(chunk, largest
             by_piece[p * L.piece_runs + r] = (int(row["seg"]), int(row["start"]) + r * B.RUN_ELEMS)
     assert by_chunk == by_piece
     assert sum(min(B.RUN_ELEMS, L.segments[s].off + L.segments[s].n_pad - at) for s, at in by_piece.values()) == L.n_total
+
+
+@pytest.mark.parametrize("spans,ms", [
+    ([], 0.0), ([(5, 5), (9, 3)], 0.0), ([(0, 2_000_000)], 2.0), ([(0, 2_000_000), (1_000_000, 3_000_000)], 3.0),
+    ([(4_000_000, 5_000_000), (0, 3_000_000), (1_000_000, 2_000_000), (3_000_000, 3_500_000)], 4.5)])
+def test_time_covered_by_overlapping_spans(spans, ms):
+    from stellatrain_b200.utils.stats import covered_ms
+
+    assert covered_ms(spans) == ms
