@@ -1228,9 +1228,10 @@ __global__ void __launch_bounds__(kEmitThreads, 2) k_refill(SelectArgs A) {
 // host launchers
 // ------------------------------------------------------------------------------------------------
 bool one_pass_possible(const SelectArgs& A) {
-  // list positions and counts are 32-bit, top-k keeps its undecided items behind the lists (2 n slots)
-  return A.compressor != kRandomk && A.pieces != nullptr && A.n_total < (1u << 30) &&
-         (A.compressor != kTopk || (uint64_t)A.cand_cap >= 2ull * A.n_total);
+  // list positions and counts are 32-bit; behind the lists, of one slot per item, lie as many slots for top-k's undecided
+  // items and for the candidates of threshold-v16's fill
+  const uint64_t slots = A.compressor == kTopk ? 2ull * A.n_total : A.compressor == kThresholdv16 ? A.n_total / 8u : A.n_total;
+  return A.compressor != kRandomk && A.pieces != nullptr && A.n_total < (1u << 30) && A.cand_cap >= slots;
 }
 
 cudaError_t launch_select_one_pass(const SelectArgs& A, cudaStream_t stream) {

@@ -167,8 +167,7 @@ class GpuBucket:
         self._opt_host = opt
         self.opt = _dev_bytes(opt, device)
         self.scratch = scratch if scratch is not None else CandidateScratch(device)
-        # lists of the one-pass chain: a slot per element; top-k keeps its undecided items behind them
-        self.scratch.reserve(2 * n if one_pass_topk and n < 1 << 30 else n)
+        self.scratch.reserve(self._scratch_items(n))
         self.handle = _ext().BucketHandle()
         self.wiring: Optional[Wiring] = None
         # library-collective baseline: a second handle whose only destination is a local send buffer
@@ -180,6 +179,15 @@ class GpuBucket:
         self.grad_tab_host: Optional[torch.Tensor] = None
         self.grad_tab_dev: Optional[torch.Tensor] = None
         self._bind()
+
+    def _scratch_items(self, n: int) -> int:
+        """Candidate slots a select of n elements can need.  The one-pass chain keeps a list slot per item, and behind the
+        lists top-k its undecided items, threshold-v16 (whose items are blocks of 16) the candidates of its fill."""
+        if self.compressor == "thresholdv16":
+            return n // 8
+        if self.compressor == "topk" and self.fused_select and n < 1 << 30:
+            return 2 * n
+        return n if self.compressor != "randomk" else B.ALIGN
 
     def _make_pieces(self) -> None:
         """Tables of the streaming and emitting kernels' work, and the counters of the latter."""
@@ -474,8 +482,8 @@ class GpuBucket:
 
 
 class CandidateScratch:
-    """Scratch for the lists and undecided items of a select, shared by all buckets that run their selects on one
-    stream (worst case: every item of the largest bucket)."""
+    """Scratch for the lists and undecided items of a select, 8 bytes each, shared by all buckets that run their selects
+    on one stream (worst case: every item of the largest bucket)."""
 
     def __init__(self, device: torch.device) -> None:
         self.device = device
