@@ -50,12 +50,10 @@ def fill_grads(b, gen, scale=1e-2, mode="normal"):
 @pytest.mark.parametrize("mode", ["normal", "ties", "zero", "shrinking"])
 @pytest.mark.parametrize("fused", [True, False])
 def test_select_matches_oracle(compressor, mode, fused):
-    """Bit-equal streams, residuals and thresholds against the plain-PyTorch rule, for the two-pass chain and
-    for the one-pass chain that takes over once a threshold compressor has its thresholds.  "shrinking" halves
-    the gradient scale every step, so the threshold is far too high and the one-pass chain has to complete
-    the stream from a scan of the tensor."""
-    if compressor == "topk" and fused:
-        pytest.skip("top-k has no persistent threshold: always the two-pass chain")
+    """Bit-equal entries, residuals and thresholds against the plain-PyTorch rule, for the four-kernel chain and for the
+    one-pass chain that takes over once every tensor has been through one select.  "shrinking" halves the gradient scale
+    every step, so the threshold (top-k: the cut under the previous one) is far too high and the one-pass chain has to
+    complete the stream from the whole tensor; "zero" leaves top-k a previous threshold of zero."""
     torch.manual_seed(0)
     gen = torch.Generator(device="cuda").manual_seed(1234)
     b = make_bucket(compressor, 0.99, fused_select=fused)
