@@ -206,8 +206,8 @@ struct BucketHandle : public st::BucketHandle {
     check(st::BucketHandle::group_reduce(as_ptr<CUstream_st>(stream)), "launch_group_reduce");
   }
 
-  // The one-pass chain of the threshold compressors runs when it is enabled, possible for this bucket and every
-  // tensor has its threshold; otherwise the four-kernel chain.
+  // The one-pass chain runs when it is enabled, possible for this bucket (not random-k) and every tensor has its threshold
+  // (top-k: has been through one select); otherwise the four-kernel chain, or the two kernels of random-k.
   void py_select(uint64_t stream) {
     check(st::BucketHandle::select(as_ptr<CUstream_st>(stream)), "launch_select");
   }

@@ -16,7 +16,10 @@
 //   refill  top-k only: tensors whose candidates fell short of k (the distribution dropped below the cut) are selected
 //           from r itself.  Their histogram was taken by `emit`; with no such tensor this kernel returns at once.
 // 12 bytes per element cross HBM (read g, read r, write r) against 16 to 20 of the four-kernel chain, which remains for a
-// tensor's first select.  The results are those of the four-kernel chain; only the order of a top-k stream differs.
+// tensor's first select.  The entries are those of the four-kernel chain, with one exception: a threshold-v16 block that holds
+// nothing is never sent, and a tensor with fewer blocks that hold something than its budget says "no entry" for the rest.  The
+// order differs: top-k's entries come as its pieces get to them, and a threshold-v16 stream that is short of blocks over the
+// threshold has those first, in index order, and the fill behind them.
 //
 // What bounds it, 64 MB bucket (16.8 M elements, 201 MB of traffic, 31 us at the 6.5 TB/s of a plain copy), one B200:
 //   scan    memory: 35.5 us for threshold-v16, 36 us for top-k at 0.1 %, 39 us at 1 % (list and histogram).  Runs of one
@@ -284,23 +287,17 @@ __global__ void __launch_bounds__(kScanThreads, 4) k_scan(SelectArgs A) {
           before += (all >> (8 * j)) & 0xFFu;
         }
         __syncwarp();
-        // Histogram of the candidates.  The top bin, which holds many of them, is not counted: `emit` knows their number.
-        const uint32_t centre = top_centre(ss);
-        const uint32_t piece = seg_rel >> piece_shift;      // of the tensor
-        const uint32_t first_piece = ((ch.run0 + rel / kRunElems) >> A.piece_shift) - piece;
-        uint32_t* const gh = A.hist_top + (size_t)(first_piece + (piece & (hist_copies(sd.n_pad) - 1u))) * kHistBins;
-        for (uint32_t q0 = 0; q0 < n_half; q0 += 32u) {
-          const uint32_t q = q0 + lane;
-          uint32_t b = kHistBins - 1;
-          if (q < n_half) {
-            const uint2 e = first[q];
-            if (n_half <= kStage) dst[q] = e;
-            b = top_bin(e.y & 0x7fffffffu, centre);
-          }
-          if (MODE == kScanTop) {
+        if (n_half <= kStage)
+          for (uint32_t q = lane; q < n_half; q += 32u) dst[q] = stage[q];
+        if (MODE == kScanTop) {
+          // Histogram of the candidates.  The top bin, which holds many of them, is not counted: `emit` knows their number.
+          const uint32_t centre = top_centre(ss);
+          const uint32_t piece = seg_rel >> piece_shift;      // of the tensor
+          const uint32_t first_piece = ((ch.run0 + rel / kRunElems) >> A.piece_shift) - piece;
+          uint32_t* const gh = A.hist_top + (size_t)(first_piece + (piece & (hist_copies(sd.n_pad) - 1u))) * kHistBins;
+          for (uint32_t q = lane; q < n_half; q += 32u) {
+            const uint32_t b = top_bin(first[q].y & 0x7fffffffu, centre);
             if (b != (uint32_t)(kHistBins - 1)) atomicAdd(gh + b, 1u);
-          } else if (n_half > kStage) {
-            break;
           }
         }
         __syncwarp();

@@ -6,7 +6,7 @@
 Times, with CUDA events after warm-up, the select chain and the apply chain (scatter, apply) over all buckets
 of a parameter-size list, and reports achieved HBM bandwidth against the measured copy bandwidth of the
 machine (``MEASURED_PEAKS.json`` next to the repository root when present).  Algorithmic traffic of one select,
-per element: the two-pass chain (pass1, plan, pass2, cand) reads g and r and writes r in pass 1 and reads r
+per element: the four-kernel chain (pass1, plan, pass2, cand) reads g and r and writes r in pass 1 and reads r
 again in pass 2 = 16 bytes; the one-pass chain (scan, emit and, top-k, refill) reads g and r and
 writes r = 12 bytes; both write 4 more when the consumed gradient is zeroed (``--zero-grad 1``, the engine's
 "flat" gradient mode; its default mode hands the kernels autograd's own tensors and zeroes nothing).  The sparse
@@ -108,7 +108,9 @@ def main() -> None:
     out = {
         "compressor": args.compressor, "optimizer": args.optimizer, "elements": n_total, "buckets": len(buckets),
         "segments": len(numels), "entries_per_step": entries,
-        "select_chain": "one-pass (scan, emit)" if one_pass else "two-pass (pass1, plan, pass2, cand)",
+        "select_chain": ("random-k (ef_only, randomk)" if args.compressor == "randomk"
+                         else "four-kernel (pass1, plan, pass2, cand)" if not one_pass
+                         else "one-pass (scan, emit, refill)" if args.compressor == "topk" else "one-pass (scan, emit)"),
         "select_bytes_per_element": sel_bytes / n_total,
         "select_ms": sel, "select_GBps": sel_bytes / sel / 1e6,
         "select_frac_of_measured_copy": sel_bytes / sel / 1e6 / peaks["hbm_gbs"],
