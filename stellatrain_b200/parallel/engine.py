@@ -926,6 +926,8 @@ class SparseDPEngine:
         if sd["world"] != self.world:
             raise ValueError(f"checkpoint world size {sd['world']} != {self.world}: receive slots and "
                              f"per-rank k depend on it")
+        if any(abs(bsd["ratio"] - rt.bucket.ratio) > 1e-12 for rt, bsd in zip(self.buckets, sd["buckets"])):
+            self.capture_version += 1     # stream sizes and work tables are launch arguments: captured steps are stale now
         for rt, bsd, it in zip(self.buckets, sd["buckets"], sd["iteration"]):
             rt.bucket.load_state_dict(bsd)
             rt.select_count = rt.apply_count = it

@@ -713,3 +713,37 @@ def test_captured_iteration_joins_the_streams_that_took_part(used):
 
     for a, b in zip(run(True), run(False)):
         assert torch.equal(a, b)
+
+
+def test_a_checkpoint_with_another_ratio_makes_a_captured_step_stale():
+    """Its launches carry the sizes and tables of the old ratio; a checkpoint with the same ratio leaves it usable."""
+    import torch.nn as nn
+
+    from stellatrain_b200.parallel.engine import EngineConfig, SparseDPEngine
+    from stellatrain_b200.parallel.graphs import GraphedStep
+
+    def make(ratio):
+        torch.manual_seed(4)
+        m = nn.Linear(64, 90).cuda()
+        return m, SparseDPEngine(m, EngineConfig(compressor="topk", ratio=ratio, min_ratio=0.9, optimizer="sgd", staleness=0,
+                                                 optimizer_options={"lr": 0.1}))
+
+    m, e = make(0.95)
+    x = torch.randn(8, 64, device="cuda")
+
+    def step(inp):
+        loss = m(inp).square().mean()
+        loss.backward()
+        return loss
+
+    graphed = GraphedStep(e, step, [x], warmup=2)
+    e.load_state_dict(e.state_dict())
+    assert not graphed.stale
+    graphed.replay()
+    other = make(0.9)[1]
+    e.load_state_dict(other.state_dict())
+    assert graphed.stale
+    with pytest.raises(RuntimeError, match="stale"):
+        graphed.replay()
+    e.close()
+    other.close()
