@@ -84,6 +84,7 @@ class BucketLayout:
     segments: list[Segment] = field(default_factory=list)
     n_total: int = 0
     cap: int = 0
+    min_piece_entries: int = 1024     # see piece_runs
     narrow_wire: bool = False   # tensors below NARROW_LIMIT padded elements send 4-byte (u16 index, bf16 value) entries
 
     def __post_init__(self) -> None:
@@ -179,17 +180,21 @@ class BucketLayout:
     @property
     def piece_runs(self) -> int:
         """Runs per piece, a power of two: the largest that gives every SM a piece and no piece more entries than its CTA
-        places in one round, as long as all pieces are resident together.
+        places in one round, as long as all pieces are resident together and hold ``min_piece_entries``.
 
         Every CTA of the emitting kernel sums the tensor's counts and (top-k) reads its histograms, so few large pieces are
         right where the entries are few: 1 % of 16 M elements.  Elsewhere they leave SMs idle and make a CTA work round
         after round.  A captured step of one tensor, pieces of 128 runs against those of this rule, us: top-k at 10 %
         300 k elements 82 / 39, 1 M 86 / 46, 3 M 115 / 78, 16 M 256 / 222; threshold-v16 at 10 % 300 k 55 / 32, 3 M
-        102 / 70, 16 M 219 / 190; threshold-v at 10 % 3 M 69 / 51.  At 1 % 3 M measure 43 / 43."""
+        102 / 70, 16 M 219 / 190; threshold-v at 10 % 3 M 69 / 51.  Splitting a tensor costs a trip to L2 per count and
+        counter: at 1 % of 300 k elements in 40 tensors a bound of 0, 256 or 512 entries made threshold-v 28, 27 and 27 us
+        from 25 and threshold-v16 29, 27 and 27 from 26.  Top-k has no such bound (0): the kernels that make up for
+        candidates that fell short read whole pieces, and with a new batch per pass 1 % of 3 M elements took 60 us in pieces
+        of 128 runs, 48 in 16."""
         total = self.n_total // RUN_ELEMS
         runs = MAX_PIECE_RUNS
-        while runs > MIN_PIECE_RUNS and (total < PIECES_WANTED * runs or
-                                         (self.cap * runs > PIECE_ENTRIES * total and total <= PIECES_AT_ONCE * (runs // 2))):
+        while (runs > MIN_PIECE_RUNS and self.cap * (runs // 2) >= self.min_piece_entries * total and
+               (total < PIECES_WANTED * runs or (self.cap * runs > PIECE_ENTRIES * total and total <= PIECES_AT_ONCE * (runs // 2)))):
             runs //= 2
         return runs
 

@@ -135,6 +135,8 @@ class GpuBucket:
         self.vmax = torch.zeros(ns, **f32) if (optimizer == "adam" and amsgrad) else None
         self.last = torch.zeros(ns, dtype=torch.int32, device=device) if smart_momentum else None
 
+        if compressor == "topk":
+            layout.min_piece_entries = 0
         layout.set_ratio(ratio, self.k_world)
         self.cap_max = max(layout.max_cap(self.min_ratio, self.k_world), layout.cap, 1)
         n_segs = len(layout.segments)

@@ -200,15 +200,16 @@ def test_bundles_train_bit_for_bit_like_one_task_per_tensor(sizes, bundle_elems,
         assert torch.equal(a, b)
 
 
-@pytest.mark.parametrize("chunk,largest,ratio,piece_runs", [
-    (1024, 500_001, 0.99, 8), (8192, 500_001, 0.5, 8), (1 << 18, 500_001, 0.99, 8), (8192, 3_000_003, 0.99, 16),
-    (8192, 18_000_001, 0.99, 128), (1 << 18, 18_000_001, 0.97, 64), (1024, 18_000_001, 0.9, 32), (8192, 40_000_000, 0.5, 128)])
-def test_runs_and_pieces_of_the_one_pass_select_tile_every_tensor(chunk, largest, ratio, piece_runs):
+@pytest.mark.parametrize("chunk,largest,ratio,min_entries,piece_runs", [
+    (1024, 500_001, 0.99, 0, 8), (1024, 500_001, 0.99, 1024, 128), (8192, 500_001, 0.5, 1024, 8), (1 << 18, 500_001, 0.99, 0, 8),
+    (8192, 3_000_003, 0.99, 0, 16), (8192, 18_000_001, 0.99, 0, 128), (1 << 18, 18_000_001, 0.97, 1024, 64),
+    (1024, 18_000_001, 0.9, 1024, 32), (8192, 40_000_000, 0.5, 1024, 128)])
+def test_runs_and_pieces_of_the_one_pass_select_tile_every_tensor(chunk, largest, ratio, min_entries, piece_runs):
     """Every element belongs to exactly one run, and a run found through its chunk has the place its piece gives it."""
     from stellatrain_b200.parallel import buckets as B
 
     numels = [1, 16, 17, 1023, 1025, 131071, 131072, 131073, largest]
-    L = B.BucketLayout([str(i) for i in range(len(numels))], numels, chunk_elems=chunk)
+    L = B.BucketLayout([str(i) for i in range(len(numels))], numels, chunk_elems=chunk, min_piece_entries=min_entries)
     L.set_ratio(ratio, 1)
     assert L.piece_runs == piece_runs
     by_chunk, by_piece = {}, {}
