@@ -25,8 +25,9 @@
 //   scan    memory: 35.5 us for threshold-v16, 36 us for top-k at 0.1 %, 39 us at 1 % (list and histogram).  Runs of one
 //           warp need no barrier and no shared state, so a late load holds up nothing else; with one CTA per 8192 elements
 //           that scanned, chained counts over CTAs and emitted by itself the same traffic took 54 us.
-//   emit    latency, a chain of about twelve trips to L2: 15 us for threshold-v16, 19 us (0.1 %) to 27 us (1 %) for top-k.
-//   refill  1.4 us when there is nothing to do.
+//   emit    latency, a chain of about twelve trips to L2: 15 us for threshold-v16, 19 us (0.1 %) to 31 us (1 %) for top-k; at
+//           10 % the entries count: 28 us for threshold-v16, 45 us for top-k.
+//   refill  1.4 to 2.5 us when there is nothing to do, 95 us for a bucket that is one tensor (42 us at 3 M elements).
 #include "select_common.cuh"
 
 namespace st {
@@ -885,7 +886,8 @@ __device__ __forceinline__ uint32_t collect_unlisted(const SelectArgs& A, const 
 }
 
 // Thread 0 of the last CTA of a top-k tensor: what the next select starts from.  Every candidate costs a list entry and a
-// histogram count, candidates that fall short cost two more passes over the tensor (twice the time).  How many more
+// histogram count; candidates that fall short cost two more passes over the tensor by the emitting kernels (a step of 16 M
+// elements takes up to 125 us more, one of 3 M 60) and hold up the whole bucket.  How many more
 // candidates there were than entries says how near the cut came to falling short.  The threshold of one batch differs from
 // that of the next, so the window grows at once when few were spare and shrinks by a few per cent a step when many were.
 __device__ __forceinline__ void step_top(const SelectArgs& A, const Job& J, SegState ss, uint32_t t_key, uint32_t listed) {
