@@ -25,6 +25,8 @@ namespace st {
 
 namespace {
 constexpr int kThreads = 256;
+constexpr int kSms = 148;
+constexpr int kSingleEntries = 4;      // entries that a thread of k_apply_single has under way
 }
 
 // One warp waits (bounded) for the arrival flags of all sources, one lane per source, and leaves the outcome
@@ -104,11 +106,14 @@ struct StepConsts {
 };
 
 // 1 - beta^tick in double, as the reference computes it (adam.cpp:41-42).  Two double-precision powers take about
-// 1.5 us: every kernel below sends its own loads off first and computes them while those travel.
-__device__ __forceinline__ void bias_corrections(const OptState& o, float* bc) {
-  bc[0] = (float)(1.0 - pow((double)o.beta1, (double)o.tick));
-  bc[1] = (float)(1.0 - pow((double)o.beta2, (double)o.tick));
+// 1.5 us: every kernel below sends its own loads off first and computes them, one in each of two warps, while those travel.
+__device__ __forceinline__ float bias_correction(const OptState& o, uint32_t moment) {
+  return (float)(1.0 - pow((double)(moment == 0u ? o.beta1 : o.beta2), (double)o.tick));
 }
+
+// a b + c d, c d rounded by itself.  Which of the products that is the compiler may choose in the plain expression, and kernels
+// that share the rule have to agree.
+__device__ __forceinline__ float weighted_sum(float a, float b, float c, float d) { return fmaf(a, b, __fmul_rn(c, d)); }
 
 // The optimiser rule for element `s` of the state range (`rc`: its record with the merged gradient in x, `x`: its
 // parameter).  Writes the record back with the accumulator cleared and the stamp of this epoch; returns the new value.
@@ -121,7 +126,7 @@ __device__ __forceinline__ float update_element(const ApplyArgs& A, const OptSta
       mu = powf(o.momentum, (float)(c.m_iter - A.last[s]));
     if (o.weight_decay != 0.f) g += o.weight_decay * x;
     if (o.momentum != 0.f) {
-      const float b = o.first ? g : rc.z * mu + (1.f - o.dampening) * g;
+      const float b = o.first ? g : weighted_sum(1.f - o.dampening, g, rc.z, mu);
       g = o.nesterov ? g + mu * b : b;
       m_new = b;
     }
@@ -130,8 +135,8 @@ __device__ __forceinline__ float update_element(const ApplyArgs& A, const OptSta
   } else {
     if (o.maximize) g = -g;
     if (o.weight_decay != 0.f) g += o.weight_decay * x;
-    const float mt = o.beta1 * rc.z + (1.f - o.beta1) * g;
-    const float vt = o.beta2 * rc.w + (1.f - o.beta2) * g * g;
+    const float mt = weighted_sum(o.beta1, rc.z, 1.f - o.beta1, g);
+    const float vt = weighted_sum(o.beta2, rc.w, __fmul_rn(1.f - o.beta2, g), g);
     const float mh = mt / c.bc1;
     float vh = vt / c.bc2;
     if (o.amsgrad && A.vmax != nullptr) {
@@ -174,7 +179,7 @@ __global__ void __launch_bounds__(kThreads) k_apply(ApplyArgs A) {
       if (in_range) old = atomicExch(reinterpret_cast<uint32_t*>(&A.rec[s].y), epoch);
     };
     if (i < A.ent_hi) claim();
-    if (threadIdx.x == 0 && o.kind != 0) bias_corrections(o, s_bc);
+    if ((threadIdx.x & 31u) == 0u && threadIdx.x < 64u && o.kind != 0) s_bc[threadIdx.x >> 5] = bias_correction(o, threadIdx.x >> 5);
     if (A.cksum_local != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
       // the scatter kernel has read the whole stream of this source: does it add up to what was sent?
       const uint32_t got = atomicExch(A.rsum + src, 0u);
@@ -220,8 +225,15 @@ __global__ void __launch_bounds__(kThreads) k_apply(ApplyArgs A) {
 
 // One source: its stream names every element at most once (each select emits an element once, also where the narrow wire
 // format's rounding leaves something of it in the residual; random-k strides through the tensor with a step coprime to its
-// size), so there is nothing to merge: no accumulator, no stamp to compete for, one kernel instead of two.  Bound by DRAM
-// accesses to single records: 168,000 entries of a 64 MB bucket take 10.8 us as blocks of 16 neighbours (threshold-v16; 13 us with scatter and apply) and 16.5 us one by one (top-k; 19 us).
+// size), so there is nothing to merge: no accumulator, no stamp to compete for, one kernel instead of two.
+//
+// Bound by a chain of trips (counters, entry, record and parameter) and, with scattered entries, by DRAM accesses to single
+// records.  A thread has N entries under way: a CTA's life is the chain, so fewer and fuller CTAs leave the SMs to the streaming
+// kernels of other buckets.  One entry a thread and four, us: blocks of 16 neighbours (threshold-v16) 168,000 entries of a 64 MB
+// bucket 11.0 and 6.9, 670,000 28.7 and 13.5; scattered ones (top-k) 168,000 17.2 and 14.7, but 670,000 58 and 67 (every entry
+// opens DRAM rows of its own, and the more of them compete the fewer stay open).  Up to one entry a thread on every SM there is
+// nothing to gather.  So: four entries a thread for blocks, for scattered entries as long as that is at most two CTAs per SM.
+template <int N>
 __global__ void __launch_bounds__(kThreads) k_apply_single(ApplyArgs A) {
   __shared__ float s_bc[2];
   const uint32_t epoch = *A.epoch;
@@ -233,33 +245,40 @@ __global__ void __launch_bounds__(kThreads) k_apply_single(ApplyArgs A) {
   if (ok) {
     const uint2* in = A.recv + (size_t)slot * A.slot_stride;
     const float w = A.weight[slot];
-    const uint32_t step = gridDim.x * kThreads;
-    uint32_t i = blockIdx.x * kThreads + threadIdx.x;
-    uint2 e = make_uint2(kSentinelIdx, 0u);
-    float4 rc = make_float4(0.f, 0.f, 0.f, 0.f);
-    float x = 0.f;
-    bool in_range = false;
+    const uint32_t step = gridDim.x * kThreads * N;
+    uint32_t i = blockIdx.x * kThreads * N + threadIdx.x;
+    uint2 e[N];
+    float4 rc[N];
+    float x[N];
     auto fetch = [&]() {
-      e = load_entry(A, in, i);
-      in_range = e.x < A.n_total;
-      if (in_range) {
-        rc = __ldcg(A.rec + e.x);
-        x = __ldcg(A.param + e.x);
-      } else if (e.x != kSentinelIdx) {
-        set_status(A.status, kBadIndex);
+#pragma unroll
+      for (int u = 0; u < N; ++u)
+        e[u] = i + u * kThreads < A.ent_hi ? load_entry(A, in, i + u * kThreads) : make_uint2(kSentinelIdx, 0u);
+#pragma unroll
+      for (int u = 0; u < N; ++u) {
+        if (e[u].x < A.n_total) {
+          rc[u] = __ldcg(A.rec + e[u].x);
+          x[u] = __ldcg(A.param + e[u].x);
+        } else if (e[u].x != kSentinelIdx) {
+          set_status(A.status, kBadIndex);
+        }
       }
     };
-    if (i < A.ent_hi) fetch();
-    if (threadIdx.x == 0 && o.kind != 0) bias_corrections(o, s_bc);
+    fetch();
+    if ((threadIdx.x & 31u) == 0u && threadIdx.x < 64u && o.kind != 0) s_bc[threadIdx.x >> 5] = bias_correction(o, threadIdx.x >> 5);
     __syncthreads();
     const StepConsts c = {s_bc[0], s_bc[1], o.maximize ? -o.lr : o.lr, o.tick - 1u};
-    while (i < A.ent_hi) {
-      if (in_range) {
-        rc.x += __uint_as_float(e.y) * w;      // what the merge would have left in the accumulator
-        A.param[e.x] = update_element(A, o, c, e.x, epoch, rc, x);
+    while (true) {
+#pragma unroll
+      for (int u = 0; u < N; ++u) {
+        if (e[u].x < A.n_total) {
+          rc[u].x += __uint_as_float(e[u].y) * w;      // what the merge would have left in the accumulator
+          A.param[e[u].x] = update_element(A, o, c, e[u].x, epoch, rc[u], x[u]);
+        }
       }
       i += step;
-      if (i < A.ent_hi) fetch();
+      if (i >= A.ent_hi) break;
+      fetch();
     }
   }
   __syncthreads();
@@ -330,7 +349,12 @@ cudaError_t launch_apply(const ApplyArgs& A, int max_ctas_per_source, int phase,
     dim3 grid(parts, A.world);
     if (A.use_flags) k_wait_streams<<<1, 32, 0, stream>>>(A);
     if (apply_merges_nothing(A)) {
-      k_apply_single<<<parts, kThreads, 0, stream>>>(A);
+      const uint32_t n = A.ent_hi - A.ent_lo;
+      const int wide = (int)((n + kThreads * kSingleEntries - 1) / (kThreads * kSingleEntries));
+      if (n > (uint32_t)(kSms * kThreads) && (A.blocks || wide <= 2 * kSms))
+        k_apply_single<kSingleEntries><<<wide < max_ctas_per_source ? wide : max_ctas_per_source, kThreads, 0, stream>>>(A);
+      else
+        k_apply_single<1><<<parts, kThreads, 0, stream>>>(A);
       return cudaGetLastError();
     }
     if (A.deterministic) {

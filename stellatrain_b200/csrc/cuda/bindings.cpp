@@ -175,6 +175,7 @@ struct BucketHandle : public st::BucketHandle {
     sel.zero_grad = zero_grad ? 1u : 0u;
     sel.skip_ef = skip_ef ? 1u : 0u;
     app.narrow = narrow ? 1u : 0u;
+    app.blocks = compressor == st::kThresholdv16 ? 1u : 0u;
     app.deterministic = deterministic ? 1u : 0u;   // one scatter launch per source, in rank order
     app.src_first = 0u;
   }

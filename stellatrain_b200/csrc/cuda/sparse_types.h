@@ -228,6 +228,7 @@ struct ApplyArgs {
   uint32_t narrow;
   uint32_t n_segs;
   const SegDesc* segs;
+  uint32_t blocks;                  // entries come as blocks of 16 neighbours (threshold-v16)
   // Debug checks (null = off): the scatter adds the same hash over what it reads into rsum[source], the apply
   // compares it with the word the source stored and reports kBadChecksum; with `poison` every consumed entry
   // of a wide stream is overwritten with the "no entry" marker, so a position a source fails to rewrite

@@ -399,6 +399,29 @@ def test_single_source_apply_equals_the_merging_one(optimizer, options, extra, c
             assert torch.equal(getattr(one, name), getattr(two, name))
 
 
+@pytest.mark.parametrize("compressor,n,narrow", [("topk", 378_881, False), ("topk", 3_031_039, False), ("topk", 3_031_051, False),
+                                                 ("thresholdv16", 378_897, False), ("thresholdv16", 3_200_003, False),
+                                                 ("thresholdv", 640_000, True)])
+@pytest.mark.parametrize("ctas", [3, 148 * 16])
+def test_single_source_apply_at_the_edges_of_its_grid(compressor, n, narrow, ctas):
+    """More entries than one per thread on every SM (37,888): four of them a thread, and scattered ones one a thread again past
+    303,104; the last CTA is not full.  The same bits as scatter + apply, which debug checks keep."""
+    pair = []
+    for debug in (False, True):
+        gen = torch.Generator(device="cuda").manual_seed(22)
+        sizes = [n // 10] * 10 if narrow else [n]
+        b = make_bucket(compressor, 0.9, "adam", sizes=sizes, chunk=8192, narrow=narrow, debug=debug)
+        b.handle.max_ctas_per_source = ctas
+        for _ in range(3):
+            fill_grads(b, gen)
+            b.select()
+            b.apply()
+        torch.cuda.synchronize()
+        b.check_status()
+        pair.append(b)
+    assert torch.equal(pair[0].param, pair[1].param) and torch.equal(pair[0].rec, pair[1].rec)
+
+
 def test_randomk_stream_is_valid():
     b = make_bucket("randomk", 0.9, sizes=[1000, 4096, 17])
     gen = torch.Generator(device="cuda").manual_seed(3)
