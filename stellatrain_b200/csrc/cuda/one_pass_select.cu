@@ -916,11 +916,19 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(SelectArgs A) {
 
   if (!(J.sd.reserved & kSegSkip)) {
     const SegState ss = A.state[J.pc.seg];
-    // listed items and near misses of this piece and of the tensor
+    // listed items and near misses of this piece and of the tensor; listed items in front of this piece, and of the fullest one
     unsigned long long all = 0ull;
+    uint32_t ahead = 0, most = 0;
     if (J.pc.count > 1u)
-      for (uint32_t t = tid; t < J.pc.count; t += kEmitThreads) all += A.piece_cnt[J.pc.first + t];
-    if (tid == 0) S.sum = 0ull;
+      for (uint32_t t = tid; t < J.pc.count; t += kEmitThreads) {
+        const unsigned long long n = A.piece_cnt[J.pc.first + t];
+        all += n;
+        if (MODE != kScanTop) {
+          if (t < J.pc.index) ahead += (uint32_t)n;
+          most = max(most, (uint32_t)n);
+        }
+      }
+    if (tid == 0) { S.sum = 0ull; S.at[0] = 0u; S.at[1] = 0u; }
     uint32_t total, near_total = 0;
     uint32_t ex = block_excl_scan(cnt & 0xffffu, S.tmp, total);
     if (tid <= kMaxPieceRuns) S.pre[tid] = ex;
@@ -929,13 +937,27 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(SelectArgs A) {
       if (tid <= kMaxPieceRuns) S.near[tid] = nex;
     }
     uint32_t found = total, c_near = near_total;
+    bool even = true;       // no CTA gets much more than its share when each sends the items of its own piece
     if (J.pc.count > 1u) {
 #pragma unroll
       for (int d = 16; d > 0; d >>= 1) all += __shfl_xor_sync(0xffffffffu, all, d);
-      if ((tid & 31u) == 0u && all) atomicAdd(&S.sum, all);
+      if (MODE != kScanTop) {
+        ahead = __reduce_add_sync(0xffffffffu, ahead);
+        most = __reduce_max_sync(0xffffffffu, most);
+      }
+      if ((tid & 31u) == 0u && all) {
+        atomicAdd(&S.sum, all);
+        if (MODE != kScanTop) {
+          atomicAdd(&S.at[0], ahead);
+          atomicMax(&S.at[1], most);
+        }
+      }
       __syncthreads();
       found = (uint32_t)S.sum;
       c_near = (uint32_t)(S.sum >> 32);
+      ahead = S.at[0];
+      constexpr uint32_t kPerItem = kBlock ? 16u : 1u;
+      even = S.at[1] * kPerItem <= 2u * max(kStageItems, min(found, J.kk) / J.pc.count * kPerItem);
     }
     const bool short_of = found < J.kk;
     // will this CTA store into the destinations?  Then they must have consumed the slot.
@@ -1039,14 +1061,18 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(SelectArgs A) {
           nears[nb0 + j] = area[run * kArea + n_blk - 1u - (j - S.near[run])];
         }
       }
-      // The first kk items in index order are sent.  A threshold that lags behind lets nearly everything pass, and the budget
-      // then ends within the tensor's first piece: the positions, not the pieces, are shared out among its CTAs.
+      // The first kk items in index order are sent, as a rule by the CTA of their piece.  A threshold that lags behind lets nearly
+      // everything pass, and the budget then ends within the tensor's first piece; items may also lie in a few places only: then
+      // the positions, not the pieces, are shared out among the CTAs, which costs two more trips to find the piece of a position
+      // and its runs.
       const uint32_t n_send = min(found, J.kk);
       const uint32_t lo = (uint32_t)((uint64_t)n_send * J.pc.index / J.pc.count);
       const uint32_t hi = (uint32_t)((uint64_t)n_send * (J.pc.index + 1u) / J.pc.count);
-      if (may && lo < hi) {
+      if (may && even) {
+        if (ahead < n_send) send_range<kBlock>(A, J, S, area, ahead, 0u, min(total, n_send - ahead));
+      } else if (may && lo < hi) {
         uint32_t piece = 0, base = 0;
-        if (J.pc.count > 1u) {
+        {
           uint32_t carry = 0;
           for (uint32_t t0 = 0; t0 < J.pc.count && carry <= lo; t0 += kEmitThreads) {
             const uint32_t t = t0 + tid;
@@ -1061,7 +1087,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(SelectArgs A) {
           base = S.at[1];
         }
         for (;;) {
-          if (J.pc.count > 1u) {
+          {
             const uint32_t n_runs = (min(J.piece_elems, J.sd.n_pad - piece * J.piece_elems) + kRunElems - 1u) / kRunElems;
             const uint32_t v = tid < n_runs ? A.run_cnt[((J.pc.first + piece) << A.piece_shift) + tid] & 0xffffu : 0u;
             ex = block_excl_scan(v, S.tmp, total);

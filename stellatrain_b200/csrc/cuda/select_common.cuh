@@ -108,7 +108,7 @@ __device__ __forceinline__ void finish_select(const SelectArgs& A, uint32_t epoc
   const uint32_t prev = atom_add_acq_rel_gpu(A.done_ctr, 1u);
   if (prev == gridDim.x - 1) {
     *A.done_ctr = 0;
-    __threadfence_system();
+    if (A.publish) __threadfence_system();     // without peers the end of the kernel is enough, and sooner
     if (refills != nullptr) {
       if (is_refill) *refills = 0;
       else if (ld_volatile_u32(refills) != 0u) return;

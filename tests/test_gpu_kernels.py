@@ -155,6 +155,50 @@ def test_one_pass_select_at_its_edges(compressor, mode, ratio, chunk, narrow, pi
     assert int(work[:, 4:6].abs().max()) == 0 and int(work[:, 10:].abs().max()) == 0 and int(b.counters[4]) == 0
 
 
+@pytest.mark.parametrize("compressor", ["thresholdv", "thresholdv16"])
+@pytest.mark.parametrize("where", ["everywhere", "one piece", "first piece"])
+@pytest.mark.parametrize("over", [0.7, 1.1, 3.0])
+def test_items_over_the_threshold_in_all_pieces_or_in_one(compressor, where, over):
+    """A CTA sends the listed items of its own piece unless one piece holds most of them; then the positions are shared out.
+    ``over``: items over the threshold, as a multiple of the budget."""
+    n, ratio = 3_000_003, 0.97
+    b = make_bucket(compressor, ratio, sizes=[n, 70_001], chunk=8192)
+    assert b.n_pieces > 20
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    resid_ref = torch.zeros_like(b.resid)
+    per_piece = b.layout.piece_runs * B.RUN_ELEMS
+    for step in range(3):
+        fill_grads(b, gen)
+        if where != "everywhere":
+            at = per_piece * (0 if where == "first piece" else 7)
+            b.grad[at : at + per_piece] *= 1000.0
+        grad = b.grad.clone()
+        if step > 0:        # a threshold that lets so many pass
+            block = compressor == "thresholdv16"
+            state = b.seg_state()
+            for si, (s, _, slp) in enumerate(seg_slices(b)):
+                key = (grad[slp] + b.resid[slp]).abs()
+                key = key.view(-1, 16).sum(1) if block else key
+                state["tau"][si] = float(key.sort(descending=True).values[int(over * (s.k // 16 if block else s.k))])
+            b.state.copy_(torch.from_numpy(state.view(np.uint8).reshape(-1)))
+        states = oracle_states(b)
+        b.select()
+        torch.cuda.synchronize()
+        b.check_status()
+        idx_all, val_all = read_stream(b, step + 1)
+        for si, (s, sl, slp) in enumerate(seg_slices(b)):
+            own = slp if compressor == "thresholdv16" else sl
+            want_idx, want_val, new_r = O.compress_step(compressor, grad[own], resid_ref[own], s.k, states[si], one_pass=step > 0)
+            got = torch.from_numpy(idx_all[s.out_off : s.out_off + s.k])
+            valid = got != O.SENTINEL
+            got, order = got[valid].sort()
+            want, worder = (want_idx.cpu() + s.off).sort()
+            assert torch.equal(got, want), (s.numel, step)
+            assert torch.equal(val_all[s.out_off : s.out_off + s.k][valid][order], want_val.cpu()[worder]), (s.numel, step)
+            resid_ref[own] = new_r
+        assert torch.equal(b.resid, resid_ref), step
+
+
 @pytest.mark.parametrize("compressor", ["topk", "thresholdv", "thresholdv16"])
 def test_a_ratio_change_cuts_the_bucket_anew(compressor):
     """More entries want smaller pieces; thresholds and residuals stay."""
