@@ -193,26 +193,18 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* s, uin
   __syncthreads();  // protects s against a previous call
   if (lane == 31) s[warp] = incl;
   __syncthreads();
-  uint32_t warp_off = 0, sum = 0;
-  for (int w = 0; w < nwarp; ++w) {
-    const uint32_t x = s[w];
-    if (w < warp) warp_off += x;
-    sum += x;
-  }
-  total = sum;
-  return warp_off + incl - v;
+  const uint32_t x = lane < nwarp ? s[lane] : 0u;
+  total = __reduce_add_sync(0xffffffffu, x);
+  return __reduce_add_sync(0xffffffffu, lane < warp ? x : 0u) + incl - v;
 }
 
 __device__ __forceinline__ uint32_t block_max_u32(uint32_t v, uint32_t* s) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, d));
+  v = __reduce_max_sync(0xffffffffu, v);
   __syncthreads();
   if (lane == 0) s[warp] = v;
   __syncthreads();
-  uint32_t r = 0;
-  for (int w = 0; w < nwarp; ++w) r = max(r, s[w]);
-  return r;
+  return __reduce_max_sync(0xffffffffu, lane < nwarp ? s[lane] : 0u);
 }
 
 }  // namespace st

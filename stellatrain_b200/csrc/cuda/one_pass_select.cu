@@ -44,7 +44,7 @@ constexpr uint32_t kMaxPieceElems = kMaxPieceRuns * kRunElems;
 
 constexpr int kEmitThreads = 256;
 constexpr uint32_t kStageItems = 2048;         // entries staged at a time
-constexpr uint32_t kPickMax = 2048;            // candidates that a CTA holds in registers to pick the best from
+constexpr uint32_t kPickMax = 2048;            // candidates that a CTA holds in shared memory to pick the best from
 
 // Top-k of a tensor this small is picked from registers by its one CTA of `emit`: its k-th largest value moves too much from
 // step to step to be worth predicting, and no list, histogram or cut is needed.
@@ -352,10 +352,16 @@ struct EmitShared {
   uint32_t near[kMaxPieceRuns + 1];    // near misses in front of each run of the piece
   uint32_t tmp[kEmitThreads / 32 + 1];
   uint32_t res[4];
-  uint32_t cnt[64];                 // counts of the bitwise searches
   uint32_t word[4];                 // [0] may emit, [1] last CTA of the tensor, [2], [3] bases of a batch
   unsigned long long sum;           // listed items | near misses << 32 of the tensor
   uint32_t at[2];                   // piece of the tensor that holds a position, positions in front of it
+  // where the tensor's entries go
+  uint2* out[kMaxWorld];            // its region in each destination, when entries are plain pairs
+  uint32_t n_out;                   // 0: they are not (narrow wire format, multicast, checksums)
+  uint32_t off;                     // the tensor's first element
+  uint32_t nb;
+  int dest;
+  uint64_t slot_off;
 };
 
 // Run (of the piece) that holds item j: the last one that starts at or in front of it and is not empty.
@@ -398,9 +404,23 @@ __device__ __forceinline__ Job job_of(const SelectArgs& A, bool block) {
   return J;
 }
 
-__device__ __forceinline__ void emit_and_keep(const SelectArgs& A, const Job& J, uint32_t pos, uint32_t gi, float a) {
-  const float sv = wire_value(J.nb, a);
-  emit_entry(A, J.dest, J.nb, J.slot_off, pos, gi, sv);
+// Where the tensor's entries go.  A CTA barrier follows before anybody reads it.
+__device__ __forceinline__ void note_destinations(const SelectArgs& A, const Job& J, EmitShared& S) {
+  const bool plain = J.nb == kNotNarrow && A.cksum_acc == nullptr && (J.dest >= 0 || A.out_mc == nullptr);
+  const uint32_t n = J.dest >= 0 ? 1u : (uint32_t)A.world;
+  if (threadIdx.x < n) S.out[threadIdx.x] = A.out[J.dest >= 0 ? (uint32_t)J.dest : threadIdx.x] + J.slot_off;
+  if (threadIdx.x == 0) {
+    S.n_out = plain ? n : 0u;
+    S.off = J.sd.off;
+    S.nb = J.nb;
+    S.dest = J.dest;
+    S.slot_off = J.slot_off;
+  }
+}
+
+__device__ __forceinline__ void emit_and_keep(const SelectArgs& A, const EmitShared& S, uint32_t pos, uint32_t gi, float a) {
+  const float sv = wire_value(S.nb, a);
+  emit_entry(A, S.dest, S.nb, S.slot_off, pos, gi, sv);
   A.resid[gi] = a - sv;     // exactly zero unless the wire format rounds
 }
 
@@ -464,13 +484,52 @@ __device__ __forceinline__ void plan_top(const uint32_t* gh, uint32_t copies, ui
   __syncthreads();
 }
 
+// Which pairs a CTA sends: S.stage in order; those that S.hist names; of a tensor whose values are the words of S.stage, those.
+enum Staged : uint32_t { kInOrder = 0, kNamed = 1, kWords = 2 };
+
+// Sends m of the CTA's pairs at positions pos, pos + 1, ... and takes them out of the residual.
+//
+// The kernels of this part run once per CTA and step from one section to the next: what they wait for, besides L2, is their own
+// instructions.  With the stores to the destinations inlined wherever pairs are sent, and the searches below unrolled over
+// registers, `emit` had 166 KB of code for top-k, and a section took microseconds of fetches the first time an SM came to it (the
+// last CTA's search in a tensor 7 us for 100 items).  So sections that are used twice or rarely are functions, loops are loops, and
+// items lie in shared memory: a 64 MB bucket takes 16 us instead of 23 (top-k, 1 %) and 9.6 instead of 12.9 (threshold-v16).
+__device__ __noinline__ void send_staged(const SelectArgs& A, EmitShared& S, Staged how, uint32_t m, uint32_t pos) {
+  const uint32_t* const words = reinterpret_cast<const uint32_t*>(S.stage);
+  const uint32_t n_out = S.n_out, off = S.off;
+  auto pair = [&](uint32_t q) {
+    const uint32_t i = how == kInOrder ? q : S.hist[q];
+    return how == kWords ? make_uint2(off + i, words[i]) : S.stage[i];
+  };
+  if (n_out == 0u) {
+#pragma unroll 1
+    for (uint32_t q = threadIdx.x; q < m; q += kEmitThreads) {
+      const uint2 e = pair(q);
+      emit_and_keep(A, S, pos + q, e.x, __uint_as_float(e.y));
+    }
+    return;
+  }
+  float* const resid = A.resid;
+#pragma unroll 1
+  for (uint32_t p = 0; p < n_out; ++p) {
+    uint2* const out = S.out[p] + pos;
+#pragma unroll 4
+    for (uint32_t q = threadIdx.x; q < m; q += kEmitThreads) {
+      const uint2 e = pair(q);
+      out[q] = e;
+      if (p == 0u) resid[e.x] = __uint_as_float(e.y) - __uint_as_float(e.y);      // zero, or what the next select drops
+    }
+  }
+}
+
 // Sends the `n` marked items of a CTA's batch at positions base, base + 1, ...: bit u of `sel` marks the thread's item u, `ex`
 // is the number of marked items in front of the thread's first.  They go through shared memory, so that the stores into the
-// destinations are consecutive and stand in the code once (unrolled per item they took 10 us in instruction fetches alone).
+// destinations are consecutive.
 template <int N>
-__device__ __forceinline__ void send_marked(const SelectArgs& A, const Job& J, EmitShared& S, const uint32_t (&idx)[N],
-                                            const uint32_t (&bits)[N], uint32_t sel, uint32_t ex, uint32_t n, uint32_t base) {
+__device__ __forceinline__ void send_marked(const SelectArgs& A, EmitShared& S, const uint32_t (&idx)[N], const uint32_t (&bits)[N],
+                                            uint32_t sel, uint32_t ex, uint32_t n, uint32_t base) {
   uint2* const stage = S.stage;
+#pragma unroll 1
   for (uint32_t w = 0; w < n; w += kStageItems) {
     uint32_t p = ex - w;
 #pragma unroll
@@ -481,10 +540,7 @@ __device__ __forceinline__ void send_marked(const SelectArgs& A, const Job& J, E
       }
     }
     __syncthreads();
-    const uint32_t m = min(kStageItems, n - w);
-#pragma unroll 1
-    for (uint32_t q = threadIdx.x; q < m; q += kEmitThreads)
-      emit_and_keep(A, J, base + w + q, stage[q].x, __uint_as_float(stage[q].y));
+    send_staged(A, S, kInOrder, min(kStageItems, n - w), base + w);
     __syncthreads();
   }
 }
@@ -521,127 +577,167 @@ __device__ __forceinline__ void emit_top_batch(const SelectArgs& A, const Job& J
   uint32_t q = b_und + (ex >> 16);
 #pragma unroll
   for (int u = 0; u < N; ++u)
-    if (und >> u & 1u) undecided[q++] = make_uint2(idx[u], bits[u] & 0x7fffffffu);
-  send_marked<N>(A, J, S, idx, bits, sel, ex & 0xffffu, t_sel, b_sel);
+    if (und >> u & 1u) undecided[q++] = make_uint2(idx[u], bits[u]);
+  send_marked<N>(A, S, idx, bits, sel, ex & 0xffffu, t_sel, b_sel);
 }
 
-// Where the best `take` of the CTA's (key, id) pairs end (larger key first, equal keys by lower id): the lowest-ranked one
-// taken.  `there`: bit u says whether pair u counts; 1 <= take <= number of pairs.  The CTA holds the pairs in registers and
-// finds the key bit by bit, as many bits as [key_lo, key_hi), which holds all keys, leaves open; a step is a count over the
-// CTA with one barrier, about 0.1 us whatever the data (ranking 400 pairs against one another took 25 us).  The caller has
-// cleared S.cnt behind a barrier.
-template <int N>
-__device__ __forceinline__ uint2 cut_of_best(const uint32_t (&key)[N], const uint32_t (&id)[N], uint32_t there, uint32_t take,
-                                             uint32_t key_lo, uint32_t key_hi, EmitShared& S) {
-  auto count = [&](int slot, auto pred) {
-    uint32_t n = 0;
-#pragma unroll
-    for (int u = 0; u < N; ++u) n += (there >> u & 1u) && pred(key[u], id[u]) ? 1u : 0u;
-    n = __reduce_add_sync(0xffffffffu, n);
-    if ((threadIdx.x & 31u) == 0u && n) atomicAdd(&S.cnt[slot], n);
+// Keys of the last two octaves under the largest differ from it in these bits: where the best of a distribution are looked for
+// first.
+constexpr uint32_t kTwoOctaves = 24u;
+
+// Where the best `take` of n items in S.stage end (larger key first, equal keys by lower id): {key, id - id_lo} of the
+// lowest-ranked one taken; 1 <= take <= n.  The items are pairs (id, key or signed value), or the words (keys or signed values) of
+// one tensor, whose ids count from 0.  No key lies above `top`; ids lie in [id_lo, id_lo + n_ids).
+// A radix search, 8 bits at a time with a bin per thread.  Its digits are those of the distance to `top`, so that they differ
+// where the cut is: of the `open` lowest bits first, which is a guess; a cut further away is found in all 31.
+__device__ __noinline__ uint2 find_cut(EmitShared& S, bool words, uint32_t n, uint32_t take, uint32_t top, uint32_t open,
+                                       uint32_t id_lo, uint32_t n_ids) {
+  static_assert(kEmitThreads == 256, "a bin per thread");
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, n_up = (n + kEmitThreads - 1u) & ~(kEmitThreads - 1u);
+  const uint32_t* const word = reinterpret_cast<const uint32_t*>(S.stage);
+  auto distance = [&](uint32_t i) { return top - ((words ? word[i] : S.stage[i].y) & 0x7fffffffu); };
+  auto id_of = [&](uint32_t i) { return words ? i : S.stage[i].x - id_lo; };
+  uint32_t prefix = 0, rem = take, ties = 0, d = 0;
+  bool by_id = false;
+#pragma unroll 1
+  for (;;) {
+    // among the values whose bits from `open` upwards are `prefix`: the digit of the rem-th smallest
+    const uint32_t w = min(open, 8u), shift = open - w;
+    S.hist[tid] = 0u;
     __syncthreads();
-    return S.cnt[slot];
-  };
-  uint32_t t = key_lo, n_ge = 0xFFFFFFFFu;      // a key that at least `take` pairs reach
-  for (int bit = 31 - __clz((key_hi - key_lo) | 1u); bit >= 0 && n_ge != take; --bit) {
-    const uint32_t trial = t + (1u << bit);
-    const uint32_t n = count(bit, [&](uint32_t k, uint32_t) { return k >= trial; });
-    if (n >= take) { t = trial; n_ge = n; }
-  }
-  uint32_t last;
-  if (n_ge == take) {
-    // exactly the pairs from t upwards: the smallest key among them, and the highest id that has it
-    uint32_t mn = 0xFFFFFFFFu, mx = 0;
-#pragma unroll
-    for (int u = 0; u < N; ++u)
-      if ((there >> u & 1u) && key[u] >= t) mn = min(mn, key[u]);
-    t = ~block_max_u32(~mn, S.tmp);
-#pragma unroll
-    for (int u = 0; u < N; ++u)
-      if ((there >> u & 1u) && key[u] == t) mx = max(mx, id[u]);
-    last = block_max_u32(mx, S.tmp);
-  } else {
-    // t is the take-th largest key itself and more pairs share it than are wanted
-    const uint32_t need = take - count(31, [&](uint32_t k, uint32_t) { return k > t; });
-    last = 0;                      // the need-th smallest id among equal keys: the largest that fewer ids lie under
-    for (int bit = 31; bit >= 0; --bit) {
-      const uint32_t trial = last | 1u << bit;
-      if (count(32 + bit, [&](uint32_t k, uint32_t i) { return k == t && i < trial; }) < need) last = trial;
+#pragma unroll 4
+    for (uint32_t i = tid; i < n_up; i += kEmitThreads) {
+      uint32_t bin = 256u;
+      if (i < n) {
+        uint32_t v = distance(i);
+        const bool counts = !by_id || v == d;
+        if (by_id) v = id_of(i);
+        if (counts && v >> open == prefix) bin = v >> shift & ((1u << w) - 1u);
+      }
+      int same;
+      __match_all_sync(0xffffffffu, bin, &same);      // equal values would queue up at one counter
+      if (bin < 256u && (!same || lane == 0u)) atomicAdd(&S.hist[bin], same ? 32u : 1u);
+    }
+    __syncthreads();
+    const uint32_t h = S.hist[tid];
+    if (tid == 0) S.res[2] = 0u;
+    uint32_t total;
+    const uint32_t ex = block_excl_scan(h, S.tmp, total);
+    if (ex < rem && ex + h >= rem) { S.res[0] = tid; S.res[1] = rem - ex; S.res[2] = h; }
+    __syncthreads();
+    ties = S.res[2];
+    if (ties == 0u) {      // the guess was wrong
+      open = 31u;
+      prefix = 0u;
+      continue;
+    }
+    prefix = prefix << w | S.res[0];
+    rem = S.res[1];
+    open = shift;
+    if (by_id) {
+      if (open == 0u) break;
+      continue;
+    }
+    if (rem == ties) break;
+    if (open == 0u) {      // more items share the key than are wanted: the rem-th smallest id
+      d = prefix;
+      by_id = true;
+      open = 32u - __clz(n_ids);
+      prefix = 0u;
     }
   }
-  return make_uint2(t, last);
+  uint32_t last = prefix;
+  if (!by_id) {
+    // all items that share these bits: the furthest of them, and the highest id there
+    uint32_t mx = 0;
+#pragma unroll 4
+    for (uint32_t i = tid; i < n; i += kEmitThreads)
+      if (distance(i) >> open == prefix) mx = max(mx, distance(i));
+    d = block_max_u32(mx, S.tmp);
+    mx = 0;
+#pragma unroll 4
+    for (uint32_t i = tid; i < n; i += kEmitThreads)
+      if (distance(i) == d) mx = max(mx, id_of(i));
+    last = block_max_u32(mx, S.tmp);
+  }
+  return make_uint2(top - d, last);
 }
 
-// The best `take` of c candidates: their ids go to S.hist, the lowest-ranked one last.  Returns its key.
-// 1 <= take <= c <= N * kEmitThreads.
-template <int N>
-__device__ __forceinline__ uint32_t pick_best(const uint2* cand, uint32_t c, uint32_t take, uint32_t key_lo, uint32_t key_hi,
-                                              EmitShared& S) {
-  static_assert(N * kEmitThreads <= (int)kPickMax && kPickMax <= 2048, "the ids fit EmitShared::hist");
+// The best `take` of c <= kPickMax candidates (id, key or signed value): they come to S.stage, and S.hist names those taken, the
+// lowest-ranked one last.  Returns its key.  `top`, `open`: see find_cut.
+__device__ __forceinline__ uint32_t pick_few(const uint2* cand, uint32_t c, uint32_t take, uint32_t top, uint32_t open,
+                                             uint32_t id_lo, uint32_t n_ids, EmitShared& S) {
+  static_assert(kPickMax <= kStageItems && kPickMax <= 2048, "the candidates fit EmitShared::stage, their numbers EmitShared::hist");
+  constexpr int kPer = kPickMax / kEmitThreads;
   const uint32_t tid = threadIdx.x;
-  uint32_t key[N], id[N], there = 0;
+  uint2 e[kPer];
 #pragma unroll
-  for (int u = 0; u < N; ++u) {
-    const uint32_t i = u * kEmitThreads + tid;
-    const uint2 e = i < c ? __ldcg(cand + i) : make_uint2(0u, 0u);
-    there |= (uint32_t)(i < c) << u;
-    id[u] = e.x;
-    key[u] = e.y;
-  }
-  if (tid < 64u) S.cnt[tid] = 0u;
-  if (tid == 64u) S.word[2] = 0u;
+  for (int u = 0; u < kPer; ++u)
+    if (u * kEmitThreads + tid < c) e[u] = __ldcg(cand + u * kEmitThreads + tid);
+#pragma unroll
+  for (int u = 0; u < kPer; ++u)
+    if (u * kEmitThreads + tid < c) S.stage[u * kEmitThreads + tid] = e[u];
+  if (tid == 0) S.word[2] = 0u;
   __syncthreads();
-  const uint2 cut = cut_of_best<N>(key, id, there, take, key_lo, key_hi, S);
-#pragma unroll
-  for (int u = 0; u < N; ++u) {
-    if ((there >> u & 1u) && (key[u] > cut.x || (key[u] == cut.x && id[u] <= cut.y))) {
-      const bool is_last = key[u] == cut.x && id[u] == cut.y;
-      S.hist[is_last ? take - 1u : atomicAdd(&S.word[2], 1u)] = id[u];
-    }
+  const uint2 cut = find_cut(S, false, c, take, top, open, id_lo, n_ids);
+  __syncthreads();      // the search is through with S.hist
+#pragma unroll 1
+  for (uint32_t i = tid; i < c; i += kEmitThreads) {
+    const uint32_t key = S.stage[i].y & 0x7fffffffu, id = S.stage[i].x - id_lo;
+    if (key > cut.x || (key == cut.x && id <= cut.y))
+      S.hist[key == cut.x && id == cut.y ? take - 1u : atomicAdd(&S.word[2], 1u)] = i;
   }
   __syncthreads();
   return cut.x;
 }
 
-__device__ __forceinline__ uint32_t pick_few(const uint2* cand, uint32_t c, uint32_t take, uint32_t key_lo, uint32_t key_hi,
-                                             EmitShared& S) {
-  return c <= (uint32_t)kEmitThreads ? pick_best<1>(cand, c, take, key_lo, key_hi, S)
-                                     : pick_best<kPickMax / kEmitThreads>(cand, c, take, key_lo, key_hi, S);
-}
-
-// Top-k of a small tensor, from registers: every thread holds N of its elements.  Returns the k-th largest key.
-template <int N>
+// Top-k of a small tensor: its values lie in shared memory.  Returns the k-th largest key.
 __device__ __forceinline__ uint32_t top_direct(const SelectArgs& A, const Job& J, EmitShared& S) {
+  static_assert(kTopDirect == 2u * kStageItems && kTopDirect == 16u * kEmitThreads, "the values are the words of EmitShared::stage");
   const uint32_t tid = threadIdx.x;
-  uint32_t key[N], id[N], bits[N], there = 0;
+  uint4* const words = reinterpret_cast<uint4*>(S.stage);
+  uint32_t top = 0;
+  uint4 a[4];
 #pragma unroll
-  for (int u = 0; u < N / 4; ++u) {
-    const uint32_t i = (u * kEmitThreads + tid) * 4u;
-    const bool act = i < J.sd.n_pad;
-    const float4 a = act ? *reinterpret_cast<const float4*>(A.resid + J.sd.off + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-    there |= (act ? 15u : 0u) << (4 * u);
-    const float v[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      id[4 * u + e] = J.sd.off + i + e;
-      bits[4 * u + e] = __float_as_uint(v[e]);
-      key[4 * u + e] = key_bits(v[e]);
-    }
+  for (int u = 0; u < 4; ++u) {
+    const uint32_t i = u * kEmitThreads + tid;
+    a[u] = i * 4u < J.sd.n_pad ? *reinterpret_cast<const uint4*>(A.resid + J.sd.off + i * 4u) : make_uint4(0u, 0u, 0u, 0u);
   }
-  if (tid < 64u) S.cnt[tid] = 0u;
-  __syncthreads();
-  const uint2 cut = cut_of_best<N>(key, id, there, J.kk, 0u, 0x7fffffffu, S);
-  uint32_t take = 0;
 #pragma unroll
-  for (int u = 0; u < N; ++u)
-    take |= (uint32_t)((there >> u & 1u) && (key[u] > cut.x || (key[u] == cut.x && id[u] <= cut.y))) << u;
+  for (int u = 0; u < 4; ++u) {
+    words[u * kEmitThreads + tid] = a[u];
+    top = max(max(max(top, a[u].x & 0x7fffffffu), max(a[u].y & 0x7fffffffu, a[u].z & 0x7fffffffu)), a[u].w & 0x7fffffffu);
+  }
+  top = block_max_u32(top, S.tmp);
+  const uint2 cut = find_cut(S, true, J.sd.n_pad, J.kk, top, kTwoOctaves, 0u, J.sd.n_pad);
+  uint32_t take = 0;      // bit 4 u + e: element e of the thread's u-th four
+#pragma unroll 1
+  for (uint32_t u = 0; u < 4u; ++u) {
+    const uint32_t i = (u * kEmitThreads + tid) * 4u;
+    const uint4 v = words[u * kEmitThreads + tid];
+    const uint32_t key[4] = {v.x & 0x7fffffffu, v.y & 0x7fffffffu, v.z & 0x7fffffffu, v.w & 0x7fffffffu};
+#pragma unroll
+    for (uint32_t e = 0; e < 4u; ++e)
+      take |= (uint32_t)(i < J.sd.n_pad && (key[e] > cut.x || (key[e] == cut.x && i + e <= cut.y))) << (4u * u + e);
+  }
   uint32_t total;
   const uint32_t ex = block_excl_scan(__popc(take), S.tmp, total);
-  send_marked<N>(A, J, S, id, bits, take, ex, total, 0u);
+#pragma unroll 1
+  for (uint32_t w = 0; w < total; w += 2048u) {
+    uint32_t p = ex - w;
+#pragma unroll 1
+    for (uint32_t left = take; left != 0u; left &= left - 1u, ++p) {
+      const uint32_t b = __ffs(left) - 1u;
+      if (p < 2048u) S.hist[p] = ((b >> 2) * kEmitThreads + tid) * 4u + (b & 3u);
+    }
+    __syncthreads();
+    send_staged(A, S, kWords, min(2048u, total - w), w);
+    __syncthreads();
+  }
   return cut.x;
 }
 
-// The same for more pairs than registers hold: a radix search over the bits that the keys of `cand` leave open, 11 at a time.
+// The same for more items than shared memory holds: a radix search over the bits that the keys of `cand` leave open, 11 at a time.
 // Fixed digits of the whole key put nearly all pairs, which lie close together, on one counter: 25,000 adds to one address of
 // shared memory took longer than all passes over the pairs.  Ids lie in [id_lo, id_lo + n_ids).
 __device__ __forceinline__ uint2 cut_of_many(const uint2* cand, uint32_t c, uint32_t take, uint32_t id_lo, uint32_t n_ids,
@@ -656,7 +752,7 @@ __device__ __forceinline__ uint2 cut_of_many(const uint2* cand, uint32_t c, uint
       for (int u = 0; u < kIlp; ++u) e[u] = i0 + u * kEmitThreads < c ? __ldcg(cand + i0 + u * kEmitThreads) : make_uint2(0u, 0u);
 #pragma unroll
       for (int u = 0; u < kIlp; ++u)
-        if (i0 + u * kEmitThreads < c) f(e[u]);
+        if (i0 + u * kEmitThreads < c) f(make_uint2(e[u].x, e[u].y & 0x7fffffffu));
     }
   };
   // The digit of the rem-th value, counted from the largest (`down`) or the smallest one: S.res = {digit, values still to be
@@ -731,8 +827,9 @@ __device__ __forceinline__ uint2 cut_of_many(const uint2* cand, uint32_t c, uint
 // by one CTA of 1024 threads, which drew a stream position per item from one address and copied a block with one thread,
 // this took up to 0.1 ms for the 25,000 undecided items of a 64 MB bucket whose gradients had changed in scale.
 template <bool kBlock>
-__device__ __forceinline__ uint32_t send_best(const SelectArgs& A, const Job& J, EmitShared& S, const uint2* cand, uint32_t c,
-                                              uint32_t take, uint32_t done, uint2* list) {
+__device__ __noinline__ uint32_t send_best(const SelectArgs& A, EmitShared& S, const uint2* cand, uint32_t c, uint32_t take,
+                                           uint32_t done, uint2* list) {
+  const Job J = job_of(A, kBlock);
   constexpr uint32_t kPerItem = kBlock ? 16u : 1u;
   constexpr int kIlp = kStageItems / kEmitThreads;
   const uint32_t tid = threadIdx.x;
@@ -743,7 +840,8 @@ __device__ __forceinline__ uint32_t send_best(const SelectArgs& A, const Job& J,
 #pragma unroll
     for (int u = 0; u < kIlp; ++u) {
       const uint32_t i = i0 + u * kEmitThreads + tid;
-      const uint2 e = i < c ? __ldcg(cand + i) : make_uint2(0xFFFFFFFFu, 0u);
+      uint2 e = i < c ? __ldcg(cand + i) : make_uint2(0xFFFFFFFFu, 0u);
+      e.y &= 0x7fffffffu;
       id[u] = e.x;
       const bool is_last = e.y == cut.x && e.x == cut.y;
       if (is_last) list[take - 1u].x = e.x;
@@ -771,9 +869,7 @@ __device__ __forceinline__ uint32_t send_best(const SelectArgs& A, const Job& J,
     }
     __syncthreads();
     const uint32_t p0 = done * kPerItem + t0;      // the last block may be cut off at k
-    const uint32_t m = min(min(kStageItems, take * kPerItem - t0), J.sd.k > p0 ? J.sd.k - p0 : 0u);
-#pragma unroll 1
-    for (uint32_t q = tid; q < m; q += kEmitThreads) emit_and_keep(A, J, p0 + q, stage[q].x, __uint_as_float(stage[q].y));
+    send_staged(A, S, kInOrder, min(min(kStageItems, take * kPerItem - t0), J.sd.k > p0 ? J.sd.k - p0 : 0u), p0);
     __syncthreads();
   }
   return cut.x;
@@ -784,49 +880,66 @@ __device__ __forceinline__ uint32_t settle_top(const SelectArgs& A, const Job& J
                                                uint32_t c, uint32_t rem, uint32_t key_lo, uint32_t key_hi) {
   const uint32_t done = J.kk - rem;
   if (c <= kPickMax) {
-    const uint32_t t_key = pick_few(undecided, c, rem, key_lo, key_hi, S);
-#pragma unroll 1
-    for (uint32_t q = threadIdx.x; q < rem; q += kEmitThreads) {
-      const uint32_t gi = S.hist[q];
-      emit_and_keep(A, J, done + q, gi, __ldcg(A.resid + gi));
-    }
+    const uint32_t t_key = pick_few(undecided, c, rem, key_hi - 1u, 32u - __clz(key_hi - 1u - key_lo), J.sd.off, J.sd.n_pad, S);
+    send_staged(A, S, kNamed, rem, done);
     return t_key;
   }
-  return send_best<false>(A, J, S, undecided, c, rem, done, A.cand + J.sd.off);
+  return send_best<false>(A, S, undecided, c, rem, done, A.cand + J.sd.off);
 }
 
 // Sends the items [j0, j1) of one piece at positions base + j; items and positions are in index order.  The dependent loads
-// (list, residual) of four entries per thread travel together; the entries then pass through shared memory as above.
+// (list, residual) of a thread travel together; the entries then pass through shared memory as above.
 template <bool kBlock>
 __device__ __forceinline__ void send_range(const SelectArgs& A, const Job& J, EmitShared& S, const uint2* lists,
                                            uint32_t base, uint32_t j0, uint32_t j1) {
   constexpr uint32_t kPerItem = kBlock ? 16u : 1u, kArea = kBlock ? kRunBlocks : kRunElems;
-  constexpr uint32_t kIlp = kStageItems / kEmitThreads;
-  uint2* const stage = S.stage;
   const uint32_t end = j1 * kPerItem;
+#pragma unroll 1
   for (uint32_t t0 = j0 * kPerItem; t0 < end; t0 += kStageItems) {
-    uint2 e[kIlp];
+    if (kBlock) {
+      // four lanes to a block
+      constexpr int kPer = kStageItems / 4 / kEmitThreads;
+      uint32_t gi[kPer];
+      float4 a[kPer];
 #pragma unroll
-    for (int u = 0; u < (int)kIlp; ++u) {
-      const uint32_t t = t0 + u * kEmitThreads + threadIdx.x;
-      e[u] = make_uint2(0u, 0u);
-      if (t < end) {
-        const uint32_t j = t / kPerItem, run = run_of(S.pre, j);
-        e[u] = lists[run * kArea + (j - S.pre[run])];
-        if (kBlock) e[u].x = e[u].x * 16u + (t & 15u);
+      for (int u = 0; u < kPer; ++u) {
+        const uint32_t t = t0 + (u * kEmitThreads + threadIdx.x) * 4u, j = t / 16u, run = run_of(S.pre, j);
+        if (t < end) gi[u] = lists[run * kArea + (j - S.pre[run])].x * 16u + (t & 15u);
       }
-    }
 #pragma unroll
-    for (int u = 0; u < (int)kIlp; ++u) {
-      if (kBlock && t0 + u * kEmitThreads + threadIdx.x < end) e[u].y = __float_as_uint(__ldcg(A.resid + e[u].x));
-      stage[u * kEmitThreads + threadIdx.x] = e[u];
+      for (int u = 0; u < kPer; ++u)
+        if (t0 + (u * kEmitThreads + threadIdx.x) * 4u < end) a[u] = __ldcg(reinterpret_cast<const float4*>(A.resid + gi[u]));
+#pragma unroll
+      for (int u = 0; u < kPer; ++u) {
+        const uint32_t q = (u * kEmitThreads + threadIdx.x) * 4u;
+        if (t0 + q < end) {
+          uint4* const to = reinterpret_cast<uint4*>(&S.stage[q]);
+          to[0] = make_uint4(gi[u], __float_as_uint(a[u].x), gi[u] + 1u, __float_as_uint(a[u].y));
+          to[1] = make_uint4(gi[u] + 2u, __float_as_uint(a[u].z), gi[u] + 3u, __float_as_uint(a[u].w));
+        }
+      }
+    } else {
+      // 256 consecutive items to a warp: a lane's items are 32 apart, and its run moves on with them
+      constexpr int kPer = kStageItems / kEmitThreads;
+      const uint32_t q0 = (threadIdx.x & ~31u) * kPer + (threadIdx.x & 31u);
+      uint32_t run = run_of(S.pre, t0 + q0);
+      uint2 e[kPer];
+#pragma unroll
+      for (int u = 0; u < kPer; ++u) {
+        const uint32_t j = t0 + q0 + u * 32u;
+        if (j < end) {
+          while (S.pre[run + 1u] <= j) ++run;
+          e[u] = lists[run * kArea + (j - S.pre[run])];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kPer; ++u)
+        if (t0 + q0 + u * 32u < end) S.stage[q0 + u * 32u] = e[u];
     }
     __syncthreads();
     // a truncated last block leaves the residual exact: only emitted elements are cleared
-    const uint32_t p0 = base * kPerItem + t0, m = min(min(kStageItems, end - t0), J.sd.k > p0 ? J.sd.k - p0 : 0u);
-#pragma unroll 1
-    for (uint32_t q = threadIdx.x; q < m; q += kEmitThreads)
-      emit_and_keep(A, J, p0 + q, stage[q].x, __uint_as_float(stage[q].y));
+    const uint32_t p0 = base * kPerItem + t0;
+    send_staged(A, S, kInOrder, min(min(kStageItems, end - t0), J.sd.k > p0 ? J.sd.k - p0 : 0u), p0);
     __syncthreads();
   }
 }
@@ -835,8 +948,8 @@ __device__ __forceinline__ void send_range(const SelectArgs& A, const Job& J, Em
 // the fill.  A listed block is sent whenever the stream is short; what the narrow wire format's rounding leaves of it in the
 // residual waits for the next select, so that a stream names an element once.  The lists, and not the residual, say which
 // blocks these are: other CTAs of the tensor may be sending them now.  Returns the number collected by this CTA.
-__device__ __forceinline__ uint32_t collect_unlisted(const SelectArgs& A, const Job& J, EmitShared& S, const uint2* area,
-                                                     uint32_t total, uint2* cand) {
+__device__ __noinline__ uint32_t collect_unlisted(const SelectArgs& A, EmitShared& S, const uint2* area, uint32_t total, uint2* cand) {
+  const Job J = job_of(A, true);
   constexpr uint32_t kQuads = kEmitThreads / 4, kKeys = 8;      // blocks side by side; keys a lane keeps per round
   static_assert(kMaxPieceElems / 16u / 32u <= 2048u, "a bit per block of a piece fits EmitShared::hist");
   const uint32_t tid = threadIdx.x, first = J.pc.start >> 4;
@@ -885,6 +998,31 @@ __device__ __forceinline__ uint32_t collect_unlisted(const SelectArgs& A, const 
   return done;
 }
 
+// The candidates do not reach down to the k-th largest value: a histogram of the rest.
+__device__ __noinline__ void count_rest(const SelectArgs& A, EmitShared& S) {
+  const uint32_t tid = threadIdx.x;
+  const Job J = job_of(A, false);
+  const uint32_t cut = top_cut(A.state[J.pc.seg], J.sd.n_pad);
+  for (uint32_t b = tid; b < (uint32_t)kHistBins; b += kEmitThreads) S.hist[b] = 0u;
+  __syncthreads();
+  uint32_t zeros = 0;
+#pragma unroll 4
+  for (uint32_t i = tid * 4u; i < J.len; i += kEmitThreads * 4u) {
+    const float4 a = *reinterpret_cast<const float4*>(A.resid + J.pc.start + i);
+    const uint32_t key[4] = {key_bits(a.x), key_bits(a.y), key_bits(a.z), key_bits(a.w)};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if (key[e] == 0u) ++zeros;
+      else if (key[e] < cut) atomicAdd(&S.hist[rest_bin(key[e], cut)], 1u);
+    }
+  }
+  block_excl_scan(zeros, S.tmp, zeros);
+  uint32_t* gh = A.hist_rest + (size_t)J.pc.seg * kHistBins;
+  for (uint32_t b = tid; b < (uint32_t)kHistBins; b += kEmitThreads)
+    if (S.hist[b]) atomicAdd(gh + b, S.hist[b]);
+  if (tid == 0) A.run_cnt[blockIdx.x << A.piece_shift] = zeros;     // this CTA has read its own counts
+}
+
 // Thread 0 of the last CTA of a top-k tensor: what the next select starts from.  Every candidate costs a list entry and a
 // histogram count; candidates that fall short cost two more passes over the tensor by the emitting kernels (a step of 16 M
 // elements takes up to 125 us more, one of 3 M 60) and hold up the whole bucket.  How many more
@@ -906,7 +1044,7 @@ __device__ __forceinline__ void step_top(const SelectArgs& A, const Job& J, SegS
 }  // namespace
 
 template <int MODE>
-__global__ void __launch_bounds__(kEmitThreads, 4) k_emit(SelectArgs A) {
+__global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const __grid_constant__ SelectArgs A) {
   __shared__ EmitShared S;
   constexpr bool kBlock = MODE == kScanBlock;
   const uint32_t tid = threadIdx.x;
@@ -929,6 +1067,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(SelectArgs A) {
         }
       }
     if (tid == 0) { S.sum = 0ull; S.at[0] = 0u; S.at[1] = 0u; }
+    note_destinations(A, J, S);
     uint32_t total, near_total = 0;
     uint32_t ex = block_excl_scan(cnt & 0xffffu, S.tmp, total);
     if (tid <= kMaxPieceRuns) S.pre[tid] = ex;
@@ -973,44 +1112,26 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(SelectArgs A) {
       const bool direct = J.sd.n_pad <= kTopDirect;
       if (direct) {
         if (may) {
-          const uint32_t t_key = J.sd.n_pad <= 4u * kEmitThreads ? top_direct<4>(A, J, S) : top_direct<16>(A, J, S);
+          const uint32_t t_key = top_direct(A, J, S);
           if (tid == 0) step_top(A, J, ss, t_key, 0u);
         }
       } else if (short_of && ok) {
-        // the candidates do not reach down to the k-th largest value: a histogram of the rest, for `refill`
-        const uint32_t cut = top_cut(ss, J.sd.n_pad);
-        for (uint32_t b = tid; b < (uint32_t)kHistBins; b += kEmitThreads) S.hist[b] = 0u;
-        __syncthreads();
-        uint32_t zeros = 0;
-#pragma unroll 4
-        for (uint32_t i = tid * 4u; i < J.len; i += kEmitThreads * 4u) {
-          const float4 a = *reinterpret_cast<const float4*>(A.resid + J.pc.start + i);
-          const uint32_t key[4] = {key_bits(a.x), key_bits(a.y), key_bits(a.z), key_bits(a.w)};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            if (key[e] == 0u) ++zeros;
-            else if (key[e] < cut) atomicAdd(&S.hist[rest_bin(key[e], cut)], 1u);
-          }
-        }
-        block_excl_scan(zeros, S.tmp, zeros);
-        uint32_t* gh = A.hist_rest + (size_t)J.pc.seg * kHistBins;
-        for (uint32_t b = tid; b < (uint32_t)kHistBins; b += kEmitThreads)
-          if (S.hist[b]) atomicAdd(gh + b, S.hist[b]);
-        if (tid == 0) A.run_cnt[blockIdx.x << A.piece_shift] = zeros;     // this CTA has read its own counts
+        count_rest(A, S);      // for `refill`
       } else if (!short_of) {
         plan_top(A.hist_top + (size_t)J.pc.first * kHistBins, hist_copies(J.sd.n_pad), found, J.kk, false, S);
         top_bin_range(S.res[0], top_centre(ss), key_lo, key_hi);
         if (may) {
           constexpr int kItems = 8;
+#pragma unroll 1
           for (uint32_t j0 = 0; j0 < total; j0 += kEmitThreads * kItems) {
             uint32_t idx[kItems], bits[kItems];
+            uint32_t j = j0 + tid * kItems, run = run_of(S.pre, j);      // the stream keeps the lists' order: the update reads it faster
 #pragma unroll
-            for (int u = 0; u < kItems; ++u) {
-              const uint32_t j = j0 + tid * kItems + u;     // the stream keeps the lists' order: the update reads it faster
+            for (int u = 0; u < kItems; ++u, ++j) {
               idx[u] = kSentinelIdx;
               bits[u] = 0u;
               if (j < total) {
-                const uint32_t run = run_of(S.pre, j);
+                while (S.pre[run + 1u] <= j) ++run;
                 const uint2 e = area[run * kArea + (j - S.pre[run])];
                 idx[u] = e.x;
                 bits[u] = e.y;
@@ -1048,7 +1169,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(SelectArgs A) {
       const bool rescan = kBlock && short_of && (!ss.inited || c_near < J.kk - found);
       uint32_t collected = 0;
       if (rescan) {
-        collected = collect_unlisted(A, J, S, area, total, nears);
+        collected = collect_unlisted(A, S, area, total, nears);
       } else if (kBlock && short_of && near_total) {
         // the fill needs the tensor's near misses in one place
         if (tid == 0) S.word[2] = J.pc.count == 1u ? 0u : atomicAdd(&J.wp->cand_cnt, near_total);
@@ -1115,17 +1236,19 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(SelectArgs A) {
           const uint32_t c = !rescan ? c_near : J.pc.count == 1u ? collected : __ldcg(&J.wp->cand_cnt);
           const uint32_t take = min(need, c);
           if (take && c <= kPickMax) {
-            t_key = pick_few(nears, c, take, 0u, 0x7fffffffu, S);
+            // none reaches the threshold, and the best lie in the two octaves under it
+            const uint32_t top = ss.inited ? max(__float_as_uint(ss.tau), 1u) - 1u : 0x7fffffffu;
+            t_key = pick_few(nears, c, take, top, ss.inited ? kTwoOctaves : 31u, J.sd.off >> 4, J.sd.n_pad >> 4, S);
 #pragma unroll 1
             for (uint32_t e = tid; e < take * 16u; e += kEmitThreads) {
               const uint32_t q = e >> 4, p = (found + q) * 16u + (e & 15u);
               if (p < J.sd.k) {   // only the lowest-ranked block can be cut off
-                const uint32_t gi = S.hist[q] * 16u + (e & 15u);
-                emit_and_keep(A, J, p, gi, __ldcg(A.resid + gi));
+                const uint32_t gi = S.stage[S.hist[q]].x * 16u + (e & 15u);
+                emit_and_keep(A, S, p, gi, __ldcg(A.resid + gi));
               }
             }
           } else if (take) {
-            t_key = send_best<true>(A, J, S, nears, c, take, found, A.cand + (J.sd.off >> 4));
+            t_key = send_best<true>(A, S, nears, c, take, found, A.cand + (J.sd.off >> 4));
           }
           // fewer blocks with anything in them than the budget: the rest of the stream says "no entry"
 #pragma unroll 1
@@ -1174,7 +1297,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(SelectArgs A) {
 }
 
 // Top-k tensors whose candidates fell short: the exact selection from the residual, with the histogram that `emit` took.
-__global__ void __launch_bounds__(kEmitThreads, 2) k_refill(SelectArgs A) {
+__global__ void __launch_bounds__(kEmitThreads, 2) k_refill(const __grid_constant__ SelectArgs A) {
   __shared__ EmitShared S;
   if (ld_volatile_u32(A.refills) == 0u) return;     // the same for every CTA: it is cleared behind the last one
   const uint32_t tid = threadIdx.x;
@@ -1182,6 +1305,7 @@ __global__ void __launch_bounds__(kEmitThreads, 2) k_refill(SelectArgs A) {
   const bool ok = ld_volatile_u32(A.status) == kOk;
   if (!(J.sd.reserved & kSegSkip) && J.wp->refill != 0u) {
     if (tid == 0) S.word[0] = ok && acks_arrived(A, J.epoch) ? 1u : 0u;
+    note_destinations(A, J, S);
     const SegState ss = A.state[J.pc.seg];
     const uint32_t cut = top_cut(ss, J.sd.n_pad), found = J.wp->found;      // found < kk items reach the cut
     uint32_t* gh = A.hist_rest + (size_t)J.pc.seg * kHistBins;
@@ -1209,7 +1333,7 @@ __global__ void __launch_bounds__(kEmitThreads, 2) k_refill(SelectArgs A) {
         for (int e = 0; e < 4; ++e) zero |= (uint32_t)((bits[e] & 0x7fffffffu) == 0u) << e;
         const uint32_t ex = block_excl_scan(__popc(zero), S.tmp, total);
         while (zero && base + ex + __popc(zero) > rem) zero &= ~(0x80000000u >> __clz(zero));      // the budget ends here
-        send_marked<4>(A, J, S, idx, bits, zero, ex, min(total, rem - base), J.kk - rem + base);
+        send_marked<4>(A, S, idx, bits, zero, ex, min(total, rem - base), J.kk - rem + base);
         base += total;
       }
     }

@@ -86,8 +86,7 @@ __device__ __forceinline__ void publish_checksums(const SelectArgs& A, uint32_t 
 
 // The receive slot about to be overwritten was last used two epochs ago; every destination must have consumed
 // it.  One thread calls this right before its CTA stores into the destinations.
-__device__ __forceinline__ bool acks_arrived(const SelectArgs& A, uint32_t epoch) {
-  if (!A.use_acks || epoch <= 2u) return true;
+static __device__ __noinline__ bool wait_acks(const SelectArgs& A, uint32_t epoch) {
   const uint64_t want = (uint64_t)epoch - 2u;
   for (int p = 0; p < A.world; ++p) {
     if (!wait_ge_bounded(A.ack_local + (size_t)(epoch & 1u) * A.world + p, want, A.timeout_ns)) {
@@ -96,6 +95,10 @@ __device__ __forceinline__ bool acks_arrived(const SelectArgs& A, uint32_t epoch
     }
   }
   return true;
+}
+
+__device__ __forceinline__ bool acks_arrived(const SelectArgs& A, uint32_t epoch) {
+  return !A.use_acks || epoch <= 2u || wait_acks(A, epoch);
 }
 
 // Completion of a select chain, called by thread 0 of every CTA of its last kernel after a CTA barrier: the last
