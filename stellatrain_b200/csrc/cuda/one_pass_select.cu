@@ -166,11 +166,12 @@ __global__ void __launch_bounds__(kScanThreads, 4) k_scan(SelectArgs A) {
   // gradient pointer (a second level of dependent loads) are fetched.
   const Chunk ch = A.chunks[blockIdx.x];
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  // Listed elements of half a run meet here, so that all lanes take part in storing (and, top-k, counting) them.  A fuller
-  // half goes straight to the list.
-  constexpr uint32_t kStage = MODE == kScanBlock ? 1u : 96u;
-  __shared__ uint2 s_stage[kScanWarps][kStage];
-  uint2* const stage = s_stage[warp];
+  // Half a run that has listed elements, and their places in it: all lanes take part in storing (and, top-k, counting) them.  The
+  // lists of top-k are instructions before they are traffic: with the listed values stored from registers, one predicated store
+  // for each of a lane's sixteen, this kernel issued 157 warp instructions per 128 elements at 1 % and took 37 us where
+  // threshold-v16 takes 29 (64 MB bucket).
+  __shared__ float4 s_half[MODE == kScanBlock ? 1 : kScanWarps][MODE == kScanBlock ? 1 : kHalf / 4];
+  __shared__ uint16_t s_place[MODE == kScanBlock ? 1 : kScanWarps][MODE == kScanBlock ? 1 : kHalf];
   if (blockIdx.x == 0 && threadIdx.x == 0 && A.stamps != nullptr) A.stamps[0] = global_timer_ns();
 
   const uint32_t piece_shift = A.piece_shift + kRunShift;      // of elements
@@ -205,7 +206,9 @@ __global__ void __launch_bounds__(kScanThreads, 4) k_scan(SelectArgs A) {
     if (MODE == kScanBlock && ss.inited)
       near_lo = __float_as_uint(fmaxf(ss.tau * (1.f - window_or(ss.reserved[0], kWindowDefault)), 0.f));
 
-    uint32_t n_list = 0, mx = 0;        // entries listed so far; largest key of this lane
+    const float cut_value = __uint_as_float(cut);
+    uint32_t n_list = 0;                // entries listed so far
+    float mx = 0.f;                     // largest magnitude of this lane
     uint32_t own[2] = {0u, 0u};         // block mode: keys of two of the run's blocks, numbers h * 32 + (lane & 3) * 8 + lane / 4
     uint2* list = A.cand + (MODE == kScanBlock ? start >> 4 : start);
 #pragma unroll
@@ -252,10 +255,12 @@ __global__ void __launch_bounds__(kScanThreads, 4) k_scan(SelectArgs A) {
           const uint32_t key = __float_as_uint(quad_l1(a));   // the same value in the four lanes of a block
           if ((lane & 3u) == (uint32_t)j) own[h] = key;
         } else {
-          const uint32_t k0 = key_bits(a.x), k1 = key_bits(a.y), k2 = key_bits(a.z), k3 = key_bits(a.w);
-          mask |= (k0 >= cut ? 1u << (4 * j) : 0u) | (k1 >= cut ? 2u << (4 * j) : 0u) |
-                  (k2 >= cut ? 4u << (4 * j) : 0u) | (k3 >= cut ? 8u << (4 * j) : 0u);
-          if (MODE == kScanElem) mx = max(mx, max(max(k0, k1), max(k2, k3)));
+          // magnitudes compare as their bits do, and nothing reaches a cut that is no number
+          if (fabsf(a.x) >= cut_value) mask |= 1u << (4 * j);
+          if (fabsf(a.y) >= cut_value) mask |= 2u << (4 * j);
+          if (fabsf(a.z) >= cut_value) mask |= 4u << (4 * j);
+          if (fabsf(a.w) >= cut_value) mask |= 8u << (4 * j);
+          if (MODE == kScanElem) mx = fmaxf(mx, fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w))));
         }
       }
       if (MODE == kScanElem && n_valid < (h + 1) * kHalf) {
@@ -271,33 +276,37 @@ __global__ void __launch_bounds__(kScanThreads, 4) k_scan(SelectArgs A) {
         n4 = (n4 & 0xFu) | (n4 & 0xF0u) << 4 | (n4 & 0xF00u) << 8 | (n4 & 0xF000u) << 12;
         const uint32_t incl = warp_incl_scan(n4), ex = incl - n4;
         const uint32_t all = __shfl_sync(0xffffffffu, incl, 31);
-        const uint32_t n_half = (all & 0xFFu) + ((all >> 8) & 0xFFu) + ((all >> 16) & 0xFFu) + (all >> 24);
-        uint2* const dst = list + n_list;
-        uint2* const first = n_half <= kStage ? stage : dst;
-        uint32_t before = 0;
+        const uint32_t c0 = all & 0xFFu, c1 = c0 + ((all >> 8) & 0xFFu), c2 = c1 + ((all >> 16) & 0xFFu), n_half = c2 + (all >> 24);
+        // the lane's next place for an element of each float4, 16 bits each
+        uint32_t at01 = (ex & 0xFFu) | (c0 + ((ex >> 8) & 0xFFu)) << 16;
+        uint32_t at23 = (c1 + ((ex >> 16) & 0xFFu)) | (c2 + (ex >> 24)) << 16;
+        float4* const half = s_half[warp];
+        uint16_t* const place = s_place[warp];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          if (mask & (15u << (4 * j))) {
-            const uint32_t at = start + h0 + j * 128u;
-            uint2* to = first + before + ((ex >> (8 * j)) & 0xFFu);
-            if (mask & (1u << (4 * j))) *to++ = make_uint2(at, __float_as_uint(rv[j].x));
-            if (mask & (2u << (4 * j))) *to++ = make_uint2(at + 1u, __float_as_uint(rv[j].y));
-            if (mask & (4u << (4 * j))) *to++ = make_uint2(at + 2u, __float_as_uint(rv[j].z));
-            if (mask & (8u << (4 * j))) *to++ = make_uint2(at + 3u, __float_as_uint(rv[j].w));
-          }
-          before += (all >> (8 * j)) & 0xFFu;
+        for (int j = 0; j < 4; ++j) half[j * 32 + lane] = rv[j];
+        for (uint32_t left = mask; left != 0u; left &= left - 1u) {
+          const uint32_t bit = __ffs(left) - 1u, shift = (bit & 4u) << 2;
+          const uint32_t at = bit & 8u ? at23 : at01;
+          place[(at >> shift) & 0xFFFFu] = (uint16_t)((bit >> 2) * 128u + lane * 4u + (bit & 3u));
+          if (bit & 8u) at23 += 1u << shift; else at01 += 1u << shift;
         }
         __syncwarp();
-        if (n_half <= kStage)
-          for (uint32_t q = lane; q < n_half; q += 32u) dst[q] = stage[q];
+        const float* const value = reinterpret_cast<const float*>(half);
+        uint2* const dst = list + n_list;
+        // Histogram of top-k's candidates.  The top bin, which holds many of them, is not counted: `emit` knows their number.
+        uint32_t* gh = nullptr;
+        uint32_t centre = 0;
         if (MODE == kScanTop) {
-          // Histogram of the candidates.  The top bin, which holds many of them, is not counted: `emit` knows their number.
-          const uint32_t centre = top_centre(ss);
+          centre = top_centre(ss);
           const uint32_t piece = seg_rel >> piece_shift;      // of the tensor
           const uint32_t first_piece = ((ch.run0 + rel / kRunElems) >> A.piece_shift) - piece;
-          uint32_t* const gh = A.hist_top + (size_t)(first_piece + (piece & (hist_copies(sd.n_pad) - 1u))) * kHistBins;
-          for (uint32_t q = lane; q < n_half; q += 32u) {
-            const uint32_t b = top_bin(first[q].y & 0x7fffffffu, centre);
+          gh = A.hist_top + (size_t)(first_piece + (piece & (hist_copies(sd.n_pad) - 1u))) * kHistBins;
+        }
+        for (uint32_t q = lane; q < n_half; q += 32u) {
+          const uint32_t i = place[q], bits = __float_as_uint(value[i]);
+          dst[q] = make_uint2(start + h * kHalf + i, bits);
+          if (MODE == kScanTop) {
+            const uint32_t b = top_bin(bits & 0x7fffffffu, centre);
             if (b != (uint32_t)(kHistBins - 1)) atomicAdd(gh + b, 1u);
           }
         }
@@ -325,9 +334,9 @@ __global__ void __launch_bounds__(kScanThreads, 4) k_scan(SelectArgs A) {
       }
     }
     if (MODE == kScanElem) {
-      mx = __reduce_max_sync(0xffffffffu, mx);
+      const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
       // runs that do not raise the maximum leave its one address alone
-      if (lane == 0 && mx > ld_volatile_u32(&A.work[ch.seg].max_bits)) atomicMax(&A.work[ch.seg].max_bits, mx);
+      if (lane == 0 && top > ld_volatile_u32(&A.work[ch.seg].max_bits)) atomicMax(&A.work[ch.seg].max_bits, top);
     }
     if (lane == 0) {
       const uint32_t run = ch.run0 + rel / kRunElems;
