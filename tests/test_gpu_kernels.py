@@ -466,6 +466,27 @@ def test_single_source_apply_at_the_edges_of_its_grid(compressor, n, narrow, cta
     assert torch.equal(pair[0].param, pair[1].param) and torch.equal(pair[0].rec, pair[1].rec)
 
 
+@pytest.mark.parametrize("sizes,ratio", [([1, 1025, 131072, 131073, 400_001], 0.5), ([3_000_003, 17], 0.97)])
+def test_randomk_positions_of_a_tensor_in_pieces(sizes, ratio):
+    """The pieces of a tensor share its positions out: position j holds element (start + j stride) mod n, as one CTA wrote it."""
+    b = make_bucket("randomk", ratio, sizes=sizes, chunk=8192)
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    for step in range(2):
+        fill_grads(b, gen)
+        a = b.grad + b.resid
+        b.select()
+        torch.cuda.synchronize()
+        b.check_status()
+        idx, val = read_stream(b, step + 1)
+        for s, _, _ in seg_slices(b):
+            i = idx[s.out_off : s.out_off + s.k] - s.off
+            assert (i >= 0).all() and (i < s.numel).all()
+            assert s.k < 3 or (np.diff(i) % s.numel == np.diff(i)[0] % s.numel).all()
+            assert torch.equal(val[s.out_off : s.out_off + s.k], a[torch.from_numpy(i + s.off).cuda()].cpu())
+        a[torch.from_numpy(idx).cuda()] = 0.0
+        assert torch.equal(b.resid, a)
+
+
 def test_randomk_stream_is_valid():
     b = make_bucket("randomk", 0.9, sizes=[1000, 4096, 17])
     gen = torch.Generator(device="cuda").manual_seed(3)
