@@ -220,13 +220,16 @@ struct BucketHandle : public st::BucketHandle {
     const uint32_t zero_grad = sel.zero_grad;
     float* const grad = sel.grad;
     sel.grad = as_ptr<float>(input);
-    sel.fresh = 1u;
+    sel.fresh = n;
+    float* const resid = sel.resid;
+    if (one_pass_next()) sel.resid = sel.grad;      // read in place, see SelectArgs::fresh
     sel.zero_grad = 0u;
     uint32_t words[2] = {0u, 0u};
     cudaError_t e = cudaMemsetAsync(sel.status + 1, 0, sizeof(uint32_t), s);
     if (e == cudaSuccess) e = st::BucketHandle::select(s);
     sel.grad = grad;
     sel.fresh = 0u;
+    sel.resid = resid;
     sel.zero_grad = zero_grad;
     st::UnpackArgs U = {app.recv, app.slot_stride, app.cap, n, sel.epoch, as_ptr<int32_t>(idx), as_ptr<float>(val), sel.status + 1};
     if (e == cudaSuccess) e = st::launch_unpack(U, s);

@@ -23,9 +23,10 @@ struct BucketHandle {
   bool last_select_fused = false;
 
   bool can_fuse() const { return one_pass_possible(sel); }
+  bool one_pass_next() const { return fused_enabled && thresholds_ready && can_fuse(); }
 
   cudaError_t select(cudaStream_t stream) {
-    const bool fused = fused_enabled && thresholds_ready && can_fuse();
+    const bool fused = one_pass_next();
     const cudaError_t e = fused ? launch_select_one_pass(sel, stream) : launch_select(sel, randomk_seed, stream);
     thresholds_ready = true;       // the four-kernel chain leaves every tensor with a threshold
     last_select_fused = fused;

@@ -158,6 +158,29 @@ static_assert(kHistBins == 2048 && kHistShift == 20 && kFar < 1u << 24, "bins of
 }  // namespace
 
 // ------------------------------------------------------------------------------------------------
+// the residual
+// ------------------------------------------------------------------------------------------------
+namespace {
+
+__device__ __forceinline__ float number_or_zero(float x) { return x == x ? x : 0.f; }
+
+// Elements of the residual.  A tensor compressed by itself has none: A.resid is the caller's tensor then, which is read where it
+// lies, up to its last element, with NaN as zero (scan's policy), and never written.  Half of the traffic of scan: with a copy of
+// the tensor as its residual, 38.6 M elements took 63 us.
+__device__ __forceinline__ float4 resid4(const SelectArgs& A, uint32_t i) {
+  if (!A.fresh) return __ldcg(reinterpret_cast<const float4*>(A.resid + i));
+  const float4 a = load4_guarded(A.resid, i, A.fresh);
+  return make_float4(number_or_zero(a.x), number_or_zero(a.y), number_or_zero(a.z), number_or_zero(a.w));
+}
+
+__device__ __forceinline__ float resid1(const SelectArgs& A, uint32_t i) {
+  if (!A.fresh) return __ldcg(A.resid + i);
+  return i < A.fresh ? number_or_zero(A.resid[i]) : 0.f;
+}
+
+}  // namespace
+
+// ------------------------------------------------------------------------------------------------
 // scan
 // ------------------------------------------------------------------------------------------------
 template <int MODE>
@@ -245,7 +268,7 @@ __global__ void __launch_bounds__(kScanThreads, 4) k_scan(SelectArgs A) {
             if (!(a.z == a.z)) a.z = 0.f;
             if (!(a.w == a.w)) a.w = 0.f;
           }
-          if (i < len) {
+          if (i < len && !A.fresh) {
             *reinterpret_cast<float4*>(r + i) = a;
             if (A.zero_grad) store4_guarded(g, i, g_valid, make_float4(0.f, 0.f, 0.f, 0.f));
           }
@@ -430,7 +453,7 @@ __device__ __forceinline__ void note_destinations(const SelectArgs& A, const Job
 __device__ __forceinline__ void emit_and_keep(const SelectArgs& A, const EmitShared& S, uint32_t pos, uint32_t gi, float a) {
   const float sv = wire_value(S.nb, a);
   emit_entry(A, S.dest, S.nb, S.slot_off, pos, gi, sv);
-  A.resid[gi] = a - sv;     // exactly zero unless the wire format rounds
+  if (!A.fresh) A.resid[gi] = a - sv;     // exactly zero unless the wire format rounds
 }
 
 // True in every thread of the CTA that finishes its tensor last; orders the other CTAs' stores in front of what follows.
@@ -518,7 +541,7 @@ __device__ __noinline__ void send_staged(const SelectArgs& A, EmitShared& S, Sta
     }
     return;
   }
-  float* const resid = A.resid;
+  float* const resid = A.fresh ? nullptr : A.resid;
 #pragma unroll 1
   for (uint32_t p = 0; p < n_out; ++p) {
     uint2* const out = S.out[p] + pos;
@@ -526,7 +549,7 @@ __device__ __noinline__ void send_staged(const SelectArgs& A, EmitShared& S, Sta
     for (uint32_t q = threadIdx.x; q < m; q += kEmitThreads) {
       const uint2 e = pair(q);
       out[q] = e;
-      if (p == 0u) resid[e.x] = __uint_as_float(e.y) - __uint_as_float(e.y);      // zero, or what the next select drops
+      if (p == 0u && resid != nullptr) resid[e.x] = __uint_as_float(e.y) - __uint_as_float(e.y);      // zero, or what the next select drops
     }
   }
 }
@@ -710,7 +733,8 @@ __device__ __forceinline__ uint32_t top_direct(const SelectArgs& A, const Job& J
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
     const uint32_t i = u * kEmitThreads + tid;
-    a[u] = i * 4u < J.sd.n_pad ? *reinterpret_cast<const uint4*>(A.resid + J.sd.off + i * 4u) : make_uint4(0u, 0u, 0u, 0u);
+    const float4 v = i * 4u < J.sd.n_pad ? resid4(A, J.sd.off + i * 4u) : make_float4(0.f, 0.f, 0.f, 0.f);
+    a[u] = make_uint4(__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w));
   }
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
@@ -872,7 +896,7 @@ __device__ __noinline__ uint32_t send_best(const SelectArgs& A, EmitShared& S, c
       uint2 e = make_uint2(0u, 0u);
       if (t < take * kPerItem) {
         e.x = __ldcg(&list[t / kPerItem].x) * kPerItem + t % kPerItem;
-        e.y = __float_as_uint(__ldcg(A.resid + e.x));
+        e.y = __float_as_uint(resid1(A, e.x));
       }
       stage[u * kEmitThreads + tid] = e;
     }
@@ -917,7 +941,7 @@ __device__ __forceinline__ void send_range(const SelectArgs& A, const Job& J, Em
       }
 #pragma unroll
       for (int u = 0; u < kPer; ++u)
-        if (t0 + (u * kEmitThreads + threadIdx.x) * 4u < end) a[u] = __ldcg(reinterpret_cast<const float4*>(A.resid + gi[u]));
+        if (t0 + (u * kEmitThreads + threadIdx.x) * 4u < end) a[u] = resid4(A, gi[u]);
 #pragma unroll
       for (int u = 0; u < kPer; ++u) {
         const uint32_t q = (u * kEmitThreads + threadIdx.x) * 4u;
@@ -970,7 +994,7 @@ __device__ __noinline__ uint32_t collect_unlisted(const SelectArgs& A, EmitShare
     atomicOr(&S.hist[b >> 5], 1u << (b & 31u));
   }
   __syncthreads();
-  const float* src = A.resid + J.pc.start + (tid & 3u) * 4u;
+  const uint32_t src = J.pc.start + (tid & 3u) * 4u;
   uint32_t done = 0;
   for (uint32_t b0 = 0; b0 < n_blk; b0 += kQuads * kKeys * 4u) {
     uint32_t key[kKeys], there = 0;
@@ -981,7 +1005,7 @@ __device__ __noinline__ uint32_t collect_unlisted(const SelectArgs& A, EmitShare
       for (uint32_t q = 0; q < 4u; ++q) {   // independent loads in flight
         const uint32_t b = b0 + (s * 4u + q) * kQuads + (tid >> 2);
         const bool take = b < n_blk && !(S.hist[b >> 5] >> (b & 31u) & 1u);
-        a[q] = take ? __ldcg(reinterpret_cast<const float4*>(src + b * 16u)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        a[q] = take ? resid4(A, src + b * 16u) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
 #pragma unroll
       for (uint32_t q = 0; q < 4u; ++q) {
@@ -1017,7 +1041,7 @@ __device__ __noinline__ void count_rest(const SelectArgs& A, EmitShared& S) {
   uint32_t zeros = 0;
 #pragma unroll 4
   for (uint32_t i = tid * 4u; i < J.len; i += kEmitThreads * 4u) {
-    const float4 a = *reinterpret_cast<const float4*>(A.resid + J.pc.start + i);
+    const float4 a = resid4(A, J.pc.start + i);
     const uint32_t key[4] = {key_bits(a.x), key_bits(a.y), key_bits(a.z), key_bits(a.w)};
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -1253,7 +1277,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const __grid_constant_
               const uint32_t q = e >> 4, p = (found + q) * 16u + (e & 15u);
               if (p < J.sd.k) {   // only the lowest-ranked block can be cut off
                 const uint32_t gi = S.stage[S.hist[q]].x * 16u + (e & 15u);
-                emit_and_keep(A, S, p, gi, __ldcg(A.resid + gi));
+                emit_and_keep(A, S, p, gi, resid1(A, gi));
               }
             }
           } else if (take) {
@@ -1334,7 +1358,7 @@ __global__ void __launch_bounds__(kEmitThreads, 2) k_refill(const __grid_constan
       for (uint32_t i0 = 0; i0 < len && base < rem; i0 += kEmitThreads * 4u) {
         const uint32_t i = i0 + tid * 4u;
         const bool act = i < len;
-        const float4 a = act ? *reinterpret_cast<const float4*>(A.resid + J.pc.start + i) : make_float4(1.f, 1.f, 1.f, 1.f);
+        const float4 a = act ? resid4(A, J.pc.start + i) : make_float4(1.f, 1.f, 1.f, 1.f);
         const uint32_t at = J.pc.start + i, idx[4] = {at, at + 1u, at + 2u, at + 3u};
         const uint32_t bits[4] = {__float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(a.z), __float_as_uint(a.w)};
         uint32_t zero = 0, total;
@@ -1354,7 +1378,7 @@ __global__ void __launch_bounds__(kEmitThreads, 2) k_refill(const __grid_constan
         for (int u = 0; u < kItems / 4; ++u) {
           const uint32_t i = i0 + (u * kEmitThreads + tid) * 4u;
           const bool act = i < len;
-          const float4 a = act ? *reinterpret_cast<const float4*>(A.resid + J.pc.start + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+          const float4 a = act ? resid4(A, J.pc.start + i) : make_float4(0.f, 0.f, 0.f, 0.f);
           const float v[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
           for (int e = 0; e < 4; ++e) {

@@ -147,7 +147,8 @@ struct SelectArgs {
   uint32_t compressor;         // Compressor
   uint32_t zero_grad;          // write zeros over consumed gradients
   uint32_t skip_ef;            // 1: the residual already holds g + r (re-selection), skip the add
-  uint32_t fresh;              // 1: there is no residual yet (r is written, not read); `grad` holds exactly one tensor
+  uint32_t fresh;              // not 0: `grad` holds exactly one tensor, of so many elements, and there is no residual: the
+                               // four-kernel chain writes r and does not read it, the one-pass chain has the tensor in its place
   // exchange
   int32_t world, rank;
   uint2* out[kMaxWorld];       // per destination: its receive area for source `rank`, slot 0

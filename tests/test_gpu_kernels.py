@@ -259,6 +259,34 @@ def test_compress_reads_the_tensor_in_place(compressor, n, form):
 
 
 @pytest.mark.parametrize("compressor", ["topk", "thresholdv", "thresholdv16"])
+@pytest.mark.parametrize("n", [4095, 400_003])
+def test_compress_of_values_that_change_in_scale(compressor, n):
+    """The ways of the chain that read the tensor once more (too few candidates, the fill from all blocks), at its ragged end and
+    with NaN in it: the pairs of the plain rule, and the tensor as it was."""
+    import stellatrain_b200 as st
+
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    name, state = f"{compressor} {n} scales", O.ThresholdState()
+    st.configure_compression(compressor)
+    try:
+        for call, scale in enumerate([1.0, 1.0, 0.01, 0.01, 30.0, 0.2, 0.0]):
+            x = torch.randn(n, generator=gen, device="cuda") * (1e-2 * scale)
+            if call == 5:
+                x[: n - 100] = 0.0
+            x[n - 2] = float("nan")
+            before = x.clone()
+            idx, val = st.compress(name, x, 0.97)
+            assert torch.equal(x.nan_to_num(7.0), before.nan_to_num(7.0))
+            x = x.nan_to_num(0.0)
+            assert torch.equal(val, x[idx.long()]) and len(torch.unique(idx)) == len(idx)
+            want, _, _ = O.compress_step(compressor, x, torch.zeros_like(x), int((1.0 - 0.97) * n), state, one_pass=call > 0)
+            want = want[want < n].sort().values
+            assert torch.equal(idx.long().sort().values, want), call
+    finally:
+        st.configure_compression("thresholdv16")
+
+
+@pytest.mark.parametrize("compressor", ["topk", "thresholdv", "thresholdv16"])
 def test_compress_under_capture_is_refused_and_leaves_no_trace(compressor):
     """The refused call must not count as the tensor's first select, which is the one that measures the threshold."""
     import stellatrain_b200 as st
