@@ -332,8 +332,8 @@ PYBIND11_MODULE(_C, m) {
 
   // Native step engine: C++ hooks on the parameters, bucket bookkeeping, stream and event choreography.
   py::class_<st::NativeEngine>(m, "NativeEngine")
-      .def(py::init<int, uint64_t, uint64_t, int, int>(), py::arg("device"), py::arg("sparse_stream"), py::arg("second_stream"),
-           py::arg("staleness"), py::arg("grad_accumulation"))
+      .def(py::init<int, uint64_t, uint64_t, uint64_t, int, int>(), py::arg("device"), py::arg("sparse_stream"),
+           py::arg("second_stream"), py::arg("apply_stream"), py::arg("staleness"), py::arg("grad_accumulation"))
       .def("add_bucket",
            [](st::NativeEngine& e, BucketHandle& h, py::object select_handle, int n_params, bool steal, uint64_t table_host,
               int table_ring, uint64_t table_dev, py::object flat_grad, const std::vector<uint32_t>& seg_off,

@@ -25,9 +25,14 @@ struct BucketHandle {
   bool can_fuse() const { return one_pass_possible(sel); }
   bool one_pass_next() const { return fused_enabled && thresholds_ready && can_fuse(); }
 
-  cudaError_t select(cudaStream_t stream) {
+  // `before_emit` (or null): what has to be done before entries are stored; the one-pass chain streams beside it.
+  cudaError_t select(cudaStream_t stream, cudaEvent_t before_emit = nullptr) {
     const bool fused = one_pass_next();
-    const cudaError_t e = fused ? launch_select_one_pass(sel, stream) : launch_select(sel, randomk_seed, stream);
+    if (!fused && before_emit != nullptr) {
+      const cudaError_t w = cudaStreamWaitEvent(stream, before_emit, 0);
+      if (w != cudaSuccess) return w;
+    }
+    const cudaError_t e = fused ? launch_select_one_pass(sel, stream, before_emit) : launch_select(sel, randomk_seed, stream);
     thresholds_ready = true;       // the four-kernel chain leaves every tensor with a threshold
     last_select_fused = fused;
     return e;

@@ -9,9 +9,9 @@ namespace st {
 cudaError_t launch_select(const SelectArgs& args, uint32_t randomk_seed, cudaStream_t stream);
 
 // One-pass variant for tensors that have been through one select already: two kernels, three for top-k.  Usable when
-// one_pass_possible() says so.
+// one_pass_possible() says so.  `before_emit` (or null): an event that the kernels behind the streaming one wait for.
 bool one_pass_possible(const SelectArgs& args);
-cudaError_t launch_select_one_pass(const SelectArgs& args, cudaStream_t stream);
+cudaError_t launch_select_one_pass(const SelectArgs& args, cudaStream_t stream, cudaEvent_t before_emit);
 
 // Bounded wait + scatter-add + sparse optimiser of one bucket: two kernels on `stream` (one for a single source), plus the copy of
 // the owners' new parameter values when the optimiser state is partitioned.  phase 0 = all, 1 = scatter and

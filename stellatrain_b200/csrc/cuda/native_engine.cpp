@@ -63,6 +63,11 @@ struct NativeEngine::Impl {
   // `second` is null when there is one stream: buckets of several ranks stay in one order for all of them, and an emulated
   // slow link has one token bucket.
   cudaStream_t sparse = nullptr, second = nullptr;
+  // The update of the previous iteration and the streaming kernel of this one touch nothing in common: with one rank the update
+  // runs on a stream of its own.  The kernels behind the streaming one wait for it: they advance the select epoch, by which the
+  // update knows whether there is anything to apply (nothing after a flush).  Captured steps with this, and with streaming kernels
+  // one priority level under the others: ViT-B/16 272 -> 249 us, ResNet-152 173.5 -> 165.7, GPT-2 490 -> 482, ResNet-50 106.
+  cudaStream_t aside = nullptr;
   int staleness = 1, ga = 1;
   std::vector<BucketRec> buckets;
   std::vector<ParamRec> params;
@@ -97,16 +102,16 @@ struct NativeEngine::Impl {
     return reinterpret_cast<uint64_t*>(b.capture_row.data_ptr());
   }
 
-  void apply(BucketRec& b) {
-    check(b.spec.handle->apply(b.lane, 0));
-    check(cudaEventRecord(b.apply_done, b.lane));
+  void apply(BucketRec& b, cudaStream_t stream) {
+    check(b.spec.handle->apply(stream, 0));
+    check(cudaEventRecord(b.apply_done, stream));
     b.apply_done_set = true;
     b.has_pending_apply = false;
     b.apply_count += 1;
     kernels += b.spec.handle->apply_kernels();
   }
 
-  void select(BucketRec& b) {
+  void select(BucketRec& b, cudaEvent_t before_emit) {
     BucketHandle* h = b.spec.select_handle ? b.spec.select_handle : b.spec.handle;
     if (b.spec.handle->has_group) {
       check(b.spec.handle->group_reduce(b.lane));
@@ -117,7 +122,7 @@ struct NativeEngine::Impl {
       shaped += b.spec.shaped_bytes;
       kernels += 1;
     }
-    check(h->select(b.lane));
+    check(h->select(b.lane, before_emit));
     if (!capturing) {
       check(cudaEventRecord(b.select_done, b.lane));
       b.select_done_set = true;
@@ -191,9 +196,21 @@ struct NativeEngine::Impl {
     }
     check(cudaEventRecord(b.grad_ready, cur));
     check(cudaStreamWaitEvent(b.lane, b.grad_ready, 0));
-    if (staleness == 1 && b.has_pending_apply) apply(b);
-    select(b);
-    if (staleness == 0) apply(b);
+    if (staleness == 1 && b.has_pending_apply) {
+      // a single bucket launched call by call is bound by the host: no second stream there
+      if (aside != nullptr && (capturing || buckets.size() > 1)) {
+        check(cudaStreamWaitEvent(aside, b.grad_ready, 0));
+        if (!capturing && b.select_done_set) check(cudaStreamWaitEvent(aside, b.select_done, 0));     // the stream it reads
+        apply(b, aside);
+        select(b, b.apply_done);
+      } else {
+        apply(b, b.lane);
+        select(b, nullptr);
+      }
+    } else {
+      select(b, nullptr);
+    }
+    if (staleness == 0) apply(b, b.lane);
     else b.has_pending_apply = true;
     release.clear();   // after the launches, see above
   }
@@ -219,11 +236,13 @@ at::Tensor tensor_of(PyObject* obj, const char* what) {
 
 }  // namespace
 
-NativeEngine::NativeEngine(int device, uint64_t sparse_stream, uint64_t second_stream, int staleness, int grad_accumulation)
+NativeEngine::NativeEngine(int device, uint64_t sparse_stream, uint64_t second_stream, uint64_t apply_stream, int staleness,
+                           int grad_accumulation)
     : impl_(new Impl) {
   impl_->device = device;
   impl_->sparse = reinterpret_cast<cudaStream_t>(static_cast<uintptr_t>(sparse_stream));
   impl_->second = reinterpret_cast<cudaStream_t>(static_cast<uintptr_t>(second_stream));
+  impl_->aside = reinterpret_cast<cudaStream_t>(static_cast<uintptr_t>(apply_stream));
   impl_->staleness = staleness;
   impl_->ga = grad_accumulation < 1 ? 1 : grad_accumulation;
   impl_->shared = std::make_shared<Shared>();
@@ -349,7 +368,7 @@ void NativeEngine::flush(uint64_t stream) {
   impl_->check(cudaStreamWaitEvent(impl_->sparse, ev, 0));
   if (impl_->second) impl_->check(cudaStreamWaitEvent(impl_->second, ev, 0));
   for (auto& b : impl_->buckets)
-    if (b.has_pending_apply) impl_->apply(b);
+    if (b.has_pending_apply) impl_->apply(b, b.lane);      // behind the select, which waited for the update before it
   for (cudaStream_t lane : {impl_->sparse, impl_->second}) {
     if (lane == nullptr) continue;
     impl_->check(cudaEventRecord(ev, lane));

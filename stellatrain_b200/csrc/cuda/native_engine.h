@@ -38,7 +38,9 @@ struct NativeBucketSpec {
 
 class NativeEngine {
  public:
-  NativeEngine(int device, uint64_t sparse_stream, uint64_t second_stream, int staleness, int grad_accumulation);
+  // `apply_stream` (or 0): where the updates of a bucket may run beside its streaming kernel, see Impl::aside.
+  NativeEngine(int device, uint64_t sparse_stream, uint64_t second_stream, uint64_t apply_stream, int staleness,
+               int grad_accumulation);
   ~NativeEngine();
   NativeEngine(const NativeEngine&) = delete;
   NativeEngine& operator=(const NativeEngine&) = delete;

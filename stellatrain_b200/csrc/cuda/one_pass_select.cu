@@ -28,6 +28,8 @@
 //   emit    latency, a chain of about twelve trips to L2: 15 us for threshold-v16, 19 us (0.1 %) to 31 us (1 %) for top-k; at
 //           10 % the entries count: 28 us for threshold-v16, 45 us for top-k.
 //   refill  1.4 to 2.5 us when there is nothing to do, 95 us for a bucket that is one tensor (42 us at 3 M elements).
+#include "launch.h"
+#include "launchers.h"
 #include "select_common.cuh"
 
 namespace st {
@@ -1416,17 +1418,19 @@ bool one_pass_possible(const SelectArgs& A) {
   return A.compressor != kRandomk && A.pieces != nullptr && A.n_total < (1u << 30) && A.cand_cap >= slots;
 }
 
-cudaError_t launch_select_one_pass(const SelectArgs& A, cudaStream_t stream) {
+cudaError_t launch_select_one_pass(const SelectArgs& A, cudaStream_t stream, cudaEvent_t before_emit) {
   if (A.n_chunks == 0 || A.n_segs == 0) return cudaSuccess;
   if (A.world > kMaxWorld || !one_pass_possible(A) || (1u << A.piece_shift) > kMaxPieceRuns) return cudaErrorInvalidValue;
+  cudaError_t e = A.compressor == kThresholdv16  ? launch_streaming(k_scan<kScanBlock>, A.n_chunks, kScanThreads, stream, A)
+                  : A.compressor == kThresholdv ? launch_streaming(k_scan<kScanElem>, A.n_chunks, kScanThreads, stream, A)
+                                                : launch_streaming(k_scan<kScanTop>, A.n_chunks, kScanThreads, stream, A);
+  if (e == cudaSuccess && before_emit != nullptr) e = cudaStreamWaitEvent(stream, before_emit, 0);
+  if (e != cudaSuccess) return e;
   if (A.compressor == kThresholdv16) {
-    k_scan<kScanBlock><<<A.n_chunks, kScanThreads, 0, stream>>>(A);
     k_emit<kScanBlock><<<A.n_pieces, kEmitThreads, 0, stream>>>(A);
   } else if (A.compressor == kThresholdv) {
-    k_scan<kScanElem><<<A.n_chunks, kScanThreads, 0, stream>>>(A);
     k_emit<kScanElem><<<A.n_pieces, kEmitThreads, 0, stream>>>(A);
   } else {
-    k_scan<kScanTop><<<A.n_chunks, kScanThreads, 0, stream>>>(A);
     k_emit<kScanTop><<<A.n_pieces, kEmitThreads, 0, stream>>>(A);
     k_refill<<<A.n_pieces, kEmitThreads, 0, stream>>>(A);
   }

@@ -200,6 +200,9 @@ class SparseDPEngine:
         # ranks, Python hooks and a shaped link keep one stream.
         self._second_stream: Optional[torch.cuda.Stream] = None
         self._second_high = high
+        # Also with one rank and the native engine: updates run beside the streaming kernel of their bucket's next select, whose
+        # emission waits for them (and with it everybody who waits for the bucket's stream).
+        self._apply_stream: Optional[torch.cuda.Stream] = None
         self.iteration = 0            # completed optimiser iterations (selects issued per bucket)
         self.micro_step = 0
         self._failed: Optional[SparseStepError] = None
@@ -230,6 +233,8 @@ class SparseDPEngine:
         numels = [params[i][1].numel() for i in order]
         groups = B.plan_buckets(numels, int(cfg.bucket_mb * (1 << 20) / 4))
         self.scratch = CandidateScratch(self.device)
+        if self.transport == "local" and self._use_native():
+            self._apply_stream = torch.cuda.Stream(device=self.device, priority=self._second_high)
         if self.transport == "local" and self._use_native() and len(groups) > 1:
             self._second_stream = torch.cuda.Stream(device=self.device, priority=self._second_high)
         scratches = [self.scratch, CandidateScratch(self.device) if self._second_stream is not None else self.scratch]
@@ -452,6 +457,7 @@ class SparseDPEngine:
         self.native = C.NativeEngine(self.device.index if self.device.index is not None else torch.cuda.current_device(),
                                      self.sparse_stream.cuda_stream,
                                      self._second_stream.cuda_stream if self._second_stream is not None else 0,
+                                     self._apply_stream.cuda_stream if self._apply_stream is not None else 0,
                                      self.cfg.staleness, self.cfg.grad_accumulation)
         for bi, rt in enumerate(self.buckets):
             b = rt.bucket

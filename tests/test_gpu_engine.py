@@ -715,6 +715,47 @@ def test_captured_iteration_joins_the_streams_that_took_part(used):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("compressor", ["topk", "thresholdv16", "randomk"])
+@pytest.mark.parametrize("bucket_mb", [0.02, 64.0])
+def test_updates_beside_the_streaming_kernel_equal_those_in_front_of_it(compressor, bucket_mb):
+    """Staleness 1: the native engine runs the update of the previous iteration beside the next select, in captured steps and, with
+    several buckets, in eager ones; the Python hooks run it in front.  Same bits, also for the replay behind a flush, which has
+    nothing to apply."""
+    import torch.nn as nn
+
+    from stellatrain_b200.parallel.engine import EngineConfig, SparseDPEngine
+    from stellatrain_b200.parallel.graphs import GraphedStep
+
+    def run(native):
+        torch.manual_seed(3)
+        m = nn.Sequential(nn.Linear(64, 120), nn.ReLU(), nn.Linear(120, 100), nn.ReLU(), nn.Linear(100, 10)).cuda()
+        e = SparseDPEngine(m, EngineConfig(compressor=compressor, ratio=0.9, optimizer="adam", staleness=1, bucket_mb=bucket_mb,
+                                           chunk_elems=1024, optimizer_options={"lr": 1e-2}, native_hooks=native))
+        assert (len(e.buckets) > 2) == (bucket_mb < 1.0)
+
+        def step(x):
+            loss = m(x).square().mean()
+            loss.backward()
+            return loss
+
+        gen = torch.Generator(device="cuda").manual_seed(8)
+        xs = [torch.randn(32, 64, device="cuda", generator=gen) for _ in range(9)]
+        graphed = GraphedStep(e, step, [xs[0]], warmup=4)
+        for i, x in enumerate(xs):
+            graphed.copy_inputs(x)
+            graphed.replay()
+            if i == 4:
+                e.synchronize()
+        e.synchronize()
+        out = [p.detach().clone() for p in m.parameters()] + [rt.bucket.resid.clone() for rt in e.buckets]
+        out += [rt.bucket.counters[:4].clone() for rt in e.buckets]
+        e.close()
+        return out
+
+    for a, b in zip(run(True), run(False)):
+        assert torch.equal(a, b)
+
+
 def test_a_checkpoint_with_another_ratio_makes_a_captured_step_stale():
     """Its launches carry the sizes and tables of the old ratio; a checkpoint with the same ratio leaves it usable."""
     import torch.nn as nn
