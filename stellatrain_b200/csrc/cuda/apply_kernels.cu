@@ -20,6 +20,7 @@
 //            the owners' flags and copies the values into the local replica, so replicas agree bit for
 //            bit.  The reference keeps full optimiser state in every process.
 #include "device_utils.cuh"
+#include "launch.h"
 
 namespace st {
 
@@ -45,11 +46,14 @@ __global__ void k_wait_streams(ApplyArgs A) {
     }
   }
   __syncwarp();
+  next_may_begin();      // not before: the wide grid behind this must not take places while a peer is late
   if (threadIdx.x == 0 && A.stamps != nullptr) A.stamps[2] = global_timer_ns();
 }
 
 __global__ void __launch_bounds__(kThreads) k_scatter(ApplyArgs A) {
   const int src = blockIdx.y + A.src_first;
+  next_may_begin();
+  behind_previous();
   const uint32_t epoch = *A.epoch;
   const uint32_t slot = epoch & 1u;
   if (epoch >= ld_volatile_u32(A.sel_epoch)) return;
@@ -155,11 +159,14 @@ __device__ __forceinline__ float update_element(const ApplyArgs& A, const OptSta
 __global__ void __launch_bounds__(kThreads) k_apply(ApplyArgs A) {
   __shared__ float s_bc[2];
   const int src = blockIdx.y;
+  // nothing but the previous update writes what these need, and that was done in front of the first kernel of this chain
+  const OptState o = *A.opt;
+  if ((threadIdx.x & 31u) == 0u && threadIdx.x < 64u && o.kind != 0) s_bc[threadIdx.x >> 5] = bias_correction(o, threadIdx.x >> 5);
+  behind_previous();
   const uint32_t epoch = *A.epoch;
   const uint32_t slot = epoch & 1u;
   if (epoch >= ld_volatile_u32(A.sel_epoch)) return;
   const bool ok = ld_volatile_u32(A.status) == kOk;
-  const OptState o = *A.opt;
 
   if (ok) {
     const uint64_t src_off = (size_t)slot * A.slot_stride + (size_t)src * A.cap;
@@ -179,7 +186,6 @@ __global__ void __launch_bounds__(kThreads) k_apply(ApplyArgs A) {
       if (in_range) old = atomicExch(reinterpret_cast<uint32_t*>(&A.rec[s].y), epoch);
     };
     if (i < A.ent_hi) claim();
-    if ((threadIdx.x & 31u) == 0u && threadIdx.x < 64u && o.kind != 0) s_bc[threadIdx.x >> 5] = bias_correction(o, threadIdx.x >> 5);
     if (A.cksum_local != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
       // the scatter kernel has read the whole stream of this source: does it add up to what was sent?
       const uint32_t got = atomicExch(A.rsum + src, 0u);
@@ -347,7 +353,9 @@ cudaError_t launch_apply(const ApplyArgs& A, int max_ctas_per_source, int phase,
     if (parts < 1) parts = 1;
     if (parts > max_ctas_per_source) parts = max_ctas_per_source;
     dim3 grid(parts, A.world);
-    if (A.use_flags) k_wait_streams<<<1, 32, 0, stream>>>(A);
+    cudaError_t e = cudaSuccess;
+    if (A.use_flags) e = launch_first(k_wait_streams, dim3(1), 32, stream, A);
+    if (e != cudaSuccess) return e;
     if (apply_merges_nothing(A)) {
       const uint32_t n = A.ent_hi - A.ent_lo;
       const int wide = (int)((n + kThreads * kSingleEntries - 1) / (kThreads * kSingleEntries));
@@ -361,12 +369,15 @@ cudaError_t launch_apply(const ApplyArgs& A, int max_ctas_per_source, int phase,
       ApplyArgs one = A;
       for (int src = 0; src < A.world; ++src) {   // one launch per source: a fixed order of additions
         one.src_first = (uint32_t)src;
-        k_scatter<<<dim3(parts, 1), kThreads, 0, stream>>>(one);
+        e = src == 0 && !A.use_flags ? launch_first(k_scatter, dim3(parts, 1), kThreads, stream, one)
+                                     : launch_behind(k_scatter, dim3(parts, 1), kThreads, stream, one);
+        if (e != cudaSuccess) return e;
       }
     } else {
-      k_scatter<<<grid, kThreads, 0, stream>>>(A);
+      e = A.use_flags ? launch_behind(k_scatter, grid, kThreads, stream, A) : launch_first(k_scatter, grid, kThreads, stream, A);
     }
-    k_apply<<<grid, kThreads, 0, stream>>>(A);
+    if (e == cudaSuccess) e = launch_behind(k_apply, grid, kThreads, stream, A);
+    if (e != cudaSuccess) return e;
   }
   if (A.owner_mode && (phase == 0 || phase == 2)) {
     uint32_t longest = 0;

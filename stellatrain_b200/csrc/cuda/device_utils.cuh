@@ -7,6 +7,12 @@
 
 namespace st {
 
+// Launches that begin before the kernel in front of them has ended (launch_behind): what that kernel writes may be read, and what
+// it reads be written, behind behind_previous() only.  Every kernel launched this way calls it in every CTA, so that the end of a
+// kernel implies the end of all in front of it.  next_may_begin(): the following kernel's CTAs may take places that become free.
+__device__ __forceinline__ void behind_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void next_may_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ uint64_t global_timer_ns() {
   uint64_t t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));

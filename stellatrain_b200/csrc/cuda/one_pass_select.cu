@@ -198,6 +198,7 @@ __global__ void __launch_bounds__(kScanThreads, 4) k_scan(SelectArgs A) {
   __shared__ float4 s_half[MODE == kScanBlock ? 1 : kScanWarps][MODE == kScanBlock ? 1 : kHalf / 4];
   __shared__ uint16_t s_place[MODE == kScanBlock ? 1 : kScanWarps][MODE == kScanBlock ? 1 : kHalf];
   if (blockIdx.x == 0 && threadIdx.x == 0 && A.stamps != nullptr) A.stamps[0] = global_timer_ns();
+  next_may_begin();
 
   const uint32_t piece_shift = A.piece_shift + kRunShift;      // of elements
   for (uint32_t rel = warp * kRunElems; rel < ch.len; rel += kScanWarps * kRunElems) {
@@ -1084,11 +1085,14 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const __grid_constant_
   constexpr bool kBlock = MODE == kScanBlock;
   const uint32_t tid = threadIdx.x;
   const Job J = job_of(A, kBlock);
+  // all of this was written in front of `scan`
+  const SegState ss = A.state[J.pc.seg];
+  note_destinations(A, J, S);
+  behind_previous();
   const uint32_t cnt = tid < J.pc.n_runs ? A.run_cnt[(blockIdx.x << A.piece_shift) + tid] : 0u;
   const bool ok = ld_volatile_u32(A.status) == kOk;
 
   if (!(J.sd.reserved & kSegSkip)) {
-    const SegState ss = A.state[J.pc.seg];
     // listed items and near misses of this piece and of the tensor; listed items in front of this piece, and of the fullest one
     unsigned long long all = 0ull;
     uint32_t ahead = 0, most = 0;
@@ -1102,7 +1106,6 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const __grid_constant_
         }
       }
     if (tid == 0) { S.sum = 0ull; S.at[0] = 0u; S.at[1] = 0u; }
-    note_destinations(A, J, S);
     uint32_t total, near_total = 0;
     uint32_t ex = block_excl_scan(cnt & 0xffffu, S.tmp, total);
     if (tid <= kMaxPieceRuns) S.pre[tid] = ex;
@@ -1328,12 +1331,14 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const __grid_constant_
   }
 
   __syncthreads();
+  next_may_begin();
   if (tid == 0) finish_select(A, J.epoch, MODE == kScanTop ? A.refills : nullptr);
 }
 
 // Top-k tensors whose candidates fell short: the exact selection from the residual, with the histogram that `emit` took.
 __global__ void __launch_bounds__(kEmitThreads, 2) k_refill(const __grid_constant__ SelectArgs A) {
   __shared__ EmitShared S;
+  behind_previous();
   if (ld_volatile_u32(A.refills) == 0u) return;     // the same for every CTA: it is cleared behind the last one
   const uint32_t tid = threadIdx.x;
   const Job J = job_of(A, false);
@@ -1426,15 +1431,12 @@ cudaError_t launch_select_one_pass(const SelectArgs& A, cudaStream_t stream, cud
                                                 : launch_streaming(k_scan<kScanTop>, A.n_chunks, kScanThreads, stream, A);
   if (e == cudaSuccess && before_emit != nullptr) e = cudaStreamWaitEvent(stream, before_emit, 0);
   if (e != cudaSuccess) return e;
-  if (A.compressor == kThresholdv16) {
-    k_emit<kScanBlock><<<A.n_pieces, kEmitThreads, 0, stream>>>(A);
-  } else if (A.compressor == kThresholdv) {
-    k_emit<kScanElem><<<A.n_pieces, kEmitThreads, 0, stream>>>(A);
-  } else {
-    k_emit<kScanTop><<<A.n_pieces, kEmitThreads, 0, stream>>>(A);
-    k_refill<<<A.n_pieces, kEmitThreads, 0, stream>>>(A);
-  }
-  return cudaGetLastError();
+  void (*const emit)(SelectArgs) = A.compressor == kThresholdv16 ? k_emit<kScanBlock>
+                                   : A.compressor == kThresholdv ? k_emit<kScanElem> : k_emit<kScanTop>;
+  e = before_emit == nullptr ? launch_behind(emit, A.n_pieces, kEmitThreads, stream, A)
+                             : launch_first(emit, A.n_pieces, kEmitThreads, stream, A);
+  if (e == cudaSuccess && A.compressor == kTopk) e = launch_behind(k_refill, A.n_pieces, kEmitThreads, stream, A);
+  return e;
 }
 
 }  // namespace st
