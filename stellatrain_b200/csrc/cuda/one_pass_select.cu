@@ -169,14 +169,19 @@ __device__ __forceinline__ float number_or_zero(float x) { return x == x ? x : 0
 // Elements of the residual.  A tensor compressed by itself has none: A.resid is the caller's tensor then, which is read where it
 // lies, up to its last element, with NaN as zero (scan's policy), and never written.  Half of the traffic of scan: with a copy of
 // the tensor as its residual, 38.6 M elements took 63 us.
+// FRESH: A.fresh is not 0, or kRuntime.
+constexpr int kRuntime = 2;
+
+template <int FRESH = kRuntime>
 __device__ __forceinline__ float4 resid4(const SelectArgs& A, uint32_t i) {
-  if (!A.fresh) return __ldcg(reinterpret_cast<const float4*>(A.resid + i));
+  if (FRESH == 0 || (FRESH == kRuntime && !A.fresh)) return __ldcg(reinterpret_cast<const float4*>(A.resid + i));
   const float4 a = load4_guarded(A.resid, i, A.fresh);
   return make_float4(number_or_zero(a.x), number_or_zero(a.y), number_or_zero(a.z), number_or_zero(a.w));
 }
 
+template <int FRESH = kRuntime>
 __device__ __forceinline__ float resid1(const SelectArgs& A, uint32_t i) {
-  if (!A.fresh) return __ldcg(A.resid + i);
+  if (FRESH == 0 || (FRESH == kRuntime && !A.fresh)) return __ldcg(A.resid + i);
   return i < A.fresh ? number_or_zero(A.resid[i]) : 0.f;
 }
 
@@ -185,7 +190,9 @@ __device__ __forceinline__ float resid1(const SelectArgs& A, uint32_t i) {
 // ------------------------------------------------------------------------------------------------
 // scan
 // ------------------------------------------------------------------------------------------------
-template <int MODE>
+// FRESH: A.fresh is not 0 (a tensor compressed by itself).  Known when the kernel is compiled, as the tests for it cost 2 % of a
+// captured step otherwise.
+template <int MODE, bool FRESH>
 __global__ void __launch_bounds__(kScanThreads, 4) k_scan(SelectArgs A) {
   // The run's place is all the first loads of r need: they are on their way while the tensor's descriptor, threshold and
   // gradient pointer (a second level of dependent loads) are fetched.
@@ -209,7 +216,7 @@ __global__ void __launch_bounds__(kScanThreads, 4) k_scan(SelectArgs A) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const uint32_t i = j * 128u + lane * 4u;
-      rv[j] = i < len && !A.fresh ? *reinterpret_cast<const float4*>(r + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      rv[j] = i < len && !FRESH ? *reinterpret_cast<const float4*>(r + i) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     const SegDesc sd = A.segs[ch.seg];
     const bool tab = A.grad_tab != nullptr;
@@ -223,7 +230,7 @@ __global__ void __launch_bounds__(kScanThreads, 4) k_scan(SelectArgs A) {
       continue;
     }
     const uint32_t n_valid = sd.n > seg_rel ? min(len, sd.n - seg_rel) : 0u;
-    const uint32_t g_valid = tab || A.fresh ? n_valid : len;   // gradients handed over per tensor are not padded
+    const uint32_t g_valid = tab || FRESH ? n_valid : len;   // gradients handed over per tensor are not padded
     const bool add = !A.skip_ef;
     // a tensor without a threshold yet lists nothing: `emit` then takes the exact top items from the residual
     const uint32_t tau_bits = ss.inited ? __float_as_uint(ss.tau) : 0xFFFFFFFFu;
@@ -245,7 +252,7 @@ __global__ void __launch_bounds__(kScanThreads, 4) k_scan(SelectArgs A) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const uint32_t i = h0 + j * 128u;
-          rv[j] = i < len && !A.fresh ? *reinterpret_cast<const float4*>(r + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+          rv[j] = i < len && !FRESH ? *reinterpret_cast<const float4*>(r + i) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
       }
       if (add) {
@@ -271,7 +278,7 @@ __global__ void __launch_bounds__(kScanThreads, 4) k_scan(SelectArgs A) {
             if (!(a.z == a.z)) a.z = 0.f;
             if (!(a.w == a.w)) a.w = 0.f;
           }
-          if (i < len && !A.fresh) {
+          if (i < len && !FRESH) {
             *reinterpret_cast<float4*>(r + i) = a;
             if (A.zero_grad) store4_guarded(g, i, g_valid, make_float4(0.f, 0.f, 0.f, 0.f));
           }
@@ -727,6 +734,7 @@ __device__ __forceinline__ uint32_t pick_few(const uint2* cand, uint32_t c, uint
 }
 
 // Top-k of a small tensor: its values lie in shared memory.  Returns the k-th largest key.
+template <bool FRESH>
 __device__ __forceinline__ uint32_t top_direct(const SelectArgs& A, const Job& J, EmitShared& S) {
   static_assert(kTopDirect == 2u * kStageItems && kTopDirect == 16u * kEmitThreads, "the values are the words of EmitShared::stage");
   const uint32_t tid = threadIdx.x;
@@ -736,7 +744,7 @@ __device__ __forceinline__ uint32_t top_direct(const SelectArgs& A, const Job& J
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
     const uint32_t i = u * kEmitThreads + tid;
-    const float4 v = i * 4u < J.sd.n_pad ? resid4(A, J.sd.off + i * 4u) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 v = i * 4u < J.sd.n_pad ? resid4<FRESH>(A, J.sd.off + i * 4u) : make_float4(0.f, 0.f, 0.f, 0.f);
     a[u] = make_uint4(__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w));
   }
 #pragma unroll
@@ -925,7 +933,7 @@ __device__ __forceinline__ uint32_t settle_top(const SelectArgs& A, const Job& J
 
 // Sends the items [j0, j1) of one piece at positions base + j; items and positions are in index order.  The dependent loads
 // (list, residual) of a thread travel together; the entries then pass through shared memory as above.
-template <bool kBlock>
+template <bool kBlock, bool FRESH>
 __device__ __forceinline__ void send_range(const SelectArgs& A, const Job& J, EmitShared& S, const uint2* lists,
                                            uint32_t base, uint32_t j0, uint32_t j1) {
   constexpr uint32_t kPerItem = kBlock ? 16u : 1u, kArea = kBlock ? kRunBlocks : kRunElems;
@@ -944,7 +952,7 @@ __device__ __forceinline__ void send_range(const SelectArgs& A, const Job& J, Em
       }
 #pragma unroll
       for (int u = 0; u < kPer; ++u)
-        if (t0 + (u * kEmitThreads + threadIdx.x) * 4u < end) a[u] = resid4(A, gi[u]);
+        if (t0 + (u * kEmitThreads + threadIdx.x) * 4u < end) a[u] = resid4<FRESH>(A, gi[u]);
 #pragma unroll
       for (int u = 0; u < kPer; ++u) {
         const uint32_t q = (u * kEmitThreads + threadIdx.x) * 4u;
@@ -1079,7 +1087,7 @@ __device__ __forceinline__ void step_top(const SelectArgs& A, const Job& J, SegS
 
 }  // namespace
 
-template <int MODE>
+template <int MODE, bool FRESH>
 __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const __grid_constant__ SelectArgs A) {
   __shared__ EmitShared S;
   constexpr bool kBlock = MODE == kScanBlock;
@@ -1150,7 +1158,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const __grid_constant_
       const bool direct = J.sd.n_pad <= kTopDirect;
       if (direct) {
         if (may) {
-          const uint32_t t_key = top_direct(A, J, S);
+          const uint32_t t_key = top_direct<FRESH>(A, J, S);
           if (tid == 0) step_top(A, J, ss, t_key, 0u);
         }
       } else if (short_of && ok) {
@@ -1228,7 +1236,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const __grid_constant_
       const uint32_t lo = (uint32_t)((uint64_t)n_send * J.pc.index / J.pc.count);
       const uint32_t hi = (uint32_t)((uint64_t)n_send * (J.pc.index + 1u) / J.pc.count);
       if (may && even) {
-        if (ahead < n_send) send_range<kBlock>(A, J, S, area, ahead, 0u, min(total, n_send - ahead));
+        if (ahead < n_send) send_range<kBlock, FRESH>(A, J, S, area, ahead, 0u, min(total, n_send - ahead));
       } else if (may && lo < hi) {
         uint32_t piece = 0, base = 0;
         {
@@ -1254,7 +1262,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const __grid_constant_
             __syncthreads();
           }
           const uint2* const lists = A.cand + (kBlock ? J.sd.off >> 4 : J.sd.off) + (size_t)piece * (kArea << A.piece_shift);
-          send_range<kBlock>(A, J, S, lists, base, lo > base ? lo - base : 0u, min(hi - base, total));
+          send_range<kBlock, FRESH>(A, J, S, lists, base, lo > base ? lo - base : 0u, min(hi - base, total));
           base += total;
           ++piece;
           if (base >= hi || piece >= J.pc.count) break;
@@ -1282,7 +1290,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const __grid_constant_
               const uint32_t q = e >> 4, p = (found + q) * 16u + (e & 15u);
               if (p < J.sd.k) {   // only the lowest-ranked block can be cut off
                 const uint32_t gi = S.stage[S.hist[q]].x * 16u + (e & 15u);
-                emit_and_keep(A, S, p, gi, resid1(A, gi));
+                emit_and_keep(A, S, p, gi, resid1<FRESH>(A, gi));
               }
             }
           } else if (take) {
@@ -1426,15 +1434,17 @@ bool one_pass_possible(const SelectArgs& A) {
 cudaError_t launch_select_one_pass(const SelectArgs& A, cudaStream_t stream, cudaEvent_t before_emit) {
   if (A.n_chunks == 0 || A.n_segs == 0) return cudaSuccess;
   if (A.world > kMaxWorld || !one_pass_possible(A) || (1u << A.piece_shift) > kMaxPieceRuns) return cudaErrorInvalidValue;
-  cudaError_t e = A.compressor == kThresholdv16  ? launch_streaming(k_scan<kScanBlock>, A.n_chunks, kScanThreads, stream, A)
-                  : A.compressor == kThresholdv ? launch_streaming(k_scan<kScanElem>, A.n_chunks, kScanThreads, stream, A)
-                                                : launch_streaming(k_scan<kScanTop>, A.n_chunks, kScanThreads, stream, A);
+  using Kernel = void (*)(SelectArgs);
+  const Kernel scan[2][3] = {{k_scan<kScanTop, false>, k_scan<kScanElem, false>, k_scan<kScanBlock, false>},
+                             {k_scan<kScanTop, true>, k_scan<kScanElem, true>, k_scan<kScanBlock, true>}};
+  const Kernel emit[2][3] = {{k_emit<kScanTop, false>, k_emit<kScanElem, false>, k_emit<kScanBlock, false>},
+                             {k_emit<kScanTop, true>, k_emit<kScanElem, true>, k_emit<kScanBlock, true>}};
+  const int fresh = A.fresh ? 1 : 0, mode = A.compressor == kThresholdv16 ? kScanBlock : A.compressor == kThresholdv ? kScanElem : kScanTop;
+  cudaError_t e = launch_streaming(scan[fresh][mode], A.n_chunks, kScanThreads, stream, A);
   if (e == cudaSuccess && before_emit != nullptr) e = cudaStreamWaitEvent(stream, before_emit, 0);
   if (e != cudaSuccess) return e;
-  void (*const emit)(SelectArgs) = A.compressor == kThresholdv16 ? k_emit<kScanBlock>
-                                   : A.compressor == kThresholdv ? k_emit<kScanElem> : k_emit<kScanTop>;
-  e = before_emit == nullptr ? launch_behind(emit, A.n_pieces, kEmitThreads, stream, A)
-                             : launch_first(emit, A.n_pieces, kEmitThreads, stream, A);
+  e = before_emit == nullptr ? launch_behind(emit[fresh][mode], A.n_pieces, kEmitThreads, stream, A)
+                             : launch_first(emit[fresh][mode], A.n_pieces, kEmitThreads, stream, A);
   if (e == cudaSuccess && A.compressor == kTopk) e = launch_behind(k_refill, A.n_pieces, kEmitThreads, stream, A);
   return e;
 }
