@@ -22,11 +22,13 @@
 // threshold has those first, in index order, and the fill behind them.
 //
 // What bounds it, 64 MB bucket (16.8 M elements, 201 MB of traffic, 31 us at the 6.5 TB/s of a plain copy), one B200:
-//   scan    memory: 35.5 us for threshold-v16, 36 us for top-k at 0.1 %, 39 us at 1 % (list and histogram).  Runs of one
+//   scan    memory: 35.5 us for threshold-v16 (29 where L2 holds part of a single bucket), 36 us for top-k at 0.1 %, 39 us at 1 %
+//           (list and histogram).  Runs of one
 //           warp need no barrier and no shared state, so a late load holds up nothing else; with one CTA per 8192 elements
 //           that scanned, chained counts over CTAs and emitted by itself the same traffic took 54 us.
-//   emit    latency, a chain of about twelve trips to L2: 15 us for threshold-v16, 19 us (0.1 %) to 31 us (1 %) for top-k; at
-//           10 % the entries count: 28 us for threshold-v16, 45 us for top-k.
+//   emit    latency, a chain of about ten trips to L2, and its own instructions (see send_staged): 9.6 us for threshold-v16, 16 us
+//           for top-k at 1 %; the slowest sections of the latter are the sum of the histograms (3 us) and the last CTA's
+//           search (3 us).
 //   refill  1.4 to 2.5 us when there is nothing to do, 95 us for a bucket that is one tensor (42 us at 3 M elements).
 #include "launch.h"
 #include "launchers.h"
@@ -1443,8 +1445,10 @@ cudaError_t launch_select_one_pass(const SelectArgs& A, cudaStream_t stream, cud
   cudaError_t e = launch_streaming(scan[fresh][mode], A.n_chunks, kScanThreads, stream, A);
   if (e == cudaSuccess && before_emit != nullptr) e = cudaStreamWaitEvent(stream, before_emit, 0);
   if (e != cudaSuccess) return e;
-  e = before_emit == nullptr ? launch_behind(emit[fresh][mode], A.n_pieces, kEmitThreads, stream, A)
-                             : launch_first(emit[fresh][mode], A.n_pieces, kEmitThreads, stream, A);
+  // With peers every CTA of the emission ends in a system-wide fence; begun beside the scan it took 40 us on one of two boxes, 23
+  // behind it (64 MB bucket, eight destinations).
+  e = before_emit == nullptr && !A.publish ? launch_behind(emit[fresh][mode], A.n_pieces, kEmitThreads, stream, A)
+                                           : launch_first(emit[fresh][mode], A.n_pieces, kEmitThreads, stream, A);
   if (e == cudaSuccess && A.compressor == kTopk) e = launch_behind(k_refill, A.n_pieces, kEmitThreads, stream, A);
   return e;
 }
