@@ -628,21 +628,25 @@ __device__ __forceinline__ void emit_top_batch(const SelectArgs& A, const Job& J
 // Keys of the last two octaves under the largest differ from it in these bits: where the best of a distribution are looked for
 // first.
 constexpr uint32_t kTwoOctaves = 24u;
+constexpr uint32_t kNoCut = 0xFFFFFFFFu;       // a search that found none; no key
 
 // Where the best `take` of n items in S.stage end (larger key first, equal keys by lower id): {key, id - id_lo} of the
 // lowest-ranked one taken; 1 <= take <= n.  The items are pairs (id, key or signed value), or the words (keys or signed values) of
 // one tensor, whose ids count from 0.  No key lies above `top`; ids lie in [id_lo, id_lo + n_ids).
 // A radix search, 8 bits at a time with a bin per thread.  Its digits are those of the distance to `top`, so that they differ
-// where the cut is: of the `open` lowest bits first, which is a guess; a cut further away is found in all 31.
-__device__ __noinline__ uint2 find_cut(EmitShared& S, bool words, uint32_t n, uint32_t take, uint32_t top, uint32_t open,
-                                       uint32_t id_lo, uint32_t n_ids) {
+// where the cut is: of the `open` lowest bits first, which is a guess; a cut further away is found in all 31.  Keys have no more
+// than those, so a search that covers them fails only where the items are not what the caller says (a key over `top`, fewer than
+// `take` of them): it then reports kBadCandidate and returns kNoCut.  At most twelve digits in all.
+__device__ __noinline__ uint2 find_cut(EmitShared& S, uint32_t* status, bool words, uint32_t n, uint32_t take, uint32_t top,
+                                       uint32_t open, uint32_t id_lo, uint32_t n_ids) {
   static_assert(kEmitThreads == 256, "a bin per thread");
   const uint32_t tid = threadIdx.x, lane = tid & 31u, n_up = (n + kEmitThreads - 1u) & ~(kEmitThreads - 1u);
   const uint32_t* const word = reinterpret_cast<const uint32_t*>(S.stage);
   auto distance = [&](uint32_t i) { return top - ((words ? word[i] : S.stage[i].y) & 0x7fffffffu); };
   auto id_of = [&](uint32_t i) { return words ? i : S.stage[i].x - id_lo; };
   uint32_t prefix = 0, rem = take, ties = 0, d = 0;
-  bool by_id = false;
+  bool by_id = false, all_bits = open >= 31u;
+  top = min(top, 0x7fffffffu);      // a threshold with its sign bit set lies over every key
 #pragma unroll 1
   for (;;) {
     // among the values whose bits from `open` upwards are `prefix`: the digit of the rem-th smallest
@@ -670,9 +674,14 @@ __device__ __noinline__ uint2 find_cut(EmitShared& S, bool words, uint32_t n, ui
     if (ex < rem && ex + h >= rem) { S.res[0] = tid; S.res[1] = rem - ex; S.res[2] = h; }
     __syncthreads();
     ties = S.res[2];
-    if (ties == 0u) {      // the guess was wrong
-      open = 31u;
+    if (ties == 0u) {
+      if (all_bits || by_id) {
+        if (tid == 0) set_status(status, kBadCandidate);
+        return make_uint2(kNoCut, 0u);
+      }
+      open = 31u;      // the guess was wrong
       prefix = 0u;
+      all_bits = true;
       continue;
     }
     prefix = prefix << w | S.res[0];
@@ -708,9 +717,9 @@ __device__ __noinline__ uint2 find_cut(EmitShared& S, bool words, uint32_t n, ui
 }
 
 // The best `take` of c <= kPickMax candidates (id, key or signed value): they come to S.stage, and S.hist names those taken, the
-// lowest-ranked one last.  Returns its key.  `top`, `open`: see find_cut.
-__device__ __forceinline__ uint32_t pick_few(const uint2* cand, uint32_t c, uint32_t take, uint32_t top, uint32_t open,
-                                             uint32_t id_lo, uint32_t n_ids, EmitShared& S) {
+// lowest-ranked one last.  Returns its key, or kNoCut (S.hist then names none).  `top`, `open`: see find_cut.
+__device__ __forceinline__ uint32_t pick_few(const SelectArgs& A, const uint2* cand, uint32_t c, uint32_t take, uint32_t top,
+                                             uint32_t open, uint32_t id_lo, uint32_t n_ids, EmitShared& S) {
   static_assert(kPickMax <= kStageItems && kPickMax <= 2048, "the candidates fit EmitShared::stage, their numbers EmitShared::hist");
   constexpr int kPer = kPickMax / kEmitThreads;
   const uint32_t tid = threadIdx.x;
@@ -723,8 +732,9 @@ __device__ __forceinline__ uint32_t pick_few(const uint2* cand, uint32_t c, uint
     if (u * kEmitThreads + tid < c) S.stage[u * kEmitThreads + tid] = e[u];
   if (tid == 0) S.word[2] = 0u;
   __syncthreads();
-  const uint2 cut = find_cut(S, false, c, take, top, open, id_lo, n_ids);
+  const uint2 cut = find_cut(S, A.status, false, c, take, top, open, id_lo, n_ids);
   __syncthreads();      // the search is through with S.hist
+  if (cut.x == kNoCut) return kNoCut;
 #pragma unroll 1
   for (uint32_t i = tid; i < c; i += kEmitThreads) {
     const uint32_t key = S.stage[i].y & 0x7fffffffu, id = S.stage[i].x - id_lo;
@@ -735,7 +745,7 @@ __device__ __forceinline__ uint32_t pick_few(const uint2* cand, uint32_t c, uint
   return cut.x;
 }
 
-// Top-k of a small tensor: its values lie in shared memory.  Returns the k-th largest key.
+// Top-k of a small tensor: its values lie in shared memory.  Returns the k-th largest key, or kNoCut.
 template <bool FRESH>
 __device__ __forceinline__ uint32_t top_direct(const SelectArgs& A, const Job& J, EmitShared& S) {
   static_assert(kTopDirect == 2u * kStageItems && kTopDirect == 16u * kEmitThreads, "the values are the words of EmitShared::stage");
@@ -755,7 +765,8 @@ __device__ __forceinline__ uint32_t top_direct(const SelectArgs& A, const Job& J
     top = max(max(max(top, a[u].x & 0x7fffffffu), max(a[u].y & 0x7fffffffu, a[u].z & 0x7fffffffu)), a[u].w & 0x7fffffffu);
   }
   top = block_max_u32(top, S.tmp);
-  const uint2 cut = find_cut(S, true, J.sd.n_pad, J.kk, top, kTwoOctaves, 0u, J.sd.n_pad);
+  const uint2 cut = find_cut(S, A.status, true, J.sd.n_pad, J.kk, top, kTwoOctaves, 0u, J.sd.n_pad);
+  if (cut.x == kNoCut) return kNoCut;
   uint32_t take = 0;      // bit 4 u + e: element e of the thread's u-th four
 #pragma unroll 1
   for (uint32_t u = 0; u < 4u; ++u) {
@@ -921,13 +932,14 @@ __device__ __noinline__ uint32_t send_best(const SelectArgs& A, EmitShared& S, c
   return cut.x;
 }
 
-// Top-k, last CTA of a tensor: the best `rem` of the `c` undecided items complete the stream.  Returns the k-th largest key.
+// Top-k, last CTA of a tensor: the best `rem` of the `c` undecided items complete the stream.  Returns the k-th largest key, or
+// kNoCut.
 __device__ __forceinline__ uint32_t settle_top(const SelectArgs& A, const Job& J, EmitShared& S, const uint2* undecided,
                                                uint32_t c, uint32_t rem, uint32_t key_lo, uint32_t key_hi) {
   const uint32_t done = J.kk - rem;
   if (c <= kPickMax) {
-    const uint32_t t_key = pick_few(undecided, c, rem, key_hi - 1u, 32u - __clz(key_hi - 1u - key_lo), J.sd.off, J.sd.n_pad, S);
-    send_staged(A, S, kNamed, rem, done);
+    const uint32_t t_key = pick_few(A, undecided, c, rem, key_hi - 1u, 32u - __clz(key_hi - 1u - key_lo), J.sd.off, J.sd.n_pad, S);
+    if (t_key != kNoCut) send_staged(A, S, kNamed, rem, done);
     return t_key;
   }
   return send_best<false>(A, S, undecided, c, rem, done, A.cand + J.sd.off);
@@ -1161,7 +1173,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const __grid_constant_
       if (direct) {
         if (may) {
           const uint32_t t_key = top_direct<FRESH>(A, J, S);
-          if (tid == 0) step_top(A, J, ss, t_key, 0u);
+          if (tid == 0 && t_key != kNoCut) step_top(A, J, ss, t_key, 0u);
         }
       } else if (short_of && ok) {
         count_rest(A, S);      // for `refill`
@@ -1195,7 +1207,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const __grid_constant_
           const uint32_t c = J.pc.count == 1u ? noted : __ldcg(&J.wp->cand_cnt);
           if (may && rem != 0u && rem <= c) {
             const uint32_t t_key = settle_top(A, J, S, undecided, c, rem, key_lo, key_hi);
-            if (tid == 0) step_top(A, J, ss, t_key, found);
+            if (tid == 0 && t_key != kNoCut) step_top(A, J, ss, t_key, found);
           } else if (may && tid == 0) {
             set_status(A.status, kBadCandidate);   // cannot happen: the histogram counted these very items
           }
@@ -1286,9 +1298,9 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const __grid_constant_
           if (take && c <= kPickMax) {
             // none reaches the threshold, and the best lie in the two octaves under it
             const uint32_t top = ss.inited ? max(__float_as_uint(ss.tau), 1u) - 1u : 0x7fffffffu;
-            t_key = pick_few(nears, c, take, top, ss.inited ? kTwoOctaves : 31u, J.sd.off >> 4, J.sd.n_pad >> 4, S);
+            t_key = pick_few(A, nears, c, take, top, ss.inited ? kTwoOctaves : 31u, J.sd.off >> 4, J.sd.n_pad >> 4, S);
 #pragma unroll 1
-            for (uint32_t e = tid; e < take * 16u; e += kEmitThreads) {
+            for (uint32_t e = tid; t_key != kNoCut && e < take * 16u; e += kEmitThreads) {
               const uint32_t q = e >> 4, p = (found + q) * 16u + (e & 15u);
               if (p < J.sd.k) {   // only the lowest-ranked block can be cut off
                 const uint32_t gi = S.stage[S.hist[q]].x * 16u + (e & 15u);
@@ -1313,7 +1325,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const __grid_constant_
               else if (J.sd.k < found) st.tau = st.tau + 0.01f * ((float)found / (float)J.sd.k) * max_abs;
             }
           } else if (!st.inited) {
-            if (short_of && may) {   // first threshold: the smallest selected key plus the first additive step
+            if (short_of && may && t_key != kNoCut) {   // first threshold: the smallest selected key plus the first additive step
               const float t0 = __uint_as_float(t_key);
               st.tau_inc = 0.01f * t0;
               st.tau = t0 + st.tau_inc;
@@ -1410,7 +1422,7 @@ __global__ void __launch_bounds__(kEmitThreads, 2) k_refill(const __grid_constan
       const uint32_t c = J.pc.count == 1u ? noted : __ldcg(&J.wp->cand_cnt);
       if (may && rem != 0u && (zero_fill || rem <= c)) {
         const uint32_t t_key = zero_fill ? 0u : settle_top(A, J, S, undecided, c, rem, key_lo, key_hi);
-        if (tid == 0) step_top(A, J, ss, t_key, 0u);
+        if (tid == 0 && t_key != kNoCut) step_top(A, J, ss, t_key, 0u);
       } else if (may && tid == 0) {
         set_status(A.status, kBadCandidate);
       }

@@ -199,6 +199,72 @@ def test_items_over_the_threshold_in_all_pieces_or_in_one(compressor, where, ove
         assert torch.equal(b.resid, resid_ref), step
 
 
+def set_seg_state(b, **fields):
+    state = b.seg_state()
+    for k, v in fields.items():
+        state[k] = v
+    b.state.copy_(torch.from_numpy(state.view(np.uint8).reshape(-1)))
+
+
+@pytest.mark.parametrize("tau", [-0.5, -0.0, float("nan"), float("inf")])
+def test_a_block_threshold_that_no_block_reaches(tau):
+    """A restored threshold may be anything.  One that no block reaches, also by its sign bit, leaves the whole stream to the
+    fill: the best blocks of the tensor, few (searched in shared memory) or many."""
+    sizes = [1000, 30_000, 70_001]
+    b = make_bucket("thresholdv16", 0.97, sizes=sizes)
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    for step in range(4):
+        fill_grads(b, gen)
+        if step >= 2:
+            set_seg_state(b, tau=np.float32(tau))
+        a = b.grad + b.resid
+        b.select()
+        torch.cuda.synchronize()
+        b.check_status()
+        if step < 2:
+            continue
+        idx, val = read_stream(b, step + 1)
+        for s, _, slp in seg_slices(b):
+            key = a[slp].view(-1, 4).abs()
+            key = ((key[:, 0] + key[:, 1]) + (key[:, 2] + key[:, 3])).view(-1, 4)
+            key = (key[:, 0] + key[:, 1]) + (key[:, 2] + key[:, 3])
+            blocks = key.sort(descending=True, stable=True).indices[: (s.k + 15) // 16]
+            want = (blocks[:, None] * 16 + torch.arange(16, device="cuda")).reshape(-1)[: s.k] + s.off      # the last one is cut off
+            got = torch.from_numpy(idx[s.out_off : s.out_off + s.k])
+            assert torch.equal(got.sort().values, want.cpu().sort().values), (s.numel, step)
+            assert torch.equal(val[s.out_off : s.out_off + s.k], a[got.cuda()].cpu())
+            left = a[slp].clone()
+            left[want - s.off] = 0.0
+            assert torch.equal(b.resid[slp], left)
+
+
+def test_a_fill_whose_candidates_are_not_there_is_reported():
+    """The fill's candidates and their count come from counters that every select leaves at zero.  Were they ever wrong, the
+    search for the cut must end: with an error, and nothing stored past it."""
+    n, ratio = 300_000, 0.99
+    b = make_bucket("thresholdv16", ratio, sizes=[n], chunk=8192)
+    assert b.n_pieces > 1
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    for _ in range(2):
+        fill_grads(b, gen)
+        b.select()
+    torch.cuda.synchronize()
+    b.check_status()
+    # as many blocks with something in them as the budget has: the fill wants every candidate
+    wanted = (b.layout.segments[0].k + 15) // 16
+    b.resid.zero_()
+    b.grad.zero_()
+    b.grad.view(-1)[: wanted * 96 : 96] = 1.0
+    set_seg_state(b, tau=np.float32(1e30), r0=np.float32(1.0).view(np.uint32))
+    lists = b.scratch.buf.view(-1, 2)
+    first = b.layout.n_total // 16
+    lists[first : first + 5] = torch.tensor([0, 0x7F000000], dtype=torch.int32, device="cuda")      # five leftovers over the threshold
+    b.work.view(1, B.SEG_WORK_WORDS)[0, 4] = 5                                                       # in front of the candidates
+    b.select()
+    torch.cuda.synchronize()
+    assert int(b.status.item()) == 4
+
+
 @pytest.mark.parametrize("compressor", ["topk", "thresholdv", "thresholdv16"])
 def test_a_ratio_change_cuts_the_bucket_anew(compressor):
     """More entries want smaller pieces; thresholds and residuals stay."""
