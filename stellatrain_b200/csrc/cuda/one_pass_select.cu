@@ -241,7 +241,9 @@ __global__ void __launch_bounds__(kScanThreads, 4) k_scan(SelectArgs A) {
     if (MODE == kScanBlock && ss.inited)
       near_lo = __float_as_uint(fmaxf(ss.tau * (1.f - window_or(ss.reserved[0], kWindowDefault)), 0.f));
 
-    const float cut_value = __uint_as_float(cut);
+    // Magnitudes compare as their bits do; nothing reaches a cut over the bits of infinity, also with the sign bit set (a restored
+    // threshold may be anything): all of those become one that is no number.
+    const float cut_value = __uint_as_float(min(cut, 0x7fc00000u));
     uint32_t n_list = 0;                // entries listed so far
     float mx = 0.f;                     // largest magnitude of this lane
     uint32_t own[2] = {0u, 0u};         // block mode: keys of two of the run's blocks, numbers h * 32 + (lane & 3) * 8 + lane / 4
@@ -290,7 +292,6 @@ __global__ void __launch_bounds__(kScanThreads, 4) k_scan(SelectArgs A) {
           const uint32_t key = __float_as_uint(quad_l1(a));   // the same value in the four lanes of a block
           if ((lane & 3u) == (uint32_t)j) own[h] = key;
         } else {
-          // magnitudes compare as their bits do, and nothing reaches a cut that is no number
           if (fabsf(a.x) >= cut_value) mask |= 1u << (4 * j);
           if (fabsf(a.y) >= cut_value) mask |= 2u << (4 * j);
           if (fabsf(a.z) >= cut_value) mask |= 4u << (4 * j);

@@ -238,6 +238,39 @@ def test_a_block_threshold_that_no_block_reaches(tau):
             assert torch.equal(b.resid[slp], left)
 
 
+@pytest.mark.parametrize("threshold", [-0.5, -0.0, float("nan"), float("inf")])
+def test_an_element_threshold_that_no_element_reaches(threshold):
+    """The same for elements: threshold-v then sends nothing and keeps everything, top-k (whose state is its previous k-th
+    largest value) finds its entries in the whole tensor."""
+    sizes = [1000, 30_000, 300_000]
+    v, top = make_bucket("thresholdv", 0.97, sizes=sizes), make_bucket("topk", 0.97, sizes=sizes)
+    gen = torch.Generator(device="cuda").manual_seed(10)
+    for step in range(4):
+        for b in (v, top):
+            fill_grads(b, gen)
+        if step >= 2:
+            set_seg_state(v, tau=np.float32(threshold))
+            set_seg_state(top, r1=np.float32(threshold).view(np.uint32))
+        a_v, a_top = v.grad + v.resid, top.grad + top.resid
+        for b in (v, top):
+            b.select()
+            torch.cuda.synchronize()
+            b.check_status()
+        if step < 2:
+            continue
+        idx, _ = read_stream(v, step + 1)
+        assert np.all(idx == O.SENTINEL) and torch.equal(v.resid, a_v)
+        idx, val = read_stream(top, step + 1)
+        for s, sl, slp in seg_slices(top):
+            want = a_top[sl].abs().sort(descending=True, stable=True).indices[: s.k] + s.off
+            got = torch.from_numpy(idx[s.out_off : s.out_off + s.k])
+            assert torch.equal(got.sort().values, want.cpu().sort().values), (s.numel, step)
+            assert torch.equal(val[s.out_off : s.out_off + s.k], a_top[got.cuda()].cpu())
+            left = a_top[slp].clone()
+            left[want - s.off] = 0.0
+            assert torch.equal(top.resid[slp], left)
+
+
 def test_a_fill_whose_candidates_are_not_there_is_reported():
     """The fill's candidates and their count come from counters that every select leaves at zero.  Were they ever wrong, the
     search for the cut must end: with an error, and nothing stored past it."""
