@@ -29,7 +29,9 @@
 //   emit    latency, a chain of about ten trips to L2, and its own instructions (see send_staged): 9.6 us for threshold-v16, 16 us
 //           for top-k at 1 %; the slowest sections of the latter are the sum of the histograms (3 us) and the last CTA's
 //           search (3 us).
-//   refill  1.4 to 2.5 us when there is nothing to do, 95 us for a bucket that is one tensor (42 us at 3 M elements).
+//   refill  1.4 to 2.5 us when there is nothing to do; one tensor of 16.8 M elements (3 M) whose gradients fell to a third takes
+//           94 us (23) here and 83 us (20) in `emit`, where a CTA counts a piece of 131,072 elements (16,384); where they fell to a
+//           hundredth, so that the cut lies in a wide bin, 366 us (71), most of them for the ranking by the last CTA.
 #include "launch.h"
 #include "launchers.h"
 #include "select_common.cuh"
@@ -171,19 +173,17 @@ __device__ __forceinline__ float number_or_zero(float x) { return x == x ? x : 0
 // Elements of the residual.  A tensor compressed by itself has none: A.resid is the caller's tensor then, which is read where it
 // lies, up to its last element, with NaN as zero (scan's policy), and never written.  Half of the traffic of scan: with a copy of
 // the tensor as its residual, 38.6 M elements took 63 us.
-// FRESH: A.fresh is not 0, or kRuntime.
-constexpr int kRuntime = 2;
-
-template <int FRESH = kRuntime>
+// FRESH: A.fresh is not 0.
+template <bool FRESH>
 __device__ __forceinline__ float4 resid4(const SelectArgs& A, uint32_t i) {
-  if (FRESH == 0 || (FRESH == kRuntime && !A.fresh)) return __ldcg(reinterpret_cast<const float4*>(A.resid + i));
+  if (!FRESH) return __ldcg(reinterpret_cast<const float4*>(A.resid + i));
   const float4 a = load4_guarded(A.resid, i, A.fresh);
   return make_float4(number_or_zero(a.x), number_or_zero(a.y), number_or_zero(a.z), number_or_zero(a.w));
 }
 
-template <int FRESH = kRuntime>
+template <bool FRESH>
 __device__ __forceinline__ float resid1(const SelectArgs& A, uint32_t i) {
-  if (FRESH == 0 || (FRESH == kRuntime && !A.fresh)) return __ldcg(A.resid + i);
+  if (!FRESH) return __ldcg(A.resid + i);
   return i < A.fresh ? number_or_zero(A.resid[i]) : 0.f;
 }
 
@@ -896,10 +896,11 @@ __device__ __forceinline__ uint2 cut_of_many(const uint2* cand, uint32_t c, uint
 // the lowest-ranked one last.  Returns its key.  `list` is the area of the tensor's lists, which nobody reads any more.  Ranked
 // by one CTA of 1024 threads, which drew a stream position per item from one address and copied a block with one thread,
 // this took up to 0.1 ms for the 25,000 undecided items of a 64 MB bucket whose gradients had changed in scale.
-template <bool kBlock>
-__device__ __noinline__ uint32_t send_best(const SelectArgs& A, EmitShared& S, const uint2* cand, uint32_t c, uint32_t take,
-                                           uint32_t done, uint2* list) {
-  const Job J = job_of(A, kBlock);
+// Rare, but inline: as a function of its own the loops over the candidates took a quarter longer (a threshold-v16 tensor of 16.8 M
+// elements whose threshold is far too high, 10 % kept: 5.4 to 6.3 ms against 3.5; 1 %: 2.8 against 2.4).
+template <bool kBlock, bool FRESH>
+__device__ __forceinline__ uint32_t send_best(const SelectArgs& A, const Job& J, EmitShared& S, const uint2* cand, uint32_t c,
+                                              uint32_t take, uint32_t done, uint2* list) {
   constexpr uint32_t kPerItem = kBlock ? 16u : 1u;
   constexpr int kIlp = kStageItems / kEmitThreads;
   const uint32_t tid = threadIdx.x;
@@ -933,7 +934,7 @@ __device__ __noinline__ uint32_t send_best(const SelectArgs& A, EmitShared& S, c
       uint2 e = make_uint2(0u, 0u);
       if (t < take * kPerItem) {
         e.x = __ldcg(&list[t / kPerItem].x) * kPerItem + t % kPerItem;
-        e.y = __float_as_uint(resid1(A, e.x));
+        e.y = __float_as_uint(resid1<FRESH>(A, e.x));
       }
       stage[u * kEmitThreads + tid] = e;
     }
@@ -947,6 +948,7 @@ __device__ __noinline__ uint32_t send_best(const SelectArgs& A, EmitShared& S, c
 
 // Top-k, last CTA of a tensor: the best `rem` of the `c` undecided items complete the stream.  Returns the k-th largest key, or
 // kNoCut.
+template <bool FRESH>
 __device__ __forceinline__ uint32_t settle_top(const SelectArgs& A, const Job& J, EmitShared& S, const uint2* undecided,
                                                uint32_t c, uint32_t rem, uint32_t key_lo, uint32_t key_hi) {
   const uint32_t done = J.kk - rem;
@@ -955,7 +957,7 @@ __device__ __forceinline__ uint32_t settle_top(const SelectArgs& A, const Job& J
     if (t_key != kNoCut) send_staged(A, S, kNamed, rem, done);
     return t_key;
   }
-  return send_best<false>(A, S, undecided, c, rem, done, A.cand + J.sd.off);
+  return send_best<false, FRESH>(A, J, S, undecided, c, rem, done, A.cand + J.sd.off);
 }
 
 // Sends the items [j0, j1) of one piece at positions base + j; items and positions are in index order.  The dependent loads
@@ -1019,6 +1021,7 @@ __device__ __forceinline__ void send_range(const SelectArgs& A, const Job& J, Em
 // the fill.  A listed block is sent whenever the stream is short; what the narrow wire format's rounding leaves of it in the
 // residual waits for the next select, so that a stream names an element once.  The lists, and not the residual, say which
 // blocks these are: other CTAs of the tensor may be sending them now.  Returns the number collected by this CTA.
+template <bool FRESH>
 __device__ __noinline__ uint32_t collect_unlisted(const SelectArgs& A, EmitShared& S, const uint2* area, uint32_t total, uint2* cand) {
   const Job J = job_of(A, true);
   constexpr uint32_t kQuads = kEmitThreads / 4, kKeys = 8;      // blocks side by side; keys a lane keeps per round
@@ -1043,7 +1046,7 @@ __device__ __noinline__ uint32_t collect_unlisted(const SelectArgs& A, EmitShare
       for (uint32_t q = 0; q < 4u; ++q) {   // independent loads in flight
         const uint32_t b = b0 + (s * 4u + q) * kQuads + (tid >> 2);
         const bool take = b < n_blk && !(S.hist[b >> 5] >> (b & 31u) & 1u);
-        a[q] = take ? resid4(A, src + b * 16u) : make_float4(0.f, 0.f, 0.f, 0.f);
+        a[q] = take ? resid4<FRESH>(A, src + b * 16u) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
 #pragma unroll
       for (uint32_t q = 0; q < 4u; ++q) {
@@ -1070,6 +1073,7 @@ __device__ __noinline__ uint32_t collect_unlisted(const SelectArgs& A, EmitShare
 }
 
 // The candidates do not reach down to the k-th largest value: a histogram of the rest.
+template <bool FRESH>
 __device__ __noinline__ void count_rest(const SelectArgs& A, EmitShared& S) {
   const uint32_t tid = threadIdx.x;
   const Job J = job_of(A, false);
@@ -1079,7 +1083,7 @@ __device__ __noinline__ void count_rest(const SelectArgs& A, EmitShared& S) {
   uint32_t zeros = 0;
 #pragma unroll 4
   for (uint32_t i = tid * 4u; i < J.len; i += kEmitThreads * 4u) {
-    const float4 a = resid4(A, J.pc.start + i);
+    const float4 a = resid4<FRESH>(A, J.pc.start + i);
     const uint32_t key[4] = {key_bits(a.x), key_bits(a.y), key_bits(a.z), key_bits(a.w)};
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -1189,7 +1193,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const __grid_constant_
           if (tid == 0 && t_key != kNoCut) step_top(A, J, ss, t_key, 0u);
         }
       } else if (short_of && ok) {
-        count_rest(A, S);      // for `refill`
+        count_rest<FRESH>(A, S);      // for `refill`
       } else if (!short_of) {
         plan_top(A.hist_top + (size_t)J.pc.first * kHistBins, hist_copies(J.sd.n_pad), found, J.kk, false, S);
         top_bin_range(S.res[0], top_centre(ss), key_lo, key_hi);
@@ -1219,7 +1223,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const __grid_constant_
         if (!short_of) {
           const uint32_t c = J.pc.count == 1u ? noted : __ldcg(&J.wp->cand_cnt);
           if (may && rem != 0u && rem <= c) {
-            const uint32_t t_key = settle_top(A, J, S, undecided, c, rem, key_lo, key_hi);
+            const uint32_t t_key = settle_top<FRESH>(A, J, S, undecided, c, rem, key_lo, key_hi);
             if (tid == 0 && t_key != kNoCut) step_top(A, J, ss, t_key, found);
           } else if (may && tid == 0) {
             set_status(A.status, kBadCandidate);   // cannot happen: the histogram counted these very items
@@ -1242,7 +1246,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const __grid_constant_
       const bool rescan = kBlock && short_of && (!ss.inited || c_near < J.kk - found);
       uint32_t collected = 0;
       if (rescan) {
-        collected = collect_unlisted(A, S, area, total, nears);
+        collected = collect_unlisted<FRESH>(A, S, area, total, nears);
       } else if (kBlock && short_of && near_total) {
         // the fill needs the tensor's near misses in one place
         if (tid == 0) S.word[2] = J.pc.count == 1u ? 0u : atomicAdd(&J.wp->cand_cnt, near_total);
@@ -1321,7 +1325,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const __grid_constant_
               }
             }
           } else if (take) {
-            t_key = send_best<true>(A, S, nears, c, take, found, A.cand + (J.sd.off >> 4));
+            t_key = send_best<true, FRESH>(A, J, S, nears, c, take, found, A.cand + (J.sd.off >> 4));
           }
           // fewer blocks with anything in them than the budget: the rest of the stream says "no entry"
 #pragma unroll 1
@@ -1371,6 +1375,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const __grid_constant_
 }
 
 // Top-k tensors whose candidates fell short: the exact selection from the residual, with the histogram that `emit` took.
+template <bool FRESH>
 __global__ void __launch_bounds__(kEmitThreads, 2) k_refill(const __grid_constant__ SelectArgs A) {
   __shared__ EmitShared S;
   behind_previous();
@@ -1400,7 +1405,7 @@ __global__ void __launch_bounds__(kEmitThreads, 2) k_refill(const __grid_constan
       for (uint32_t i0 = 0; i0 < len && base < rem; i0 += kEmitThreads * 4u) {
         const uint32_t i = i0 + tid * 4u;
         const bool act = i < len;
-        const float4 a = act ? resid4(A, J.pc.start + i) : make_float4(1.f, 1.f, 1.f, 1.f);
+        const float4 a = act ? resid4<FRESH>(A, J.pc.start + i) : make_float4(1.f, 1.f, 1.f, 1.f);
         const uint32_t at = J.pc.start + i, idx[4] = {at, at + 1u, at + 2u, at + 3u};
         const uint32_t bits[4] = {__float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(a.z), __float_as_uint(a.w)};
         uint32_t zero = 0, total;
@@ -1420,7 +1425,7 @@ __global__ void __launch_bounds__(kEmitThreads, 2) k_refill(const __grid_constan
         for (int u = 0; u < kItems / 4; ++u) {
           const uint32_t i = i0 + (u * kEmitThreads + tid) * 4u;
           const bool act = i < len;
-          const float4 a = act ? resid4(A, J.pc.start + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+          const float4 a = act ? resid4<FRESH>(A, J.pc.start + i) : make_float4(0.f, 0.f, 0.f, 0.f);
           const float v[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
@@ -1434,7 +1439,7 @@ __global__ void __launch_bounds__(kEmitThreads, 2) k_refill(const __grid_constan
     if (last_of_tensor(J, S)) {
       const uint32_t c = J.pc.count == 1u ? noted : __ldcg(&J.wp->cand_cnt);
       if (may && rem != 0u && (zero_fill || rem <= c)) {
-        const uint32_t t_key = zero_fill ? 0u : settle_top(A, J, S, undecided, c, rem, key_lo, key_hi);
+        const uint32_t t_key = zero_fill ? 0u : settle_top<FRESH>(A, J, S, undecided, c, rem, key_lo, key_hi);
         if (tid == 0 && t_key != kNoCut) step_top(A, J, ss, t_key, 0u);
       } else if (may && tid == 0) {
         set_status(A.status, kBadCandidate);
@@ -1474,7 +1479,8 @@ cudaError_t launch_select_one_pass(const SelectArgs& A, cudaStream_t stream, cud
   // behind it (64 MB bucket, eight destinations).
   e = before_emit == nullptr && !A.publish ? launch_behind(emit[fresh][mode], A.n_pieces, kEmitThreads, stream, A)
                                            : launch_first(emit[fresh][mode], A.n_pieces, kEmitThreads, stream, A);
-  if (e == cudaSuccess && A.compressor == kTopk) e = launch_behind(k_refill, A.n_pieces, kEmitThreads, stream, A);
+  if (e == cudaSuccess && A.compressor == kTopk)
+    e = launch_behind(A.fresh ? k_refill<true> : k_refill<false>, A.n_pieces, kEmitThreads, stream, A);
   return e;
 }
 
