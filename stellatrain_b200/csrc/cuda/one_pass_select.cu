@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(kScanThreads, 4) k_scan(SelectArgs A) {
 namespace {
 
 struct EmitShared {
-  uint2 stage[kStageItems];
+  alignas(16) uint2 stage[kStageItems];      // also read and written four words at a time
   uint32_t hist[2048];
   uint32_t pre[kMaxPieceRuns + 1];     // listed items in front of each run of the piece
   uint32_t near[kMaxPieceRuns + 1];    // near misses in front of each run of the piece
@@ -408,6 +408,8 @@ struct EmitShared {
   int dest;
   uint64_t slot_off;
 };
+static_assert(alignof(EmitShared) % alignof(uint4) == 0 && offsetof(EmitShared, stage) % alignof(uint4) == 0,
+              "16-byte accesses to EmitShared::stage");
 
 // Run (of the piece) that holds item j: the last one that starts at or in front of it and is not empty.
 __device__ __forceinline__ uint32_t run_of(const uint32_t* pre, uint32_t j) {
