@@ -64,7 +64,8 @@ struct NativeEngine::Impl {
   // slow link has one token bucket.
   cudaStream_t sparse = nullptr, second = nullptr;
   // The update of the previous iteration and the streaming kernel of this one touch nothing in common: with one rank the update
-  // runs on a stream of its own.  The kernels behind the streaming one wait for it: they advance the select epoch, by which the
+  // runs on a stream of its own when the one-pass chain is next (the other chains and random-k have no kernel that may begin in
+  // front of the update's end: theirs stays on the bucket's lane).  The kernels behind the streaming one wait for it: they advance the select epoch, by which the
   // update knows whether there is anything to apply (nothing after a flush).  Captured steps with this, and with streaming kernels
   // one priority level under the others: ViT-B/16 272 -> 249 us, ResNet-152 173.5 -> 165.7, GPT-2 490 -> 482, ResNet-50 106.
   cudaStream_t aside = nullptr;
@@ -198,7 +199,8 @@ struct NativeEngine::Impl {
     check(cudaStreamWaitEvent(b.lane, b.grad_ready, 0));
     if (staleness == 1 && b.has_pending_apply) {
       // a single bucket launched call by call is bound by the host: no second stream there
-      if (aside != nullptr && (capturing || buckets.size() > 1)) {
+      const BucketHandle* h = b.spec.select_handle ? b.spec.select_handle : b.spec.handle;
+      if (aside != nullptr && h->one_pass_next() && (capturing || buckets.size() > 1)) {
         check(cudaStreamWaitEvent(aside, b.grad_ready, 0));
         if (!capturing && b.select_done_set) check(cudaStreamWaitEvent(aside, b.select_done, 0));     // the stream it reads
         apply(b, aside);

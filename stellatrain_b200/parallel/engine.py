@@ -200,8 +200,9 @@ class SparseDPEngine:
         # ranks, Python hooks and a shaped link keep one stream.
         self._second_stream: Optional[torch.cuda.Stream] = None
         self._second_high = high
-        # Also with one rank and the native engine: updates run beside the streaming kernel of their bucket's next select, whose
-        # emission waits for them (and with it everybody who waits for the bucket's stream).
+        # Also with one rank and the native engine: updates run beside the streaming kernel of their bucket's next one-pass select,
+        # whose emission waits for them (and with it everybody who waits for the bucket's stream).  In front of any other select
+        # they stay on the bucket's stream.
         self._apply_stream: Optional[torch.cuda.Stream] = None
         self.iteration = 0            # completed optimiser iterations (selects issued per bucket)
         self.micro_step = 0

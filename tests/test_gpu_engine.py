@@ -756,6 +756,35 @@ def test_updates_beside_the_streaming_kernel_equal_those_in_front_of_it(compress
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("compressor,beside", [("thresholdv16", True), ("randomk", False)])
+def test_updates_leave_their_buckets_stream_only_for_a_one_pass_select(compressor, beside, tmp_path):
+    """Eager steps of several buckets.  In front of a select that waits for the update in any case (random-k, the four-kernel
+    chain) a third stream would only add waits and make the updates of both lanes queue up."""
+    import json
+
+    model = small_net()
+    eng = make_engine(model, compressor=compressor, ratio=0.9, optimizer="sgd", staleness=1, optimizer_options={"lr": 0.01})
+    assert len(eng.buckets) > 2 and len(eng.sparse_streams) == 2
+    data = batches(8)
+    for x, y in data[:4]:
+        F.cross_entropy(model(x), y).backward()
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        for x, y in data[4:]:
+            F.cross_entropy(model(x), y).backward()
+        torch.cuda.synchronize()
+    prof.export_chrome_trace(str(tmp_path / "trace.json"))
+    streams = {}
+    for e in json.loads((tmp_path / "trace.json").read_text())["traceEvents"]:
+        if e.get("cat") == "kernel" and " st::k_" in " " + e["name"]:
+            kind = "update" if "k_apply_single" in e["name"] else "select"
+            streams.setdefault(kind, set()).add(e["args"]["stream"])
+    assert len(streams["select"]) == 2
+    assert streams["update"].isdisjoint(streams["select"]) if beside else streams["update"] == streams["select"]
+    eng.synchronize()
+    eng.close()
+
+
 def test_a_checkpoint_with_another_ratio_makes_a_captured_step_stale():
     """Its launches carry the sizes and tables of the old ratio; a checkpoint with the same ratio leaves it usable."""
     import torch.nn as nn
