@@ -837,15 +837,20 @@ class SparseDPEngine:
         if not self._pending_weights:
             return
         it = self.iterations_started()
-        # eager: the bucket's own stream carries the applies; a replayed graph carries them on the stream it is launched on
+        # Eager: the row is written on the bucket's own stream.  That is behind the apply which wanted the old one and in front
+        # of the apply which wants the new one, whether they run on the same stream or (`_apply_stream`) on another: the select
+        # of iteration i - 1 has waited for its iteration's apply, and the apply of iteration i + 1 waits for the select of
+        # iteration i, which follows the row.  A replayed graph carries everything on the stream it is launched on.
         keep = []
         for entry in self._pending_weights:
             since, w, done = entry
             for step in (0, 1):
                 if it == since + step and done == step:
                     for bi, rt in enumerate(self.buckets):
-                        with torch.cuda.stream(stream if stream is not None else self.stream_of_bucket(bi)):
+                        on = stream if stream is not None else self.stream_of_bucket(bi)
+                        with torch.cuda.stream(on):
                             rt.bucket.set_weight_row((since + step + 1) & 1, w)
+                        w.record_stream(on)      # the copy may run long after the last reference to `w` is gone
                     entry[2] = done = step + 1
             if done < 2:
                 keep.append(entry)

@@ -635,6 +635,46 @@ def test_rank_weights_switch_at_a_named_iteration_without_draining(staleness):
 
 
 @pytest.mark.parametrize("staleness", [0, 1])
+@pytest.mark.parametrize("late", ["first", "second"])
+def test_weight_rows_keep_their_place_when_a_buckets_stream_is_late(staleness, late):
+    """Rows of the merge-weight table are written on the buckets' streams, updates may run on another.  One lane is held back
+    by 2 ms in front of every iteration's rows while host and compute stream run ahead: weights that change twice still count
+    from exactly the iterations named."""
+    from stellatrain_b200 import _build
+
+    hold = torch.tensor([2_000_000], dtype=torch.int64, device="cuda")
+    steps, changes = 10, {2: ([0.5], 4), 5: ([2.0], 7)}      # announced in front of iteration 2 / 5, from iteration 4 / 7 on
+
+    def run(n_steps, changes, held):
+        model = _CoefficientNet().cuda()
+        eng = make_engine(model, compressor="topk", ratio=0.9, optimizer="sgd", staleness=staleness,
+                          optimizer_options={"lr": 1.0}, bucket_mb=0.002)
+        assert len(eng.buckets) > 2 and len(eng.sparse_streams) == 2
+        g = torch.Generator(device="cuda").manual_seed(78)
+        coeffs = [[torch.randn(p.numel(), device="cuda", generator=g) for p in model.ps] for _ in range(n_steps)]
+        for i, c in enumerate(coeffs):
+            if i in changes:
+                eng.set_rank_weights(changes[i][0], from_iteration=changes[i][1])
+            if held:
+                s = eng.sparse_streams[0 if late == "first" else 1]
+                _build.load_extension("_C").delay(hold.data_ptr(), 10_000_000, s.cuda_stream)
+            model(c).backward()
+        eng.synchronize()
+        eng.check_status()
+        out = [p.detach().clone() for p in model.ps]
+        eng.close()
+        return out
+
+    for a, b in zip(run(steps, changes, True), run(steps, changes, False)):
+        assert torch.equal(a, b)
+    # updates of iterations 0..3 count once, of 4..6 half, of 7..9 twice
+    ends = {n: run(n, {}, False) for n in (0, 4, 7, steps)}
+    for i, got in enumerate(run(steps, changes, True)):
+        p = [ends[n][i] for n in (0, 4, 7, steps)]
+        torch.testing.assert_close(got - p[0], (p[1] - p[0]) + 0.5 * (p[2] - p[1]) + 2.0 * (p[3] - p[2]), rtol=1e-5, atol=1e-4)
+
+
+@pytest.mark.parametrize("staleness", [0, 1])
 @pytest.mark.parametrize("grad_mode", ["steal", "flat"])
 def test_bucket_chains_on_two_streams_equal_one_stream(staleness, grad_mode):
     """One rank, several buckets: the native engine lets them take turns on two streams, Python hooks use one.  Same bits,
