@@ -346,8 +346,8 @@ cudaError_t launch_apply(const ApplyArgs& A, int max_ctas_per_source, int phase,
   if (A.cap == 0 || A.world <= 0) return cudaSuccess;
   if (A.world > kMaxWorld) return cudaErrorInvalidValue;
   if (A.ent_hi < A.ent_lo || A.ent_hi > A.cap) return cudaErrorInvalidValue;
-  // one entry per thread: the update of an entry is a chain of dependent random accesses, so the
-  // only way to hide its latency is to have every entry in flight at once
+  // The update of an entry is a chain of dependent random accesses: its latency is hidden by many entries in flight at once.  One
+  // entry per thread where streams are merged; the update of a single source may have four, see k_apply_single.
   if (phase == 0 || phase == 1) {
     int parts = (int)((A.ent_hi - A.ent_lo + kThreads - 1) / kThreads);
     if (parts < 1) parts = 1;

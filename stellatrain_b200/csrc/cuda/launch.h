@@ -31,8 +31,7 @@ inline cudaError_t launch_first(void (*kernel)(Params...), dim3 grid, int thread
 }
 
 // Kernel directly behind another kernel of the stream, with no event in between: it may begin while that one ends, see
-// behind_previous().  Worth 0.1 to 0.6 % of a captured step; not for
-// emission to peers, see launch_select_one_pass.
+// behind_previous().  Worth 0.1 to 0.6 % of a captured step; not for emission to peers, see launch_select_one_pass.
 template <typename... Params, typename... Args>
 inline cudaError_t launch_behind(void (*kernel)(Params...), dim3 grid, int threads, cudaStream_t stream, const Args&... args) {
   cudaLaunchAttribute attr{};

@@ -23,9 +23,9 @@
 //
 // What bounds it, 64 MB bucket (16.8 M elements, 201 MB of traffic, 31 us at the 6.5 TB/s of a plain copy), one B200:
 //   scan    memory: 35.5 us for threshold-v16 (29 where L2 holds part of a single bucket), 36 us for top-k at 0.1 %, 39 us at 1 %
-//           (list and histogram).  Runs of one
-//           warp need no barrier and no shared state, so a late load holds up nothing else; with one CTA per 8192 elements
-//           that scanned, chained counts over CTAs and emitted by itself the same traffic took 54 us.
+//           (list and histogram).  Runs of one warp need no barrier and no shared state, so a late load holds up nothing else;
+//           with one CTA per 8192 elements that scanned, chained counts over CTAs and emitted by itself the same traffic took
+//           54 us.
 //   emit    latency, a chain of about ten trips to L2, and its own instructions (see send_staged): 9.6 us for threshold-v16, 16 us
 //           for top-k at 1 %; the slowest sections of the latter are the sum of the histograms (3 us) and the last CTA's
 //           search (3 us).
@@ -52,7 +52,7 @@ constexpr int kEmitThreads = 256;
 constexpr uint32_t kStageItems = 2048;         // entries staged at a time
 constexpr uint32_t kPickMax = 2048;            // candidates that a CTA holds in shared memory to pick the best from
 
-// Top-k of a tensor this small is picked from registers by its one CTA of `emit`: its k-th largest value moves too much from
+// Top-k of a tensor this small is picked from shared memory by its one CTA of `emit`: its k-th largest value moves too much from
 // step to step to be worth predicting, and no list, histogram or cut is needed.
 constexpr uint32_t kTopDirect = 4096;
 constexpr float kTopWindowDefault = 0.1f;
@@ -1478,7 +1478,7 @@ cudaError_t launch_select_one_pass(const SelectArgs& A, cudaStream_t stream, cud
   if (e == cudaSuccess && before_emit != nullptr) e = cudaStreamWaitEvent(stream, before_emit, 0);
   if (e != cudaSuccess) return e;
   // With peers every CTA of the emission ends in a system-wide fence; begun beside the scan it took 40 us on one of two boxes, 23
-  // behind it (64 MB bucket, eight destinations).
+  // behind it (64 MB bucket, eight destinations; 20 since entries are read once for all of them).
   e = before_emit == nullptr && !A.publish ? launch_behind(emit[fresh][mode], A.n_pieces, kEmitThreads, stream, A)
                                            : launch_first(emit[fresh][mode], A.n_pieces, kEmitThreads, stream, A);
   if (e == cudaSuccess && A.compressor == kTopk)
