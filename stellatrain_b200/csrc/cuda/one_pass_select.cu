@@ -539,8 +539,8 @@ enum Staged : uint32_t { kInOrder = 0, kNamed = 1, kWords = 2 };
 // The kernels of this part run once per CTA and step from one section to the next: what they wait for, besides L2, is their own
 // instructions.  With the stores to the destinations inlined wherever pairs are sent, and the searches below unrolled over
 // registers, `emit` had 166 KB of code for top-k, and a section took microseconds of fetches the first time an SM came to it (the
-// last CTA's search in a tensor 7 us for 100 items).  So sections that are used twice or rarely are functions, loops are loops, and
-// items lie in shared memory: a 64 MB bucket takes 16 us instead of 23 (top-k, 1 %) and 9.6 instead of 12.9 (threshold-v16).
+// last CTA's search in a tensor 7 us for 100 items).  So sections that are used twice are functions, loops are loops, and items
+// lie in shared memory: a 64 MB bucket takes 16 us instead of 23 (top-k, 1 %) and 9.6 instead of 12.9 (threshold-v16).
 __device__ __noinline__ void send_staged(const SelectArgs& A, EmitShared& S, Staged how, uint32_t m, uint32_t pos) {
   const uint32_t* const words = reinterpret_cast<const uint32_t*>(S.stage);
   const uint32_t n_out = S.n_out, off = S.off;
@@ -1022,10 +1022,11 @@ __device__ __forceinline__ void send_range(const SelectArgs& A, const Job& J, Em
 // Threshold-v16: the blocks of a piece that hold something and are not on its lists (`total` listed blocks), as candidates of
 // the fill.  A listed block is sent whenever the stream is short; what the narrow wire format's rounding leaves of it in the
 // residual waits for the next select, so that a stream names an element once.  The lists, and not the residual, say which
-// blocks these are: other CTAs of the tensor may be sending them now.  Returns the number collected by this CTA.
+// blocks these are: other CTAs of the tensor may be sending them now.  Returns the number collected by this CTA.  Inline: as a
+// function of its own it made the select of a tensor of 3 M elements whose threshold is twice too high 476 us instead of 461.
 template <bool FRESH>
-__device__ __noinline__ uint32_t collect_unlisted(const SelectArgs& A, EmitShared& S, const uint2* area, uint32_t total, uint2* cand) {
-  const Job J = job_of(A, true);
+__device__ __forceinline__ uint32_t collect_unlisted(const SelectArgs& A, const Job& J, EmitShared& S, const uint2* area,
+                                                     uint32_t total, uint2* cand) {
   constexpr uint32_t kQuads = kEmitThreads / 4, kKeys = 8;      // blocks side by side; keys a lane keeps per round
   static_assert(kMaxPieceElems / 16u / 32u <= 2048u, "a bit per block of a piece fits EmitShared::hist");
   const uint32_t tid = threadIdx.x, first = J.pc.start >> 4;
@@ -1248,7 +1249,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const __grid_constant_
       const bool rescan = kBlock && short_of && (!ss.inited || c_near < J.kk - found);
       uint32_t collected = 0;
       if (rescan) {
-        collected = collect_unlisted<FRESH>(A, S, area, total, nears);
+        collected = collect_unlisted<FRESH>(A, J, S, area, total, nears);
       } else if (kBlock && short_of && near_total) {
         // the fill needs the tensor's near misses in one place
         if (tid == 0) S.word[2] = J.pc.count == 1u ? 0u : atomicAdd(&J.wp->cand_cnt, near_total);
