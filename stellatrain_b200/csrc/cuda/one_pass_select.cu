@@ -174,17 +174,28 @@ __device__ __forceinline__ float number_or_zero(float x) { return x == x ? x : 0
 // lies, up to its last element, with NaN as zero (scan's policy), and never written.  Half of the traffic of scan: with a copy of
 // the tensor as its residual, 38.6 M elements took 63 us.
 // FRESH: A.fresh is not 0.
+//
+// Four elements are read in two parts, so that a thread's loads travel together: `load4` for all of them, without a branch, then
+// `resid4` for each, which adds what the tensor's end cut off.  With a branch around every load they went one after the other:
+// `compress` of 16.8 M elements at 1 %, us of emit and refill, where the values fell to a thirtieth 705 (with this 478), to a third
+// 270 (194), grew thirtyfold 1063 (806); threshold-v16, fallen to a third, 185 (107).
 template <bool FRESH>
-__device__ __forceinline__ float4 resid4(const SelectArgs& A, uint32_t i) {
-  if (!FRESH) return __ldcg(reinterpret_cast<const float4*>(A.resid + i));
-  const float4 a = load4_guarded(A.resid, i, A.fresh);
+__device__ __forceinline__ float4 load4(const SelectArgs& A, uint32_t i) {
+  return !FRESH || i + 4u <= A.fresh ? __ldcg(reinterpret_cast<const float4*>(A.resid + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+template <bool FRESH>
+__device__ __forceinline__ float4 resid4(const SelectArgs& A, uint32_t i, float4 a) {
+  if (!FRESH) return a;
+  if (i < A.fresh && i + 4u > A.fresh) a = load4_guarded(A.resid, i, A.fresh);
   return make_float4(number_or_zero(a.x), number_or_zero(a.y), number_or_zero(a.z), number_or_zero(a.w));
 }
 
 template <bool FRESH>
 __device__ __forceinline__ float resid1(const SelectArgs& A, uint32_t i) {
   if (!FRESH) return __ldcg(A.resid + i);
-  return i < A.fresh ? number_or_zero(A.resid[i]) : 0.f;
+  const float a = __ldcg(A.resid + min(i, A.fresh - 1u));
+  return i < A.fresh ? number_or_zero(a) : 0.f;
 }
 
 }  // namespace
@@ -767,17 +778,18 @@ __device__ __forceinline__ uint32_t top_direct(const SelectArgs& A, const Job& J
   const uint32_t tid = threadIdx.x;
   uint4* const words = reinterpret_cast<uint4*>(S.stage);
   uint32_t top = 0;
-  uint4 a[4];
+  float4 v[4];
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
-    const uint32_t i = u * kEmitThreads + tid;
-    const float4 v = i * 4u < J.sd.n_pad ? resid4<FRESH>(A, J.sd.off + i * 4u) : make_float4(0.f, 0.f, 0.f, 0.f);
-    a[u] = make_uint4(__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w));
+    const uint32_t i = (u * kEmitThreads + tid) * 4u;
+    v[u] = i < J.sd.n_pad ? load4<FRESH>(A, J.sd.off + i) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
-    words[u * kEmitThreads + tid] = a[u];
-    top = max(max(max(top, a[u].x & 0x7fffffffu), max(a[u].y & 0x7fffffffu, a[u].z & 0x7fffffffu)), a[u].w & 0x7fffffffu);
+    const float4 e = resid4<FRESH>(A, J.sd.off + (u * kEmitThreads + tid) * 4u, v[u]);
+    const uint4 a = make_uint4(__float_as_uint(e.x), __float_as_uint(e.y), __float_as_uint(e.z), __float_as_uint(e.w));
+    words[u * kEmitThreads + tid] = a;
+    top = max(max(max(top, a.x & 0x7fffffffu), max(a.y & 0x7fffffffu, a.z & 0x7fffffffu)), a.w & 0x7fffffffu);
   }
   top = block_max_u32(top, S.tmp);
   const uint2 cut = find_cut(S, A.status, true, J.sd.n_pad, J.kk, top, kTwoOctaves, 0u, J.sd.n_pad);
@@ -983,14 +995,15 @@ __device__ __forceinline__ void send_range(const SelectArgs& A, const Job& J, Em
       }
 #pragma unroll
       for (int u = 0; u < kPer; ++u)
-        if (t0 + (u * kEmitThreads + threadIdx.x) * 4u < end) a[u] = resid4<FRESH>(A, gi[u]);
+        if (t0 + (u * kEmitThreads + threadIdx.x) * 4u < end) a[u] = load4<FRESH>(A, gi[u]);
 #pragma unroll
       for (int u = 0; u < kPer; ++u) {
         const uint32_t q = (u * kEmitThreads + threadIdx.x) * 4u;
         if (t0 + q < end) {
+          const float4 v = resid4<FRESH>(A, gi[u], a[u]);
           uint4* const to = reinterpret_cast<uint4*>(&S.stage[q]);
-          to[0] = make_uint4(gi[u], __float_as_uint(a[u].x), gi[u] + 1u, __float_as_uint(a[u].y));
-          to[1] = make_uint4(gi[u] + 2u, __float_as_uint(a[u].z), gi[u] + 3u, __float_as_uint(a[u].w));
+          to[0] = make_uint4(gi[u], __float_as_uint(v.x), gi[u] + 1u, __float_as_uint(v.y));
+          to[1] = make_uint4(gi[u] + 2u, __float_as_uint(v.z), gi[u] + 3u, __float_as_uint(v.w));
         }
       }
     } else {
@@ -1045,15 +1058,19 @@ __device__ __forceinline__ uint32_t collect_unlisted(const SelectArgs& A, const 
 #pragma unroll
     for (uint32_t s = 0; s < kKeys; ++s) {
       float4 a[4];
+      uint32_t left_out = 0;
 #pragma unroll
       for (uint32_t q = 0; q < 4u; ++q) {   // independent loads in flight
         const uint32_t b = b0 + (s * 4u + q) * kQuads + (tid >> 2);
         const bool take = b < n_blk && !(S.hist[b >> 5] >> (b & 31u) & 1u);
-        a[q] = take ? resid4<FRESH>(A, src + b * 16u) : make_float4(0.f, 0.f, 0.f, 0.f);
+        a[q] = take ? load4<FRESH>(A, src + b * 16u) : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (FRESH && !take) left_out |= 1u << q;
       }
 #pragma unroll
       for (uint32_t q = 0; q < 4u; ++q) {
-        const uint32_t k = __float_as_uint(quad_l1(a[q]));
+        // a block left out stays zero: no end of the tensor lies behind ~0
+        const uint32_t at = left_out >> q & 1u ? kSentinelIdx : src + (b0 + (s * 4u + q) * kQuads + (tid >> 2)) * 16u;
+        const uint32_t k = __float_as_uint(quad_l1(resid4<FRESH>(A, at, a[q])));
         if ((tid & 3u) == q) key[s] = k;
       }
       there |= (key[s] != 0u ? 1u : 0u) << s;
@@ -1084,16 +1101,26 @@ __device__ __noinline__ void count_rest(const SelectArgs& A, EmitShared& S) {
   for (uint32_t b = tid; b < (uint32_t)kHistBins; b += kEmitThreads) S.hist[b] = 0u;
   __syncthreads();
   uint32_t zeros = 0;
-#pragma unroll 4
-  for (uint32_t i = tid * 4u; i < J.len; i += kEmitThreads * 4u) {
-    const float4 a = resid4<FRESH>(A, J.pc.start + i);
+  auto count = [&](const float4& a) {
     const uint32_t key[4] = {key_bits(a.x), key_bits(a.y), key_bits(a.z), key_bits(a.w)};
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       if (key[e] == 0u) ++zeros;
       else if (key[e] < cut) atomicAdd(&S.hist[rest_bin(key[e], cut)], 1u);
     }
+  };
+  constexpr int kQuads = 4;
+  uint32_t i = tid * 4u;
+#pragma unroll 1
+  for (; i + (kQuads - 1) * kEmitThreads * 4u < J.len; i += kQuads * kEmitThreads * 4u) {
+    float4 a[kQuads];
+#pragma unroll
+    for (int u = 0; u < kQuads; ++u) a[u] = load4<FRESH>(A, J.pc.start + i + u * kEmitThreads * 4u);
+#pragma unroll
+    for (int u = 0; u < kQuads; ++u) count(resid4<FRESH>(A, J.pc.start + i + u * kEmitThreads * 4u, a[u]));
   }
+#pragma unroll 1
+  for (; i < J.len; i += kEmitThreads * 4u) count(resid4<FRESH>(A, J.pc.start + i, load4<FRESH>(A, J.pc.start + i)));
   block_excl_scan(zeros, S.tmp, zeros);
   uint32_t* gh = A.hist_rest + (size_t)J.pc.seg * kHistBins;
   for (uint32_t b = tid; b < (uint32_t)kHistBins; b += kEmitThreads)
@@ -1408,7 +1435,7 @@ __global__ void __launch_bounds__(kEmitThreads, 2) k_refill(const __grid_constan
       for (uint32_t i0 = 0; i0 < len && base < rem; i0 += kEmitThreads * 4u) {
         const uint32_t i = i0 + tid * 4u;
         const bool act = i < len;
-        const float4 a = act ? resid4<FRESH>(A, J.pc.start + i) : make_float4(1.f, 1.f, 1.f, 1.f);
+        const float4 a = act ? resid4<FRESH>(A, J.pc.start + i, load4<FRESH>(A, J.pc.start + i)) : make_float4(1.f, 1.f, 1.f, 1.f);
         const uint32_t at = J.pc.start + i, idx[4] = {at, at + 1u, at + 2u, at + 3u};
         const uint32_t bits[4] = {__float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(a.z), __float_as_uint(a.w)};
         uint32_t zero = 0, total;
@@ -1424,11 +1451,17 @@ __global__ void __launch_bounds__(kEmitThreads, 2) k_refill(const __grid_constan
       constexpr int kItems = 16;
       for (uint32_t i0 = 0; i0 < len; i0 += kEmitThreads * kItems) {
         uint32_t idx[kItems], bits[kItems];
+        float4 raw[kItems / 4];
+#pragma unroll
+        for (int u = 0; u < kItems / 4; ++u) {
+          const uint32_t i = i0 + (u * kEmitThreads + tid) * 4u;
+          raw[u] = i < len ? load4<FRESH>(A, J.pc.start + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
 #pragma unroll
         for (int u = 0; u < kItems / 4; ++u) {
           const uint32_t i = i0 + (u * kEmitThreads + tid) * 4u;
           const bool act = i < len;
-          const float4 a = act ? resid4<FRESH>(A, J.pc.start + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+          const float4 a = resid4<FRESH>(A, J.pc.start + i, raw[u]);
           const float v[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
