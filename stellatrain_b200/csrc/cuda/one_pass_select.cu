@@ -476,10 +476,11 @@ __device__ __forceinline__ void note_destinations(const SelectArgs& A, const Job
   }
 }
 
+template <bool FRESH>
 __device__ __forceinline__ void emit_and_keep(const SelectArgs& A, const EmitShared& S, uint32_t pos, uint32_t gi, float a) {
   const float sv = wire_value(S.nb, a);
   emit_entry(A, S.dest, S.nb, S.slot_off, pos, gi, sv);
-  if (!A.fresh) A.resid[gi] = a - sv;     // exactly zero unless the wire format rounds
+  if (!FRESH) A.resid[gi] = a - sv;     // exactly zero unless the wire format rounds
 }
 
 // True in every thread of the CTA that finishes its tensor last; orders the other CTAs' stores in front of what follows.
@@ -550,8 +551,10 @@ enum Staged : uint32_t { kInOrder = 0, kNamed = 1, kWords = 2 };
 // The kernels of this part run once per CTA and step from one section to the next: what they wait for, besides L2, is their own
 // instructions.  With the stores to the destinations inlined wherever pairs are sent, and the searches below unrolled over
 // registers, `emit` had 166 KB of code for top-k, and a section took microseconds of fetches the first time an SM came to it (the
-// last CTA's search in a tensor 7 us for 100 items).  So sections that are used twice are functions, loops are loops, and items
+// last CTA's search in a tensor 7 us for 100 items).  Without a residual nothing is taken out of it, and the code for that is left
+// out (top-k, one tensor of 38.6 M elements: 28.9 us, 27.6 without).  So sections that are used twice are functions, loops are loops, and items
 // lie in shared memory: a 64 MB bucket takes 16 us instead of 23 (top-k, 1 %) and 9.6 instead of 12.9 (threshold-v16).
+template <bool FRESH>
 __device__ __noinline__ void send_staged(const SelectArgs& A, EmitShared& S, Staged how, uint32_t m, uint32_t pos) {
   const uint32_t* const words = reinterpret_cast<const uint32_t*>(S.stage);
   const uint32_t n_out = S.n_out, off = S.off;
@@ -563,13 +566,13 @@ __device__ __noinline__ void send_staged(const SelectArgs& A, EmitShared& S, Sta
 #pragma unroll 1
     for (uint32_t q = threadIdx.x; q < m; q += kEmitThreads) {
       const uint2 e = pair(q);
-      emit_and_keep(A, S, pos + q, e.x, __uint_as_float(e.y));
+      emit_and_keep<FRESH>(A, S, pos + q, e.x, __uint_as_float(e.y));
     }
     return;
   }
-  float* const resid = A.fresh ? nullptr : A.resid;
+  float* const resid = A.resid;
   auto take_out = [&](const uint2& e) {
-    if (resid != nullptr) resid[e.x] = __uint_as_float(e.y) - __uint_as_float(e.y);      // zero, or what the next select drops
+    if (!FRESH) resid[e.x] = __uint_as_float(e.y) - __uint_as_float(e.y);      // zero, or what the next select drops
   };
   if (n_out == 1u) {
     uint2* const out = S.out[0] + pos;
@@ -595,7 +598,7 @@ __device__ __noinline__ void send_staged(const SelectArgs& A, EmitShared& S, Sta
 // Sends the `n` marked items of a CTA's batch at positions base, base + 1, ...: bit u of `sel` marks the thread's item u, `ex`
 // is the number of marked items in front of the thread's first.  They go through shared memory, so that the stores into the
 // destinations are consecutive.
-template <int N>
+template <bool FRESH, int N>
 __device__ __forceinline__ void send_marked(const SelectArgs& A, EmitShared& S, const uint32_t (&idx)[N], const uint32_t (&bits)[N],
                                             uint32_t sel, uint32_t ex, uint32_t n, uint32_t base) {
   uint2* const stage = S.stage;
@@ -610,14 +613,14 @@ __device__ __forceinline__ void send_marked(const SelectArgs& A, EmitShared& S, 
       }
     }
     __syncthreads();
-    send_staged(A, S, kInOrder, min(kStageItems, n - w), base + w);
+    send_staged<FRESH>(A, S, kInOrder, min(kStageItems, n - w), base + w);
     __syncthreads();
   }
 }
 
 // Sends the items over the threshold's bin and notes those inside it.  `emitted` / `noted`: counts so far when one CTA
 // has the whole tensor; several CTAs draw theirs from the tensor's counters, once per batch.
-template <int N>
+template <bool FRESH, int N>
 __device__ __forceinline__ void emit_top_batch(const SelectArgs& A, const Job& J, EmitShared& S, uint2* undecided,
                                                const uint32_t (&idx)[N], const uint32_t (&bits)[N], uint32_t key_lo,
                                                uint32_t key_hi, uint32_t& emitted, uint32_t& noted) {
@@ -648,7 +651,7 @@ __device__ __forceinline__ void emit_top_batch(const SelectArgs& A, const Job& J
 #pragma unroll
   for (int u = 0; u < N; ++u)
     if (und >> u & 1u) undecided[q++] = make_uint2(idx[u], bits[u]);
-  send_marked<N>(A, S, idx, bits, sel, ex & 0xffffu, t_sel, b_sel);
+  send_marked<FRESH, N>(A, S, idx, bits, sel, ex & 0xffffu, t_sel, b_sel);
 }
 
 // Keys of the last two octaves under the largest differ from it in these bits: where the best of a distribution are looked for
@@ -815,7 +818,7 @@ __device__ __forceinline__ uint32_t top_direct(const SelectArgs& A, const Job& J
       if (p < 2048u) S.hist[p] = ((b >> 2) * kEmitThreads + tid) * 4u + (b & 3u);
     }
     __syncthreads();
-    send_staged(A, S, kWords, min(2048u, total - w), w);
+    send_staged<FRESH>(A, S, kWords, min(2048u, total - w), w);
     __syncthreads();
   }
   return cut.x;
@@ -954,7 +957,7 @@ __device__ __forceinline__ uint32_t send_best(const SelectArgs& A, const Job& J,
     }
     __syncthreads();
     const uint32_t p0 = done * kPerItem + t0;      // the last block may be cut off at k
-    send_staged(A, S, kInOrder, min(min(kStageItems, take * kPerItem - t0), J.sd.k > p0 ? J.sd.k - p0 : 0u), p0);
+    send_staged<FRESH>(A, S, kInOrder, min(min(kStageItems, take * kPerItem - t0), J.sd.k > p0 ? J.sd.k - p0 : 0u), p0);
     __syncthreads();
   }
   return cut.x;
@@ -968,7 +971,7 @@ __device__ __forceinline__ uint32_t settle_top(const SelectArgs& A, const Job& J
   const uint32_t done = J.kk - rem;
   if (c <= kPickMax) {
     const uint32_t t_key = pick_few(A, undecided, c, rem, key_hi - 1u, 32u - __clz(key_hi - 1u - key_lo), J.sd.off, J.sd.n_pad, S);
-    if (t_key != kNoCut) send_staged(A, S, kNamed, rem, done);
+    if (t_key != kNoCut) send_staged<FRESH>(A, S, kNamed, rem, done);
     return t_key;
   }
   return send_best<false, FRESH>(A, J, S, undecided, c, rem, done, A.cand + J.sd.off);
@@ -1027,7 +1030,7 @@ __device__ __forceinline__ void send_range(const SelectArgs& A, const Job& J, Em
     __syncthreads();
     // a truncated last block leaves the residual exact: only emitted elements are cleared
     const uint32_t p0 = base * kPerItem + t0;
-    send_staged(A, S, kInOrder, min(min(kStageItems, end - t0), J.sd.k > p0 ? J.sd.k - p0 : 0u), p0);
+    send_staged<FRESH>(A, S, kInOrder, min(min(kStageItems, end - t0), J.sd.k > p0 ? J.sd.k - p0 : 0u), p0);
     __syncthreads();
   }
 }
@@ -1244,7 +1247,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const __grid_constant_
                 bits[u] = e.y;
               }
             }
-            emit_top_batch<kItems>(A, J, S, undecided, idx, bits, key_lo, key_hi, emitted, noted);
+            emit_top_batch<FRESH, kItems>(A, J, S, undecided, idx, bits, key_lo, key_hi, emitted, noted);
           }
         }
       }
@@ -1351,7 +1354,7 @@ __global__ void __launch_bounds__(kEmitThreads, 4) k_emit(const __grid_constant_
               const uint32_t q = e >> 4, p = (found + q) * 16u + (e & 15u);
               if (p < J.sd.k) {   // only the lowest-ranked block can be cut off
                 const uint32_t gi = S.stage[S.hist[q]].x * 16u + (e & 15u);
-                emit_and_keep(A, S, p, gi, resid1<FRESH>(A, gi));
+                emit_and_keep<FRESH>(A, S, p, gi, resid1<FRESH>(A, gi));
               }
             }
           } else if (take) {
@@ -1443,7 +1446,7 @@ __global__ void __launch_bounds__(kEmitThreads, 2) k_refill(const __grid_constan
         for (int e = 0; e < 4; ++e) zero |= (uint32_t)((bits[e] & 0x7fffffffu) == 0u) << e;
         const uint32_t ex = block_excl_scan(__popc(zero), S.tmp, total);
         while (zero && base + ex + __popc(zero) > rem) zero &= ~(0x80000000u >> __clz(zero));      // the budget ends here
-        send_marked<4>(A, S, idx, bits, zero, ex, min(total, rem - base), J.kk - rem + base);
+        send_marked<FRESH, 4>(A, S, idx, bits, zero, ex, min(total, rem - base), J.kk - rem + base);
         base += total;
       }
     }
@@ -1469,7 +1472,7 @@ __global__ void __launch_bounds__(kEmitThreads, 2) k_refill(const __grid_constan
             idx[4 * u + e] = act && (bits[4 * u + e] & 0x7fffffffu) ? J.pc.start + i + e : kSentinelIdx;
           }
         }
-        emit_top_batch<kItems>(A, J, S, undecided, idx, bits, key_lo, key_hi, emitted, noted);
+        emit_top_batch<FRESH, kItems>(A, J, S, undecided, idx, bits, key_lo, key_hi, emitted, noted);
       }
     }
     if (last_of_tensor(J, S)) {
