@@ -29,9 +29,9 @@
 //   emit    latency, a chain of about ten trips to L2, and its own instructions (see send_staged): 9.6 us for threshold-v16, 16 us
 //           for top-k at 1 %; the slowest sections of the latter are the sum of the histograms (3 us) and the last CTA's
 //           search (3 us).
-//   refill  1.4 to 2.5 us when there is nothing to do; one tensor of 16.8 M elements (3 M) whose gradients fell to a third takes
-//           94 us (23) here and 83 us (20) in `emit`, where a CTA counts a piece of 131,072 elements (16,384); where they fell to a
-//           hundredth, so that the cut lies in a wide bin, 366 us (71), most of them for the ranking by the last CTA.
+//   refill  1.4 to 2.5 us when there is nothing to do; one tensor of 16.8 M normal values (3 M), residual empty, that fell to a
+//           third takes 104 us (22) here and 65 us (15) in `emit`, where a CTA counts a piece of 131,072 elements (16,384); where they
+//           fell to a hundredth, so that the cut lies in a wide bin, 729 us (112), most of them for the ranking by the last CTA.
 #include "launch.h"
 #include "launchers.h"
 #include "select_common.cuh"
@@ -176,9 +176,9 @@ __device__ __forceinline__ float number_or_zero(float x) { return x == x ? x : 0
 // FRESH: A.fresh is not 0.
 //
 // Four elements are read in two parts, so that a thread's loads travel together: `load4` for all of them, without a branch, then
-// `resid4` for each, which adds what the tensor's end cut off.  With a branch around every load they went one after the other:
-// `compress` of 16.8 M elements at 1 %, us of emit and refill, where the values fell to a thirtieth 705 (with this 478), to a third
-// 270 (194), grew thirtyfold 1063 (806); threshold-v16, fallen to a third, 185 (107).
+// `resid4` for each, which adds what the tensor's end cut off.  With a branch around every load they went one after the other: a
+// `compress` of 16.8 M elements (top-k, 1 %) whose values had fallen to a thirtieth took 778 us and now 551, fallen to a third 338
+// and 256, grown thirtyfold 1497 and 1206; `emit` of threshold-v16, values fallen to a third, 185 and 106.
 template <bool FRESH>
 __device__ __forceinline__ float4 load4(const SelectArgs& A, uint32_t i) {
   return !FRESH || i + 4u <= A.fresh ? __ldcg(reinterpret_cast<const float4*>(A.resid + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -551,9 +551,9 @@ enum Staged : uint32_t { kInOrder = 0, kNamed = 1, kWords = 2 };
 // The kernels of this part run once per CTA and step from one section to the next: what they wait for, besides L2, is their own
 // instructions.  With the stores to the destinations inlined wherever pairs are sent, and the searches below unrolled over
 // registers, `emit` had 166 KB of code for top-k, and a section took microseconds of fetches the first time an SM came to it (the
-// last CTA's search in a tensor 7 us for 100 items).  Without a residual nothing is taken out of it, and the code for that is left
-// out (top-k, one tensor of 38.6 M elements: 28.9 us, 27.6 without).  So sections that are used twice are functions, loops are loops, and items
-// lie in shared memory: a 64 MB bucket takes 16 us instead of 23 (top-k, 1 %) and 9.6 instead of 12.9 (threshold-v16).
+// last CTA's search in a tensor 7 us for 100 items).  So sections that are used twice are functions, loops are loops, and items
+// lie in shared memory: a 64 MB bucket takes 16 us instead of 23 (top-k, 1 %) and 9.6 instead of 12.9 (threshold-v16).  Without a
+// residual the code that takes pairs out of it is left out as well (top-k, one tensor of 38.6 M elements: 28.9 us, now 27.6).
 template <bool FRESH>
 __device__ __noinline__ void send_staged(const SelectArgs& A, EmitShared& S, Staged how, uint32_t m, uint32_t pos) {
   const uint32_t* const words = reinterpret_cast<const uint32_t*>(S.stage);
