@@ -386,6 +386,30 @@ def test_compress_of_values_that_change_in_scale(compressor, n):
 
 
 @pytest.mark.parametrize("compressor", ["topk", "thresholdv", "thresholdv16"])
+@pytest.mark.parametrize("n", [2, 3, 6, 16_385, 16_386, 140_001, 140_002])
+def test_compress_reads_the_last_elements_however_many_there_are(compressor, n):
+    """A tensor in place is read four elements at a time, and its end by itself: tensors shorter than that, and one or two
+    elements behind the last four, which are the largest of all, on the ways that read the tensor once more."""
+    import stellatrain_b200 as st
+
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    name, state = f"{compressor} {n} end", O.ThresholdState()
+    st.configure_compression(compressor)
+    try:
+        for call, scale in enumerate([1.0, 1.0, 0.01, 30.0, 0.2]):
+            x = torch.randn(n, generator=gen, device="cuda") * (1e-2 * scale)
+            x[-2:] = 5e-2 * scale
+            k = max(1, int((1.0 - 0.9) * n)) if n > 16 else n // 2
+            idx, val = st.compress(name, x, 0.9 if n > 16 else 0.5)
+            assert torch.equal(val, x[idx.long()]) and len(torch.unique(idx)) == len(idx)
+            want, _, _ = O.compress_step(compressor, x, torch.zeros_like(x), k, state, one_pass=call > 0)
+            want = want[want < n].sort().values
+            assert torch.equal(idx.long().sort().values, want), call
+    finally:
+        st.configure_compression("thresholdv16")
+
+
+@pytest.mark.parametrize("compressor", ["topk", "thresholdv", "thresholdv16"])
 def test_compress_under_capture_is_refused_and_leaves_no_trace(compressor):
     """The refused call must not count as the tensor's first select, which is the one that measures the threshold."""
     import stellatrain_b200 as st
